@@ -6,73 +6,9 @@
 // (helpers/cuda/activations.cu:303-353, generic/loss/softmaxCrossEntropy*.cpp); lstmCell as NDArray
 // algebra (helpers/cuda/lstm.cu:45-110) and DL4J's LSTMHelpers.java:180-330 gate order [a, f, o, g].
 // Each op reads its operands once from HBM and writes once.
-#include "common.cuh"
+#include "vec8.cuh"
 
 namespace dl4j {
-
-template <typename T> struct Vec8;
-template <> struct Vec8<__nv_bfloat16> {
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[8]) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
-  }
-  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[8]) {
-    uint4 u;
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-    *reinterpret_cast<uint4*>(p) = u;
-  }
-};
-template <> struct Vec8<__half> {
-  static __device__ __forceinline__ void load(const __half* p, float (&v)[8]) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const __half2* h = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { const float2 f = __half22float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
-  }
-  static __device__ __forceinline__ void store(__half* p, const float (&v)[8]) {
-    uint4 u;
-    __half2* h = reinterpret_cast<__half2*>(&u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-    *reinterpret_cast<uint4*>(p) = u;
-  }
-};
-template <> struct Vec8<float> {
-  static __device__ __forceinline__ void load(const float* p, float (&v)[8]) {
-    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  }
-  static __device__ __forceinline__ void store(float* p, const float (&v)[8]) {
-    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
-  }
-};
-
-// Eight elements as raw 16-byte words (one for 16-bit types, two for float): lets a kernel issue the loads of several rows
-// before converting any of them.
-template <typename T> struct Raw8 { uint4 q[sizeof(T) / 2]; };
-template <typename T> __device__ __forceinline__ Raw8<T> ld_raw8(const T* p) {
-  Raw8<T> r;
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(T) / 2); ++i) r.q[i] = __ldcs(reinterpret_cast<const uint4*>(p) + i);
-  return r;
-}
-template <typename T> __device__ __forceinline__ void unpack8(const Raw8<T>& r, float (&v)[8]) {
-  Vec8<T>::load(reinterpret_cast<const T*>(&r), v);
-}
-
-template <typename T> __device__ __forceinline__ float ldf(const T* p);
-template <> __device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float ldf<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-template <> __device__ __forceinline__ float ldf<__half>(const __half* p) { return __half2float(*p); }
-template <typename T> __device__ __forceinline__ void stf(T* p, float v);
-template <> __device__ __forceinline__ void stf<float>(float* p, float v) { *p = v; }
-template <> __device__ __forceinline__ void stf<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
-template <> __device__ __forceinline__ void stf<__half>(__half* p, float v) { *p = __float2half(v); }
 
 // ----------------------------------------------------------------------------- layer norm
 // One warp per row; C % 8 == 0 and C <= 32 * 8 * LN_MAXV.  Optional residual input: x = x + res is

@@ -188,7 +188,21 @@ def layer_norm(x, gain, bias=None, dimensions=(-1,), channelsFirst=False, **kw):
     return y + bias.reshape(shape) if bias is not None else y
 
 
-op("layer_norm_bp", n_out=3)(_autobp(layer_norm, 3))
+_layer_norm_autobp = _autobp(layer_norm, 3)
+
+
+@op("layer_norm_bp", n_out=3)
+def layer_norm_bp(*args, **kw):
+    """(x, gain[, bias], dy) -> dx, dgain[, dbias].  Normalisation over the last axis on the GPU runs as one gradient kernel; other
+    axes, devices and types differentiate the forward."""
+    if len(args) == 4 and isinstance(args[0], torch.Tensor) and args[0].dim() > 0:
+        x, gain, bias, dy = args
+        if [d % x.dim() for d in (_ints(kw.get("dimensions", (-1,))) or [-1])] == [x.dim() - 1]:
+            nat = nnops._native_for(x)
+            r = nat.layer_norm_grad(x, gain, bias, dy, 1e-5) if nat is not None else None
+            if r is not None:
+                return r if bias is not None else r[:2]
+    return _layer_norm_autobp(*args, **kw)
 
 
 @op("add_layer_norm")

@@ -57,6 +57,7 @@ def _load():
             "dl4j_bitmap_decode": [vp, vp, i64, f32, vp],
             "dl4j_layer_norm_fwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, f32, i32, vp],
             "dl4j_layer_norm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp],
+            "dl4j_layer_norm_grad": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, i32, i32, i32, vp],
             "dl4j_softmax_xent": [vp, vp, vp, vp, vp, i32, i32, i64, i32, i32, vp],
             "dl4j_scatter_add_rows": [vp, vp, vp, i64, i32, i64, i64, i32, vp],
             "dl4j_softmax_xent_fwd": [vp, vp, vp, vp, vp, vp, i32, i32, i64, i32, i32, vp],
@@ -590,29 +591,31 @@ _PAD_ODD_WIDTHS = os.environ.get("DL4J_PAD_ODD_WIDTHS", "1") != "0"
 _LN_ONE_PASS = os.environ.get("DL4J_LN_BWD_ONEPASS", "0") == "1"
 
 
+def _dense16(t):
+    """Contiguous and on a 16-byte boundary (the vector kernels' requirement): a view off the grid is copied."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gain, bias, eps, res=None):
         l = require()
         shp = x.shape
         C = shp[-1]
-        x2 = x.reshape(-1, C)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
+        x2 = _dense16(x.reshape(-1, C))
         rows = x2.shape[0]
         y = torch.empty_like(x2)
         mean = torch.empty(rows, dtype=torch.float32, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         gain = getattr(gain, "_master", gain)
         bias = getattr(bias, "_master", bias) if bias is not None else None
-        g32 = gain.detach().float().contiguous().reshape(-1)
-        b32 = bias.detach().float().contiguous().reshape(-1) if bias is not None else None
+        g32 = _dense16(gain.detach().float().reshape(-1))
+        b32 = _dense16(bias.detach().float().reshape(-1)) if bias is not None else None
         r2 = s2 = None
         if res is not None:
             # y = LN(x + res): the kernel adds the residual while loading and writes the sum once (kept for the backward)
-            r2 = res.reshape(-1, C)
-            if not r2.is_contiguous():
-                r2 = r2.contiguous()
+            r2 = _dense16(res.reshape(-1, C))
             s2 = torch.empty_like(x2)
         rc = l.dl4j_layer_norm_fwd(_ptr(x2), _ptr(r2), _ptr(g32), _ptr(b32), _ptr(y), _ptr(s2), _ptr(mean), _ptr(rstd), rows, C,
                                    float(eps), _DT[x.dtype], _stream())
@@ -655,15 +658,42 @@ class _LayerNormFn(torch.autograd.Function):
                                                rows, C, _DT[x2.dtype], 1, _stream())
             _check(rc, "dl4j_layer_norm_bwd_noalloc")
         else:
-            rc = l.dl4j_layer_norm_bwd(_ptr(dy2), _ptr(x2), _ptr(g32), _ptr(mean), _ptr(rstd), _ptr(dx), _ptr(gacc), _ptr(bacc),
-                                       rows, C, _DT[x2.dtype], _stream())
-            _check(rc, "dl4j_layer_norm_bwd")
+            partial = torch.empty(4 * num_sms() * C, dtype=torch.float32, device=dy.device)
+            rc = l.dl4j_layer_norm_grad(_ptr(dy2), _ptr(x2), _ptr(g32), _ptr(mean), _ptr(rstd), _ptr(dx), _ptr(gacc), _ptr(bacc),
+                                        _ptr(partial), rows, C, 0.0, _DT[x2.dtype], 1, num_sms(), _stream())
+            _check(rc, "dl4j_layer_norm_grad")
         if gret is not None:
             gret = gret.reshape(gain.shape).to(gain.dtype)
         if bret is not None:
             bret = bret.reshape(bias.shape).to(bias.dtype)
         dx = dx.reshape(ctx.shape)
         return dx, gret, bret, None, (dx if ctx.has_res else None)
+
+
+def layer_norm_grad(x, gain, bias, dy, eps):
+    """(dx, dgain, dbias) of LN(x) over the last axis without running the forward (``dbias`` None without ``bias``): one sweep that
+    takes the row statistics on the way.  None when the case is not covered."""
+    if not available() or not x.is_cuda or x.dtype not in _DT or x.dim() < 1 or not 1 <= x.shape[-1] <= 8192 or x.numel() == 0:
+        return None
+    C = x.shape[-1]
+    for p in (gain, bias):
+        if p is not None and (p.numel() != C or not p.is_floating_point() or p.dtype == torch.float64 or p.device != x.device):
+            return None
+    if dy.numel() != x.numel() or dy.device != x.device:
+        return None
+    l = require()
+    x2 = x.detach().contiguous()
+    dy2 = dy.detach().to(x.dtype).contiguous()
+    g32 = gain.detach().float().contiguous()
+    rows = x2.numel() // C
+    dx = torch.empty_like(x2)
+    dg = torch.empty(C, dtype=torch.float32, device=x.device)
+    db = torch.empty(C, dtype=torch.float32, device=x.device) if bias is not None else None
+    partial = torch.empty(4 * num_sms() * C, dtype=torch.float32, device=x.device)
+    rc = l.dl4j_layer_norm_grad(_ptr(dy2), _ptr(x2), _ptr(g32), None, None, _ptr(dx), _ptr(dg), _ptr(db),
+                                _ptr(partial), rows, C, float(eps), _DT[x.dtype], 0, num_sms(), _stream())
+    _check(rc, "dl4j_layer_norm_grad")
+    return dx, dg.reshape(gain.shape).to(gain.dtype), None if db is None else db.reshape(bias.shape).to(bias.dtype)
 
 
 def layer_norm(x, gain, bias, eps, residual=None):
