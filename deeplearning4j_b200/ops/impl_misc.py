@@ -284,9 +284,22 @@ op("testcustom")(lambda x, **kw: x)
 
 
 # ----------------------------------------------------------------------------- gradient compression as ops
+def _out_of_place_codec(x):
+    """The native codec when it can read ``x`` and write the result to another buffer in one pass (no clone), else None."""
+    if not (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and 0 < x.numel() < 2 ** 31 - 1):
+        return None
+    from . import native
+    return native if native.available() else None
+
+
 @op("encode_threshold", n_out=2, differentiable=False)
 def encode_threshold(x, threshold=1e-3, boundary=None, **kw):
     from ..parallel import codec
+    nat = _out_of_place_codec(x)
+    if nat is not None:
+        x = x.detach()
+        r = torch.empty_like(x)
+        return r, nat.threshold_encode(x.view(-1), float(threshold), None if boundary is None else int(boundary), residual=r)
     r = x.clone().reshape(-1).float()
     msg = codec.threshold_encode(r, float(threshold), None if boundary is None else int(boundary))
     return r.reshape(x.shape).to(x.dtype), msg
@@ -303,6 +316,12 @@ def decode_threshold(x, encoded, **kw):
 @op("encode_bitmap", n_out=3, differentiable=False)
 def encode_bitmap(x, threshold=1e-3, **kw):
     from ..parallel import codec
+    nat = _out_of_place_codec(x)
+    if nat is not None:
+        x = x.detach()
+        r = torch.empty_like(x)
+        msg = nat.bitmap_encode(x.view(-1), float(threshold), residual=r)
+        return r, msg, msg[0:1].clone()
     r = x.clone().reshape(-1).float()
     msg = codec.bitmap_encode(r, float(threshold))
     return r.reshape(x.shape).to(x.dtype), msg, msg[0:1].clone()
@@ -311,6 +330,9 @@ def encode_bitmap(x, threshold=1e-3, **kw):
 @op("decode_bitmap", differentiable=False)
 def decode_bitmap(x, encoded, **kw):
     from ..parallel import codec
+    nat = _out_of_place_codec(x)
+    if nat is not None and isinstance(encoded, torch.Tensor) and encoded.device == x.device:
+        return nat.bitmap_decode(encoded, x.detach(), out=torch.empty_like(x))
     out = x.clone().float()
     codec.bitmap_decode(encoded, out)
     return out.to(x.dtype)

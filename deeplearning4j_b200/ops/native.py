@@ -51,9 +51,12 @@ def _load():
                           i32, i32, f32, i32, i32, vp],
             "dl4j_fused_update": [vp, vp, vp, vp, vp, vp, i32, vp, vp, i32, f32, i32, vp],
             "dl4j_cast_f32_bf16": [vp, vp, i64, vp],
+            "dl4j_threshold_encode_to": [vp, vp, i64, f32, vp, i32, vp],
             "dl4j_threshold_encode": [vp, i64, f32, vp, i32, vp],
             "dl4j_threshold_decode": [vp, i32, vp, i64, f32, i32, vp],
+            "dl4j_bitmap_encode_to": [vp, vp, i64, f32, vp, vp],
             "dl4j_bitmap_encode": [vp, i64, f32, vp, vp],
+            "dl4j_bitmap_decode_to": [vp, vp, vp, i64, f32, vp],
             "dl4j_bitmap_decode": [vp, vp, i64, f32, vp],
             "dl4j_layer_norm_fwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, f32, i32, vp],
             "dl4j_layer_norm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp],
@@ -1450,14 +1453,18 @@ def cast_to_bf16(src_f32, dst_bf16):
 
 
 # =========================================================================== gradient codecs
-def threshold_encode(x, tau, capacity=None, msg=None):
-    """In-place sparse threshold encode of fp32 ``x`` (residual stays in ``x``); returns the int32 message."""
+def threshold_encode(x, tau, capacity=None, msg=None, residual=None):
+    """Sparse threshold encode of fp32 ``x``; returns the int32 message.  The residual goes to ``residual`` (same size), or stays in
+    ``x`` without one."""
     l = require()
     n = x.numel()
     capacity = int(capacity if capacity is not None else n)
     if msg is None:
         msg = torch.empty(4 + capacity, dtype=torch.int32, device=x.device)
-    rc = l.dl4j_threshold_encode(_ptr(x), n, float(tau), _ptr(msg), capacity, _stream())
+    if residual is None:
+        rc = l.dl4j_threshold_encode(_ptr(x), n, float(tau), _ptr(msg), capacity, _stream())
+    else:
+        rc = l.dl4j_threshold_encode_to(_ptr(x), _ptr(residual), n, float(tau), _ptr(msg), capacity, _stream())
     _check(rc, "dl4j_threshold_encode")
     return msg
 
@@ -1470,21 +1477,23 @@ def threshold_decode(msg, target, scale=1.0, atomics=False, capacity=None):
     return target
 
 
-def bitmap_encode(x, tau, msg=None):
+def bitmap_encode(x, tau, msg=None, residual=None):
     l = require()
     n = x.numel()
     if msg is None:
         msg = torch.empty(4 + (n + 15) // 16, dtype=torch.int32, device=x.device)
-    rc = l.dl4j_bitmap_encode(_ptr(x), n, float(tau), _ptr(msg), _stream())
+    rc = l.dl4j_bitmap_encode_to(_ptr(x), _ptr(x if residual is None else residual), n, float(tau), _ptr(msg), _stream())
     _check(rc, "dl4j_bitmap_encode")
     return msg
 
 
-def bitmap_decode(msg, target, scale=1.0):
+def bitmap_decode(msg, target, scale=1.0, out=None):
+    """Adds the decoded steps to ``target`` in place, or writes the sum to ``out``."""
     l = require()
-    rc = l.dl4j_bitmap_decode(_ptr(msg), _ptr(target), target.numel(), float(scale), _stream())
+    out = target if out is None else out
+    rc = l.dl4j_bitmap_decode_to(_ptr(msg), _ptr(target), _ptr(out), target.numel(), float(scale), _stream())
     _check(rc, "dl4j_bitmap_decode")
-    return target
+    return out
 
 
 # =========================================================================== word2vec / t-SNE
