@@ -44,6 +44,7 @@ struct GemmParams {
   int tma_aux;            // same for the auxiliary pre-activation output
   int bias_mma;           // the bias is added on the tensor core: one extra K=16 step ones[128 x 1] x bias[1 x N] per tile
   int raster_gn;          // tile raster: column-tile groups of this width, column index fastest inside a group
+  int relu_last;          // ReLU after the residual has been added (a residual block's output; inference)
   int res_act;            // != 0: `residual` holds pre-activations z and the result is multiplied by act'(z) instead of added to
                           // (the data-gradient GEMM of a layer that feeds an activation writes dz directly)
 };
@@ -416,6 +417,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                   }
               }
             }
+            if (p.relu_last) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+            }
             if (p.out_fp32) {
 #pragma unroll
               for (int j = 0; j < 8; ++j)
@@ -509,6 +514,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 v[j] = p.res_act ? mul_act_grad(v[j], z, p.res_act) : v[j] + z;
               }
             }
+          }
+          if (p.relu_last) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
           }
           if (p.out_fp32) {
             float* o = reinterpret_cast<float*>(p.C) + c_off + (long)row * p.ldc + col0;
@@ -618,9 +627,10 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   GemmParams p;
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.ld_aux = ld_aux; p.ld_res = ld_res; p.C = C; p.aux = aux; p.bias = bias;
   // `act` carries two ids: bits 0-7 the forward activation applied to the result, bits 8-15 an activation whose derivative at
-  // `residual` multiplies the result (then `residual` is not added)
+  // `residual` multiplies the result (then `residual` is not added); bit 16 applies ReLU after the residual
   p.residual = residual; p.bias_fp32 = bias_fp32; p.out_fp32 = out_fp32; p.act = act & 0xff; p.res_act = (act >> 8) & 0xff;
-  if (p.res_act && (!residual || p.act)) return -DL4J_ERR_BAD_ARG;
+  p.relu_last = (act >> 16) & 1;
+  if (p.res_act && (!residual || p.act || p.relu_last)) return -DL4J_ERR_BAD_ARG;
   p.atomic_out = atomic_out;
   p.splits = splits; p.fmt = fmt; p.alpha = alpha; p.status = dl4j_status_word(dev);
   p.batch1 = batch1; p.batch2 = batch2; p.c_stride_b1 = c_bs[0]; p.c_stride_b2 = c_bs[1];

@@ -190,10 +190,117 @@ class ComputationGraph(BaseNetwork):
         self._fuse_plan = plan
         return plan
 
+    # ------------------------------------------------------------------ inference: batch norm folded into the convolutions
+    def _fold_specs(self):
+        """Convolutions whose only consumer is a batch norm and which the native kernels run: conv vertex -> (batch-norm vertex,
+        kind, convolution layer, batch-norm layer)."""
+        specs = getattr(self, "_fold_specs_cache", None)
+        if specs is not None:
+            return specs
+        from .activations import ActivationIdentity
+        from .conf.base import CNN2DFormat
+        from .layers.conv import BatchNormalization, ConvolutionLayer
+        conf, outs, consumers = self.conf, set(self.conf.networkOutputs), {}
+        for n in self.order:
+            for i in conf.vertexInputs[n]:
+                consumers.setdefault(i, []).append(n)
+
+        def plain(n, cls):
+            v = conf.vertices.get(n)
+            return isinstance(v, LayerVertex) and type(v.layer) is cls and v.preProcessor is None and n not in outs \
+                and getattr(v.layer, "dropOut", None) is None and getattr(v.layer, "weightNoise", None) is None
+        specs = {}
+        for n in self.order:
+            cs = consumers.get(n, [])
+            if not plain(n, ConvolutionLayer) or len(cs) != 1 or not plain(cs[0], BatchNormalization):
+                continue
+            c, b = conf.vertices[n].layer, conf.vertices[cs[0]].layer
+            if not isinstance(c.activation, ActivationIdentity) or c.cnn2dDataFormat != CNN2DFormat.NCHW or b.cnn2DFormat != CNN2DFormat.NCHW \
+                    or len(c.kernelSize) != 2 or c.nOut % 8 or (b.nOut or b.nIn) != c.nOut:
+                continue
+            k, s, p = tuple(c.kernelSize), tuple(c.stride), tuple(c.padding)
+            if k == (1, 1) and p == (0, 0) and c.nIn % 8 == 0:
+                kind = "1x1"
+            elif s == (1, 1) and c.nIn % 8 == 0 and k[0] * k[1] <= 64 and 0 <= min(p) and max(p) <= 255:
+                kind = "kxk"
+            elif s == (2, 2) and tuple(c.dilation) == (1, 1) and c.nIn <= 4:
+                kind = "stem"
+            else:
+                continue
+            specs[n] = (cs[0], kind, c, b)
+        self._fold_specs_cache = specs
+        return specs
+
+    def _fold(self, x):
+        """Folded weights of this forward pass: conv vertex -> (weights [O, kH * kW * I] bf16, bias fp32); {} when the network, its
+        types or the device are not covered.  Computed anew in every call, by one launch over all convolutions."""
+        from ..ops import native, nnops
+        specs = self._fold_specs()
+        if not specs or nnops._FORCE_TORCH or not x.is_cuda or x.dtype != torch.bfloat16 or not self.flat_params.is_cuda \
+                or self.flat_params.dtype != torch.float32 or not native.available():
+            return {}
+        sig = (self.flat_params.device,) + tuple((b.eps, b.useLogStd, b.lockGammaBeta, b.gamma, b.beta) for _, _, _, b in specs.values())
+        t = getattr(self, "_fold_table", None)
+        if t is None or t["sig"] != sig:
+            import struct
+            off = {e.key: e.offset for e in self.entries}
+            rows, blocks, where, wo, bo = b"", [], {}, 0, 0
+            for i, (n, (bn, _, c, b)) in enumerate(specs.items()):
+                S = c.kernelSize[0] * c.kernelSize[1]
+                g = lambda k: off.get(k, -1)
+                rows += struct.pack("<8q4i3fi", off[n + "_W"], g(n + "_b"), g(bn + "_gamma"), g(bn + "_beta"), off[bn + "_mean"],
+                                    off[bn + ("_log10stdev" if b.useLogStd else "_var")], wo, bo, c.nOut, c.nIn, S, int(bool(b.useLogStd)),
+                                    float(b.eps), float(b.gamma), float(b.beta), len(blocks))
+                blocks += [i] * c.nOut
+                where[n] = (wo, c.nOut, S * c.nIn, bo)
+                wo += (c.nOut * S * c.nIn + 63) // 64 * 64
+                bo += (c.nOut + 63) // 64 * 64
+            dev = self.flat_params.device
+            t = self._fold_table = {"sig": sig, "where": where, "w": wo, "b": bo, "rows": torch.frombuffer(bytearray(rows), dtype=torch.uint8).to(dev),
+                                    "blocks": torch.tensor(blocks, dtype=torch.int32).to(dev)}
+        w = torch.empty(t["w"], dtype=torch.bfloat16, device=x.device)
+        b = torch.empty(t["b"], dtype=torch.float32, device=x.device)
+        native.bn_fold(t["rows"], t["blocks"], self.flat_params, w, b)
+        return {n: (w[o:o + O * K].view(O, K), b[ob:ob + O]) for n, (o, O, K, ob) in t["where"].items()}
+
+    def _folded_conv(self, n, folded, x, relu, residual=None):
+        """relu?(batchnorm(conv(x)) [+ residual]) with the folded weights of vertex ``n``."""
+        from ..ops import native
+        from .layers.conv import _pad_for_mode, _stem_space_to_depth, conv_out_size
+        _, kind, c, _ = self._fold_specs()[n]
+        w, b = folded[n]
+        kH, kW = c.kernelSize
+        if kind == "1x1":
+            if tuple(c.stride) != (1, 1):
+                x = native._SubsampleFn.apply(x, int(c.stride[0]), int(c.stride[1]))
+            x = native._dense16(native._dense_cl(x)) if x.data_ptr() % 16 else native._dense_cl(x)
+            if residual is not None:
+                residual = native._dense_cl(residual)
+                if residual.shape != (x.shape[0], c.nOut, x.shape[2], x.shape[3]) or residual.dtype != x.dtype or residual.data_ptr() % 16:
+                    y = native.conv_infer_1x1(x, w, b, False) + residual
+                    return torch.relu(y) if relu else y
+            return native.conv_infer_1x1(x, w, b, relu, residual)
+        x, pad = _pad_for_mode(x, c.kernelSize, c.stride, c.padding, c.dilation, c._mode())
+        act = relu and residual is None
+        if kind == "stem":
+            y = _stem_space_to_depth(x, w.view(c.nOut, kH, kW, c.nIn).permute(0, 3, 1, 2), b, (kH, kW), tuple(pad), relu=act)
+        else:
+            x = native._dense_cl(x)
+            d = tuple(c.dilation)
+            if min(x.shape[2] + 2 * pad[0] - (kH - 1) * d[0], x.shape[3] + 2 * pad[1] - (kW - 1) * d[1]) < 1:
+                raise ValueError(f"convolution '{n}': kernel {kH}x{kW} does not fit the padded {x.shape[2]}x{x.shape[3]} input")
+            y = native.conv_infer_kxk(x if x.data_ptr() % 16 == 0 else x.clone(), w, b, kH, kW, pad, d, act)
+        if residual is not None:
+            z = native.add_relu(y, residual) if relu else None
+            y = z if z is not None else (torch.relu(y + residual) if relu else y + residual)
+        return y
+
     def _forward(self, inputs: dict, training, fmasks=None, ctx=None, stop_at_preout=False):
         ctx = ctx if ctx is not None else {}
         fuse = self._fusion_plan() if ctx.get("fuse") else {}
         bias_of = self._fuse_bias if fuse else {}
+        folded = self._fold(next(iter(inputs.values()))) if fuse and not training and not fmasks else {}
+        folded_bn = {self._fold_specs()[n][0]: n for n in folded}
 
         def pre_bias(bn_name):
             c = bias_of.get(bn_name)
@@ -212,6 +319,19 @@ class ComputationGraph(BaseNetwork):
             in_masks = [masks.get(i) for i in conf.vertexInputs[n]]
             act = fuse.get(n)
             extra = {}
+            if n in folded:
+                # the batch norm (and a ReLU right behind it) is in this convolution; one that feeds a residual add runs at the add
+                nxt = fuse.get(self._fold_specs()[n][0], (None,))[0]
+                acts[n] = ins[0] if nxt == "defer" else self._folded_conv(n, folded, ins[0], nxt == "bn_relu")
+                masks[n] = in_masks[0]
+                continue
+            if n in folded_bn:
+                acts[n], masks[n] = ins[0], in_masks[0]
+                continue
+            if act is not None and act[0] == "bn_add_relu" and act[1] in folded_bn:
+                acts[n] = self._folded_conv(folded_bn[act[1]], folded, acts[act[1]], True, residual=acts[act[2]])
+                masks[n] = in_masks[0]
+                continue
             if act is not None and act[0] == "conv_nobias":
                 act, extra = None, {"skip_bias": True}
             elif act is None and n in bias_of:
@@ -271,7 +391,7 @@ class ComputationGraph(BaseNetwork):
         if featureMasks is not None:
             fm = {n: _as_tensor(m, self.device) for n, m in zip(self.conf.networkInputs, featureMasks)}
         with torch.no_grad():
-            acts = self._forward(ins, bool(train), fm)
+            acts = self._forward(ins, bool(train), fm, None if train else {"fuse": True})
         return [INDArray(acts[o].float() if acts[o].dtype in (torch.bfloat16, torch.float16) else acts[o]) for o in self.conf.networkOutputs]
 
     def outputSingle(self, *inputs, train=False):

@@ -169,10 +169,10 @@ class ConvolutionLayer(FeedForwardLayer):
 Convolution2D = ConvolutionLayer
 
 
-def _stem_space_to_depth(x, W, b, k, pad):
+def _stem_space_to_depth(x, W, b, k, pad, relu=False):
     """Stride-2 convolution over a few input channels (an RGB stem) rewritten as a stride-1 convolution over a 2x2
     space-to-depth view: ``y[oh] = sum_kh W[kh] x[2 oh + kh]`` with ``kh = 2 a + bh`` becomes
-    ``sum_a sum_bh W'[bh][a] x'[bh][oh + a]``.  The rewritten problem has 4x the channels (padded to 16) and half the
+    ``sum_a sum_bh W'[bh][a] x'[bh][oh + a]``.  ``relu``: applied in the convolution's epilogue (inference).  The rewritten problem has 4x the channels (padded to 16) and half the
     taps per axis, which the tensor-core convolution kernels handle well; the 3-channel original does not."""
     N, C, H, Wd = x.shape
     kH, kW = k
@@ -199,10 +199,11 @@ def _stem_space_to_depth(x, W, b, k, pad):
         # stride-1 convolution over the space-to-depth view on the native kernels; the KW2 taps of a filter row times the
         # padded channels are one 64-element run per output pixel, loaded as a single K slice
         from ...ops import native as nat
-        z = nat.conv2d(xs, Wsd, b, (0, 0), (1, 1), fuse_w=True)
+        z = nat.conv2d(xs, Wsd, b, (0, 0), (1, 1), fuse_w=True, relu=relu)
         if z is not None:
             return z
-    return F.conv2d(xs, Wsd, b)
+    z = F.conv2d(xs, Wsd, b.to(xs.dtype) if b is not None else None)
+    return torch.relu(z) if relu else z
 
 
 def nnops_conv2d(x, W, b, stride, pad, dilation, groups=1):

@@ -1068,9 +1068,10 @@ class _Conv2dFn(torch.autograd.Function):
         return dx, dW, db, None, None, None, None
 
 
-def conv2d(x, W, bias, pad, dil, fuse_w=False, path=None):
+def conv2d(x, W, bias, pad, dil, fuse_w=False, path=None, relu=False):
     """Stride-1 convolution on the native implicit-GEMM kernels, or None when the case is not covered (the caller then
-    uses the library path): 16-bit CUDA activation, channel counts multiples of 8, non-negative output size."""
+    uses the library path): 16-bit CUDA activation, channel counts multiples of 8, non-negative output size.  ``relu`` (inference
+    only: no gradient) applies ReLU in the epilogue."""
     if not (available() and x.is_cuda and x.dim() == 4 and x.dtype in (torch.bfloat16, torch.float16)):
         return None
     Wm = getattr(W, "_master", W)
@@ -1087,8 +1088,53 @@ def conv2d(x, W, bias, pad, dil, fuse_w=False, path=None):
         return None
     if fuse_w and (pad[1] != 0 or dil[1] != 1 or kW * x.shape[1] > 64):
         fuse_w = False
+    if relu:
+        assert not (torch.is_grad_enabled() and (x.requires_grad or W.requires_grad)) and Wm.dtype == x.dtype and bias.dtype == torch.float32
+        x = _dense_cl(x)
+        return conv_infer_kxk(x, _dense16(W.permute(0, 2, 3, 1)), bias.contiguous(), kH, kW, pad, dil, True, fuse_w)
     return _Conv2dFn.apply(x, W, bias, (int(pad[0]), int(pad[1])), (int(dil[0]), int(dil[1])), bool(fuse_w),
                            {None: 0, "tap": 2, "halo": 4}[path])
+
+
+# --------------------------------------------------------------------------- inference convolutions with batch norm folded in
+def bn_fold(table, block_entry, params, w_out, b_out):
+    """Folded weights (bf16, channels-last) and biases (fp32) of every convolution in ``table`` (``csrc/bn_fold.cu``), one launch."""
+    l = require()
+    if not hasattr(l.dl4j_bn_fold, "_typed"):
+        vp, i32 = ctypes.c_void_p, ctypes.c_int
+        l.dl4j_bn_fold.argtypes = [vp, vp, i32, vp, vp, vp, vp]
+        l.dl4j_bn_fold.restype = i32
+        l.dl4j_bn_fold._typed = True
+    _check(l.dl4j_bn_fold(_ptr(table), _ptr(block_entry), block_entry.numel(), _ptr(params), _ptr(w_out), _ptr(b_out), _stream()),
+           "dl4j_bn_fold")
+
+
+def conv_infer_1x1(x, w, b, relu, residual=None):
+    """relu?(x * w + b [+ residual]) for a dense channels-last x [N, Cin, H, W] and w [Cout, Cin] bf16, b fp32; one GEMM."""
+    l = require()
+    N, C, H, W = x.shape
+    O = w.shape[0]
+    M = N * H * W
+    y = torch.empty((N, H, W, O), dtype=x.dtype, device=x.device)
+    act = (1 << 16 if residual is not None else 1) if relu else 0
+    rc = l.dl4j_gemm(x.data_ptr(), w.data_ptr(), y.data_ptr(), None, b.data_ptr(), None if residual is None else residual.data_ptr(), M, O, C,
+                     C, C, O, 0, O, 0, 0, _DT[x.dtype], 1, 0, act, 0, 1, 1.0, _pick_block_n(M, O), num_sms(), _stream())
+    _check(rc, "dl4j_gemm")
+    return y.permute(0, 3, 1, 2)
+
+
+def conv_infer_kxk(x, w, b, kH, kW, pad, dil, relu, fuse_w=False):
+    """relu?(conv(x, w) + b), stride 1, for a dense channels-last x and w [Cout, kH * kW * Cin] bf16 (channels-last), b fp32."""
+    l = require()
+    _conv_sigs(l)
+    N, C, H, W = x.shape
+    O = w.shape[0]
+    OH, OW = H + 2 * pad[0] - (kH - 1) * dil[0], W + 2 * pad[1] - (kW - 1) * dil[1]
+    y = torch.empty((N, OH, OW, O), dtype=x.dtype, device=x.device)
+    rc = l.dl4j_conv2d(0, x.data_ptr(), w.data_ptr(), y.data_ptr(), b.data_ptr(), N, H, W, C, OH, OW, O, kH, kW, pad[0], pad[1], dil[0], dil[1],
+                       _DT[x.dtype], 1, int(bool(relu)), int(bool(fuse_w)), _stream())
+    _check(rc, "dl4j_conv2d")
+    return y.permute(0, 3, 1, 2)
 
 
 def conv_weight_cl(W):

@@ -1,0 +1,79 @@
+"""Inference with batch norm folded into the convolutions against the layer-by-layer executor in fp32 on the CPU."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _net(cin, hw, width, layers, has_bias=True, log_std=True, lock=False, residual=True):
+    from deeplearning4j_b200 import DataType, nn
+    from deeplearning4j_b200.nn.conf.base import ConvolutionMode, InputType, PoolingType
+    from deeplearning4j_b200.nn.conf.graphconf import ElementWiseVertex
+    from deeplearning4j_b200.nn.graph import ComputationGraph
+    from deeplearning4j_b200.nn.layers.conv import BatchNormalization, ConvolutionLayer, GlobalPoolingLayer
+    from deeplearning4j_b200.nn.layers.core import ActivationLayer, OutputLayer
+
+    def build(compute):
+        b = nn.NeuralNetConfiguration.Builder().seed(3).activation("IDENTITY").convolutionMode(ConvolutionMode.Same)
+        if compute:
+            b = b.computeDataType(DataType.BFLOAT16)
+        gb = b.graphBuilder()
+        gb.addInputs("in").setInputTypes(InputType.convolutional(hw, hw + 3, cin))
+        prev, first = "in", None
+        for i, (k, s, n) in enumerate(layers):
+            gb.addLayer(f"c{i}", ConvolutionLayer([k, k], [s, s], nOut=n, hasBias=has_bias), prev)
+            gb.addLayer(f"n{i}", BatchNormalization(useLogStd=log_std, lockGammaBeta=lock, gamma=1.5, beta=0.25), f"c{i}")
+            prev = f"n{i}"
+            if i + 1 < len(layers) or not residual:
+                gb.addLayer(f"a{i}", ActivationLayer("RELU"), prev)
+                prev = f"a{i}"
+            if i == 0:
+                first = prev
+        if residual:
+            gb.addVertex("add", ElementWiseVertex("Add"), prev, first)
+            gb.addLayer("ra", ActivationLayer("RELU"), "add")
+            prev = "ra"
+        gb.addLayer("pool", GlobalPoolingLayer(PoolingType.AVG), prev)
+        gb.addLayer("out", OutputLayer("MCXENT", nOut=10, activation="SOFTMAX"), "pool")
+        return ComputationGraph(gb.setOutputs("out").build())
+    gpu, cpu = build(True), build(False)
+    gpu.device = torch.device("cuda")
+    gpu.init(), cpu.init()
+    g = torch.Generator().manual_seed(5)
+    p = torch.empty(cpu.numParams())
+    for e in cpu.entries:
+        seg = p[e.offset:e.end]
+        if e.spec.kind == "weight" and len(e.spec.shape) >= 2 and min(e.spec.shape) > 1:
+            fan = e.spec.numel / (e.spec.shape[0] if len(e.spec.shape) == 4 else e.spec.shape[1])
+            seg.normal_(0, (1.0 / fan) ** 0.5, generator=g)
+        else:
+            seg.normal_(0, 0.1, generator=g)
+            if e.spec.name == "gamma" or e.spec.name == "var":
+                seg.add_(1.0)
+    gpu.setParams(p), cpu.setParams(p)
+    return gpu, cpu
+
+
+@pytest.mark.parametrize("layers,opts", [
+    ([(3, 1, 16), (1, 1, 8), (3, 1, 8), (1, 1, 16)], {}),                                  # bottleneck, residual in the GEMM epilogue
+    ([(3, 1, 24), (3, 1, 24)], {}),                                                        # basic block: residual after a k x k convolution
+    ([(7, 2, 16), (1, 2, 40), (5, 1, 8)], {"residual": False}),                            # stem, strided 1x1, 5x5
+    ([(3, 2, 16), (3, 1, 12), (1, 1, 16)], {"residual": False, "has_bias": False, "log_std": False}),   # 12 channels: not on the 8 grid
+    ([(1, 1, 16), (1, 1, 16)], {"lock": True}),
+])
+@pytest.mark.parametrize("cin,hw,n", [(3, 12, 2), (16, 9, 1), (8, 17, 5)])
+def test_folded_output_matches_fp32(layers, opts, cin, hw, n):
+    gpu, cpu = _net(cin, hw, 16, layers, **opts)
+    x = torch.randn(n, cin, hw, hw + 3, generator=torch.Generator().manual_seed(n))
+    want = cpu.output(x)[0].t
+    for xin in (x.cuda(), x.cuda().to(memory_format=torch.channels_last)):
+        got = gpu.output(xin)[0].t.cpu()
+        # bf16 weights and activations: 2^-9 per rounding, at most 2 roundings per layer, on logits of order one
+        assert (got - want).norm() <= 2 ** -8 * (2 * len(layers)) ** 0.5 * want.norm() * 2
+    got2 = gpu.output(x.cuda(), train=False)[0].t.cpu()
+    acts = gpu.feedForward(x.cuda())                                  # the unfused executor still exposes every activation
+    assert torch.allclose(acts["out"].t.float().cpu(), got2, atol=2e-2)
+    gpu.setParams(gpu.params().t * 0.5)                               # nothing is kept from one call to the next
+    cpu.setParams(cpu.params().t * 0.5)
+    want = cpu.output(x)[0].t
+    assert (gpu.output(x.cuda())[0].t.cpu() - want).norm() <= 2 ** -8 * (2 * len(layers)) ** 0.5 * want.norm() * 2
