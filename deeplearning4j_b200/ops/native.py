@@ -101,12 +101,16 @@ def lib():
 
 
 def available() -> bool:
+    # asked before every launch: once torch has initialised CUDA there is a device, and is_available() (environment look-ups on
+    # each call, 2 us) need not be asked again
+    if _LIB is not None and torch.cuda.is_initialized():
+        return True
     return torch.cuda.is_available() and _load() is not None
 
 
 def require():
     """Fail loudly when a GPU is present but the native library is not."""
-    if torch.cuda.is_available() and _load() is None:
+    if _LIB is None and torch.cuda.is_available() and _load() is None:
         raise RuntimeError(f"deeplearning4j_b200 native library unavailable on a GPU machine: {_LIB_ERR}")
     return _LIB
 
@@ -123,10 +127,11 @@ def _ptr(t):
 def _stream():
     """Current torch stream handle; also binds the current device's context to this thread for the
     library's own CUDA runtime instance (autograd worker threads may not have one bound yet)."""
-    rc = _LIB.dl4j_bind_device(torch.cuda.current_device())
+    dev = torch.cuda.current_device()
+    rc = _LIB.dl4j_bind_device(dev)
     if rc != 0:
         raise RuntimeError(f"dl4j_bind_device failed with CUDA error {rc}")
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(dev))       # the raw handle: a Stream object costs 10 us a launch
 
 
 def _check(rc, what):

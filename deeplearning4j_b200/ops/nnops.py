@@ -10,6 +10,8 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
+from . import native
+
 _FORCE_TORCH = False
 
 
@@ -27,14 +29,12 @@ def set_force_torch(v: bool):
 def have_fused() -> bool:
     if _FORCE_TORCH or not torch.cuda.is_available():
         return False
-    from . import native
     return native.available()
 
 
 def _native_for(x: torch.Tensor):
     if _FORCE_TORCH or not x.is_cuda:
         return None
-    from . import native
     return native if native.available() else None
 
 
