@@ -1,4 +1,4 @@
-// Fused scaled-dot-product attention, backward pass (head size 64, bf16).
+// Fused scaled-dot-product attention, backward pass (head sizes up to 64, bf16).
 #include "flash_common.cuh"
 
 using namespace dl4j;
@@ -9,7 +9,9 @@ using namespace dl4j;
 //     ->  P, dS staged in shared memory (bf16)  ->  dV += P^T dO_i, dK += dS^T Q_i (accumulated in TMEM over i),
 //     dQ_i = dS K_j (TMEM, added to the fp32 dQ buffer with vector atomics: four key blocks contribute to it).
 // P^T and dS^T are the same shared-memory tiles read through MN-major descriptors, so nothing is transposed.
-// D = rowsum(dO * O) and the forward's log-sum-exp come from the caller.
+// D = rowsum(dO * O) and the forward's log-sum-exp come from the caller.  Keys past Tk and causally hidden ones are taken out by the same
+// bits as masked keys; a causal key block starts at its own query block.  With a single key block nothing else contributes to dQ and
+// it is written in bf16 directly.
 namespace dl4j {
 
 constexpr int FB_THREADS = 64 + 512;              // warp 0 TMA, warp 1 MMA, 16 compute warps (four threads per row)
@@ -22,11 +24,15 @@ struct FlashBwdParams {
   const float* lse;          // [B, H, Tq]
   const float* dvec;         // [B, H, Tq]  rowsum(dO * O)
   const float* key_mask;     // [B, Tk] or null
-  float* dq;                 // [B, H, Tq, 64] fp32, zero on entry
-  __nv_bfloat16* dk;         // [B, Tk, H, 64]
-  __nv_bfloat16* dv;         // [B, Tk, H, 64]
-  long o_bs, o_ts;           // element strides of dk / dv between batch entries and between keys (heads are 64 apart)
-  int B, H, Tq, Tk;
+  float* dq;                 // [B, H, Tq, D] fp32, zero on entry; null: dq16 is written directly (one key block)
+  __nv_bfloat16* dq16;       // [B, Tq, H, D]
+  __nv_bfloat16* dk;         // [B, Tk, H, D]
+  __nv_bfloat16* dv;         // [B, Tk, H, D]
+  long q_bs, q_ts;           // element strides of dq16 between batch entries and between queries (heads are D apart)
+  long o_bs, o_ts;           // element strides of dk / dv between batch entries and between keys
+  int B, H, Tq, Tk, D;
+  int causal;
+  int nan_empty;             // rows without any key: their weights are NaN instead of 0
   float scale;
   int* status;
   const unsigned long long* seed;   // dropout seed of the forward pass (device memory), read when drop_thr != 0
@@ -60,12 +66,16 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k_blocks = p.Tk / FB_BLK;
+  const int k_blocks = (p.Tk + FB_BLK - 1) / FB_BLK;
   const int kb = blockIdx.x % k_blocks;
   const int h = (blockIdx.x / k_blocks) % p.H;
   const int b = blockIdx.x / (k_blocks * p.H);
   const int k0 = kb * FB_BLK;
-  const int nq = (p.Tq + FB_BLK - 1) / FB_BLK;
+  // first query block that sees these keys.  Queries without any key (under a causal mask there are some exactly when key 0 is masked)
+  // make every dV of the example NaN where that is asked for, so all blocks are visited then.
+  const bool empties = p.causal && p.nan_empty && p.key_mask != nullptr && p.key_mask[(long)b * p.Tk] == 0.f;
+  const int i0 = p.causal && !empties ? kb : 0;
+  const int nq = max((p.Tq + FB_BLK - 1) / FB_BLK - i0, 0);    // query blocks to visit; loop indices count from i0
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_do);
@@ -97,8 +107,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         const int st = i & 1;
         if (!mbar_wait_bounded(&qdo_empty[st], (uint32_t)(((i >> 1) & 1) ^ 1), p.status, DL4J_ERR_TIMEOUT_PRODUCER)) break;
         mbar_expect_tx(&qdo_full[st], 2 * FB_TILE);
-        tma_load_4d(q_s + st * FB_TILE, &tmap_q, &qdo_full[st], 0, i * FB_BLK, h, b);
-        tma_load_4d(do_s + st * FB_TILE, &tmap_do, &qdo_full[st], 0, i * FB_BLK, h, b);
+        tma_load_4d(q_s + st * FB_TILE, &tmap_q, &qdo_full[st], 0, (i0 + i) * FB_BLK, h, b);
+        tma_load_4d(do_s + st * FB_TILE, &tmap_do, &qdo_full[st], 0, (i0 + i) * FB_BLK, h, b);
       }
     }
   } else if (warp == 1) {
@@ -131,7 +141,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       const uint64_t d_dsk = make_smem_desc_sw128(ads, 16, 1024), d_kmn = make_smem_desc_sw128(ak, FB_BLK * 128, 1024);
       const uint64_t d_do_mn0 = make_smem_desc_sw128(smem_u32(do_s), FB_BLK * 128, 1024), d_q_mn0 = make_smem_desc_sw128(smem_u32(q_s), FB_BLK * 128, 1024);
       constexpr uint64_t STAGE_STEP = (uint64_t)(FB_TILE >> 4);     // second Q / dO stage: same descriptor, start address + one tile
-      if (ok) ok = issue_s(0);
+      if (ok && nq > 0) ok = issue_s(0);
       for (int i = 0; i < nq && ok; ++i) {
         const int st = i & 1;
         const uint64_t d_do_st = d_do_mn0 + (st ? STAGE_STEP : 0), d_q_st = d_q_mn0 + (st ? STAGE_STEP : 0);
@@ -168,15 +178,15 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     const int cq = cw >> 2;                         // column quarter (32 columns) owned by this thread
     const int r = q * 32 + lane;
     const int t = threadIdx.x - 64;                 // 0..511
-    if (t < FB_BLK) mask_s[t] = p.key_mask ? p.key_mask[(long)b * p.Tk + k0 + t] : 1.f;
+    if (t < FB_BLK) mask_s[t] = k0 + t >= p.Tk ? 0.f : (p.key_mask ? p.key_mask[(long)b * p.Tk + k0 + t] : 1.f);
     asm volatile("bar.sync 1, 512;" ::: "memory");
     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     const float k2 = p.scale * FA_LOG2E;
     // key mask of this thread's 32 columns as a bit word; without masked keys the inner loop has no select at all
-    uint32_t mbits = 0;
+    uint32_t key_bits = 0;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) mbits |= (mask_s[cq * 32 + j] != 0.f ? 1u : 0u) << j;
-    const bool all_keys = mbits == 0xffffffffu;
+    for (int j = 0; j < 32; ++j) key_bits |= (mask_s[cq * 32 + j] != 0.f ? 1u : 0u) << j;
+    const uint32_t in_bits = fa_low_bits(p.Tk - (k0 + cq * 32));      // keys that exist
     const float sc = p.scale;
     constexpr bool drop = DROP;
     uint32_t seed_lo = 0u, seed_hi = 0u;
@@ -185,7 +195,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     bool ok = true;
     const long rbase = ((long)b * p.H + h) * p.Tq;
     // per-row log-sum-exp and D of the next query block are fetched one block ahead (+inf: exp2(-inf) = 0 past the end)
-    float lse_n = r < p.Tq ? p.lse[rbase + r] : INFINITY, dv_n = r < p.Tq ? p.dvec[rbase + r] : 0.f;
+    const int t0 = i0 * FB_BLK + r;
+    float lse_n = t0 < p.Tq ? p.lse[rbase + t0] : INFINITY, dv_n = t0 < p.Tq ? p.dvec[rbase + t0] : 0.f;
     auto dq_flush = [&](int blk) -> bool {
       // dQ_blk: 64 columns per row, 16 per thread (all four column groups take part)
       if (!mbar_wait_bounded(dq_full, (uint32_t)(blk & 1), p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) return false;
@@ -196,19 +207,32 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(dq_empty);
-      const int tqb = blk * FB_BLK + r;
-      if (tqb < p.Tq) {
-        float4* dst = reinterpret_cast<float4*>(p.dq + (rbase + tqb) * FA_D + cq * 16);
+      const int tqb = (i0 + blk) * FB_BLK + r;
+      if (tqb < p.Tq && p.dq == nullptr) {
+        uint4* dst = reinterpret_cast<uint4*>(p.dq16 + b * p.q_bs + tqb * p.q_ts + (long)h * p.D + cq * 16);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          uint4 u;
+          __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) hh[e] = __floats2bfloat162_rn(__uint_as_float(v0[8 * j + 2 * e]), __uint_as_float(v0[8 * j + 2 * e + 1]));
+          if (cq * 16 + 8 * j < p.D) dst[j] = u;
+        }
+      } else if (tqb < p.Tq) {
+        float4* dst = reinterpret_cast<float4*>(p.dq + (rbase + tqb) * p.D + cq * 16);
 #pragma unroll
         for (int j = 0; j < 4; ++j)      // fire-and-forget 16-byte reductions at L2
-          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "r"(v0[4 * j]), "r"(v0[4 * j + 1]),
+          if (cq * 16 + 4 * j < p.D) asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "r"(v0[4 * j]), "r"(v0[4 * j + 1]),
                        "r"(v0[4 * j + 2]), "r"(v0[4 * j + 3])
                        : "memory");
       }
       return true;
     };
     for (int i = 0; i < nq && ok; ++i) {
-      const int tq = i * FB_BLK + r;
+      const int tq = (i0 + i) * FB_BLK + r;
+      uint32_t mbits = key_bits;
+      if (p.causal && i0 + i <= kb) mbits &= fa_low_bits(tq + 1 - (k0 + cq * 32));     // the diagonal block
+      const bool all_keys = __all_sync(0xffffffffu, mbits == 0xffffffffu);
       const float lse = lse_n, dv_r = dv_n;
       if (i + 1 < nq) {
         const int tn = tq + FB_BLK;
@@ -252,6 +276,10 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
             de[j] = pv * fmaf(__uint_as_float(dpv[j]), sc, -dvs);
           }
         }
+        if (p.nan_empty && lse == -INFINITY) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) { pe[j] = ((in_bits >> j) & 1u) ? __int_as_float(0x7fffffff) : 0.f; de[j] = 0.f; }
+        }
         fa_store_row(p_s, r, cq * 32, 32, pe);
         fa_store_row(ds_s, r, cq * 32, 32, de);
       }
@@ -267,10 +295,14 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     if (ok && mbar_wait_bounded(fin_full, 0, p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) {
       tc_fence_after();
       // accumulator rows are keys here: thread r owns key k0 + r; column groups 0, 1 -> dV, 2, 3 -> dK
-      const long orow = (long)b * p.o_bs + (long)(k0 + r) * p.o_ts + (long)h * FA_D + (cq & 1) * 32;
+      const long orow = (long)b * p.o_bs + (long)(k0 + r) * p.o_ts + (long)h * p.D + (cq & 1) * 32;
       uint32_t v0[32];
       tmem_ld_32x32(taddr + (cq < 2 ? T_DV : T_DK) + (cq & 1) * 32, v0);
       tmem_ld_wait();
+      if (nq == 0) {                                   // no query sees these keys: nothing was accumulated
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v0[j] = 0u;
+      }
       uint4* dst = reinterpret_cast<uint4*>((cq < 2 ? p.dv : p.dk) + orow);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -278,7 +310,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&u);
 #pragma unroll
         for (int e = 0; e < 4; ++e) hh[e] = __floats2bfloat162_rn(__uint_as_float(v0[8 * j + 2 * e]), __uint_as_float(v0[8 * j + 2 * e + 1]));
-        dst[j] = u;
+        if (k0 + r < p.Tk && (cq & 1) * 32 + 8 * j < p.D) dst[j] = u;
       }
     }
     tc_fence_before();
@@ -294,32 +326,39 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
 }  // namespace dl4j
 
-// q / k / v / dout: [B, H, T, 64] bf16 views (element strides {sb, sh, st}); lse, dvec [B, H, Tq] fp32; dq [B, H, Tq, 64] fp32
-// zeroed by the caller; dk, dv bf16 addressed as base + b * o_bs + key * o_ts + head * 64.  Limits: Tk a multiple of 128.
+// q / k / v / dout: [B, H, T, D] bf16 views (element strides {sb, sh, st}), D a multiple of 8 up to 64; lse, dvec [B, H, Tq] fp32;
+// dq_acc [B, H, Tq, D] fp32 zeroed by the caller, or null with at most 128 keys: dq is then written here, addressed as
+// base + b * q_bs + query * q_ts + head * D; dk, dv bf16 addressed as base + b * o_bs + key * o_ts + head * D.
+// flags as in dl4j_flash_attn_fwd.
 DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* dvec,
-                                 const float* key_mask, float* dq, void* dk, void* dv, int B, int H, int Tq, int Tk, const long* q_strides,
-                                 const long* k_strides, const long* v_strides, const long* do_strides, long o_bs, long o_ts, float scale,
-                                 float dropout_p, const void* seed, void* stream_) {
-  if (B < 1 || H < 1 || Tq < 1 || Tk < FB_BLK || Tk % FB_BLK) return -DL4J_ERR_BAD_ARG;
+                                 const float* key_mask, float* dq_acc, void* dq, void* dk, void* dv, int B, int H, int Tq, int Tk, int D,
+                                 const long* q_strides, const long* k_strides, const long* v_strides, const long* do_strides, long q_bs,
+                                 long q_ts, long o_bs, long o_ts, float scale, int flags, float dropout_p, const void* seed, void* stream_) {
+  if (B < 1 || H < 1 || Tq < 1 || Tk < 1 || D < 8 || D > FA_D || D % 8) return -DL4J_ERR_BAD_ARG;
   if (dropout_p < 0.f || dropout_p >= 1.f || (dropout_p > 0.f && !seed)) return -DL4J_ERR_BAD_ARG;
+  if (!dq_acc && (!dq || Tk > FB_BLK)) return -DL4J_ERR_BAD_ARG;
   CUtensorMap tq, tk, tv, tdo;
-  int r = fa_encode(&tq, q, B, H, Tq, q_strides[0], q_strides[1], q_strides[2], FB_BLK);
+  int r = fa_encode(&tq, q, B, H, Tq, D, q_strides[0], q_strides[1], q_strides[2], FB_BLK);
   if (r) return -1000 - r;
-  r = fa_encode(&tk, k, B, H, Tk, k_strides[0], k_strides[1], k_strides[2], FB_BLK);
+  r = fa_encode(&tk, k, B, H, Tk, D, k_strides[0], k_strides[1], k_strides[2], FB_BLK);
   if (r) return -1000 - r;
-  r = fa_encode(&tv, v, B, H, Tk, v_strides[0], v_strides[1], v_strides[2], FB_BLK);
+  r = fa_encode(&tv, v, B, H, Tk, D, v_strides[0], v_strides[1], v_strides[2], FB_BLK);
   if (r) return -1000 - r;
-  r = fa_encode(&tdo, dout, B, H, Tq, do_strides[0], do_strides[1], do_strides[2], FB_BLK);
+  r = fa_encode(&tdo, dout, B, H, Tq, D, do_strides[0], do_strides[1], do_strides[2], FB_BLK);
   if (r) return -1000 - r;
   int dev = 0;
   cudaGetDevice(&dev);
   FlashBwdParams p;
   p.lse = lse; p.dvec = dvec; p.key_mask = key_mask;
-  p.dq = dq;
+  p.dq = dq_acc;
+  p.dq16 = reinterpret_cast<__nv_bfloat16*>(dq);
+  p.q_bs = q_bs; p.q_ts = q_ts;
   p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
   p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
   p.o_bs = o_bs; p.o_ts = o_ts;
-  p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk;
+  p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.D = D;
+  p.causal = flags & 1;
+  p.nan_empty = (flags >> 1) & 1;
   p.scale = scale;
   p.status = dl4j_status_word(dev);
   p.seed = reinterpret_cast<const unsigned long long*>(seed);
@@ -329,7 +368,7 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   auto kern = p.drop_thr ? flash_attn_bwd_kernel<true> : flash_attn_bwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  kern<<<B * H * (Tk / FB_BLK), FB_THREADS, smem, (cudaStream_t)stream_>>>(tq, tk, tv, tdo, p);
+  kern<<<B * H * ((Tk + FB_BLK - 1) / FB_BLK), FB_THREADS, smem, (cudaStream_t)stream_>>>(tq, tk, tv, tdo, p);
   return (int)cudaGetLastError();
 }
 
@@ -339,18 +378,18 @@ namespace dl4j {
 // dvec[b, h, t] = sum_d dO[b, h, t, d] * O[b, t, h, d]; eight threads per row, 8 elements each
 __global__ void __launch_bounds__(256)
 attn_dvec_kernel(const __nv_bfloat16* __restrict__ dO, long sb, long sh, long st, const __nv_bfloat16* __restrict__ O, float* __restrict__ dvec,
-                 int B, int H, int T) {
+                 int B, int H, int T, int D) {
   const long rows = (long)B * H * T;
   const long g = blockIdx.x * 256L + threadIdx.x;
   const long row = g >> 3;
   const int part = (int)(g & 7);
   float acc = 0.f;
-  if (row < rows) {
+  if (row < rows && part * 8 < D) {
     const int t = (int)(row % T);
     const int h = (int)((row / T) % H);
     const int b = (int)(row / ((long)T * H));
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(dO + b * sb + h * sh + t * st) + part);
-    const uint4 c = __ldg(reinterpret_cast<const uint4*>(O + (((long)b * T + t) * H + h) * FA_D) + part);
+    const uint4 c = __ldg(reinterpret_cast<const uint4*>(O + (((long)b * T + t) * H + h) * D) + part);
     const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&a);
     const __nv_bfloat162* ch = reinterpret_cast<const __nv_bfloat162*>(&c);
 #pragma unroll
@@ -365,42 +404,41 @@ attn_dvec_kernel(const __nv_bfloat16* __restrict__ dO, long sb, long sh, long st
   if (row < rows && part == 0) dvec[row] = acc;
 }
 
-// dq (bf16, addressed base + b * o_bs + t * o_ts + h * 64) = acc [B, H, T, 64] fp32; the accumulator is cleared for its next use
+// dq (bf16, addressed base + b * o_bs + t * o_ts + h * D) = acc [B, H, T, D] fp32
 __global__ void __launch_bounds__(256)
-attn_dq_finish_kernel(float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long o_bs, long o_ts, int B, int H, int T) {
-  const long n8 = (long)B * H * T * (FA_D / 8);
+attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long o_bs, long o_ts, int B, int H, int T, int D) {
+  const int parts = D / 8;
+  const long n8 = (long)B * H * T * parts;
   for (long g = blockIdx.x * 256L + threadIdx.x; g < n8; g += (long)gridDim.x * 256) {
-    const int part = (int)(g & 7);
-    const long row = g >> 3;
+    const int part = (int)(g % parts);
+    const long row = g / parts;
     const int t = (int)(row % T);
     const int h = (int)((row / T) % H);
     const int b = (int)(row / ((long)T * H));
-    float4* src = reinterpret_cast<float4*>(acc) + 2 * g;
-    const float4 x = src[0], y = src[1];
+    const float4* src = reinterpret_cast<const float4*>(acc) + 2 * g;
+    const float4 x = __ldcs(src), y = __ldcs(src + 1);
     uint4 u;
     __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&u);
     hh[0] = __floats2bfloat162_rn(x.x, x.y); hh[1] = __floats2bfloat162_rn(x.z, x.w);
     hh[2] = __floats2bfloat162_rn(y.x, y.y); hh[3] = __floats2bfloat162_rn(y.z, y.w);
-    reinterpret_cast<uint4*>(out + b * o_bs + t * o_ts + (long)h * FA_D)[part] = u;
-    src[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-    src[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<uint4*>(out + b * o_bs + t * o_ts + (long)h * D)[part] = u;
   }
 }
 
 }  // namespace dl4j
 
-DL4J_API int dl4j_attn_dvec(const void* dout, const long* do_strides, const void* out, float* dvec, int B, int H, int T, void* stream) {
+DL4J_API int dl4j_attn_dvec(const void* dout, const long* do_strides, const void* out, float* dvec, int B, int H, int T, int D, void* stream) {
   const long threads = (long)B * H * T * 8;
   attn_dvec_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(dout), do_strides[0], do_strides[1], do_strides[2], reinterpret_cast<const __nv_bfloat16*>(out),
-      dvec, B, H, T);
+      dvec, B, H, T, D);
   return (int)cudaGetLastError();
 }
 
-DL4J_API int dl4j_attn_dq_finish(float* acc, void* out, long o_bs, long o_ts, int B, int H, int T, void* stream) {
-  const long n8 = (long)B * H * T * 8;
+DL4J_API int dl4j_attn_dq_finish(const float* acc, void* out, long o_bs, long o_ts, int B, int H, int T, int D, void* stream) {
+  const long n8 = (long)B * H * T * (D / 8);
   long blocks = (n8 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  attn_dq_finish_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(acc, reinterpret_cast<__nv_bfloat16*>(out), o_bs, o_ts, B, H, T);
+  attn_dq_finish_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(acc, reinterpret_cast<__nv_bfloat16*>(out), o_bs, o_ts, B, H, T, D);
   return (int)cudaGetLastError();
 }

@@ -1,8 +1,11 @@
-// Fused scaled-dot-product attention forward for head size 64 (bf16), one CTA per (batch, head, 128-query block), two
+// Fused scaled-dot-product attention forward for head sizes up to 64 (bf16), one CTA per (batch, head, 128-query block), two
 // CTAs resident per SM so that one CTA's softmax overlaps the other's loads and MMAs:
 //     for each block of 128 keys:  S = Q K_j^T (tcgen05, fp32 in TMEM)  ->  online softmax in registers  ->
 //     P_j (bf16) staged in shared memory  ->  P_j V_j (tcgen05, TMEM)  ->  O = O * alpha + P_j V_j in registers
-//     finally: normalise, store O [B, Tq, H, 64] and the row log-sum-exp [B, H, Tq].
+//     finally: normalise, store O [B, Tq, H, D] and the row log-sum-exp [B, H, Tq].
+// Any number of keys: the last block's missing keys are zero rows that a bit mask takes out of the softmax; the same bits carry the
+// key mask and the causal mask, and causal blocks past the diagonal are not visited.  When the gradient is what the caller wants, O is
+// not stored: the row sums of dO * O that the backward kernel needs are taken from the fp32 accumulators instead.
 // The score matrix never reaches HBM (AttentionHelper.cpp computes matmul, scale, mask add, softmax over the full
 // score matrix and a second matmul as separate ops).  Warp 0 issues the TMA loads (K / V blocks through a 3-slot
 // ring), warp 1 the MMAs, warps 2-9 do the softmax: two threads per query row, each owning half of the columns.
@@ -20,10 +23,15 @@ constexpr int FF_TMEM_COLS = 256;             // S: 0..127, P V: 128..191
 constexpr uint32_t FF_T_PV = 128;
 
 struct FlashFwdParams {
-  __nv_bfloat16* out;        // [B, Tq, H, 64]
+  __nv_bfloat16* out;        // [B, Tq, H, D] or null
   float* lse;                // [B, H, Tq]
   const float* key_mask;     // [B, Tk] (non-zero = keep) or null
-  int B, H, Tq, Tk;
+  const __nv_bfloat16* dout; // gradient of the output, element strides do_b / do_h / do_t, or null
+  long do_b, do_h, do_t;
+  float* dvec;               // [B, H, Tq] rowsum(dO * O), written when dout is given
+  int B, H, Tq, Tk, D;
+  int causal;                // key index <= query index
+  float empty;               // value of a row without any key: 0 or NaN
   float scale;
   int* status;
   const unsigned long long* seed;   // device-resident dropout seed (read when drop_thr != 0)
@@ -53,10 +61,11 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q_blocks = (p.Tq + FF_BM - 1) / FF_BM;
-  const int qb = blockIdx.x % q_blocks;
+  const int qb = q_blocks - 1 - blockIdx.x % q_blocks;          // causal: the longest rows start first
   const int h = (blockIdx.x / q_blocks) % p.H;
   const int b = blockIdx.x / (q_blocks * p.H);
-  const int nb = p.Tk / FF_BN;
+  const int nb_all = (p.Tk + FF_BN - 1) / FF_BN;
+  const int nb = p.causal ? min(nb_all, qb + 1) : nb_all;
   const int q0 = qb * FF_BM;
 
   if (threadIdx.x == 0) {
@@ -168,11 +177,11 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     // Key mask: block 0 is staged here, block j + 1 is fetched into a register at the top of block j and stored at its end, so
     // no global-memory latency sits between the barriers.  Without a mask the loops below have no select at all.
     const bool has_mask = p.key_mask != nullptr;
-    if (has_mask && t < FF_BN) mask_s[t] = p.key_mask[(long)b * p.Tk + t];
+    if (has_mask && t < FF_BN) mask_s[t] = t < p.Tk ? p.key_mask[(long)b * p.Tk + t] : 0.f;
     asm volatile("bar.sync 1, 256;" ::: "memory");
     for (int j = 0; j < nb; ++j) {
       float mask_next = 1.f;
-      if (has_mask && j + 1 < nb && t < FF_BN) mask_next = p.key_mask[(long)b * p.Tk + (j + 1) * FF_BN + t];
+      if (has_mask && j + 1 < nb && t < FF_BN) mask_next = (j + 1) * FF_BN + t < p.Tk ? p.key_mask[(long)b * p.Tk + (j + 1) * FF_BN + t] : 0.f;
       float* xj = xch + (j & 1) * (2 * FF_BM);       // exchange buffer of this block (the other parity may still be read)
       if (!mbar_wait_bounded(s_full, (uint32_t)(j & 1), p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) *fail_s = 1;
       tc_fence_after();
@@ -184,7 +193,10 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
         for (int i = 0; i < 32; ++i) { mb0 |= (mk[i] != 0.f ? 1u : 0u) << i; mb1 |= (mk[32 + i] != 0.f ? 1u : 0u) << i; }
       }
-      const bool all_keys = (mb0 & mb1) == 0xffffffffu;
+      int lim = p.Tk - (j * FF_BN + ch * 64);          // keys of this thread's 64 that exist (and that its row may see)
+      if (p.causal) lim = min(lim, q0 + r + 1 - (j * FF_BN + ch * 64));
+      if (lim < 64) { mb0 &= fa_low_bits(lim); mb1 &= fa_low_bits(lim - 32); }
+      const bool all_keys = __all_sync(0xffffffffu, (mb0 & mb1) == 0xffffffffu);     // warp-uniform: tcgen05.ld follows
       float m = -INFINITY;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -253,17 +265,42 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       xl[ch * FF_BM + r] = run_l;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       const float l = run_l + xl[(ch ^ 1) * FF_BM + r];
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float inv = l > 0.f ? 1.f / l : p.empty;
       const int tq = q0 + r;
+      if (p.dout) {            // uniform: D = sum over the head dimension of dO * O, this thread's 32 columns, then both halves
+        float d = 0.f;
+        if (tq < p.Tq) {
+          const uint4* src = reinterpret_cast<const uint4*>(p.dout + b * p.do_b + h * p.do_h + tq * p.do_t + ch * 32);
+#pragma unroll
+          for (int jj = 0; jj < 4; ++jj) {
+            if (ch * 32 + jj * 8 < p.D) {
+              const uint4 u = __ldg(src + jj);
+              const __nv_bfloat162* hh = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 g = __bfloat1622float2(hh[i]);
+                d = fmaf(g.x, o[jj * 8 + 2 * i] * inv, fmaf(g.y, o[jj * 8 + 2 * i + 1] * inv, d));
+              }
+            }
+          }
+        }
+        float* xd = xch + ((nb + 1) & 1) * (2 * FF_BM);
+        xd[ch * FF_BM + r] = d;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (ch == 0 && tq < p.Tq) p.dvec[((long)b * p.H + h) * p.Tq + tq] = d + xd[FF_BM + r];
+      }
       if (tq < p.Tq) {
-        uint4* dst = reinterpret_cast<uint4*>(p.out + (((long)b * p.Tq + tq) * p.H + h) * FA_D + ch * 32);
+        uint4* dst = reinterpret_cast<uint4*>(p.out + (((long)b * p.Tq + tq) * p.H + h) * p.D + ch * 32);
+        if (p.out) {
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
+          if (ch * 32 + jj * 8 >= p.D) break;
           uint4 u;
           __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&u);
 #pragma unroll
           for (int i = 0; i < 4; ++i) hh[i] = __floats2bfloat162_rn(o[jj * 8 + 2 * i] * inv, o[jj * 8 + 2 * i + 1] * inv);
           dst[jj] = u;
+        }
         }
         if (p.lse && ch == 0) {
           const float mref = (run_m == -INFINITY) ? 0.f : run_m;
@@ -286,21 +323,23 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 
 using namespace dl4j;
 
-// q / k / v: [B, H, T, 64] bf16 views with element strides {sb, sh, st} (head dimension contiguous, strides multiples of 8,
-// base 16-byte aligned).  out [B, Tq, H, 64] bf16 contiguous, lse [B, H, Tq] fp32, key_mask [B, Tk] fp32 or null.
-// Limits: Tk a multiple of 128.  dropout_p > 0: `seed` points to a 64-bit seed in device memory; pass the same seed and
-// probability to the backward pass.
+// q / k / v (and dout): [B, H, T, D] bf16 views with element strides {sb, sh, st} (head dimension contiguous, strides multiples of 8,
+// base 16-byte aligned), D a multiple of 8 up to 64.  out [B, Tq, H, D] bf16 contiguous or null, lse [B, H, Tq] fp32, key_mask [B, Tk]
+// fp32 or null.  With dout, dvec [B, H, Tq] receives rowsum(dO * O).  flags: 1 causal (key index <= query index), 2 a row without any
+// key is NaN (0 otherwise).  dropout_p > 0: `seed` points to a 64-bit seed in device memory; pass the same seed and probability to
+// the backward pass.
 DL4J_API int dl4j_flash_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const float* key_mask, int B, int H,
-                                 int Tq, int Tk, const long* q_strides, const long* k_strides, const long* v_strides, float scale,
-                                 float dropout_p, const void* seed, void* stream_) {
-  if (B < 1 || H < 1 || Tq < 1 || Tk < FF_BN || Tk % FF_BN) return -DL4J_ERR_BAD_ARG;
-  if (dropout_p < 0.f || dropout_p >= 1.f || (dropout_p > 0.f && !seed)) return -DL4J_ERR_BAD_ARG;
+                                 int Tq, int Tk, int D, const long* q_strides, const long* k_strides, const long* v_strides, float scale,
+                                 int flags, const void* dout, const long* do_strides, float* dvec, float dropout_p, const void* seed,
+                                 void* stream_) {
+  if (B < 1 || H < 1 || Tq < 1 || Tk < 1 || D < 8 || D > FA_D || D % 8) return -DL4J_ERR_BAD_ARG;
+  if (dropout_p < 0.f || dropout_p >= 1.f || (dropout_p > 0.f && !seed) || (dout && !dvec)) return -DL4J_ERR_BAD_ARG;
   CUtensorMap tq, tk, tv;
-  int r = fa_encode(&tq, q, B, H, Tq, q_strides[0], q_strides[1], q_strides[2], FF_BM);
+  int r = fa_encode(&tq, q, B, H, Tq, D, q_strides[0], q_strides[1], q_strides[2], FF_BM);
   if (r) return -1000 - r;
-  r = fa_encode(&tk, k, B, H, Tk, k_strides[0], k_strides[1], k_strides[2], FF_BN);
+  r = fa_encode(&tk, k, B, H, Tk, D, k_strides[0], k_strides[1], k_strides[2], FF_BN);
   if (r) return -1000 - r;
-  r = fa_encode(&tv, v, B, H, Tk, v_strides[0], v_strides[1], v_strides[2], FF_BN);
+  r = fa_encode(&tv, v, B, H, Tk, D, v_strides[0], v_strides[1], v_strides[2], FF_BN);
   if (r) return -1000 - r;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -308,7 +347,12 @@ DL4J_API int dl4j_flash_attn_fwd(const void* q, const void* k, const void* v, vo
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.lse = lse;
   p.key_mask = key_mask;
-  p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk;
+  p.dout = reinterpret_cast<const __nv_bfloat16*>(dout);
+  p.do_b = dout ? do_strides[0] : 0; p.do_h = dout ? do_strides[1] : 0; p.do_t = dout ? do_strides[2] : 0;
+  p.dvec = dvec;
+  p.B = B; p.H = H; p.Tq = Tq; p.Tk = Tk; p.D = D;
+  p.causal = flags & 1;
+  p.empty = (flags & 2) ? __builtin_nanf("") : 0.f;
   p.scale = scale;
   p.status = dl4j_status_word(dev);
   p.seed = reinterpret_cast<const unsigned long long*>(seed);

@@ -29,6 +29,9 @@ __device__ __forceinline__ void fa_store_row(uint8_t* tile, int r, int col0, int
   }
 }
 
+// low `n` bits set, n clamped to 0 .. 32
+__device__ __forceinline__ uint32_t fa_low_bits(int n) { return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u); }
+
 // Dropout on the attention weights (AttentionHelper.cpp applies it to the softmax output): the keep decision of element
 // (batch*head, query row, key column) is a pure function of a 64-bit seed and those three indices, so the backward pass
 // regenerates the forward's mask instead of storing it.  One Philox4x32-7 block yields 8 x 16 bits = the decisions of 8
@@ -59,11 +62,12 @@ __device__ __forceinline__ uint32_t fa_keep32(uint32_t seed_lo, uint32_t seed_hi
 
 }  // namespace dl4j
 
-// Tensor map over a [B, H, T, 64] bf16 view given by its element strides (unit stride along the head dimension)
-static inline int fa_encode(CUtensorMap* map, const void* base, int B, int H, int T, long sb, long sh, long st, uint32_t box_rows) {
+// Tensor map over a [B, H, T, D] bf16 view (D <= 64) given by its element strides (unit stride along the head dimension).  The box is
+// 64 columns wide whatever D is: the copy engine fills the columns D .. 63 and the rows past T with zeros.
+static inline int fa_encode(CUtensorMap* map, const void* base, int B, int H, int T, int D, long sb, long sh, long st, uint32_t box_rows) {
   dl4j_PFN_encodeTiled enc = dl4j_get_encode_tiled();
   if (!enc) return -1;
-  cuuint64_t dims[4] = {(cuuint64_t)dl4j::FA_D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)st * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
   cuuint32_t box[4] = {(cuuint32_t)dl4j::FA_D, box_rows, 1, 1};
   cuuint32_t es[4] = {1, 1, 1, 1};

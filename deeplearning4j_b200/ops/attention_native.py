@@ -27,7 +27,10 @@ def _ok_view(t):
 
 
 def _prep(t):
-    return t if _ok_view(t) else t.contiguous()
+    if _ok_view(t):
+        return t
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def _bgemm(l, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, alpha, H, Bn, a_bs, b_bs, c_bs, dtype, out_fp32=0):
@@ -57,24 +60,24 @@ def _typed_softmax(l):
 
 class _AttentionFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, key_mask, scale, dropout_p=0.0):
+    def forward(ctx, q, k, v, key_mask, scale, dropout_p=0.0, flags=0):
         l = native.require()
         _typed_softmax(l)
         q, k, v = _prep(q), _prep(k), _prep(v)
         Bn, H, Tq, D = q.shape
         Tk = k.shape[2]
         dt = q.dtype
-        ctx.flash = (USE_FLASH or dropout_p > 0.0) and flash_supported(q, k, v)
+        ctx.flash = (USE_FLASH or dropout_p > 0.0 or flags) and flash_supported(q, k, v)
         if ctx.flash:
             # fused kernel: the score matrix stays in tensor memory; only O and the row log-sum-exp are written
             seed = _next_dropout_seed(q.device) if dropout_p > 0.0 else None
-            O, lse = flash_forward(q, k, v, key_mask, scale, dropout_p, seed)
             mk = key_mask.to(torch.float32).contiguous() if key_mask is not None else None
+            O, lse = flash_forward(q, k, v, mk, scale, dropout_p, seed, flags)
             ctx.save_for_backward(q, k, v, O, lse, mk, seed)
-            ctx.scale, ctx.dropout_p = scale, float(dropout_p)
+            ctx.scale, ctx.dropout_p, ctx.flags = scale, float(dropout_p), flags
             return O.permute(0, 2, 1, 3)
         if dropout_p > 0.0:
-            raise RuntimeError("attention dropout needs the fused kernels (head size 64, key length a multiple of 128)")
+            raise RuntimeError("attention dropout needs the fused kernels (head size up to 64, key length a multiple of 128)")
         P = torch.empty((Bn, H, Tq, Tk), dtype=dt, device=q.device)
         # S = scale * Q K^T
         _bgemm(l, q.data_ptr(), k.data_ptr(), P.data_ptr(), Tq, Tk, D, q.stride(2), k.stride(2), Tk, 0, 0, scale, H, Bn,
@@ -96,7 +99,14 @@ class _AttentionFn(torch.autograd.Function):
     def backward(ctx, dO):
         l = native.require()
         if ctx.flash:
-            return _flash_backward(ctx, dO)
+            q, k, v, O, lse, mk, seed = ctx.saved_tensors
+            dO = _prep(dO)
+            dvec = torch.empty_like(lse)             # D_r = sum_d dO * O per query row, laid out like the log-sum-exp
+            Bn, H, Tq, D = q.shape
+            rc = _flash_lib().dl4j_attn_dvec(native._ptr(dO), _LONG3(*dO.stride()[:3]), native._ptr(O), native._ptr(dvec), Bn, H, Tq, D,
+                                             native._stream())
+            native._check(rc, "dl4j_attn_dvec")
+            return (*_flash_backward(q, k, v, dO, lse, dvec, mk, ctx.scale, ctx.flags, ctx.dropout_p, seed), None, None, None, None)
         q, k, v, P = ctx.saved_tensors
         Bn, H, Tq, D = q.shape
         Tk = k.shape[2]
@@ -134,31 +144,62 @@ class _AttentionFn(torch.autograd.Function):
         cbs, ldc = obs(dk_t)
         _bgemm(l, dP.data_ptr(), q.data_ptr(), dk_t.data_ptr(), Tk, D, Tq, Tk, q.stride(2), ldc, 1, 1, 1.0, H, Bn,
                pbs, (q.stride(1), q.stride(0)), cbs, dt)
-        return dq_t.permute(0, 2, 1, 3), dk_t.permute(0, 2, 1, 3), dv_t.permute(0, 2, 1, 3), None, None, None
+        return dq_t.permute(0, 2, 1, 3), dk_t.permute(0, 2, 1, 3), dv_t.permute(0, 2, 1, 3), None, None, None, None
 
 
-def attention(q, k, v, mask, scale, dropout_p=0.0):
+def _bad_mask(q, k, mask):
+    return mask is not None and (mask.dim() != 2 or mask.shape[0] != q.shape[0] or mask.shape[1] != k.shape[2])
+
+
+def _empty_rows_are_zero(D, Tq, Tk):
+    """What a query whose keys are all masked gets.  The lengths that have always run on these kernels give 0; on the others, which
+    the softmax over -inf served before, and with a causal mask it is NaN, and stays so."""
+    return Tk % 128 == 0 or (D % 8 == 0 and Tk % 8 == 0 and Tq % 8 == 0 and Tk <= 1024)
+
+
+def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
     """q, k, v: [B, H, T, D]; ``mask``: None or a [B, Tk] key mask (non-zero = attend); ``dropout_p``: probability of dropping an
-    attention weight (training).  Returns None when the case is not covered by the native kernels.
+    attention weight (training); ``causal``: query i sees the keys 0 .. i.  Returns None when the case is not covered by the native
+    kernels.
 
-    Head sizes below 64 run on the fused head-size-64 kernels with zero-padded heads (Q K^T is unchanged by zero columns, the
-    padded columns of V give output columns that are sliced away), so no score matrix is materialised for them either."""
+    bf16 with head sizes up to 64 runs on the fused kernels for any number of queries and keys (the copy engine zero-fills narrower
+    heads and the last key block); other head sizes and fp16 on batched GEMMs with a materialised score matrix."""
     if not native.available() or q.dim() != 4 or q.dtype not in (torch.bfloat16, torch.float16):
         return None
-    if mask is not None and (mask.dim() != 2 or mask.shape[0] != q.shape[0] or mask.shape[1] != k.shape[2]):
+    if _bad_mask(q, k, mask):
         return None
     D, Tk, Tq = q.shape[3], k.shape[2], q.shape[2]
     scale = float(scale) if scale is not None else D ** -0.5
-    if D < 64 and D % 8 == 0 and q.dtype == torch.bfloat16 and Tk % 128 == 0 and Tk == v.shape[2] and q.shape[:2] == k.shape[:2]:
-        pad = (0, 64 - D)
-        qp, kp, vp = (torch.nn.functional.pad(t, pad) for t in (q, k, v))
-        return _AttentionFn.apply(qp, kp, vp, mask, scale, float(dropout_p))[..., :D]
     fused = flash_supported(q, k, v)
-    if dropout_p > 0.0 and not fused:
+    if dropout_p > 0.0 and (not fused or Tk % 128 or causal):
         return None
-    if D % 8 or Tk % 8 or Tq % 8 or (Tk > 1024 and not fused):
+    if fused and (USE_FLASH or dropout_p > 0.0):
+        flags = (1 if causal else 0) | (0 if _empty_rows_are_zero(D, Tq, Tk) and not causal else 2)
+        return _AttentionFn.apply(q, k, v, mask, scale, float(dropout_p), flags)
+    if causal or D % 8 or Tk % 8 or Tq % 8 or Tk > 1024:
         return None
     return _AttentionFn.apply(q, k, v, mask, scale, float(dropout_p))
+
+
+def attention_grad(q, k, v, mask, scale, dout, causal=False):
+    """(dq, dk, dv) without materialising the output: the forward kernel hands the row sums of dO * O straight to the backward kernel.
+    None when the fused kernels do not cover the case."""
+    if not USE_FLASH or not native.available() or not flash_supported(q, k, v) or _bad_mask(q, k, mask) or dout.dim() != 4 \
+            or dout.device != q.device or dout.shape != (*q.shape[:3], v.shape[3]):
+        return None
+    q, k, v, dout = _prep(q.detach()), _prep(k.detach()), _prep(v.detach()), _prep(dout.detach().to(q.dtype))
+    Bn, H, Tq, D = q.shape
+    scale = float(scale) if scale is not None else D ** -0.5
+    flags = (1 if causal else 0) | (0 if _empty_rows_are_zero(D, Tq, k.shape[2]) and not causal else 2)
+    mk = mask.detach().to(torch.float32).contiguous() if mask is not None else None
+    stats = torch.empty((2, Bn, H, Tq), dtype=torch.float32, device=q.device)
+    lse, dvec = stats[0], stats[1]
+    rc = _flash_lib().dl4j_flash_attn_fwd(native._ptr(q), native._ptr(k), native._ptr(v), None, native._ptr(lse), native._ptr(mk), Bn, H, Tq,
+                                          k.shape[2], D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), scale,
+                                          flags, native._ptr(dout), _LONG3(*dout.stride()[:3]), native._ptr(dvec), 0.0, None,
+                                          native._stream())
+    native._check(rc, "dl4j_flash_attn_fwd")
+    return _flash_backward(q, k, v, dout, lse, dvec, mk, scale, flags, 0.0, None)
 
 
 # Dropout seeds live on the device: every fused forward call with dropout takes a private copy of the running seed and
@@ -184,40 +225,32 @@ def _next_dropout_seed(device):
 
 
 _LONG3 = ctypes.c_long * 3
-_DQ_ACC = {}
 USE_FLASH = True      # False: batched GEMMs + separate softmax kernels with a materialised score matrix (cross-check path)
 
 
-def _flash_backward(ctx, dO):
+def _flash_lib():
     l = native.require()
     if not hasattr(l.dl4j_flash_attn_bwd, "_typed"):
-        vp, i32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+        vp, i32, f32, lng = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_long
         lp = ctypes.POINTER(ctypes.c_long)
-        l.dl4j_flash_attn_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, lp, lp, lp, lp, ctypes.c_long, ctypes.c_long, f32,
-                                          f32, vp, vp]
+        l.dl4j_flash_attn_fwd.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, lp, lp, lp, f32, i32, vp, lp, vp, f32, vp, vp]
+        l.dl4j_flash_attn_fwd.restype = ctypes.c_int
+        l.dl4j_flash_attn_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, lp, lp, lp, lp, lng, lng, lng,
+                                          lng, f32, i32, f32, vp, vp]
         l.dl4j_flash_attn_bwd.restype = ctypes.c_int
-        l.dl4j_attn_dvec.argtypes = [vp, lp, vp, vp, i32, i32, i32, vp]
+        l.dl4j_attn_dvec.argtypes = [vp, lp, vp, vp, i32, i32, i32, i32, vp]
         l.dl4j_attn_dvec.restype = ctypes.c_int
-        l.dl4j_attn_dq_finish.argtypes = [vp, vp, ctypes.c_long, ctypes.c_long, i32, i32, i32, vp]
+        l.dl4j_attn_dq_finish.argtypes = [vp, vp, lng, lng, i32, i32, i32, i32, vp]
         l.dl4j_attn_dq_finish.restype = ctypes.c_int
         l.dl4j_flash_attn_bwd._typed = True
-    q, k, v, O, lse, mk, seed = ctx.saved_tensors
+    return l
+
+
+def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
+    l = _flash_lib()
     Bn, H, Tq, D = q.shape
     Tk = k.shape[2]
-    dO = _prep(dO)                                           # [B, H, Tq, D] view
-    def st(t):
-        return _LONG3(t.stride(0), t.stride(1), t.stride(2))
-    # D_r = sum_d dO * O per query row, laid out like the log-sum-exp
-    dvec = torch.empty((Bn, H, Tq), dtype=torch.float32, device=q.device)
-    rc = l.dl4j_attn_dvec(native._ptr(dO), st(dO), native._ptr(O), native._ptr(dvec), Bn, H, Tq, native._stream())
-    native._check(rc, "dl4j_attn_dvec")
-    # fp32 dQ accumulator: allocated zeroed once per shape, the finishing kernel clears it again after reading it
-    key = (q.device, Bn, H, Tq)
-    dq_acc = _DQ_ACC.get(key)
-    if dq_acc is None:
-        dq_acc = _DQ_ACC[key] = torch.zeros((Bn, H, Tq, D), dtype=torch.float32, device=q.device)
-    same_len = Tq == Tk
-    if same_len:
+    if Tq == Tk:
         # one packed [B, T, 3, H, D] gradient buffer, so the gradient of the fused q/k/v projection is a plain view
         dqkv = torch.empty((Bn, Tq, 3, H, D), dtype=q.dtype, device=q.device)
         dq_t, dk_t, dv_t = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
@@ -225,41 +258,38 @@ def _flash_backward(ctx, dO):
         dq_t = torch.empty((Bn, Tq, H, D), dtype=q.dtype, device=q.device)
         dk_t = torch.empty((Bn, Tk, H, D), dtype=q.dtype, device=q.device)
         dv_t = torch.empty((Bn, Tk, H, D), dtype=q.dtype, device=q.device)
-
+    # more than one key block adds into a query's gradient: an fp32 accumulator, its own for every call (streams and threads may
+    # run the same shape at the same time)
+    acc = torch.zeros((Bn, H, Tq, D), dtype=torch.float32, device=q.device) if Tk > 128 else None
+    stream = native._stream()
     rc = l.dl4j_flash_attn_bwd(native._ptr(q), native._ptr(k), native._ptr(v), native._ptr(dO), native._ptr(lse), native._ptr(dvec),
-                               native._ptr(mk), native._ptr(dq_acc), native._ptr(dk_t), native._ptr(dv_t), Bn, H, Tq, Tk,
-                               st(q), st(k), st(v), st(dO), dk_t.stride(0), dk_t.stride(1), float(ctx.scale), float(ctx.dropout_p),
-                               native._ptr(seed), native._stream())
+                               native._ptr(mk), native._ptr(acc), native._ptr(dq_t), native._ptr(dk_t), native._ptr(dv_t), Bn, H, Tq, Tk, D,
+                               _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), _LONG3(*dO.stride()[:3]),
+                               dq_t.stride(0), dq_t.stride(1), dk_t.stride(0), dk_t.stride(1), scale, flags, dropout_p, native._ptr(seed),
+                               stream)
     native._check(rc, "dl4j_flash_attn_bwd")
-    rc = l.dl4j_attn_dq_finish(native._ptr(dq_acc), native._ptr(dq_t), dq_t.stride(0), dq_t.stride(1), Bn, H, Tq, native._stream())
-    native._check(rc, "dl4j_attn_dq_finish")
-    return dq_t.permute(0, 2, 1, 3), dk_t.permute(0, 2, 1, 3), dv_t.permute(0, 2, 1, 3), None, None, None
+    if acc is not None:
+        rc = l.dl4j_attn_dq_finish(native._ptr(acc), native._ptr(dq_t), dq_t.stride(0), dq_t.stride(1), Bn, H, Tq, D, stream)
+        native._check(rc, "dl4j_attn_dq_finish")
+    return dq_t.permute(0, 2, 1, 3), dk_t.permute(0, 2, 1, 3), dv_t.permute(0, 2, 1, 3)
 
 
 def flash_supported(q, k, v):
-    return (native.available() and q.dtype == torch.bfloat16 and q.dim() == 4 and q.shape[3] == 64 and k.shape[2] >= 128
-            and k.shape[2] % 128 == 0 and k.shape[2] == v.shape[2] and q.shape[:2] == k.shape[:2] and v.shape[3] == 64)
+    return (native.available() and q.is_cuda and q.dim() == 4 and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.shape[3] <= 64
+            and q.shape[3] % 8 == 0 and k.shape == v.shape and q.shape[3] == k.shape[3] and q.shape[:2] == k.shape[:2]
+            and q.numel() > 0 and k.numel() > 0)
 
 
-def flash_forward(q, k, v, key_mask, scale, dropout_p=0.0, seed=None):
-    """Fused attention forward: returns (out [B, Tq, H, 64] bf16, lse [B, H, Tq] fp32).  q, k, v: [B, H, T, 64] views."""
-    l = native.require()
-    if not hasattr(l.dl4j_flash_attn_fwd, "_typed"):
-        vp, i32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
-        lp = ctypes.POINTER(ctypes.c_long)
-        l.dl4j_flash_attn_fwd.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, lp, lp, lp, f32, f32, vp, vp]
-        l.dl4j_flash_attn_fwd.restype = ctypes.c_int
-        l.dl4j_flash_attn_fwd._typed = True
+def flash_forward(q, k, v, key_mask, scale, dropout_p=0.0, seed=None, flags=0):
+    """Fused attention forward: returns (out [B, Tq, H, D] bf16, lse [B, H, Tq] fp32).  q, k, v: [B, H, T, D] views."""
+    l = _flash_lib()
     q, k, v = _prep(q), _prep(k), _prep(v)
     Bn, H, Tq, D = q.shape
-    Tk = k.shape[2]
     out = torch.empty((Bn, Tq, H, D), dtype=q.dtype, device=q.device)
     lse = torch.empty((Bn, H, Tq), dtype=torch.float32, device=q.device)
     mk = key_mask.to(torch.float32).contiguous() if key_mask is not None else None
-
-    def st(t):
-        return _LONG3(t.stride(0), t.stride(1), t.stride(2))
-    rc = l.dl4j_flash_attn_fwd(native._ptr(q), native._ptr(k), native._ptr(v), native._ptr(out), native._ptr(lse), native._ptr(mk),
-                               Bn, H, Tq, Tk, st(q), st(k), st(v), float(scale), float(dropout_p), native._ptr(seed), native._stream())
+    rc = l.dl4j_flash_attn_fwd(native._ptr(q), native._ptr(k), native._ptr(v), native._ptr(out), native._ptr(lse), native._ptr(mk), Bn, H, Tq,
+                               k.shape[2], D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), float(scale), flags,
+                               None, None, None, float(dropout_p), native._ptr(seed), native._stream())
     native._check(rc, "dl4j_flash_attn_fwd")
     return out, lse

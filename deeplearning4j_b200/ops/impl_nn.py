@@ -311,6 +311,11 @@ def dot_product_attention_v2(q, v, k=None, attentionBias=None, qMask=None, vMask
     qq, kk, vv = (t if four else t.unsqueeze(1) for t in (q, k, v))
     sc = float(scale) if scale else 1.0
     mask = vMask
+    if useCausalMask and attentionBias is None and qMask is None and not (dropoutProbability and training):
+        nat = nnops._native_for(qq)
+        o = nat.attention(qq, kk, vv, mask, sc, causal=True) if nat is not None else None
+        if o is not None:
+            return (o if four else o.squeeze(1),)
     if useCausalMask or attentionBias is not None or qMask is not None:
         s = torch.matmul(qq, kk.transpose(-1, -2)) * sc
         if attentionBias is not None:
@@ -358,7 +363,28 @@ def multi_head_dot_product_attention(q, k, v, Wq, Wk, Wv, Wo, mask=None, scaled=
 
 
 op("dot_product_attention_bp", n_out=3)(_autobp(lambda q, k, v, **kw: dot_product_attention(q, k, v, **kw)[0], 3))
-op("dot_product_attention_v2_bp", n_out=3)(_autobp(lambda q, v, k, **kw: dot_product_attention_v2(q, v, k, **kw)[0], 3))
+_attention_v2_autobp = _autobp(lambda q, v, k, **kw: dot_product_attention_v2(q, v, k, **kw)[0], 3)
+
+
+@op("dot_product_attention_v2_bp", n_out=3)
+def dot_product_attention_v2_bp(*args, **kw):
+    """(q, v, k, dout) -> dq, dv, dk.  Where the fused kernels cover the call they compute the gradients directly, without the output
+    tensor and the autograd graph; everything else differentiates the forward."""
+    if len(args) == 4 and all(isinstance(a, torch.Tensor) for a in args) and kw.get("attentionBias") is None and kw.get("qMask") is None \
+            and not (kw.get("dropoutProbability") and kw.get("training")):
+        q, v, k, g = args
+        four = q.dim() == 4
+        nat = nnops._native_for(q)
+        if nat is not None and q.dim() in (3, 4) and k.dim() == v.dim() == q.dim():
+            qq, kk, vv = (t if four else t.unsqueeze(1) for t in (q, k, v))
+            shape = (*qq.shape[:3], vv.shape[3])
+            if g.numel() == math.prod(shape):
+                r = nat.attention_grad(qq, kk, vv, kw.get("vMask"), float(kw.get("scale", 1.0) or 1.0), g.reshape(shape),
+                                       bool(kw.get("useCausalMask", False)))
+                if r is not None:
+                    dq, dk, dv = r if four else (t.squeeze(1) for t in r)
+                    return dq, dv, dk
+    return _attention_v2_autobp(*args, **kw)
 op("multi_head_dot_product_attention_bp", n_out=7)(
     _autobp(lambda q, k, v, a, b, c, d, **kw: multi_head_dot_product_attention(q, k, v, a, b, c, d, **kw)[0], 7))
 

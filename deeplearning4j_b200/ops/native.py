@@ -1393,9 +1393,14 @@ def add_relu(a, b):
     return _AddReluFn.apply(a, b)
 
 
-def attention(q, k, v, mask, scale, dropout_p=0.0):
+def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
     from . import attention_native
-    return attention_native.attention(q, k, v, mask, scale, dropout_p)
+    return attention_native.attention(q, k, v, mask, scale, dropout_p, causal)
+
+
+def attention_grad(q, k, v, mask, scale, dout, causal=False):
+    from . import attention_native
+    return attention_native.attention_grad(q, k, v, mask, scale, dout, causal)
 
 
 # =========================================================================== fused updater

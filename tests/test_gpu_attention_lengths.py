@@ -1,0 +1,87 @@
+"""Fused attention at lengths and head sizes off the tile grid, causal and masked, against fp64; routes against the general path."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B, H, Tq, Tk, D, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    t = lambda T: torch.randn(B, T, H, D, generator=g, device="cuda").bfloat16().permute(0, 2, 1, 3)
+    return t(Tq), t(Tk), t(Tk), t(Tq), g
+
+
+def _ref(q, k, v, scale, mask, causal):
+    s = q @ k.transpose(-1, -2) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).triu(1), float("-inf"))
+    if mask is not None:
+        s = s.masked_fill(mask[:, None, None, :] == 0, float("-inf"))
+    return torch.softmax(s, -1) @ v
+
+
+@pytest.mark.parametrize("Tq,Tk", [(1, 1), (7, 5), (16, 127), (128, 128), (129, 129), (200, 200), (256, 255), (257, 384), (500, 130), (1000, 1000)])
+@pytest.mark.parametrize("D", [8, 32, 40, 64])
+@pytest.mark.parametrize("masked,causal", [(False, False), (True, False), (False, True), (True, True)])
+def test_forward_and_gradients(Tq, Tk, D, masked, causal):
+    """bf16 rounds P, dS and the results once each (2^-9 relative): 1e-2 of the norm leaves a factor of two."""
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    from deeplearning4j_b200.ops import native
+    B, H = 2, 3
+    q, k, v, do, g = _inputs(B, H, Tq, Tk, D, Tq * 1000 + Tk + D)
+    mask = None
+    if masked:
+        mask = (torch.rand(B, Tk, generator=g, device="cuda") > 0.3).float()
+        mask[:, 0] = 1.0
+    scale = D ** -0.5
+    q64, k64, v64 = (t.double().requires_grad_(True) for t in (q, k, v))
+    want = _ref(q64, k64, v64, scale, mask, causal)
+    dq, dk, dv = torch.autograd.grad(want, (q64, k64, v64), do.double())
+    got = Nd4j.exec("dot_product_attention_v2", q, v, k, None, None, mask, scale=scale, useCausalMask=causal).t
+    gq, gv, gk = (a.t for a in Nd4j.exec("dot_product_attention_v2_bp", q, v, k, do, vMask=mask, scale=scale, useCausalMask=causal))
+    # ... and through autograd
+    ql, kl, vl = (t.detach().requires_grad_(True) for t in (q, k, v))
+    from deeplearning4j_b200.ops import attention_native as an
+    aq, ak, av = torch.autograd.grad(an.attention(ql, kl, vl, mask, scale, causal=causal), (ql, kl, vl), do)
+    torch.cuda.synchronize()
+    native.check_status()
+    assert (got.double() - want).norm() <= 1e-2 * want.norm()
+    # with one visible key P is exactly 1 and dq, dk vanish: compare against the size of the terms that cancel
+    size = do.double().norm() * scale
+    for a, b in ((gq, dq), (gk, dk), (aq, dq), (ak, dk)):
+        assert (a.double() - b).norm() <= 1e-2 * (b.norm() + size)
+    for a, b in ((gv, dv), (av, dv)):
+        assert (a.double() - b).norm() <= 1e-2 * b.norm()
+
+
+@pytest.mark.parametrize("T,causal,zero", [(256, False, True), (200, False, True), (201, False, False), (130, True, False)])
+def test_rows_without_keys(T, causal, zero):
+    """Zero where the native kernels always served the length, NaN where the softmax over -inf did."""
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    q, k, v, do, _ = _inputs(2, 2, T, T, 64, T)
+    mask = torch.ones(2, T, device="cuda")
+    if causal:
+        mask[1, :3] = 0                                     # the first three queries of example 1 see nothing
+    else:
+        mask[1] = 0
+    out = Nd4j.exec("dot_product_attention_v2", q, v, k, None, None, mask, scale=0.125, useCausalMask=causal).t
+    dq, dv, dk = (a.t for a in Nd4j.exec("dot_product_attention_v2_bp", q, v, k, do, vMask=mask, scale=0.125, useCausalMask=causal))
+    bad = out[1, :, :3] if causal else out[1]
+    assert torch.isfinite(out[0]).all() and torch.isfinite(dv[0]).all()
+    if zero:
+        assert (bad == 0).all() and (dv[1] == 0).all()
+    else:
+        assert torch.isnan(bad).all() and torch.isnan(dv[1]).all()
+    assert (dq[1, :, :3] == 0).all() and torch.isfinite(dk).all()
+
+
+def test_three_dimensional_and_misaligned_inputs():
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    base = torch.randn(3 * 50 * 24 + 3, device="cuda").bfloat16()
+    q = base[3:].view(3, 50, 24)                            # off the 16-byte grid
+    k, v = torch.randn(3, 33, 24, device="cuda").bfloat16(), torch.randn(3, 33, 24, device="cuda").bfloat16()
+    out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=0.2).t
+    want = _ref(q.double()[:, None], k.double()[:, None], v.double()[:, None], 0.2, None, False)[:, 0]
+    assert out.shape == (3, 50, 24) and (out.double() - want).norm() <= 1e-2 * want.norm()
+    dq, dv, dk = Nd4j.exec("dot_product_attention_v2_bp", q, v, k, torch.ones_like(q), scale=0.2)
+    assert dq.t.shape == q.shape and dk.t.shape == k.shape and dv.t.shape == v.shape
