@@ -103,10 +103,17 @@ class LSTM(BaseRecurrentLayer):
             c = torch.zeros(mb, n, dtype=torch.float32 if x.dtype in (torch.bfloat16, torch.float16) else x.dtype, device=x.device)
         W, RW, b = p["W"], p["RW"], p["b"]
         RW4 = RW[:, :4 * n]
-        # one GEMM for all time steps' input contributions
-        zx = nnops.linear(xt.reshape(T * mb, -1), W, b).reshape(T, mb, 4 * n)
         gate, act = self.gateActivationFn, self.activation
         plain = isinstance(gate, ActivationSigmoid) and isinstance(act, ActivationTanH) and not self.PEEPHOLE
+        if T == 1 and plain and mask is None and not training and x.is_cuda and not nnops._FORCE_TORCH:
+            from ...ops import native as nat
+            if nat.lstm_step_supported(xt, W, RW, n, mb) and h.dtype == x.dtype and c.dtype == torch.float32 \
+                    and (b is None or b.dtype == torch.float32) and h.shape == c.shape == (mb, n):
+                h, c = nat.lstm_step(xt[0], W, RW, None if b is None else b.detach().reshape(-1), h, c)
+                self._store(ctx, key, (h, c))
+                return self._from_tmn(h.unsqueeze(0))
+        # one GEMM for all time steps' input contributions
+        zx = nnops.linear(xt.reshape(T * mb, -1), W, b).reshape(T, mb, 4 * n)
         if plain and mask is None and c.dtype == torch.float32 and not nnops._FORCE_TORCH:
             from ...ops import native as nat
             if nat.lstm_seq_supported(zx, n, mb) and h.dtype == zx.dtype:

@@ -45,6 +45,9 @@ def linear(x, W, b=None, activation=None, training=False):
         y = nat.linear(x, W, b, activation)
         if y is not None:
             return y
+        y = nat.linear_small(x, W, b)
+        if y is not None:
+            return activation(y, training) if activation is not None else y
     if W.dtype != x.dtype:
         W = W.to(x.dtype)
     if b is not None and x.dim() == 2 and b.dtype == x.dtype and b.numel() == W.shape[1]:
