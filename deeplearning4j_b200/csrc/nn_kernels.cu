@@ -515,17 +515,43 @@ softmax_xent_fwd_kernel(const T* __restrict__ logits, const T* __restrict__ dens
     sl += l; slz += l * v;
   };
   if (VEC) {
+    // Four 16-byte loads per thread are issued before any is used: with one at a time the loop waited out a memory latency per 2048
+    // columns (2456 x 30528 bf16: 57 us -> 41 us; reading the logits once takes 23).
+    constexpr int U = 4;
     const int C8 = C & ~7;
-    for (int j = threadIdx.x * 8; j < C8; j += SX_THREADS * 8) {
-      float v[8], l[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      Vec8<T>::load(z + j, v);
-      if (lab) Vec8<T>::load(lab + j, l);
-      float m8 = v[0];
+    for (int j0 = threadIdx.x * 8; j0 < C8; j0 += U * SX_THREADS * 8) {
+      Raw8<T> q[U];
+      float m8 = -INFINITY;
 #pragma unroll
-      for (int i = 1; i < 8; ++i) m8 = fmaxf(m8, v[i]);
+      for (int u = 0; u < U; ++u)
+        if (j0 + u * SX_THREADS * 8 < C8) q[u] = ld_raw8_keep(z + j0 + u * SX_THREADS * 8);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (j0 + u * SX_THREADS * 8 < C8) {
+          float v[8];
+          unpack8(q[u], v);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) m8 = fmaxf(m8, v[i]);
+        }
+      }
       if (m8 > mx) { se *= __expf(mx - m8); mx = m8; }
+      const float mref = mx == -INFINITY ? 0.f : mx;          // all -inf so far: every term below is exp(-inf) = 0
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { se += mx == -INFINITY ? 0.f : __expf(v[i] - mx); sl += l[i]; slz += l[i] * v[i]; }
+      for (int u = 0; u < U; ++u) {
+        const int j = j0 + u * SX_THREADS * 8;
+        if (j < C8) {
+          float v[8];
+          unpack8(q[u], v);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) se += __expf(v[i] - mref);
+          if (lab) {
+            float l[8];
+            Vec8<T>::load(lab + j, l);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { sl += l[i]; slz += l[i] * v[i]; }
+          }
+        }
+      }
     }
     for (int j = C8 + threadIdx.x; j < C; j += SX_THREADS) take(ldf(z + j), lab ? ldf(lab + j) : 0.f);
   } else {

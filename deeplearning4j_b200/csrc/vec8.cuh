@@ -55,6 +55,13 @@ template <typename T> __device__ __forceinline__ Raw8<T> ld_raw8(const T* p) {
   for (int i = 0; i < (int)(sizeof(T) / 2); ++i) r.q[i] = __ldcs(reinterpret_cast<const uint4*>(p) + i);
   return r;
 }
+// the same without the streaming hint: data that a later kernel reads again
+template <typename T> __device__ __forceinline__ Raw8<T> ld_raw8_keep(const T* p) {
+  Raw8<T> r;
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(T) / 2); ++i) r.q[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+  return r;
+}
 template <typename T> __device__ __forceinline__ void unpack8(const Raw8<T>& r, float (&v)[8]) {
   Vec8<T>::load(reinterpret_cast<const T*>(&r), v);
 }

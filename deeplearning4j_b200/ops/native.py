@@ -292,6 +292,36 @@ def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtyp
     return out
 
 
+def _long_k_splits(M, N, K):
+    """Split-K factor for a 16-bit-output GEMM with few output tiles and a long reduction (the data gradient of a vocabulary
+    projection: 2456 x 768 from K = 30522 is 60 tiles of 128 x 256 on 148 SMs).  The estimate: waves x k-blocks x 0.31 us (four MMAs
+    at one issue per ~147 clocks), against the passes a split adds over the fp32 partial result (zeroing, reductions, the cast).
+    2456 x 768 x 30522: 140 - 156 us unsplit (120 tiles of 128 x 128), 110 us split by 7, zeroing and cast included."""
+    sms, kb = num_sms(), (K + 63) // 64
+    tiles = ((M + 127) // 128) * ((N + 255) // 256)
+    if tiles >= sms or kb < 32:
+        return 1
+    best, cost1 = 1, min((tiles + sms - 1) // sms, (((M + 127) // 128) * ((N + 127) // 128) + sms - 1) // sms) * kb * 0.31
+    best_cost = cost1
+    for s in range(2, 17):
+        if kb // s < 8:
+            break
+        c = ((tiles * s + sms - 1) // sms) * ((kb + s - 1) // s) * 0.31 + M * N * (10 + 4 * s) / 5e6 + 6.0
+        if c < best_cost:
+            best, best_cost = s, c
+    return best
+
+
+def _dgrad_gemm(a, b, out=None):
+    """``a @ b`` in a's type; a long reduction over few output tiles is split and summed in fp32 before the one rounding."""
+    M, N = a.shape[0], b.shape[1]
+    s = _long_k_splits(M, N, a.shape[1])
+    if s == 1 or N % 4:
+        return gemm_raw(a, b, out=out)
+    acc = gemm_raw(a, b, out_dtype=torch.float32, atomic=True, splits=s, block_n=256)
+    return acc.to(a.dtype) if out is None else out.copy_(acc)
+
+
 class _MatmulFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, a, b):
@@ -525,7 +555,7 @@ class _LinearFn(torch.autograd.Function):
         # ---- data gradient: dx = dz @ W^T
         dx = None
         if ctx.needs_input_grad[0]:
-            dx = gemm_raw(dz, W_lp.t())
+            dx = _dgrad_gemm(dz, W_lp.t())
         # ---- weight gradient: dW^T [nOut, nIn] = dz^T @ x
         dW = None
         if ctx.needs_input_grad[1]:
@@ -565,6 +595,8 @@ def linear(x, W, b, activation):
         return None
     if not x.is_contiguous():
         x = x.contiguous()
+    # fewer rows stay with the library: forward + backward of 128 x 512 x 10001 takes 60 us of device time here against 107 there, but
+    # its two autograd products cost the caller 118 us where this function costs 296
     if ((W.shape[1] % 8) or (x.shape[1] % 8)) and _PAD_ODD_WIDTHS and x.shape[0] >= 256:
         return _linear_padded(x, W, b, act)
     if _operand_a(x) is None or _operand_b(W_lp) is None or _operand_b(W_lp.t()) is None:
@@ -575,21 +607,105 @@ def linear(x, W, b, activation):
     return _LinearFn.apply(x, W, b, act, W_lp)
 
 
+def pitch_copy(src, dst):
+    """dst <- src (2-D, unit column stride, any row pitch; fp32 -> 16-bit converts)."""
+    l = require()
+    if not hasattr(l.dl4j_pitch_copy, "_typed"):
+        vp, i32, lng = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
+        l.dl4j_pitch_copy.argtypes = [vp, i32, vp, i32, lng, i32, lng, lng, vp]
+        l.dl4j_pitch_copy.restype = i32
+        l.dl4j_pitch_copy._typed = True
+    rc = l.dl4j_pitch_copy(_ptr(src), _DT[src.dtype], _ptr(dst), _DT[dst.dtype], src.shape[0], src.shape[1], src.stride(0), dst.stride(0), _stream())
+    _check(rc, "dl4j_pitch_copy")
+    return dst
+
+
+def _pitched(rows, cols, dtype, device):
+    """Uninitialised [rows, cols] matrix whose rows start on 16-byte boundaries (and whose padding belongs to its storage)."""
+    return torch.empty((rows, (cols + 7) // 8 * 8), dtype=dtype, device=device)[:, :cols]
+
+
+def _on_pitch(t, dtype):
+    """``t`` in ``dtype`` with unit column stride and rows on 16-byte boundaries, padding included in the storage; copied if need be."""
+    P = (t.shape[1] + 7) // 8 * 8
+    if t.dtype == dtype and t.stride(1) == 1 and t.stride(0) == P and t.data_ptr() % 16 == 0 \
+            and (t.storage_offset() + t.shape[0] * P) * t.element_size() <= t.untyped_storage().nbytes():
+        return t
+    if t.stride(1) != 1 or (t.dtype != dtype and t.dtype != torch.float32):
+        t = t.to(dtype).contiguous()
+    return pitch_copy(t, _pitched(t.shape[0], t.shape[1], dtype, t.device))
+
+
+def _full_rows(t):
+    """A pitched matrix with its padding columns (whatever they hold)."""
+    return t.as_strided((t.shape[0], t.stride(0)), (t.stride(0), 1))
+
+
+class _OddLinearFn(torch.autograd.Function):
+    """``act(x @ W + b)`` for layer widths off the 8-element grid (a 77-symbol alphabet, a 30522-word vocabulary, ten classes).  TMA asks
+    for 16-byte row pitches, not for widths: the weights are copied once to such a pitch, results and their gradients live on it as
+    strided views, and the tiles' edges are clipped by the tensor maps."""
+
+    @staticmethod
+    def forward(ctx, x, W, b, act):
+        dt = x.dtype
+        M, K = x.shape
+        N = W.shape[1]
+        xp = _on_pitch(x.detach(), dt)
+        Wd = W.detach()
+        rows = Wd.stride(1) == 1 or Wd.stride(0) != 1          # row-major [K, N]; else 'f' order, stored as [N, K]
+        Wp = _on_pitch(Wd, dt) if rows else _on_pitch(Wd.t(), dt).t()
+        y = _pitched(M, N, dt, x.device)
+        z = _pitched(M, N, dt, x.device) if act in (2, 3, 4, 5, 6) and any(ctx.needs_input_grad) else None
+        b_fwd = _fwd_bias(b, dt)[0]
+        if b_fwd is not None:
+            b_fwd = _dense16(b_fwd.detach())
+        gemm_raw(xp, Wp, out=y, bias=b_fwd, act=act, aux=z)
+        ctx.act, ctx.rows, ctx.w_dtype, ctx.b_like = act, rows, W.dtype, None if b is None else (b.shape, b.dtype)
+        ctx.save_for_backward(xp, Wp, z if z is not None else (y if act == 1 else None))
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        l = require()
+        xp, Wp, saved = ctx.saved_tensors
+        M, K = xp.shape
+        N = Wp.shape[1]
+        dt = xp.dtype
+        dz = _on_pitch(dy, dt)
+        P = dz.stride(0)
+        acc = torch.zeros(P, dtype=torch.float32, device=dy.device) if ctx.b_like is not None and ctx.needs_input_grad[2] else None
+        if ctx.act:
+            out = _pitched(M, N, dt, dy.device)
+            rc = l.dl4j_bias_act_bwd(_ptr(dz), _ptr(saved), _ptr(out), _ptr(acc), M, P, ctx.act, _DT[dt], _stream())
+            _check(rc, "dl4j_bias_act_bwd")
+            dz = out
+        elif acc is not None:
+            _check(l.dl4j_bias_act_bwd(_ptr(dz), None, None, _ptr(acc), M, P, 0, _DT[dt], _stream()), "dl4j_bias_act_bwd")
+        db = None if acc is None else acc[:N].reshape(ctx.b_like[0]).to(ctx.b_like[1])
+        dx = None
+        if ctx.needs_input_grad[0]:
+            dx = _dgrad_gemm(dz, Wp.t(), out=None if K % 8 == 0 else _pitched(M, K, dt, dy.device))
+        dW = None
+        if ctx.needs_input_grad[1]:
+            a, c = (xp.t(), dz) if ctx.rows else (dz.t(), xp)
+            R, C = a.shape[0], c.shape[1]
+            splits = _wgrad_splits(((R + 127) // 128) * ((C + 255) // 256), M)
+            wide = ctx.w_dtype == torch.float32 or splits > 1       # partial sums and fp32 gradients stay in fp32
+            buf = torch.zeros((R, (C + 7) // 8 * 8), dtype=torch.float32, device=dy.device)[:, :C] if wide else _pitched(R, C, dt, dy.device)
+            gemm_raw(a, c, out=buf, atomic=wide, splits=splits)
+            if not buf.is_contiguous() or buf.dtype != ctx.w_dtype:
+                same = ctx.w_dtype in (buf.dtype, torch.float16, torch.bfloat16) and (buf.dtype == torch.float32 or buf.dtype == ctx.w_dtype)
+                buf = pitch_copy(buf, torch.empty((R, C), dtype=ctx.w_dtype, device=dy.device)) if same else buf.to(ctx.w_dtype).contiguous()
+            dW = buf if ctx.rows else buf.t()
+        return dx, dW, db, None
+
+
 def _linear_padded(x, W, b, act):
-    """Layer widths that are not multiples of 8 (a 77-symbol alphabet, ten classes): the operands are zero-padded to the next
-    multiple with differentiable ops and the fused path runs on the padded problem; the padding columns produce zeros that the
-    final slice drops, and their gradients vanish in the slice's backward."""
-    import torch.nn.functional as F
-    K, N = x.shape[1], W.shape[1]
-    Kp, Np = (K + 7) // 8 * 8, (N + 7) // 8 * 8
-    xp = F.pad(x, (0, Kp - K)) if Kp != K else x
-    Wp = F.pad(W, (0, Np - N, 0, Kp - K))                    # [Kp, Np], row-major copy in the parameter's precision
-    bp = None if b is None else F.pad(b.reshape(-1), (0, Np - N))
-    Wp_lp = Wp.detach().to(x.dtype)
-    if _operand_a(xp) is None or _operand_b(Wp_lp) is None or _operand_b(Wp_lp.t()) is None:
+    """Layer widths that are not multiples of 8, see ``_OddLinearFn``; None when the case is not covered."""
+    if W.dim() != 2 or min(x.shape[0], W.shape[0], W.shape[1]) == 0 or W.dtype not in (x.dtype, torch.float32) or not W.is_cuda:
         return None
-    y = _LinearFn.apply(xp, Wp, bp, act, Wp_lp)
-    return y[:, :N] if Np != N else y
+    return _OddLinearFn.apply(x, W, b, act)
 
 
 _PAD_ODD_WIDTHS = os.environ.get("DL4J_PAD_ODD_WIDTHS", "1") != "0"
@@ -743,7 +859,9 @@ class _SoftmaxXentFn(torch.autograd.Function):
         l = require()
         logits, stats, lab_or_idx = ctx.saved_tensors
         rows, C = logits.shape
-        grad = torch.empty((rows, C), dtype=logits.dtype, device=logits.device)
+        # logits on a 16-byte row pitch (a layer of odd width) get a gradient on the same pitch: vector stores here, no copy there
+        pitched = C % 8 and logits.stride(0) == (C + 7) // 8 * 8
+        grad = _pitched(rows, C, logits.dtype, logits.device) if pitched else torch.empty((rows, C), dtype=logits.dtype, device=logits.device)
         d = dloss.reshape(-1).float().contiguous()
         idx, lab = (lab_or_idx, None) if ctx.sparse else (None, lab_or_idx)
         rc = l.dl4j_softmax_xent_bwd(_ptr(logits), _ptr(lab), _ptr(idx), _ptr(stats[0]), _ptr(stats[1]), _ptr(d), _ptr(grad), rows, C,
