@@ -711,6 +711,115 @@ def _linear_padded(x, W, b, act):
 _PAD_ODD_WIDTHS = os.environ.get("DL4J_PAD_ODD_WIDTHS", "1") != "0"
 
 
+# =========================================================================== small fp32 layers
+def _sgemm(a, b, out, bias=None, act=0):
+    """out [M, N] (unit column stride) = act(a @ b + bias) in fp32, for operands with a unit stride in one dimension."""
+    l = require()
+    if not hasattr(l.dl4j_sgemm_small, "_typed"):
+        vp, i32, lng = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
+        l.dl4j_sgemm_small.argtypes = [vp, lng, i32, vp, lng, i32, vp, vp, lng, i32, i32, i32, i32, i32, vp]
+        l.dl4j_sgemm_small.restype = i32
+        l.dl4j_sgemm_small._typed = True
+    a_kc, b_kc = a.stride(1) == 1, b.stride(0) == 1
+    rc = l.dl4j_sgemm_small(_ptr(a), a.stride(0) if a_kc else a.stride(1), int(a_kc), _ptr(b), b.stride(1) if b_kc else b.stride(0), int(b_kc),
+                            _ptr(bias), _ptr(out), out.stride(0), a.shape[0], b.shape[1], a.shape[1], act, num_sms(), _stream())
+    _check(rc, "dl4j_sgemm_small")
+    return out
+
+
+def _unit(t):
+    return t.dim() == 2 and 1 in t.stride()
+
+
+def _sgemm_wins(M, N, most=64):
+    """Whether a product leaves a library kernel short of tiles.  A layer's forward (bias and ReLU in the epilogue) wins up to 64 tiles of
+    64 x 64: 512 x 512 x 512 15.6 us against 17.3, at 128 tiles (512 x 1024 x 1024) 47 against 36.  The bare data gradient up to 16:
+    128 x 512 x 512 8.7 us against 10.7, at 64 tiles 15 against 12.  The weight gradient stays a library product that adds into its
+    target: 7 us against 8 - 12 here."""
+    return ((M + 63) // 64) * ((N + 63) // 64) <= most
+
+
+def _plain_autograd():
+    """No forward-mode level, functorch transform or tracer is active: the cases that differentiate or record through torch operators
+    and that a custom autograd function does not serve."""
+    return torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None \
+        and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+
+
+def _own_grad(p):
+    """The parameter's preallocated fp32 gradient when the kernels may add to it in autograd's place (nobody hooked the leaf)."""
+    g = p.grad if p.is_leaf else None
+    if g is None or g.dtype != torch.float32 or p._backward_hooks or getattr(p, "_post_accumulate_grad_hooks", None) \
+            or getattr(p, "_grad_ready", None) is not None:
+        return None
+    return g
+
+
+class _Linear32Fn(torch.autograd.Function):
+    """``act(x @ W + b)`` in fp32 for small layers: bias and ReLU in the product's epilogue, the bias gradient in the pass that applies
+    the activation's, the weight gradient added straight into the parameter's."""
+
+    @staticmethod
+    def forward(ctx, x, W, b, relu):
+        y = torch.empty((x.shape[0], W.shape[1]), dtype=torch.float32, device=x.device)
+        _sgemm(x, W, y, bias=None if b is None else b.detach().reshape(-1), act=1 if relu else 0)
+        ctx.relu, ctx.refs = relu, (W, b)
+        ctx.save_for_backward(x, W, b, y if relu else None)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, W, b, y = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        if torch.is_grad_enabled():                    # create_graph: the gradient has to be differentiable itself
+            dz = dy * (y > 0).to(dy.dtype) if ctx.relu else dy
+            return (dz @ W.t() if need[0] else None, x.t() @ dz if need[1] else None,
+                    dz.sum(0).reshape(b.shape) if b is not None and need[2] else None, None)
+        l = require()
+        dy = dy.contiguous()
+        M, N = dy.shape
+        Wl, bl = ctx.refs
+        db = acc = None
+        if b is not None and need[2]:
+            acc = _own_grad(bl)
+            if acc is None or not acc.is_contiguous():
+                acc = db = torch.zeros(N, dtype=torch.float32, device=dy.device)
+        dz = dy
+        if ctx.relu or acc is not None:
+            dz = torch.empty_like(dy) if ctx.relu else dy
+            rc = l.dl4j_bias_act_bwd(_ptr(dy), _ptr(y), _ptr(dz) if ctx.relu else None, _ptr(acc), M, N, 1 if ctx.relu else 0, 2, _stream())
+            _check(rc, "dl4j_bias_act_bwd")
+        dx = dW = None
+        if need[0]:
+            dx = _sgemm(dz, W.t(), torch.empty_like(x, memory_format=torch.contiguous_format)) if _sgemm_wins(M, x.shape[1], 16) else dz @ W.t()
+        if need[1]:
+            g = _own_grad(Wl)
+            if g is not None and _unit(g):
+                g.addmm_(x.t(), dz)
+            elif W.stride(0) == 1 and W.shape[0] > 1:           # 'f' order
+                dW = (dz.t() @ x).t()
+            else:
+                dW = x.t() @ dz
+        return dx, dW, None if db is None else db.reshape(b.shape), None
+
+
+def linear32(x, W, b, relu):
+    """fp32 dense layer on the small-problem kernel, or None when the case is not covered or the library does it better."""
+    if not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.float32 or W.dtype != torch.float32 or W.dim() != 2 \
+            or W.shape[0] != x.shape[1] or min(x.shape[0], *W.shape) == 0 or not _sgemm_wins(x.shape[0], W.shape[1]) \
+            or torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled() or not _unit(x) or not W.is_cuda:
+        return None
+    if not ((W.stride(0) == 1 and W.stride(1) >= W.shape[0]) or (W.stride(1) == 1 and W.stride(0) >= W.shape[1])):
+        return None
+    if b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1] or not b.is_contiguous() or not b.is_cuda):
+        return None
+    if not _plain_autograd():
+        return None
+    if x.stride(1) != 1:
+        x = x.contiguous()
+    return _Linear32Fn.apply(x, W, b, bool(relu))
+
+
 # =========================================================================== layer norm
 _LN_ONE_PASS = os.environ.get("DL4J_LN_BWD_ONEPASS", "0") == "1"
 
@@ -1597,7 +1706,7 @@ def attention_grad(q, k, v, mask, scale, dout, causal=False):
 # =========================================================================== fused updater
 _SEG_FMT = "<qqqqqfffiii"     # offset, block_start, block_numel, state_off, shadow_off, l1, l2, wd, kernel_id, hyper, pad
 _CHUNK_FMT = "<qii"
-_CHUNK = int(os.environ.get("DL4J_UPDATER_CHUNK", "16384"))     # elements per block of the multi-segment updater launch
+_CHUNK = int(os.environ.get("DL4J_UPDATER_CHUNK", "16384"))     # most elements per block of the multi-segment updater launch
 
 
 def _cfg_index(known, cfg):
@@ -1610,36 +1719,44 @@ def _cfg_index(known, cfg):
     return len(known) - 1
 
 
+def _chunk_size(numel):
+    """Elements per block of the updater launch: enough blocks for eight per SM, between one pass of a block's 256 threads (1024) and
+    the measured best of large networks.  0.67 M parameters in 16384-element chunks were 41 blocks on 148 SMs: 34 us, now 7.7.
+    The exchange kernels of a parallel group, which walk their chunks persistently, keep the large ones."""
+    return max(1024, min(_CHUNK, numel // (8 * num_sms()) // 1024 * 1024))
+
+
 def _build_tables(upd, shadow_offsets):
-    """Static part of the segment / chunk tables for a MultiLayerUpdater."""
+    """Static part of the segment / chunk tables for a MultiLayerUpdater; the chunk table for the exchange kernels and the one for the
+    single-process launch."""
     segs = upd.segments(0, 0)
     block_ids = []
-    seg_rows, chunks = [], []
+    seg_rows, chunks, small = [], [], []
     upd._seg_chunk0 = []                 # first chunk of every segment (bucketed gradient exchange addresses chunk ranges)
+    size = _chunk_size(sum(sg[1] for sg in segs))
     for si, (off, numel, st_off, bn, bs, kid, lr, l1, l2, wd, cfg) in enumerate(segs):
         upd._seg_chunk0.append(len(chunks))
         hid = _cfg_index(block_ids, cfg)
         seg_rows.append([off, bs, bn, st_off, shadow_offsets[si] if shadow_offsets is not None else 0, l1, l2, wd, kid, hid, 0])
-        o = 0
-        while o < numel:
-            c = min(_CHUNK, numel - o)
-            chunks.append(struct.pack(_CHUNK_FMT, off + o, c, si))
-            o += c
+        for table, step in ((chunks, _CHUNK), (small, size)):
+            for o in range(0, numel, step):
+                table.append(struct.pack(_CHUNK_FMT, off + o, min(step, numel - o), si))
     upd._seg_chunk0.append(len(chunks))
-    return seg_rows, b"".join(chunks), len(chunks), len(block_ids)
+    return seg_rows, b"".join(chunks), len(chunks), b"".join(small), len(small), len(block_ids)
 
 
 def update_tables(upd, iteration, epoch, shadow_offsets=None):
     """Device chunk/segment tables + this iteration's hyper-parameter table for ``upd``; None if unsupported."""
     cache = getattr(upd, "_native_tables", None)
     if cache is None or cache["shadow"] is not shadow_offsets:
-        seg_rows, chunk_bytes, n_chunks, n_hyper = _build_tables(upd, shadow_offsets)
+        seg_rows, chunk_bytes, n_chunks, small_bytes, n_small, n_hyper = _build_tables(upd, shadow_offsets)
         if n_hyper > 8:
             upd._native_tables = {"unsupported": True, "shadow": shadow_offsets}
             return None
         dev = upd.params.device
         chunks_t = torch.frombuffer(bytearray(chunk_bytes), dtype=torch.uint8).to(dev)
-        cache = {"seg_rows": seg_rows, "chunks": chunks_t, "n_chunks": n_chunks, "n_hyper": n_hyper, "shadow": shadow_offsets,
+        small_t = torch.frombuffer(bytearray(small_bytes), dtype=torch.uint8).to(dev)
+        cache = {"seg_rows": seg_rows, "chunks": chunks_t, "n_chunks": n_chunks, "small": small_t, "n_small": n_small, "n_hyper": n_hyper, "shadow": shadow_offsets,
                  "segs_dev": None, "segs_key": None}
         upd._native_tables = cache
     if cache.get("unsupported"):
@@ -1686,7 +1803,7 @@ def fused_update(upd, iteration, epoch, shadow=None, shadow_offsets=None, grad_s
     state = upd.state
     hp = hyper.ctypes.data_as(ctypes.c_void_p)
     rc = l.dl4j_fused_update(_ptr(upd.params), _ptr(upd.grads), _ptr(state) if state.numel() else None, _ptr(shadow),
-                             _ptr(residual), _ptr(cache["chunks"]), cache["n_chunks"], _ptr(cache["segs_dev"]), hp, cache["n_hyper"],
+                             _ptr(residual), _ptr(cache["small"]), cache["n_small"], _ptr(cache["segs_dev"]), hp, cache["n_hyper"],
                              float(grad_scale), 1 if zero_grads else 0, _stream())
     _check(rc, "dl4j_fused_update")
     upd._fused_zeroes_grads = bool(zero_grads)

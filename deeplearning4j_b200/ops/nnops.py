@@ -48,6 +48,11 @@ def linear(x, W, b=None, activation=None, training=False):
         y = nat.linear_small(x, W, b)
         if y is not None:
             return activation(y, training) if activation is not None else y
+    if nat is not None and x.dtype == torch.float32:
+        relu = activation is not None and nat._act_id(activation) == 1
+        y = nat.linear32(x, W, b, relu)
+        if y is not None:
+            return y if relu or activation is None else activation(y, training)
     if W.dtype != x.dtype:
         W = W.to(x.dtype)
     if b is not None and x.dim() == 2 and b.dtype == x.dtype and b.numel() == W.shape[1]:

@@ -1,0 +1,81 @@
+"""Small fp32 dense layers on the cluster-split product, against fp64, and the autograd forms they must not break."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(M, K, N, f_order, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(M, K, generator=g, device="cuda")
+    W = torch.randn(K, N, generator=g, device="cuda") / K ** 0.5
+    W = W.t().contiguous().t() if f_order else W
+    return x, W, torch.randn(N, generator=g, device="cuda"), torch.randn(M, N, generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (3, 5, 7), (64, 32, 64), (65, 33, 63), (128, 784, 512), (128, 512, 10), (17, 1000, 129),
+                                   (200, 300, 777), (1000, 64, 64), (2, 4096, 2)])
+@pytest.mark.parametrize("f_order", [False, True])
+@pytest.mark.parametrize("act", [None, "relu", "tanh"])
+def test_forward_and_gradients(M, K, N, f_order, act):
+    """fp32 sums of at most 4096 terms: a few units of 2^-24 times the square root of the count."""
+    from deeplearning4j_b200.nn.activations import ActivationReLU, ActivationTanH
+    from deeplearning4j_b200.ops import native, nnops
+    x, W, b, dy = _case(M, K, N, f_order, M + K + N)
+    leaves = [t.detach().requires_grad_(True) for t in (x, W, b)]
+    before = native.LAUNCHES
+    y = nnops.linear(*leaves, {None: None, "relu": ActivationReLU(), "tanh": ActivationTanH()}[act])
+    assert native.LAUNCHES > before
+    got = torch.autograd.grad(y, leaves, dy)
+    ref_leaves = [t.detach().double().requires_grad_(True) for t in (x, W, b)]
+    z = ref_leaves[0] @ ref_leaves[1] + ref_leaves[2]
+    ref = {None: lambda v: v, "relu": torch.relu, "tanh": torch.tanh}[act](z)
+    want = torch.autograd.grad(ref, ref_leaves, dy.double())
+    assert (y.double() - ref).norm() <= 2e-6 * (z.norm() + ref.norm())
+    size = dy.double().norm()
+    for u, v, p in zip(got, want, leaves):
+        assert u.shape == p.shape and (u.double() - v).norm() <= 3e-6 * (v.norm() + size)
+    # the parameter's own gradient is added to
+    for t in leaves:
+        t.grad = torch.ones_like(t)
+    nnops.linear(*leaves, ActivationReLU() if act == "relu" else None).backward(dy if act != "tanh" else torch.zeros_like(dy))
+    if act != "tanh":
+        for t, v in zip(leaves, want):
+            assert (t.grad.double() - 1 - v).norm() <= 3e-6 * (v.norm() + size + t.numel() ** 0.5)
+
+
+def test_hooks_create_graph_and_transforms():
+    from deeplearning4j_b200.nn.activations import ActivationReLU
+    from deeplearning4j_b200.ops import nnops
+    x, W, b, dy = _case(8, 12, 16, False, 3)
+    Wl = W.detach().requires_grad_(True)
+    Wl.grad = torch.zeros_like(W)
+    seen = []
+    Wl.register_hook(lambda g: seen.append(g.clone()))
+    nnops.linear(x, Wl, b, None).backward(dy)
+    assert len(seen) == 1 and torch.allclose(Wl.grad, x.t() @ dy, atol=1e-5)
+    # second derivatives
+    xl = x.detach().requires_grad_(True)
+    gx = torch.autograd.grad((nnops.linear(xl, W, b, ActivationReLU()) ** 2).sum(), xl, create_graph=True)[0]
+    ggx = torch.autograd.grad(gx.sum(), xl)[0]
+    x2 = x.detach().double().requires_grad_(True)
+    g2 = torch.autograd.grad((torch.relu(x2 @ W.double() + b.double()) ** 2).sum(), x2, create_graph=True)[0]
+    assert torch.allclose(ggx.double(), torch.autograd.grad(g2.sum(), x2)[0], rtol=1e-4, atol=1e-4)
+    # transforms and forward mode go through torch operators
+    v = torch.func.vmap(lambda r: nnops.linear(r[None], W, b, None)[0])(x)
+    assert torch.allclose(v, x @ W + b, atol=1e-5)
+    with torch.autograd.forward_ad.dual_level():
+        d = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+        t = torch.autograd.forward_ad.unpack_dual(nnops.linear(d, W, b, None)).tangent
+    assert torch.allclose(t, torch.ones_like(x) @ W, atol=1e-5)
+
+
+def test_nan_and_inf_pass():
+    from deeplearning4j_b200.nn.activations import ActivationReLU
+    from deeplearning4j_b200.ops import nnops
+    x, W, b, _ = _case(4, 8, 8, True, 1)
+    x[0, 0] = float("nan")
+    x[1, 0] = float("inf")
+    y = nnops.linear(x, W, b, ActivationReLU())
+    assert torch.isnan(y[0]).all() and not torch.isfinite(y[1]).any() == bool((W[0] > 0).all() and False) or torch.isinf(y[1]).any()
+    assert torch.equal(torch.isnan(y), torch.isnan(torch.relu(x @ W + b)))
