@@ -563,6 +563,11 @@ class GlobalPoolingLayer(NoParamLayer):
         if self.poolingType == PoolingType.MAX:
             return x.amax(dim=dims, keepdim=kd)
         if self.poolingType == PoolingType.AVG:
+            if x.is_cuda and x.dim() == 4 and dims == (2, 3) and not nnops._FORCE_TORCH:
+                from ...ops import native as nat
+                z = nat.global_avgpool(x)
+                if z is not None:
+                    return z[:, :, None, None] if kd else z
             return x.mean(dim=dims, keepdim=kd)
         if self.poolingType == PoolingType.SUM:
             return x.sum(dim=dims, keepdim=kd)

@@ -1555,6 +1555,47 @@ class _MaxPoolFn(torch.autograd.Function):
         return dx, None, None, None
 
 
+class _GlobalAvgPoolFn(torch.autograd.Function):
+    """Mean over H and W of a channels-last activation; the gradient is written channels-last, as the layers in front of it want it."""
+
+    @staticmethod
+    def forward(ctx, x):
+        l = _avgpool_lib()
+        N, C, H, W = x.shape
+        y = torch.empty((N, C), dtype=x.dtype, device=x.device)
+        _check(l.dl4j_global_avgpool(0, _ptr(x), _ptr(y), N, H * W, C, _DT[x.dtype], _stream()), "dl4j_global_avgpool")
+        ctx.shape = (N, C, H, W)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        N, C, H, W = ctx.shape
+        if torch.is_grad_enabled():                    # create_graph
+            return (dy / (H * W)).reshape(N, C, 1, 1).expand(N, C, H, W)
+        dy = _dense16(dy)
+        dx = torch.empty((N, C, H, W), dtype=dy.dtype, device=dy.device, memory_format=torch.channels_last)
+        _check(_avgpool_lib().dl4j_global_avgpool(1, _ptr(dy), _ptr(dx), N, H * W, C, _DT[dy.dtype], _stream()), "dl4j_global_avgpool")
+        return dx
+
+
+def _avgpool_lib():
+    l = require()
+    if not hasattr(l.dl4j_global_avgpool, "_typed"):
+        vp, i32 = ctypes.c_void_p, ctypes.c_int
+        l.dl4j_global_avgpool.argtypes = [i32, vp, vp, i32, i32, i32, i32, vp]
+        l.dl4j_global_avgpool.restype = i32
+        l.dl4j_global_avgpool._typed = True
+    return l
+
+
+def global_avgpool(x):
+    """[N, C, H, W] 16-bit channels-last -> [N, C], or None when the case is not covered."""
+    if not available() or not x.is_cuda or x.dim() != 4 or x.dtype not in (torch.bfloat16, torch.float16) or x.numel() == 0 or x.shape[1] % 8 \
+            or x.shape[0] > 65535 or not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 or not _plain_autograd():
+        return None
+    return _GlobalAvgPoolFn.apply(x)
+
+
 def maxpool2d(x, k, s, p):
     if not (available() and x.is_cuda and x.dim() == 4 and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0):
         return None
