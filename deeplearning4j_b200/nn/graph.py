@@ -19,6 +19,25 @@ from .conf.graphconf import ElementWiseVertex
 from ..utils.crash import guard_fit
 
 
+def _dense_nhwc(t):
+    return t.dim() == 4 and t.dtype == torch.bfloat16 and t.is_cuda and t.numel() > 0 and t.is_contiguous(memory_format=torch.channels_last) \
+        and t.data_ptr() % 16 == 0
+
+
+class _Folded:
+    """One call's folded weights: buffers and, per convolution vertex, (weight offset, channels out, row length, bias offset)."""
+
+    def __init__(self, w, b, where):
+        self.w, self.b, self.where = w, b, where
+
+    def __contains__(self, n): return n in self.where
+    def __iter__(self): return iter(self.where)
+
+    def __getitem__(self, n):
+        o, O, K, ob = self.where[n]
+        return self.w[o:o + O * K].view(O, K), self.b[ob:ob + O]
+
+
 class _VertexOwner:
     """Lets a parameterised non-layer vertex (AttentionVertex) take part in the updater machinery."""
     gradientNormalization = None
@@ -238,7 +257,7 @@ class ComputationGraph(BaseNetwork):
         specs = self._fold_specs()
         if not specs or nnops._FORCE_TORCH or not x.is_cuda or x.dtype != torch.bfloat16 or not self.flat_params.is_cuda \
                 or self.flat_params.dtype != torch.float32 or not native.available():
-            return {}
+            return ()
         sig = (self.flat_params.device,) + tuple((b.eps, b.useLogStd, b.lockGammaBeta, b.gamma, b.beta) for _, _, _, b in specs.values())
         t = getattr(self, "_fold_table", None)
         if t is None or t["sig"] != sig:
@@ -261,7 +280,150 @@ class ComputationGraph(BaseNetwork):
         w = torch.empty(t["w"], dtype=torch.bfloat16, device=x.device)
         b = torch.empty(t["b"], dtype=torch.float32, device=x.device)
         native.bn_fold(t["rows"], t["blocks"], self.flat_params, w, b)
-        return {n: (w[o:o + O * K].view(O, K), b[ob:ob + O]) for n, (o, O, K, ob) in t["where"].items()}
+        return _Folded(w, b, t["where"])
+
+    # ------------------------------------------------------------------ inference: a run of folded convolutions as one native call
+    def _compile_run(self, idx, acts, folded, folded_bn, fuse):
+        """Plans the vertices from ``order[idx]`` on that are folded convolutions, their batch norms, ReLUs and residual adds: the steps
+        with their buffers' offsets in one workspace (``csrc/infer_program.cu``), or None when the run is too short to pay."""
+        from ..ops import native
+        from .conf.base import ConvolutionMode
+        from .layers.conv import same_padding
+        conf, specs = self.conf, self._fold_specs()
+        NONE = -(1 << 63)
+        env, ext, steps, size, last, region = {}, [], [], [], [], []
+
+        def get(name):                   # (buffer, N, C, H, W); buffer: tensor number or -1 - external
+            r = env.get(name)
+            if r is None and name in acts:
+                t = acts[name]
+                if not _dense_nhwc(t):
+                    return None
+                if name not in ext:
+                    ext.append(name)
+                r = env[name] = (-1 - ext.index(name),) + tuple(t.shape)
+            return r
+
+        def new(N, C, H, W):
+            size.append(N * C * H * W * 2)
+            last.append(len(steps))
+            return (len(size) - 1, N, C, H, W)
+
+        def use(r):
+            if r[0] >= 0:
+                last[r[0]] = len(steps)
+            return r[0]
+
+        def conv(n, x, relu, res=None):
+            _, kind, c, _ = specs[n]
+            wo, O, _, bo = folded.where[n]
+            kH, kW = c.kernelSize
+            _, N, C, H, W = x
+            if C != c.nIn:
+                return None
+            if kind == "1x1":
+                sH, sW = c.stride
+                if (sH, sW) != (1, 1):
+                    y = new(N, C, (H + sH - 1) // sH, (W + sW - 1) // sW)
+                    steps.append([2, N, H, W, C, y[3], y[4], C, 1, 1, sH, sW, 1, 1, 0, 0, use(x), NONE, y[0], 0, 0])
+                    x, H, W = y, y[3], y[4]
+                if res is not None and res[1:] != (N, O, H, W):
+                    return None
+                y = new(N, O, H, W)
+                steps.append([0, N, H, W, C, H, W, O, 1, 1, 0, 0, 1, 1, int(relu), native._pick_block_n(N * H * W, O), use(x),
+                              NONE if res is None else use(res), y[0], wo, bo])
+                return y
+            d, mode = c.dilation, c._mode()
+            if mode == ConvolutionMode.Causal:
+                return None
+            pad = list(c.padding)
+            if mode == ConvolutionMode.Same:
+                lo_hi = [same_padding(v, k, 1, dd) for v, k, dd in ((H, kH, d[0]), (W, kW, d[1]))]
+                if any(lo != hi for lo, hi in lo_hi):
+                    return None
+                pad = [lo for lo, _ in lo_hi]
+            OH, OW = H + 2 * pad[0] - (kH - 1) * d[0], W + 2 * pad[1] - (kW - 1) * d[1]
+            if min(OH, OW) < 1 or (res is not None and (not relu or res[1:] != (N, O, OH, OW))):
+                return None
+            y = new(N, O, OH, OW)
+            steps.append([1, N, H, W, C, OH, OW, O, kH, kW, pad[0], pad[1], d[0], d[1], int(relu and res is None), 0, use(x), NONE, y[0], wo, bo])
+            if res is not None:
+                z = new(N, O, OH, OW)
+                steps.append([3, N, OH, OW, O, OH, OW, O, 1, 1, 0, 0, 1, 1, 1, 0, use(y), use(res), z[0], 0, 0])
+                y = z
+            return y
+
+        for n in self.order[idx:]:
+            ins = conf.vertexInputs[n]
+            a = fuse.get(n)
+            mark = (len(steps), len(size), list(last))
+            y = None
+            if n in folded:
+                x = get(ins[0]) if specs[n][1] != "stem" else None
+                nxt = fuse.get(specs[n][0], (None,))[0]
+                y = None if x is None else (x if nxt == "defer" else conv(n, x, nxt == "bn_relu"))
+            elif n in folded_bn:
+                y = get(ins[0])
+            elif a is not None and a[0] == "bn_add_relu" and a[1] in folded_bn:
+                x, r = get(a[1]), get(a[2])
+                y = conv(folded_bn[a[1]], x, True, r) if x is not None and r is not None else None
+            elif a is not None and a[0] == "alias":
+                y = get(a[1])
+            if y is None:
+                del steps[mark[0]:], size[mark[1]:]
+                last[:] = mark[2]
+                break
+            env[n] = y
+            region.append(n)
+        if len(steps) < 3:
+            return None
+        inside = set(region)
+        keep = [n for n in region if n in conf.networkOutputs or any(n in conf.vertexInputs[m] for m in self.order if m not in inside)
+                or any(n in p[1:] for m, p in fuse.items() if m not in inside)]
+        for n in keep:
+            if env[n][0] >= 0:
+                last[env[n][0]] = len(steps)
+        # offsets: first fit among the buffers alive at the same time (a buffer's life starts at the step that writes it)
+        first = [0] * len(size)
+        for i, st in enumerate(steps):
+            first[st[18]] = i
+        off, placed, total = [0] * len(size), [], 0
+        for i in range(len(size)):
+            busy = sorted((off[j], off[j] + size[j]) for j in placed if last[j] >= first[i] and first[j] <= last[i])
+            at = 0
+            for lo, hi in busy:
+                if at + size[i] <= lo:
+                    break
+                at = max(at, (hi + 255) // 256 * 256)
+            off[i] = at
+            placed.append(i)
+            total = max(total, at + size[i])
+        import struct
+        where = lambda r: r if r < 0 else off[r]
+        blob = b"".join(struct.pack("<16i5q", *st[:16], where(st[16]), st[17] if st[17] == NONE else where(st[17]), off[st[18]], st[19], st[20])
+                        for st in steps)
+        return {"steps": blob, "n": len(steps), "bytes": max(total, 256), "ext": ext, "region": inside,
+                "keep": [(n,) + env[n] + (where(env[n][0]),) for n in keep]}
+
+    def _folded_run(self, idx, acts, folded, folded_bn, fuse):
+        """Runs the planned vertices from ``order[idx]`` on; returns them as a set (empty: nothing was run).  A plan depends on the shapes
+        of the activations it starts from; the eight most recent are kept."""
+        from ..ops import native
+        plans = self.__dict__.setdefault("_run_plans", {})
+        key = (idx, self._fold_table["sig"]) + tuple((n, tuple(t.shape)) for n, t in acts.items() if t.dim() == 4 and _dense_nhwc(t))
+        plan = plans.get(key)
+        if plan is None:
+            while len(plans) >= 8:
+                plans.pop(next(iter(plans)), None)
+            plan = plans[key] = self._compile_run(idx, acts, folded, folded_bn, fuse) or {"n": 0}
+        if not plan["n"]:
+            return ()
+        ins = [acts[n] for n in plan["ext"]]
+        ws = torch.empty(plan["bytes"] // 2, dtype=torch.bfloat16, device=ins[0].device)
+        native.infer_program(plan["steps"], plan["n"], ws, ins, folded.w, folded.b)
+        for n, buf, N, C, H, W, at in plan["keep"]:
+            acts[n] = acts[plan["ext"][-1 - buf]] if buf < 0 else ws.as_strided((N, C, H, W), (H * W * C, 1, W * C, C), at // 2)
+        return plan["region"]
 
     def _folded_conv(self, n, folded, x, relu, residual=None):
         """relu?(batchnorm(conv(x)) [+ residual]) with the folded weights of vertex ``n``."""
@@ -299,8 +461,9 @@ class ComputationGraph(BaseNetwork):
         ctx = ctx if ctx is not None else {}
         fuse = self._fusion_plan() if ctx.get("fuse") else {}
         bias_of = self._fuse_bias if fuse else {}
-        folded = self._fold(next(iter(inputs.values()))) if fuse and not training and not fmasks else {}
+        folded = self._fold(next(iter(inputs.values()))) if fuse and not training and not fmasks else ()
         folded_bn = {self._fold_specs()[n][0]: n for n in folded}
+        done = ()
 
         def pre_bias(bn_name):
             c = bias_of.get(bn_name)
@@ -313,7 +476,13 @@ class ComputationGraph(BaseNetwork):
         ctx["input_T"] = {k: v.shape[2] for k, v in inputs.items() if v.dim() == 3}
         preouts = ctx.setdefault("preouts", {})
         conf = self.conf
-        for n in self.order:
+        for idx, n in enumerate(self.order):
+            if n in done:
+                continue
+            if n in folded and self._fold_specs()[n][1] != "stem" and not done:
+                done = self._folded_run(idx, acts, folded, folded_bn, fuse)
+                if n in done:
+                    continue
             v = conf.vertices[n]
             ins = [acts[i] for i in conf.vertexInputs[n]]
             in_masks = [masks.get(i) for i in conf.vertexInputs[n]]

@@ -1442,6 +1442,21 @@ def conv_infer_kxk(x, w, b, kH, kW, pad, dil, relu, fuse_w=False):
     return y.permute(0, 3, 1, 2)
 
 
+def infer_program(steps, n, workspace, inputs, w, b):
+    """Issues the ``n`` steps of a planned run of folded convolutions (``csrc/infer_program.cu``)."""
+    global LAUNCHES
+    l = require()
+    if not hasattr(l.dl4j_infer_program, "_typed"):
+        vp, i32 = ctypes.c_void_p, ctypes.c_int
+        l.dl4j_infer_program.argtypes = [ctypes.c_char_p, i32, vp, vp, vp, vp, i32, i32, vp]
+        l.dl4j_infer_program.restype = i32
+        l.dl4j_infer_program._typed = True
+    ext = (ctypes.c_void_p * len(inputs))(*[t.data_ptr() for t in inputs])
+    rc = l.dl4j_infer_program(steps, n, _ptr(workspace), ext, _ptr(w), _ptr(b), _DT[workspace.dtype], num_sms(), _stream())
+    LAUNCHES += n - 1
+    _check(rc, "dl4j_infer_program")
+
+
 def conv_weight_cl(W):
     """bf16 channels-last version of an fp32 convolution kernel parameter, or None when not applicable."""
     if not (available() and W.is_cuda and W.dim() == 4 and W.dtype == torch.float32 and W.is_contiguous()):
