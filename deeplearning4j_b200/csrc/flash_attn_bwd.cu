@@ -14,10 +14,19 @@ using namespace dl4j;
 // it is written in bf16 directly.
 namespace dl4j {
 
-constexpr int FB_THREADS = 64 + 512;              // warp 0 TMA, warp 1 MMA, 16 compute warps (four threads per row)
+// warp 0 TMA, warps 1 / 18 / 19 MMA issue, warps 2 .. 17 compute (four threads per row).
+// Two things bounded this kernel at 3.4 us per block of 128 x 128 (B 32, H 12, T 512: 193 us).  One thread gets a tcgen05.mma into the
+// pipe every ~147 clocks whatever its shape, a block takes 32 of them, and S of the next block came last: three threads issue now (S + dV,
+// dP + dK, dQ; every accumulator has one issuer), S and dP of the next block first, the rest beside the threads' work.  And dQ left
+// through 16-byte reductions, 32 rows to a warp instruction, one L1 wavefront each: 2048 of the block's cycles on the data pipe that the
+// MMA operands share (82 % busy).  Each warp now stages its 32 x 16 piece in shared memory and the copy engine adds it.  Now 163 us (2.9 us a block).
+constexpr int FB_COMPUTE = 512;
+constexpr int FB_THREADS = 64 + FB_COMPUTE + 64;
 constexpr int FB_BLK = 128;                       // queries per step and keys per CTA
 constexpr int FB_TILE = FB_BLK * FA_D * 2;        // 16 KB: one [128, 64] bf16 tile
 constexpr int FB_PS = FB_BLK * FB_BLK * 2;        // 32 KB: P or dS
+constexpr int FB_DQ_SLAB = 32 * 16 * 4;           // one warp's piece of dQ
+constexpr int FB_DQ = 16 * FB_DQ_SLAB;
 constexpr int FB_TMEM_COLS = 512;                 // S 0..127, dP 128..255, dQ 256..319, dV 320..383, dK 384..447
 
 struct FlashBwdParams {
@@ -44,7 +53,7 @@ template <bool DROP>
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                      const FlashBwdParams p) {
+                      const __grid_constant__ CUtensorMap tmap_dq, const FlashBwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* k_s = smem;
@@ -53,7 +62,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint8_t* do_s = q_s + 2 * FB_TILE;              // two stages
   uint8_t* p_s = do_s + 2 * FB_TILE;
   uint8_t* ds_s = p_s + FB_PS;
-  float* mask_s = reinterpret_cast<float*>(ds_s + FB_PS);      // [128]
+  uint8_t* dq_s = ds_s + FB_PS;                   // [16 warps] 32 rows x 16 fp32 columns, 64-byte swizzle
+  float* mask_s = reinterpret_cast<float*>(dq_s + FB_DQ);      // [128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(mask_s + FB_BLK);
   uint64_t* kv_full = bars;
   uint64_t* qdo_full = bars + 1;     // [2]
@@ -63,7 +73,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint64_t* dq_full = bars + 7;
   uint64_t* dq_empty = bars + 8;
   uint64_t* fin_full = bars + 9;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* pds_empty = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_blocks = (p.Tk + FB_BLK - 1) / FB_BLK;
@@ -80,12 +91,13 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_do);
     mbar_init(kv_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 1); }
-    mbar_init(s_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 2); }
+    mbar_init(pds_empty, 3);
+    mbar_init(s_full, 2);
     mbar_init(p_full, 16);
     mbar_init(dq_full, 1);
     mbar_init(dq_empty, 16);
-    mbar_init(fin_full, 1);
+    mbar_init(fin_full, 2);
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -111,66 +123,63 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         tma_load_4d(do_s + st * FB_TILE, &tmap_do, &qdo_full[st], 0, (i0 + i) * FB_BLK, h, b);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 || warp >= 18) {
     if (lane == 0) {
+      const int role = warp == 1 ? 0 : warp - 17;                     // 0: S, dV   1: dP, dK   2: dQ
       const uint32_t id_s = make_idesc(1, 0, 0, FB_BLK, FB_BLK);      // [q, keys] = A[q, d] K-major x B[keys, d] K-major
       const uint32_t id_kv = make_idesc(1, 1, 1, FB_BLK, FA_D);       // [keys, d] = A^T (P / dS tile, MN-major) x B[q, d] MN-major
       const uint32_t id_dq = make_idesc(1, 0, 1, FB_BLK, FA_D);       // [q, d] = dS K-major x K_j[keys, d] MN-major
+      const uint32_t ak = smem_u32(k_s), ads = smem_u32(ds_s);
+      // descriptors are built once; inside the loops they only advance by a constant (one 64-bit add per operand)
+      const uint64_t d_k = make_smem_desc_sw128(role == 0 ? ak : smem_u32(v_s), 16, 1024);                            // S: K, dP: V
+      const uint64_t d_a0 = make_smem_desc_sw128(smem_u32(role == 0 ? q_s : do_s), 16, 1024);                         // S: Q, dP: dO
+      const uint64_t d_t = make_smem_desc_sw128(smem_u32(role == 0 ? p_s : ds_s), FB_BLK * 128, 1024);                // dV: P^T, dK: dS^T
+      const uint64_t d_b0 = make_smem_desc_sw128(smem_u32(role == 0 ? do_s : q_s), FB_BLK * 128, 1024);               // dV: dO, dK: Q
+      const uint64_t d_dsk = make_smem_desc_sw128(ads, 16, 1024), d_kmn = make_smem_desc_sw128(ak, FB_BLK * 128, 1024);
+      constexpr uint64_t STAGE_STEP = (uint64_t)(FB_TILE >> 4);
+      const uint32_t t_s = tmem_base + (role == 0 ? T_S : T_DP), t_kv = tmem_base + (role == 0 ? T_DV : T_DK);
       bool ok = mbar_wait_bounded(kv_full, 0, p.status, DL4J_ERR_TIMEOUT_MMA);
-      const uint32_t ak = smem_u32(k_s), av = smem_u32(v_s), ap = smem_u32(p_s), ads = smem_u32(ds_s);
-      const uint64_t dk_k = make_smem_desc_sw128(ak, 16, 1024), dv_k = make_smem_desc_sw128(av, 16, 1024);
-      const uint64_t d_q_k0 = make_smem_desc_sw128(smem_u32(q_s), 16, 1024), d_do_k0 = make_smem_desc_sw128(smem_u32(do_s), 16, 1024);
-      constexpr uint64_t STAGE_STEP_K = (uint64_t)(FB_TILE >> 4);
-      // S_i = Q_i K_j^T and dP_i = dO_i V_j^T; issued one block ahead so that they overlap the threads' work on block i - 1
+      // S_i = Q_i K_j^T or dP_i = dO_i V_j^T
       auto issue_s = [&](int i) -> bool {
         const int st = i & 1;
         if (!mbar_wait_bounded(&qdo_full[st], (uint32_t)((i >> 1) & 1), p.status, DL4J_ERR_TIMEOUT_MMA)) return false;
         tc_fence_after();
-        const uint64_t dq_k = d_q_k0 + (st ? STAGE_STEP_K : 0), ddo_k = d_do_k0 + (st ? STAGE_STEP_K : 0);
+        const uint64_t d_a = d_a0 + (st ? STAGE_STEP : 0);
 #pragma unroll
-        for (int k = 0; k < FA_D / 16; ++k) {
-          umma_f16(tmem_base + T_S, dq_k + ((uint64_t)(k * 32) >> 4), dk_k + ((uint64_t)(k * 32) >> 4), id_s, k > 0 ? 1u : 0u);
-          umma_f16(tmem_base + T_DP, ddo_k + ((uint64_t)(k * 32) >> 4), dv_k + ((uint64_t)(k * 32) >> 4), id_s, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < FA_D / 16; ++k)
+          umma_f16(t_s, d_a + ((uint64_t)(k * 32) >> 4), d_k + ((uint64_t)(k * 32) >> 4), id_s, k > 0 ? 1u : 0u);
         umma_commit(s_full);
         return true;
       };
-      // descriptors are built once; inside the loops they only advance by a constant (one 64-bit add per operand), which keeps
-      // the single issuing thread at a few instructions per MMA
-      const uint64_t d_pt = make_smem_desc_sw128(ap, FB_BLK * 128, 1024), d_dst = make_smem_desc_sw128(ads, FB_BLK * 128, 1024);
-      const uint64_t d_dsk = make_smem_desc_sw128(ads, 16, 1024), d_kmn = make_smem_desc_sw128(ak, FB_BLK * 128, 1024);
-      const uint64_t d_do_mn0 = make_smem_desc_sw128(smem_u32(do_s), FB_BLK * 128, 1024), d_q_mn0 = make_smem_desc_sw128(smem_u32(q_s), FB_BLK * 128, 1024);
-      constexpr uint64_t STAGE_STEP = (uint64_t)(FB_TILE >> 4);     // second Q / dO stage: same descriptor, start address + one tile
-      if (ok && nq > 0) ok = issue_s(0);
+      if (ok && role < 2 && nq > 0) ok = issue_s(0);
       for (int i = 0; i < nq && ok; ++i) {
         const int st = i & 1;
-        const uint64_t d_do_st = d_do_mn0 + (st ? STAGE_STEP : 0), d_q_st = d_q_mn0 + (st ? STAGE_STEP : 0);
         if (!mbar_wait_bounded(p_full, (uint32_t)(i & 1), p.status, DL4J_ERR_TIMEOUT_MMA)) { ok = false; break; }
-        tc_fence_after();
+        if (role < 2) {
+          // S / dP of block i have been read out of tensor memory (p_full), block i + 1's may overwrite them: they come first, the
+          // threads wait for them
+          if (i + 1 < nq && !(ok = issue_s(i + 1))) break;
+          tc_fence_after();
+          const uint64_t d_b = d_b0 + (st ? STAGE_STEP : 0);
 #pragma unroll
-        for (int k = 0; k < FB_BLK / 16; ++k) {
-          // reduction over the 128 query rows: 16 rows (2048 bytes) per step in the MN-major tiles
-          const uint64_t a_pt = d_pt + (uint64_t)(k * (2048 >> 4)), a_dst = d_dst + (uint64_t)(k * (2048 >> 4));
-          const uint64_t b_do = d_do_st + (uint64_t)(k * (2048 >> 4)), b_q = d_q_st + (uint64_t)(k * (2048 >> 4));
-          umma_f16(tmem_base + T_DV, a_pt, b_do, id_kv, (i > 0 || k > 0) ? 1u : 0u);
-          umma_f16(tmem_base + T_DK, a_dst, b_q, id_kv, (i > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(&qdo_empty[st]);      // Q_i / dO_i are not read again: their stage can be refilled
-        // dQ_{i-1} must have left tensor memory before dQ_i overwrites it; the threads read it out while dV / dK were issued
-        if (!mbar_wait_bounded(dq_empty, (uint32_t)((i & 1) ^ 1), p.status, DL4J_ERR_TIMEOUT_MMA)) { ok = false; break; }
-        tc_fence_after();
+          for (int k = 0; k < FB_BLK / 16; ++k)      // reduction over the 128 query rows: 16 rows (2048 bytes) per step, MN-major tiles
+            umma_f16(t_kv, d_t + (uint64_t)(k * (2048 >> 4)), d_b + (uint64_t)(k * (2048 >> 4)), id_kv, (i > 0 || k > 0) ? 1u : 0u);
+          umma_commit(&qdo_empty[st]);               // Q_i / dO_i are not read again by this thread: their stage can be refilled
+        } else {
+          // dQ_{i-1} must have left tensor memory before dQ_i overwrites it
+          if (!mbar_wait_bounded(dq_empty, (uint32_t)((i & 1) ^ 1), p.status, DL4J_ERR_TIMEOUT_MMA)) { ok = false; break; }
+          tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < FB_BLK / 16; ++k) {
-          // reduction over the 128 keys: dS K-major (two 64-key blocks of 16 KB, 32 bytes per step), K_j MN-major
-          const uint64_t a_ds = d_dsk + (uint64_t)(((k >> 2) * (FB_BLK * 128) + (k & 3) * 32) >> 4);
-          const uint64_t b_k = d_kmn + (uint64_t)(k * (2048 >> 4));
-          umma_f16(tmem_base + T_DQ, a_ds, b_k, id_dq, k > 0 ? 1u : 0u);
+          for (int k = 0; k < FB_BLK / 16; ++k) {
+            // reduction over the 128 keys: dS K-major (two 64-key blocks of 16 KB, 32 bytes per step), K_j MN-major
+            const uint64_t a_ds = d_dsk + (uint64_t)(((k >> 2) * (FB_BLK * 128) + (k & 3) * 32) >> 4);
+            umma_f16(tmem_base + T_DQ, a_ds, d_kmn + (uint64_t)(k * (2048 >> 4)), id_dq, k > 0 ? 1u : 0u);
+          }
+          umma_commit(dq_full);
         }
-        umma_commit(dq_full);
-        // S / dP of block i were read out of tensor memory before p_full(i) completed, so block i + 1 may overwrite them now
-        if (i + 1 < nq) ok = issue_s(i + 1);
+        umma_commit(pds_empty);
       }
-      if (ok) umma_commit(fin_full);
+      if (ok && role < 2) umma_commit(fin_full);
     }
   } else {
     const int cw = warp - 2;                        // 0..15
@@ -218,13 +227,20 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           for (int e = 0; e < 4; ++e) hh[e] = __floats2bfloat162_rn(__uint_as_float(v0[8 * j + 2 * e]), __uint_as_float(v0[8 * j + 2 * e + 1]));
           if (cq * 16 + 8 * j < p.D) dst[j] = u;
         }
-      } else if (tqb < p.Tq) {
-        float4* dst = reinterpret_cast<float4*>(p.dq + (rbase + tqb) * p.D + cq * 16);
+      } else if (p.dq != nullptr) {
+        uint8_t* slab = dq_s + cw * FB_DQ_SLAB;
+        if (lane == 0) bulk_wait_read<0>();           // the previous block's piece has left the slab
+        __syncwarp();
 #pragma unroll
-        for (int j = 0; j < 4; ++j)      // fire-and-forget 16-byte reductions at L2
-          if (cq * 16 + 4 * j < p.D) asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "r"(v0[4 * j]), "r"(v0[4 * j + 1]),
-                       "r"(v0[4 * j + 2]), "r"(v0[4 * j + 3])
-                       : "memory");
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<uint4*>(slab + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = make_uint4(v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int row0 = (i0 + blk) * FB_BLK + q * 32;
+        if (lane == 0) {
+          if (row0 < p.Tq && cq * 16 < p.D) tma_reduce_add_4d(&tmap_dq, slab, cq * 16, row0, h, b);
+          bulk_commit();
+        }
       }
       return true;
     };
@@ -280,6 +296,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
           for (int j = 0; j < 32; ++j) { pe[j] = ((in_bits >> j) & 1u) ? __int_as_float(0x7fffffff) : 0.f; de[j] = 0.f; }
         }
+        // block i - 1's MMAs have read P and dS (warp-uniform wait)
+        if (i >= 1 && !mbar_wait_bounded(pds_empty, (uint32_t)((i - 1) & 1), p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) { ok = false; break; }
         fa_store_row(p_s, r, cq * 32, 32, pe);
         fa_store_row(ds_s, r, cq * 32, 32, de);
       }
@@ -292,6 +310,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       if (i > 0 && !dq_flush(i - 1)) { ok = false; break; }
     }
     if (ok && nq > 0) ok = dq_flush(nq - 1);
+    if (lane == 0) bulk_wait<0>();                    // the reductions are done before the shared memory goes
     if (ok && mbar_wait_bounded(fin_full, 0, p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) {
       tc_fence_after();
       // accumulator rows are keys here: thread r owns key k0 + r; column groups 0, 1 -> dV, 2, 3 -> dK
@@ -346,6 +365,18 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   if (r) return -1000 - r;
   r = fa_encode(&tdo, dout, B, H, Tq, D, do_strides[0], do_strides[1], do_strides[2], FB_BLK);
   if (r) return -1000 - r;
+  CUtensorMap tdq;
+  memset(&tdq, 0, sizeof(tdq));
+  if (dq_acc) {
+    dl4j_PFN_encodeTiled enc = dl4j_get_encode_tiled();
+    if (!enc || (reinterpret_cast<uintptr_t>(dq_acc) & 15)) return -DL4J_ERR_BAD_ARG;
+    cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)Tq, (cuuint64_t)H, (cuuint64_t)B};
+    cuuint64_t strides[3] = {(cuuint64_t)D * 4, (cuuint64_t)Tq * D * 4, (cuuint64_t)H * Tq * D * 4};
+    cuuint32_t box[4] = {16, 32, 1, 1}, es[4] = {1, 1, 1, 1};
+    const CUresult cr = enc(&tdq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dq_acc, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return -1000 - (int)cr;
+  }
   int dev = 0;
   cudaGetDevice(&dev);
   FlashBwdParams p;
@@ -364,11 +395,11 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   p.seed = reinterpret_cast<const unsigned long long*>(seed);
   p.drop_thr = dropout_p > 0.f ? (uint32_t)(dropout_p * 65536.f + 0.5f) : 0u;
   p.inv_keep = p.drop_thr ? 65536.f / (65536.f - (float)p.drop_thr) : 1.f;
-  const size_t smem = 6 * FB_TILE + 2 * FB_PS + FB_BLK * sizeof(float) + 256 + 1024;
+  const size_t smem = 6 * FB_TILE + 2 * FB_PS + FB_DQ + FB_BLK * sizeof(float) + 256 + 1024;
   auto kern = p.drop_thr ? flash_attn_bwd_kernel<true> : flash_attn_bwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  kern<<<B * H * ((Tk + FB_BLK - 1) / FB_BLK), FB_THREADS, smem, (cudaStream_t)stream_>>>(tq, tk, tv, tdo, p);
+  kern<<<B * H * ((Tk + FB_BLK - 1) / FB_BLK), FB_THREADS, smem, (cudaStream_t)stream_>>>(tq, tk, tv, tdo, tdq, p);
   return (int)cudaGetLastError();
 }
 

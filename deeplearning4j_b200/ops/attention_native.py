@@ -22,8 +22,8 @@ _LONG2 = ctypes.c_long * 2
 
 def _ok_view(t):
     """[B, H, T, D] view usable by a rank-4 tensor map: unit inner stride, 16-byte aligned strides."""
-    return (t.dim() == 4 and t.stride(3) == 1 and t.stride(2) % 8 == 0 and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0
-            and t.data_ptr() % 16 == 0 and t.shape[3] % 8 == 0)
+    s = t.stride()
+    return len(s) == 4 and s[3] == 1 and not (s[0] | s[1] | s[2]) & 7 and t.data_ptr() % 16 == 0 and t.shape[3] % 8 == 0
 
 
 def _prep(t):
@@ -175,6 +175,8 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
         return None
     if fused and (USE_FLASH or dropout_p > 0.0):
         flags = (1 if causal else 0) | (0 if _empty_rows_are_zero(D, Tq, Tk) and not causal else 2)
+        if dropout_p == 0.0 and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)):
+            return flash_forward(q, k, v, mask, scale, flags=flags)[0].permute(0, 2, 1, 3)       # nothing to differentiate
         return _AttentionFn.apply(q, k, v, mask, scale, float(dropout_p), flags)
     if causal or D % 8 or Tk % 8 or Tq % 8 or Tk > 1024:
         return None
@@ -275,9 +277,11 @@ def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
 
 
 def flash_supported(q, k, v):
-    return (native.available() and q.is_cuda and q.dim() == 4 and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.shape[3] <= 64
-            and q.shape[3] % 8 == 0 and k.shape == v.shape and q.shape[3] == k.shape[3] and q.shape[:2] == k.shape[:2]
-            and q.numel() > 0 and k.numel() > 0)
+    if not native.available() or not q.is_cuda or not q.dtype == k.dtype == v.dtype == torch.bfloat16:
+        return False
+    qs, ks = q.shape, k.shape
+    return (len(qs) == 4 and ks == v.shape and len(ks) == 4 and qs[3] <= 64 and qs[3] % 8 == 0 and qs[3] == ks[3] and qs[:2] == ks[:2]
+            and min(qs) > 0 and min(ks) > 0)
 
 
 def flash_forward(q, k, v, key_mask, scale, dropout_p=0.0, seed=None, flags=0):

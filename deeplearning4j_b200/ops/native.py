@@ -914,19 +914,19 @@ def layer_norm_grad(x, gain, bias, dy, eps):
             return None
     if dy.numel() != x.numel() or dy.device != x.device:
         return None
-    l = require()
-    x2 = x.detach().contiguous()
-    dy2 = dy.detach().to(x.dtype).contiguous()
-    g32 = gain.detach().float().contiguous()
+    l = _LIB
+    x2 = x if x.is_contiguous() else x.contiguous()
+    dy2 = dy if dy.dtype == x.dtype and dy.is_contiguous() else dy.to(x.dtype).contiguous()
+    g32 = gain if gain.dtype == torch.float32 and gain.is_contiguous() else gain.float().contiguous()
     rows = x2.numel() // C
-    dx = torch.empty_like(x2)
-    dg = torch.empty(C, dtype=torch.float32, device=x.device)
-    db = torch.empty(C, dtype=torch.float32, device=x.device) if bias is not None else None
+    dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    dg = torch.empty(gain.shape, dtype=torch.float32, device=x.device)
+    db = torch.empty(bias.shape, dtype=torch.float32, device=x.device) if bias is not None else None
     partial = torch.empty(4 * num_sms() * C, dtype=torch.float32, device=x.device)
-    rc = l.dl4j_layer_norm_grad(_ptr(dy2), _ptr(x2), _ptr(g32), None, None, _ptr(dx), _ptr(dg), _ptr(db),
-                                _ptr(partial), rows, C, float(eps), _DT[x.dtype], 0, num_sms(), _stream())
+    rc = l.dl4j_layer_norm_grad(dy2.data_ptr(), x2.data_ptr(), g32.data_ptr(), None, None, dx.data_ptr(), dg.data_ptr(), _ptr(db),
+                                partial.data_ptr(), rows, C, float(eps), _DT[x.dtype], 0, num_sms(), _stream())
     _check(rc, "dl4j_layer_norm_grad")
-    return dx, dg.reshape(gain.shape).to(gain.dtype), None if db is None else db.reshape(bias.shape).to(bias.dtype)
+    return dx, dg.to(gain.dtype), None if db is None else db.to(bias.dtype)
 
 
 def layer_norm(x, gain, bias, eps, residual=None):
