@@ -50,6 +50,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One thread of a converged warp.  Code that issues tcgen05.mma sits under this and not under `lane == 0`: the compiler knows that a
+// single thread is active after elect.sync and keeps the instruction's descriptors in uniform registers; after a plain comparison it
+// does not, and one thread gets an instruction out per ~147 clocks instead of ~64 (mma_issue_probe.cu).  512 x 512 x 2048 GEMM:
+// 14.5 -> 10.3 us, 16384 x 768 x 3072 in 128-column tiles: 99 -> 70 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

@@ -135,7 +135,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation 
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -165,7 +165,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation 
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const int b_mn = p.mode == 0 ? 0 : 1;
       const uint32_t idesc = make_idesc(p.fmt, 0, b_mn, 128, BLOCK_N);
       const uint32_t lbo_b = b_mn ? 8192u : 16u;
@@ -371,7 +371,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation {
   // (the host launches a grid that is a multiple of tiles_n in that case)
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int sa = 0, sb = 0;
       uint32_t pa = 0, pb = 0;
       bool ok = true, first = true;
@@ -402,13 +402,13 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation {
       }
     }
   } else if ((warp == 1 || warp >= 6) && p.issuers > 1) {
-    // Several issuing warps (resident weights only): one thread gets at most one tcgen05.mma into the pipe per ~147 clocks
-    // whatever its shape, an N = 64 instruction occupies the tensor core for ~48.  Warp j takes the tiles j, j + NI, ... of this
+    // Several issuing warps (resident weights only): one elected thread gets a tcgen05.mma into the pipe per ~64 clocks,
+    // an N = 64 instruction occupies the tensor core for ~48.  Warp j takes the tiles j, j + NI, ... of this
     // CTA, each into an accumulator buffer of its own.  NACC and the number of A stages are multiples of NI (x slices per tile),
     // so a buffer or a stage always falls to the same warp and that warp sees every phase of its barriers in order.
     const int me = warp == 1 ? 0 : warp - 5;
     const int NI = p.issuers;
-    if (lane == 0 && me < NI) {
+    if (me < NI && elect_one()) {
       const int b_mn = p.mode == 0 ? 0 : 1;
       const uint32_t idesc = make_idesc(p.fmt, 0, b_mn, 128, BLOCK_N);
       const uint32_t lbo_b = b_mn ? 8192u : 16u;
@@ -454,7 +454,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation {
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int b_mn = p.mode == 0 ? 0 : 1;
       const uint32_t idesc = make_idesc(p.fmt, 0, b_mn, 128, BLOCK_N);
       const uint32_t lbo_b = b_mn ? 8192u : 16u;
@@ -652,7 +652,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy,    // {Cout, OW, 
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -683,7 +683,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy,    // {Cout, OW, 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(p.fmt, 1, 1, 128, BLOCK_N);
       int stage = 0;
       uint32_t phase = 0;

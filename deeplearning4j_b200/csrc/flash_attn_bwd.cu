@@ -15,8 +15,8 @@ using namespace dl4j;
 namespace dl4j {
 
 // warp 0 TMA, warps 1 / 18 / 19 MMA issue, warps 2 .. 17 compute (four threads per row).
-// Two things bounded this kernel at 3.4 us per block of 128 x 128 (B 32, H 12, T 512: 193 us).  One thread gets a tcgen05.mma into the
-// pipe every ~147 clocks whatever its shape, a block takes 32 of them, and S of the next block came last: three threads issue now (S + dV,
+// Two things bounded this kernel at 3.4 us per block of 128 x 128 (B 32, H 12, T 512: 193 us).  One thread got a tcgen05.mma into the
+// pipe every ~147 clocks (under lane == 0; ~64 under elect.sync), a block takes 32 of them, and S of the next block came last: three threads issue now (S + dV,
 // dP + dK, dQ; every accumulator has one issuer), S and dP of the next block first, the rest beside the threads' work.  And dQ left
 // through 16-byte reductions, 32 rows to a warp instruction, one L1 wavefront each: 2048 of the block's cycles on the data pipe that the
 // MMA operands share (82 % busy).  Each warp now stages its 32 x 16 piece in shared memory and the copy engine adds it.  Now 163 us (2.9 us a block).
@@ -111,7 +111,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   constexpr uint32_t T_S = 0, T_DP = 128, T_DQ = 256, T_DV = 320, T_DK = 384;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * FB_TILE);
       tma_load_4d(k_s, &tmap_k, kv_full, 0, k0, h, b);
       tma_load_4d(v_s, &tmap_v, kv_full, 0, k0, h, b);
@@ -124,7 +124,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       }
     }
   } else if (warp == 1 || warp >= 18) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int role = warp == 1 ? 0 : warp - 17;                     // 0: S, dV   1: dP, dK   2: dQ
       const uint32_t id_s = make_idesc(1, 0, 0, FB_BLK, FB_BLK);      // [q, keys] = A[q, d] K-major x B[keys, d] K-major
       const uint32_t id_kv = make_idesc(1, 1, 1, FB_BLK, FA_D);       // [keys, d] = A^T (P / dS tile, MN-major) x B[q, d] MN-major

@@ -89,7 +89,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, FF_TILE);
       tma_load_4d(q_s, &tmap_q, q_full, 0, q0, h, b);
       for (int t = 0; t < 2 * nb; ++t) {              // tile t: K block t/2 (even) or V block t/2 (odd)
@@ -101,7 +101,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = make_idesc(1, 0, 0, FF_BM, FF_BN);      // S = Q K^T: both operands K-major (K = head dim)
       const uint32_t idesc_o = make_idesc(1, 0, 1, FF_BM, FA_D);       // P V: V [keys, 64] is MN-major for the B operand
       const uint64_t dq = make_smem_desc_sw128(smem_u32(q_s), 16, 1024);

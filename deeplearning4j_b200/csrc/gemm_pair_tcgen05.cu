@@ -239,7 +239,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs: own A rows, own half of B)
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -289,7 +289,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank != 0) {
+    const bool elected = elect_one();
+    if (elected && rank != 0) {
       // ------------------------------------------------------------------ peer: tell the leader when a stage has landed here
       // (the loads carry no cta_group qualifier, so each CTA's loads complete on its own barrier)
       const uint32_t leader_peer_full = mapa(smem_u32(peer_full), 0);
@@ -306,7 +307,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
-    } else if (lane == 0) {
+    } else if (elected) {
       // ------------------------------------------------------------------ leader: MMA issuer for the pair
       const uint32_t idesc = make_idesc(p.fmt, A_MN ? 1 : 0, B_MN ? 1 : 0, 2 * BLOCK_M, BLOCK_N);
       constexpr uint32_t LBO_A = A_MN ? 64 * BLOCK_K * 2 : 16, LBO_B = B_MN ? 64 * BLOCK_K * 2 : 16;

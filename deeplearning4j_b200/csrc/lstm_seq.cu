@@ -22,10 +22,8 @@ constexpr int LS_UNITS = 16;                 // hidden units per CTA
 constexpr int LS_N = 4 * LS_UNITS;           // MMA N: gate rows per CTA
 constexpr int LS_M = 128;                    // MMA M: batch rows (zero padded)
 constexpr int LS_BK = 64;                    // K elements per stage (128 bytes, SWIZZLE_128B)
-constexpr int LS_ISSUERS = 3;                // MMA-issuing warps.  One thread gets at most one tcgen05.mma into the pipe per ~150 clocks
-                                             // whatever the instruction's shape (measured: 150 clk for N = 8 .. 256), while an
-                                             // M 128 x N 64 x K 16 instruction occupies the tensor core for ~48 clocks and N = 16 for
-                                             // less; three issuers, each with every third k-block, bring an N = 64 instruction down to ~50 clocks, and
+constexpr int LS_ISSUERS = 3;                // MMA-issuing warps.  One elected thread gets a tcgen05.mma into the pipe per ~64 clocks, while
+                                             // an M 128 x N 64 x K 16 instruction occupies the tensor core for ~48 clocks and N = 16 for ~39;
                                              // with the producer warp and four epilogue warps the CTA stays at 256 threads (a ninth warp
                                              // would cut the register budget to 168 and spill the epilogue).
 constexpr int LS_ACCS = LS_ISSUERS;          // one TMEM accumulator per issuer (MMAs of different threads never share one); the
@@ -145,7 +143,7 @@ lstm_seq_fwd_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // resident weights: per k-block four boxes of 16 rows (one per gate) placed 2 KB apart
       mbar_expect_tx(w_full, (uint32_t)(kblocks * LS_B_KB));
       for (int kb = 0; kb < kblocks; ++kb)
@@ -173,7 +171,7 @@ lstm_seq_fwd_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
     }
   } else if (warp < LS_EPI_WARP0) {
     const int me = warp - 1;                      // issuer index: k-blocks me, me + LS_ISSUERS, ... of every step
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(1, 0, 0, LS_M, LS_N);
       const uint32_t acc = tmem_base + (uint32_t)(me * LS_N);
       bool ok = mbar_wait_bounded(w_full, 0, p.status, DL4J_ERR_TIMEOUT_MMA);
@@ -380,7 +378,7 @@ lstm_seq_bwd_kernel(const __grid_constant__ CUtensorMap tmap_dz, const __grid_co
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(w_full, (uint32_t)(kblocks * LB_B_KB));
       for (int kb = 0; kb < kblocks; ++kb) tma_load_4d(w_smem + kb * LB_B_KB, &tmap_w, w_full, kb * LS_BK, unit0, 0, 0);
       int stage = 0;
@@ -404,7 +402,7 @@ lstm_seq_bwd_kernel(const __grid_constant__ CUtensorMap tmap_dz, const __grid_co
     }
   } else if (warp < LS_EPI_WARP0) {
     const int me = warp - 1;                      // issuer index: k-blocks me, me + LS_ISSUERS, ... of every round
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(1, 0, 0, LS_M, LB_N);
       const uint32_t acc = tmem_base + (uint32_t)(me * LB_N);
       bool ok = mbar_wait_bounded(w_full, 0, p.status, DL4J_ERR_TIMEOUT_MMA);
@@ -666,7 +664,7 @@ lstm_seq_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmap_dz, const _
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(w_full, (uint32_t)(kblocks * G_B_KB));
       for (int kb = 0; kb < kblocks; ++kb) tma_load_4d(w_smem + kb * G_B_KB, &tmap_w, w_full, (kb_base + kb) * LS_BK, grp_unit0, 0, 0);
       int stage = 0;
@@ -690,7 +688,7 @@ lstm_seq_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmap_dz, const _
     }
   } else if (warp < LS_EPI_WARP0) {
     const int me = warp - 1;                      // issuer index: k-blocks me, me + LS_ISSUERS, ... of every round
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(1, 0, 0, LS_M, GN);
       const uint32_t acc = tmem_base + (uint32_t)(me * GN);
       bool ok = mbar_wait_bounded(w_full, 0, p.status, DL4J_ERR_TIMEOUT_MMA);

@@ -1,10 +1,10 @@
 // Issue-rate probe for tcgen05.mma (cta_group::1, bf16, K = 16): one CTA, operands fixed in shared memory, `issuers` warps
 // each issuing `iters` instructions into accumulators of their own.  Reports the clocks one issuer spent per instruction.
 //
-// What it measures on a B200: a single thread completes one instruction per ~150 clocks whatever the shape (M 64 / 128,
-// N 8 .. 256), while two issuers reach ~127 clocks per M 128 x N 256 instruction each (the tensor core's own rate), four reach
-// 64 at N 128 and 48 at N 64.  Kernels whose instructions are small (the persistent LSTM: N = 64 forward, N = 16 backward)
-// therefore spread the issue over several warps.
+// What it measures on a B200: an issuing thread chosen by elect.sync gets one instruction through per ~64 clocks (M 128, N 16 .. 128;
+// 127 at N 256, the tensor core's own rate); the same loop under `if (lane == 0)` needs ~147 whatever the shape, because the compiler
+// then cannot tell that one thread is active and brings the descriptors into uniform registers the slow way.  Several issuers still
+// help below N = 128: two reach 48 clocks at N 64, four 39 at N 16.
 #include "common.cuh"
 
 namespace dl4j {
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(128, 1) mma_issue_probe_kernel(long long* out,
   tc_fence_after();
   const uint32_t tmem = *slot;
   const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0 && w < issuers) {
+  if (w < issuers && elect_one()) {
     const uint32_t idesc = make_idesc(1, mn_major, mn_major, M, N);
     const uint64_t da = make_smem_desc_sw128(smem_u32(a_s), mn_major ? 16384 : 16, 1024);
     const uint64_t db = make_smem_desc_sw128(smem_u32(b_s), mn_major ? 16384 : 16, 1024);
