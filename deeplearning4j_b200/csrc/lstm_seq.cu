@@ -48,6 +48,11 @@ struct LstmSeqParams {
   long long* trace;          // optional [T][32] clock64 stamps written by the middle CTA (null = off); see dl4j_lstm_set_trace
 };
 
+// A step's h (dz) is handed from one CTA to the others as: stores -> epilogue barrier -> release increment of the counter by one thread ->
+// acquire load by the reader's producer thread -> fence.proxy.async there -> TMA loads.  One proxy fence on that path, behind the
+// acquire, orders the generic-proxy stores before the async-proxy reads; a second one on the writer's side (every epilogue thread waited
+// there for its own stores before the release did so again) cost 0.6 us of each step: batch 64, n 1024: 6.16 -> 5.59 us forward,
+// 7.53 -> 6.92 us backward.
 // Named barrier over the four epilogue warps (barrier 0 is __syncthreads).
 __device__ __forceinline__ void epilogue_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
@@ -281,8 +286,7 @@ lstm_seq_fwd_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_con
         hd[1] = pack8(h + 8);
       }
       if (threadIdx.x == 32 * LS_EPI_WARP0) ls_stamp(p.trace, s, 21);
-      fence_proxy_async_all();
-      epilogue_bar_sync();                         // every epilogue thread's stores precede the barrier; the one fence below is cumulative
+      epilogue_bar_sync();                         // every epilogue thread's stores precede the barrier; the release below is cumulative
       if (threadIdx.x == 32 * LS_EPI_WARP0) {
         ls_stamp(p.trace, s, 22);
         red_release_add(p.counter);                // one arrive per CTA; the release orders every epilogue thread's stores
@@ -531,7 +535,6 @@ lstm_seq_bwd_kernel(const __grid_constant__ CUtensorMap tmap_dz, const __grid_co
         gd = reinterpret_cast<uint4*>(drow + 3L * p.n);      gd[0] = pack8(gg); gd[1] = pack8(gg + 8);
       }
       if (threadIdx.x == 32 * LS_EPI_WARP0 && r >= 0) ls_stamp(p.trace, r, 21);
-      fence_proxy_async_all();
       epilogue_bar_sync();
       if (threadIdx.x == 32 * LS_EPI_WARP0) {
         if (r >= 0) ls_stamp(p.trace, r, 22);
@@ -876,7 +879,6 @@ lstm_seq_bwd_cluster_kernel(const __grid_constant__ CUtensorMap tmap_dz, const _
         gd = reinterpret_cast<uint4*>(drow + 3L * p.n);      gd[0] = pack8(gg); gd[1] = pack8(gg + 8);
       }
       if (threadIdx.x == 32 * LS_EPI_WARP0 && r >= 0) ls_stamp(p.trace, r, 21);
-      fence_proxy_async_all();
       epilogue_bar_sync();
       if (threadIdx.x == 32 * LS_EPI_WARP0) {
         if (r >= 0) ls_stamp(p.trace, r, 22);

@@ -1067,7 +1067,6 @@ class _LstmSeqFn(torch.autograd.Function):
     cell-gradient kernel plus one small GEMM per step and finishes with a single large weight-gradient GEMM.
     Gate order and math: libnd4j ops/declarable/helpers/impl/lstmLayer.cpp, LSTMHelpers.java."""
 
-    _scratch = {}
     PERSISTENT_BACKWARD = True       # False: per-step cell-gradient kernel + GEMM (kept as the cross-check path)
 
     @staticmethod
@@ -1083,9 +1082,7 @@ class _LstmSeqFn(torch.autograd.Function):
         h_all[0].copy_(h0)
         cs = torch.empty((T, mb, n), dtype=torch.float32, device=dev)
         gates = torch.empty((T, mb, n4), dtype=torch.bfloat16, device=dev)
-        counter = _LstmSeqFn._scratch.get(dev)
-        if counter is None:
-            counter = _LstmSeqFn._scratch[dev] = torch.zeros(64, dtype=torch.int32, device=dev)
+        counter = torch.empty(1, dtype=torch.int32, device=dev)       # of this launch alone: two streams may run the kernel at once
         c0 = c0.contiguous()
         rc = l.dl4j_lstm_seq_fwd(_ptr(zx), _ptr(rw_t), _ptr(h_all), _ptr(c0), _ptr(cs), _ptr(gates), T, mb, n, int(bool(reverse)),
                                  _ptr(counter), _stream())
@@ -1118,7 +1115,7 @@ class _LstmSeqFn(torch.autograd.Function):
             need_h0, need_c0 = ctx.needs_input_grad[2], ctx.needs_input_grad[3]
             dh0 = torch.empty((mb, n), dtype=torch.bfloat16, device=cs.device) if need_h0 else None
             dc0 = torch.empty_like(c0) if need_c0 else None
-            counter = _LstmSeqFn._scratch[cs.device]
+            counter = torch.empty(1, dtype=torch.int32, device=cs.device)
             rc = l.dl4j_lstm_seq_bwd(_ptr(dout), _ptr(gates), _ptr(cs), _ptr(c0), _ptr(rwt), _ptr(dzx), _ptr(dc), _ptr(dh0), _ptr(dc0),
                                      T, mb, n, int(rev), _ptr(counter), stream)
             _check(rc, "dl4j_lstm_seq_bwd")

@@ -86,3 +86,25 @@ def test_one_step_matches_fp64(n, mb, n_in, bf16_params):
     a = net.rnnTimeStep(x[0]).t
     net.rnnClearPreviousState()
     assert torch.equal(a, net.rnnTimeStep(torch.zeros_like(x[0])).t)
+
+
+@pytest.mark.parametrize("n,mb", [(64, 5), (256, 128), (1024, 64)])
+def test_sequence_kernels_repeat_bit_for_bit(n, mb):
+    """h and dz pass from one block to the others through memory at every step: a reader that came too early would change the bits."""
+    from deeplearning4j_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(1)
+    T = 40
+    zx = (torch.randn(T, mb, 4 * n, generator=g, device="cuda") * 0.5).bfloat16()
+    rw = torch.randn(n, 4 * n, generator=g, device="cuda") * n ** -0.5
+    h0, c0 = torch.zeros(mb, n, device="cuda", dtype=torch.bfloat16), torch.zeros(mb, n, device="cuda")
+
+    def run():
+        z = zx.clone().requires_grad_(True)
+        out = native.lstm_seq(z, rw, h0, c0)[0]
+        out.float().square().sum().backward()
+        return out.detach(), z.grad
+    want = run()
+    for _ in range(20):
+        got = run()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    native.check_status()
