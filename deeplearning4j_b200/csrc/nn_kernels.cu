@@ -739,7 +739,7 @@ bias_act_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __rest
   }
 }
 
-// Vector form for C % 8 == 0: a thread owns 8 adjacent columns (one 16-byte load per row), eight threads span a 64-column
+// Vector form for C % 8 == 0 and 16-byte aligned buffers: a thread owns 8 adjacent columns (one 16-byte load per row), eight threads span a 64-column
 // tile (128 contiguous bytes per row) and the block's 32 row lanes walk a row slab with two independent row loads in
 // flight per thread; many small blocks keep enough warps resident to hide the load latency; one atomicAdd per column and block.
 template <typename T>
@@ -1072,7 +1072,9 @@ DL4J_API int dl4j_bias_act_bwd(const void* dy, const void* z, void* dz, float* d
                                void* stream) {
   if (rows <= 0 || C <= 0) return 0;
   if (dy == nullptr || (act != 0 && z == nullptr)) return -DL4J_ERR_BAD_ARG;
-  if (C % 8 == 0) {
+  // a contiguous gradient may start anywhere: a one-row slice of a concatenation's gradient lies at the columns before it
+  const bool aligned = (((uintptr_t)dy | (uintptr_t)(act != 0 ? z : nullptr) | (uintptr_t)dz) & 15) == 0;
+  if (C % 8 == 0 && aligned) {
     const int ct = (C + 255) / 256;
     int slabs = (148 * dl4j_launch_grid("BIAS_ACT_BWD", 6) + ct - 1) / ct;      // default: about two rounds of resident blocks (3 per SM)
     if (slabs < 1) slabs = 1;

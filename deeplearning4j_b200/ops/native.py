@@ -438,8 +438,7 @@ class _MlpFn(torch.autograd.Function):
         x, W1_lp, W2_lp, z1, y1 = ctx.saved_tensors
         W1, b1, W2, b2 = ctx.refs
         l = require()
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
+        dy2 = _dense16(dy2)
         M, N2 = dy2.shape
         N1 = z1.shape[1]
         need = ctx.needs_input_grad
@@ -525,8 +524,7 @@ class _LinearFn(torch.autograd.Function):
         x, W_lp, saved = ctx.saved_tensors
         act = ctx.act
         l = require()
-        if not dy.is_contiguous():
-            dy = dy.contiguous()
+        dy = _dense16(dy)
         M, N = dy.shape
         W, b = ctx.W_ref, ctx.b_ref
         # ---- dz and bias gradient
@@ -776,7 +774,7 @@ class _Linear32Fn(torch.autograd.Function):
             return (dz @ W.t() if need[0] else None, x.t() @ dz if need[1] else None,
                     dz.sum(0).reshape(b.shape) if b is not None and need[2] else None, None)
         l = require()
-        dy = dy.contiguous()
+        dy = _dense16(dy)
         M, N = dy.shape
         Wl, bl = ctx.refs
         db = acc = None
@@ -825,9 +823,12 @@ _LN_ONE_PASS = os.environ.get("DL4J_LN_BWD_ONEPASS", "0") == "1"
 
 
 def _dense16(t):
-    """Contiguous and on a 16-byte boundary (the vector kernels' requirement): a view off the grid is copied."""
+    """Contiguous, with the strides of its shape and on a 16-byte boundary (the vector kernels' requirement): a view off the grid is
+    copied.  An extent of one leaves its stride open, and a slice keeps the pitch it was cut from there."""
     t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
+    if t.data_ptr() % 16:
+        return t.clone(memory_format=torch.contiguous_format)
+    return t.view(-1).view(t.shape) if 1 in t.shape else t
 
 
 class _LayerNormFn(torch.autograd.Function):
