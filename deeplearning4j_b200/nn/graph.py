@@ -33,6 +33,9 @@ class _Folded:
     def __contains__(self, n): return n in self.where
     def __iter__(self): return iter(self.where)
 
+    def without(self, n):
+        return _Folded(self.w, self.b, {k: v for k, v in self.where.items() if k != n})
+
     def __getitem__(self, n):
         o, O, K, ob = self.where[n]
         return self.w[o:o + O * K].view(O, K), self.b[ob:ob + O]
@@ -282,6 +285,12 @@ class ComputationGraph(BaseNetwork):
         native.bn_fold(t["rows"], t["blocks"], self.flat_params, w, b)
         return _Folded(w, b, t["where"])
 
+    def _fold_takes(self, n, x):
+        """Whether the folded kernels read ``x`` as convolution ``n`` wants it: they take the channel count from the activation.  Anything
+        else goes through the layers, which convert it or refuse it."""
+        c = self._fold_specs()[n][2]
+        return x.dim() == 4 and x.shape[1] == c.nIn and x.dtype == torch.bfloat16 and x.device == self.flat_params.device and x.numel() > 0
+
     # ------------------------------------------------------------------ inference: a run of folded convolutions as one native call
     def _compile_run(self, idx, acts, folded, folded_bn, fuse):
         """Plans the vertices from ``order[idx]`` on that are folded convolutions, their batch norms, ReLUs and residual adds: the steps
@@ -410,7 +419,7 @@ class ComputationGraph(BaseNetwork):
         of the activations it starts from; the eight most recent are kept."""
         from ..ops import native
         plans = self.__dict__.setdefault("_run_plans", {})
-        key = (idx, self._fold_table["sig"]) + tuple((n, tuple(t.shape)) for n, t in acts.items() if t.dim() == 4 and _dense_nhwc(t))
+        key = (idx, len(folded_bn), self._fold_table["sig"]) + tuple((n, tuple(t.shape)) for n, t in acts.items() if t.dim() == 4 and _dense_nhwc(t))
         plan = plans.get(key)
         if plan is None:
             while len(plans) >= 8:
@@ -435,7 +444,9 @@ class ComputationGraph(BaseNetwork):
         if kind == "1x1":
             if tuple(c.stride) != (1, 1):
                 x = native._SubsampleFn.apply(x, int(c.stride[0]), int(c.stride[1]))
-            x = native._dense16(native._dense_cl(x)) if x.data_ptr() % 16 else native._dense_cl(x)
+            x = native._dense_cl(x)
+            if x.data_ptr() % 16:
+                x = x.clone()                    # keeps channels-last
             if residual is not None:
                 residual = native._dense_cl(residual)
                 if residual.shape != (x.shape[0], c.nOut, x.shape[2], x.shape[3]) or residual.dtype != x.dtype or residual.data_ptr() % 16:
@@ -479,6 +490,9 @@ class ComputationGraph(BaseNetwork):
         for idx, n in enumerate(self.order):
             if n in done:
                 continue
+            if n in folded and not self._fold_takes(n, acts[conf.vertexInputs[n][0]]):
+                folded = folded.without(n)
+                del folded_bn[self._fold_specs()[n][0]]
             if n in folded and self._fold_specs()[n][1] != "stem" and not done:
                 done = self._folded_run(idx, acts, folded, folded_bn, fuse)
                 if n in done:

@@ -77,3 +77,20 @@ def test_folded_output_matches_fp32(layers, opts, cin, hw, n):
     cpu.setParams(cpu.params().t * 0.5)
     want = cpu.output(x)[0].t
     assert (gpu.output(x.cuda())[0].t.cpu() - want).norm() <= 2 ** -8 * (2 * len(layers)) ** 0.5 * want.norm() * 2
+
+
+@pytest.mark.parametrize("k,residual", [(1, True), (3, True), (1, False)])
+def test_inputs_the_folded_kernels_do_not_read(k, residual):
+    """Another channel count is refused as by the layers; a view off the 16-byte grid gives what its copy gives."""
+    gpu, _ = _net(16, 9, 16, [(k, 1, 16), (1, 1, 16)], residual=residual)
+    x = torch.randn(2, 16, 9, 12, device="cuda")
+    want = gpu.output(x)[0].t
+    for c in (8, 24, 64):
+        with pytest.raises(Exception):
+            gpu.output(torch.randn(2, c, 9, 12, device="cuda"))
+    for cl in (False, True):
+        xb = x.bfloat16().contiguous(memory_format=torch.channels_last if cl else torch.contiguous_format)
+        off = torch.empty(xb.numel() + 1, dtype=xb.dtype, device="cuda")[1:].as_strided(xb.shape, xb.stride())
+        off.copy_(xb)
+        assert off.data_ptr() % 16
+        assert torch.equal(gpu.output(off)[0].t, want)
