@@ -166,7 +166,7 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
         for (int j = 0; j < 8; ++j) {
           f[j] = fmaf(f[j], sc[j], sh[j]);
           if (RES) f[j] += r[j];
-          if (relu) f[j] = fmaxf(f[j], 0.f);
+          if (relu) f[j] = relu_f(f[j]);
         }
         reinterpret_cast<uint4*>(y)[gg] = bn_pack8(f);
       }
@@ -302,7 +302,7 @@ add_relu_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __rest
     bn_unpack8(__ldg(reinterpret_cast<const uint4*>(a) + g), fa);
     bn_unpack8(__ldg(reinterpret_cast<const uint4*>(b) + g), fb);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) fa[j] = fmaxf(fa[j] + fb[j], 0.f);
+    for (int j = 0; j < 8; ++j) fa[j] = relu_f(fa[j] + fb[j]);
     reinterpret_cast<uint4*>(y)[g] = bn_pack8(fa);
   }
 }

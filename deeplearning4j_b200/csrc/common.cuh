@@ -50,6 +50,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// ReLU as the library has it: NaN passes (fmaxf returns its other operand), infinities and signs as fmaxf.
+__device__ __forceinline__ float relu_f(float v) {
+  float y;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(v));
+  return y;
+}
+
 // One thread of a converged warp.  Code that issues tcgen05.mma sits under this and not under `lane == 0`: the compiler knows that a
 // single thread is active after elect.sync and keeps the instruction's descriptors in uniform registers; after a plain comparison it
 // does not, and one thread gets an instruction out per ~147 clocks instead of ~64 (mma_issue_probe.cu).  512 x 512 x 2048 GEMM:

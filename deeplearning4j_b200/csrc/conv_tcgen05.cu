@@ -249,7 +249,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation 
           }
           if (p.act == 1) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+            for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -555,7 +555,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation {
           }
           if (p.act == 1) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+            for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {

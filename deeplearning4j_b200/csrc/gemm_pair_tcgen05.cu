@@ -113,7 +113,7 @@ __device__ __forceinline__ void umma2_commit(uint32_t bar) {
 
 __device__ __forceinline__ float apply_act(float v, int act) {
   switch (act) {
-    case 1: return fmaxf(v, 0.0f);
+    case 1: return relu_f(v);
     case 2: return gelu_erf(v);
     case 3: return gelu_tanh(v);
     case 4: return sigmoidf_(v);
@@ -127,7 +127,7 @@ __device__ __forceinline__ float apply_act(float v, int act) {
 __device__ __forceinline__ void apply_act32(float (&v)[32], int act) {
   if (act == 1) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+    for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
   } else if (act == 2) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);

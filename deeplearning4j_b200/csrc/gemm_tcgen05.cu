@@ -75,7 +75,7 @@ struct GemmSmem {
 
 __device__ __forceinline__ float apply_act(float v, int act) {
   switch (act) {
-    case 1: return fmaxf(v, 0.0f);
+    case 1: return relu_f(v);
     case 2: return gelu_erf(v);
     case 3: return gelu_tanh(v);
     case 4: return sigmoidf_(v);
@@ -112,7 +112,7 @@ __device__ __forceinline__ float mul_act_grad(float v, float z, int act) {
 __device__ __forceinline__ void apply_act32(float (&v)[32], int act) {
   if (act == 1) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+    for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
   } else if (act == 2) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
@@ -419,7 +419,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             }
             if (p.relu_last) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+              for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
             }
             if (p.out_fp32) {
 #pragma unroll
@@ -517,7 +517,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
           if (p.relu_last) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+            for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
           }
           if (p.out_fp32) {
             float* o = reinterpret_cast<float*>(p.C) + c_off + (long)row * p.ldc + col0;

@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(SG_THREADS, 2) sgemm_small_kernel(const SgemmP
       v = mine[idx];
     }
     if (p.bias) v += __ldg(p.bias + n);
-    if (p.act == 1) v = v > 0.f ? v : (v != v ? v : 0.f);       // NaN passes, as in the library's ReLU
+    if (p.act == 1) v = relu_f(v);
     p.C[m * p.ldc + n] = v;
   }
   if (splits > 1) cg::this_cluster().sync();                    // nobody leaves while its tile is being read

@@ -94,3 +94,45 @@ def test_inputs_the_folded_kernels_do_not_read(k, residual):
         off.copy_(xb)
         assert off.data_ptr() % 16
         assert torch.equal(gpu.output(off)[0].t, want)
+
+
+@pytest.mark.parametrize("layers,opts", [
+    ([(1, 1, 16), (1, 1, 16)], {}), ([(3, 1, 16), (3, 1, 16)], {}), ([(3, 1, 16), (3, 1, 16)], {"residual": False}),
+    ([(7, 2, 16), (1, 2, 40), (5, 1, 8)], {"residual": False}), ([(3, 1, 16), (3, 1, 12), (1, 1, 16)], {}),
+])
+@pytest.mark.parametrize("cin", [3, 16])
+def test_nan_reaches_the_output(layers, opts, cin):
+    """A NaN in one image makes that image's probabilities NaN and no others, as the layers give it."""
+    gpu, cpu = _net(cin, 9, 16, layers, **opts)
+    x = torch.randn(3, cin, 9, 12)
+    x[1, 0, 4, 4] = float("nan")
+    got, want = gpu.output(x.cuda())[0].t.cpu(), cpu.output(x)[0].t
+    assert torch.isnan(want[1]).all() and torch.isfinite(want[[0, 2]]).all()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+
+
+def test_epilogue_relu_passes_nan_and_infinities():
+    from deeplearning4j_b200.ops import native
+    special = torch.tensor([float("nan"), float("inf"), float("-inf"), -0.0, 0.0, -1.0, 2.0, 3e-39], device="cuda")
+    a = torch.zeros(40, 64, device="cuda", dtype=torch.bfloat16)
+    w = torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16)
+    z = special.repeat(8)
+    want = torch.relu(z).bfloat16()
+
+    def same(y):
+        assert torch.equal(torch.isnan(y), torch.isnan(want.expand_as(y))) and torch.equal(y.nan_to_num(7.0), want.expand_as(y).nan_to_num(7.0))
+    same(native.gemm_raw(a, w, bias=z, act=1))
+    same(native.gemm_raw(a, w, bias=z, act=1, out_dtype=torch.float32).bfloat16())
+    same(native.gemm_raw(a[:, :24], w[:24], bias=z, act=1, block_n=128))
+    x = torch.zeros(1, 64, 5, 8, device="cuda", dtype=torch.bfloat16).contiguous(memory_format=torch.channels_last)
+    same(native.conv_infer_1x1(x, w, z, True).permute(0, 2, 3, 1).reshape(-1, 64))
+    res = want.new_zeros(1, 64, 5, 8).contiguous(memory_format=torch.channels_last)
+    same(native.conv_infer_1x1(x, w, z, True, res).permute(0, 2, 3, 1).reshape(-1, 64))
+    for k in (3, 5):
+        y = native.conv_infer_kxk(x, torch.zeros(64, k * k * 64, device="cuda", dtype=torch.bfloat16), z, k, k, (k // 2,) * 2, (1, 1), True)
+        same(y.permute(0, 2, 3, 1).reshape(-1, 64))
+    zz = z.bfloat16().reshape(1, 64, 1, 1).expand(1, 64, 5, 8).contiguous(memory_format=torch.channels_last)
+    one, zero = torch.ones(64, device="cuda"), torch.zeros(64, device="cuda")
+    same(native.bn_act_eval(zz, None, one, zero, True).permute(0, 2, 3, 1).reshape(-1, 64))
+    same(native.bn_act_eval(zz, res, one, zero, True).permute(0, 2, 3, 1).reshape(-1, 64))
+    same(native.add_relu(zz, res).permute(0, 2, 3, 1).reshape(-1, 64))
