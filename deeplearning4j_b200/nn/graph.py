@@ -444,9 +444,7 @@ class ComputationGraph(BaseNetwork):
         if kind == "1x1":
             if tuple(c.stride) != (1, 1):
                 x = native._SubsampleFn.apply(x, int(c.stride[0]), int(c.stride[1]))
-            x = native._dense_cl(x)
-            if x.data_ptr() % 16:
-                x = x.clone()                    # keeps channels-last
+            x = native._dense_cl16(x)
             if residual is not None:
                 residual = native._dense_cl(residual)
                 if residual.shape != (x.shape[0], c.nOut, x.shape[2], x.shape[3]) or residual.dtype != x.dtype or residual.data_ptr() % 16:
@@ -458,11 +456,11 @@ class ComputationGraph(BaseNetwork):
         if kind == "stem":
             y = _stem_space_to_depth(x, w.view(c.nOut, kH, kW, c.nIn).permute(0, 3, 1, 2), b, (kH, kW), tuple(pad), relu=act)
         else:
-            x = native._dense_cl(x)
+            x = native._dense_cl16(x)
             d = tuple(c.dilation)
             if min(x.shape[2] + 2 * pad[0] - (kH - 1) * d[0], x.shape[3] + 2 * pad[1] - (kW - 1) * d[1]) < 1:
                 raise ValueError(f"convolution '{n}': kernel {kH}x{kW} does not fit the padded {x.shape[2]}x{x.shape[3]} input")
-            y = native.conv_infer_kxk(x if x.data_ptr() % 16 == 0 else x.clone(), w, b, kH, kW, pad, d, act)
+            y = native.conv_infer_kxk(x, w, b, kH, kW, pad, d, act)
         if residual is not None:
             z = native.add_relu(y, residual) if relu else None
             y = z if z is not None else (torch.relu(y + residual) if relu else y + residual)

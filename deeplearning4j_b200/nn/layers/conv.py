@@ -842,6 +842,10 @@ class BatchNormalization(FeedForwardLayer):
         ``pre_bias`` is the bias of the convolution that produced ``x`` when the executor left it out of ``x``: batch
         statistics cancel it in training (its gradient is exactly zero), so it only enters the running mean and the
         inference-time shift."""
+        if residual is not None and (residual.shape != x.shape or residual.dtype != x.dtype or residual.device != x.device):
+            # the add broadcasts or converts: the kernels read the residual element by element like x
+            y = self.forward(p, x, training, mask, ctx, pre_bias=pre_bias) + residual
+            return torch.relu(y) if fuse_relu else y
         n = self.nOut or self.nIn
         nhwc = x.dim() == 4 and self.cnn2DFormat == CNN2DFormat.NHWC
         if nhwc:

@@ -1634,6 +1634,12 @@ def _dense_cl(x):
     return x.contiguous()
 
 
+def _dense_cl16(x):
+    """``_dense_cl`` on a 16-byte boundary: a view off the grid is copied."""
+    x = _dense_cl(x)
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 class _BnActFn(torch.autograd.Function):
     """y = act(batchnorm_train(x) [+ res]) over channels-last bf16 activations; running statistics are updated in place by
     the kernel (``nn/layers/normalization/BatchNormalization.java`` semantics: biased batch variance, decay rule)."""
@@ -1641,8 +1647,8 @@ class _BnActFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, res, gamma, beta, run_mean, run_stat, use_log_std, decay, eps, relu, pre_bias=None):
         l = require()
-        x = _dense_cl(x)
-        res = _dense_cl(res) if res is not None else None
+        x = _dense_cl16(x)
+        res = _dense_cl16(res) if res is not None else None
         rows, C = _rows_c(x)
         y = torch.empty_like(x)
         save = torch.empty(2 * C, dtype=torch.float32, device=x.device)
@@ -1665,7 +1671,7 @@ class _BnActFn(torch.autograd.Function):
         l = require()
         x, y, save, work = ctx.saved_tensors
         rows, C = _rows_c(x)
-        dy = _dense_cl(dy)
+        dy = _dense_cl16(dy)
         dx = torch.empty_like(x)
         dres = torch.empty_like(x) if ctx.has_res else None
         # the kernel adds dgamma / dbeta to what its targets hold: the parameters' preallocated fp32 gradients when they have
@@ -1710,8 +1716,8 @@ def bn_act_train(x, res, gamma, beta, run_mean, run_stat, use_log_std, decay, ep
 def bn_act_eval(x, res, scale, shift, relu):
     """y = act(x * scale + shift [+ res]) with fp32 per-channel scale / shift (inference statistics folded in)."""
     l = require()
-    x = _dense_cl(x)
-    res = _dense_cl(res) if res is not None else None
+    x = _dense_cl16(x)
+    res = _dense_cl16(res) if res is not None else None
     rows, C = _rows_c(x)
     y = torch.empty_like(x)
     rc = l.dl4j_bn_apply(_ptr(x), _ptr(res), _ptr(scale.float().contiguous()), _ptr(shift.float().contiguous()), int(bool(relu)), _ptr(y),
@@ -1724,8 +1730,8 @@ class _AddReluFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, a, b):
         l = require()
-        a = _dense_cl(a)
-        b = _dense_cl(b)
+        a = _dense_cl16(a)
+        b = _dense_cl16(b)
         if b.stride() != a.stride():
             b = b.contiguous(memory_format=torch.channels_last) if a.dim() == 4 else b.contiguous()
         y = torch.empty_like(a)
@@ -1742,7 +1748,7 @@ class _AddReluFn(torch.autograd.Function):
 
 
 def add_relu(a, b):
-    if not (available() and a.is_cuda and a.dtype == torch.bfloat16 and a.shape == b.shape and a.numel() % 8 == 0 and a.dim() in (2, 4)):
+    if not (available() and a.is_cuda and a.dtype == b.dtype == torch.bfloat16 and a.device == b.device and a.shape == b.shape and a.numel() % 8 == 0 and a.dim() in (2, 4)):
         return None
     return _AddReluFn.apply(a, b)
 

@@ -136,3 +136,38 @@ def test_epilogue_relu_passes_nan_and_infinities():
     same(native.bn_act_eval(zz, None, one, zero, True).permute(0, 2, 3, 1).reshape(-1, 64))
     same(native.bn_act_eval(zz, res, one, zero, True).permute(0, 2, 3, 1).reshape(-1, 64))
     same(native.add_relu(zz, res).permute(0, 2, 3, 1).reshape(-1, 64))
+
+
+@pytest.mark.parametrize("act", ["IDENTITY", "TANH"])
+@pytest.mark.parametrize("shape", [(1, 1), (9, 12)])
+def test_residual_that_broadcasts(act, shape):
+    """Add after a batch norm with a [N, C, 1, 1] input, in a folded (identity) and an unfolded convolution; output and gradients."""
+    from deeplearning4j_b200 import DataType, nn
+    from deeplearning4j_b200.nn.conf.base import InputType, PoolingType
+    from deeplearning4j_b200.nn.conf.graphconf import ElementWiseVertex
+    from deeplearning4j_b200.nn.graph import ComputationGraph
+    from deeplearning4j_b200.nn.layers.conv import BatchNormalization, ConvolutionLayer, GlobalPoolingLayer
+    from deeplearning4j_b200.nn.layers.core import ActivationLayer, OutputLayer
+
+    def build(compute):
+        b = nn.NeuralNetConfiguration.Builder().seed(3)
+        gb = (b.computeDataType(DataType.BFLOAT16) if compute else b).graphBuilder()
+        gb.addInputs("in", "in2").setInputTypes(InputType.convolutional(9, 12, 16), InputType.convolutional(*shape, 16))
+        gb.addLayer("c", ConvolutionLayer([1, 1], [1, 1], nOut=16, activation=act), "in").addLayer("n", BatchNormalization(), "c")
+        gb.addVertex("add", ElementWiseVertex("Add"), "n", "in2").addLayer("r", ActivationLayer("RELU"), "add")
+        gb.addLayer("p", GlobalPoolingLayer(PoolingType.AVG), "r").addLayer("out", OutputLayer("MCXENT", nOut=5, activation="SOFTMAX"), "p")
+        return ComputationGraph(gb.setOutputs("out").build())
+    gpu, cpu = build(True), build(False)
+    gpu.device = torch.device("cuda")
+    gpu.init(), cpu.init()
+    gpu.setParams(cpu.params().t)
+    g = torch.Generator().manual_seed(2)
+    x, s, y = torch.randn(3, 16, 9, 12, generator=g), torch.randn(3, 16, *shape, generator=g), torch.eye(5)[:3]
+    want = cpu.output([x, s])[0].t
+    assert (gpu.output([x.cuda(), s.cuda()])[0].t.cpu() - want).norm() <= 2e-2 * want.norm()
+    off = torch.empty(s.numel() + 1, device="cuda", dtype=torch.bfloat16)[1:].view(s.shape)
+    off.copy_(s)
+    assert (gpu.output([x.cuda(), off])[0].t.cpu() - want).norm() <= 2e-2 * want.norm()
+    _, sg = gpu.computeGradientAndScore([x.cuda(), s.cuda()], y.cuda())
+    _, sc = cpu.computeGradientAndScore([x, s], y)
+    assert abs(sg - sc) <= 2e-2 * abs(sc)
