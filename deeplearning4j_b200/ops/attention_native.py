@@ -100,6 +100,8 @@ class _AttentionFn(torch.autograd.Function):
         l = native.require()
         if ctx.flash:
             q, k, v, O, lse, mk, seed = ctx.saved_tensors
+            if torch.is_grad_enabled() and seed is None:     # create_graph: the gradient has to be differentiable itself
+                return (*_grad_in_ops(q, k, v, dO, mk, ctx.scale, ctx.flags), None, None, None, None)
             dO = _prep(dO)
             dvec = torch.empty_like(lse)             # D_r = sum_d dO * O per query row, laid out like the log-sum-exp
             Bn, H, Tq, D = q.shape
@@ -147,6 +149,31 @@ class _AttentionFn(torch.autograd.Function):
         return dq_t.permute(0, 2, 1, 3), dk_t.permute(0, 2, 1, 3), dv_t.permute(0, 2, 1, 3), None, None, None, None
 
 
+def _grad_in_ops(q, k, v, dO, mask, scale, flags):
+    """(dq, dk, dv) in differentiable torch operators, for second derivatives; the fused kernels' rules for hidden keys and empty rows."""
+    s = torch.matmul(q, k.transpose(-1, -2)).float() * scale
+    hidden = None
+    if flags & 1:
+        hidden = torch.ones(s.shape[-2:], dtype=torch.bool, device=s.device).triu(1)
+    if mask is not None:
+        m = (mask == 0)[:, None, None, :]
+        hidden = m if hidden is None else hidden | m
+    if hidden is not None:
+        s = s.masked_fill(hidden, float("-inf"))
+        if not flags & 2:
+            s = s.masked_fill(hidden.expand(s.shape).all(-1, keepdim=True), 0.0)
+    p = torch.softmax(s, -1)
+    if hidden is not None and not flags & 2:
+        p = p.masked_fill(hidden, 0.0)
+    dv = torch.matmul(p.to(dO.dtype).transpose(-1, -2), dO)
+    dp = torch.matmul(dO, v.transpose(-1, -2)).float()
+    ds = p * (dp - (dp * p).sum(-1, keepdim=True)) * scale
+    if hidden is not None:
+        ds = ds.masked_fill(hidden, 0.0)
+    ds = ds.to(q.dtype)
+    return torch.matmul(ds, k), torch.matmul(ds.transpose(-1, -2), q), dv
+
+
 def _bad_mask(q, k, mask):
     return mask is not None and (mask.dim() != 2 or mask.shape[0] != q.shape[0] or mask.shape[1] != k.shape[2])
 
@@ -166,7 +193,7 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
     heads and the last key block); other head sizes and fp16 on batched GEMMs with a materialised score matrix."""
     if not native.available() or q.dim() != 4 or q.dtype not in (torch.bfloat16, torch.float16):
         return None
-    if _bad_mask(q, k, mask):
+    if _bad_mask(q, k, mask) or not native._plain_autograd():
         return None
     D, Tk, Tq = q.shape[3], k.shape[2], q.shape[2]
     scale = float(scale) if scale is not None else D ** -0.5
@@ -177,7 +204,8 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
         flags = (1 if causal else 0) | (0 if _empty_rows_are_zero(D, Tq, Tk) and not causal else 2)
         if dropout_p == 0.0 and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)):
             return flash_forward(q, k, v, mask, scale, flags=flags)[0].permute(0, 2, 1, 3)       # nothing to differentiate
-        return _AttentionFn.apply(q, k, v, mask, scale, float(dropout_p), flags)
+        # laid out here and not in forward(): second derivatives go through the saved operands
+        return _AttentionFn.apply(_prep(q), _prep(k), _prep(v), mask, scale, float(dropout_p), flags)
     if causal or D % 8 or Tk % 8 or Tq % 8 or Tk > 1024:
         return None
     return _AttentionFn.apply(q, k, v, mask, scale, float(dropout_p))
@@ -187,7 +215,7 @@ def attention_grad(q, k, v, mask, scale, dout, causal=False):
     """(dq, dk, dv) without materialising the output: the forward kernel hands the row sums of dO * O straight to the backward kernel.
     None when the fused kernels do not cover the case."""
     if not USE_FLASH or not native.available() or not flash_supported(q, k, v) or _bad_mask(q, k, mask) or dout.dim() != 4 \
-            or dout.device != q.device or dout.shape != (*q.shape[:3], v.shape[3]):
+            or not native._plain_autograd() or dout.device != q.device or dout.shape != (*q.shape[:3], v.shape[3]):
         return None
     q, k, v, dout = _prep(q.detach()), _prep(k.detach()), _prep(v.detach()), _prep(dout.detach().to(q.dtype))
     Bn, H, Tq, D = q.shape

@@ -913,7 +913,7 @@ def layer_norm_grad(x, gain, bias, dy, eps):
     for p in (gain, bias):
         if p is not None and (p.numel() != C or not p.is_floating_point() or p.dtype == torch.float64 or p.device != x.device):
             return None
-    if dy.numel() != x.numel() or dy.device != x.device:
+    if dy.numel() != x.numel() or dy.device != x.device or not _plain_autograd():
         return None
     l = _LIB
     x2 = x if x.is_contiguous() else x.contiguous()
@@ -1203,7 +1203,7 @@ def _f_ordered(w):
 def lstm_step_supported(x, W, RW, n, mb):
     """One inference step as one launch (``csrc/lstm_step.cu``) for mb * n up to LSTM_STEP_MAX."""
     return (available() and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled() and mb * n <= LSTM_STEP_MAX
-            and _f_ordered(W) and _f_ordered(RW) and W.dtype == RW.dtype)
+            and _f_ordered(W) and _f_ordered(RW) and W.dtype == RW.dtype and _plain_autograd())
 
 
 # Measured per call for two layers (whole rnnTimeStep, device / wall us; step kernel against sequence kernel): 256 x 1: 17.7 / 195 against
@@ -1239,7 +1239,8 @@ def lstm_step(x, W, RW, b, h, c):
 def linear_small(x, W, b):
     """``x @ W + b`` without a gradient for up to 32 rows of bf16 activations on the parameters themselves, or None when not covered."""
     if torch.is_grad_enabled() or not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.bfloat16 or not 1 <= x.shape[0] <= 32 \
-            or not _f_ordered(W) or W.shape[0] != x.shape[1] or W.numel() == 0 or (b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1])):
+            or not _f_ordered(W) or W.shape[0] != x.shape[1] or W.numel() == 0 or (b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1])) \
+            or not _plain_autograd():
         return None
     l = _small_sigs(require())
     x = x if x.stride(1) == 1 else x.contiguous()

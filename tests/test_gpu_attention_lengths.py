@@ -85,3 +85,39 @@ def test_three_dimensional_and_misaligned_inputs():
     assert out.shape == (3, 50, 24) and (out.double() - want).norm() <= 1e-2 * want.norm()
     dq, dv, dk = Nd4j.exec("dot_product_attention_v2_bp", q, v, k, torch.ones_like(q), scale=0.2)
     assert dq.t.shape == q.shape and dk.t.shape == k.shape and dv.t.shape == v.shape
+
+
+@pytest.mark.parametrize("T,masked,causal", [(201, True, False), (100, False, True), (1032, False, False), (104, False, False), (256, True, True)])
+def test_second_derivatives_forward_mode_and_vmap(T, masked, causal):
+    """What the calls gave through torch operators: a gradient penalty, a tangent, a mapped call."""
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    B, H, D, scale = 2, 2, 64, 0.125
+    q, k, v, do, g = _inputs(B, H, T, T, D, T)
+    mask = None
+    if masked:
+        mask = (torch.rand(B, T, generator=g, device="cuda") > 0.3).float()
+        mask[:, 0] = 1.0
+
+    def call(a, b, c):
+        from deeplearning4j_b200.ops.impl_nn import dot_product_attention_v2
+        return dot_product_attention_v2(a, c, b, vMask=mask, scale=scale, useCausalMask=causal)[0]
+    # second derivatives, of views that the kernels copy as well
+    for lay in (lambda t: t, lambda t: t.transpose(-1, -2).contiguous().transpose(-1, -2)):
+        ql, kl, vl = (lay(t.detach()).requires_grad_(True) for t in (q, k, v))
+        gq = torch.autograd.grad(call(ql, kl, vl), ql, do, create_graph=True)[0]
+        second = torch.autograd.grad((gq.float() ** 2).sum(), (ql, kl, vl))
+        q6, k6, v6 = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+        gq6 = torch.autograd.grad(_ref(q6, k6, v6, scale, mask, causal), q6, do.double(), create_graph=True)[0]
+        want = torch.autograd.grad((gq6 ** 2).sum(), (q6, k6, v6))
+        assert (gq.double() - gq6).norm() <= 1e-2 * gq6.norm()
+        for a, b in zip(second, want):
+            assert (a.double() - b).norm() <= 4e-2 * b.norm()
+    with torch.autograd.forward_ad.dual_level():
+        d = torch.autograd.forward_ad.make_dual(q, do)
+        t = torch.autograd.forward_ad.unpack_dual(call(d, k, v)).tangent
+    q6 = q.double()
+    want = torch.func.jvp(lambda a: _ref(a, k.double(), v.double(), scale, mask, causal), (q6,), (do.double(),))[1]
+    assert t is not None and (t.double() - want).norm() <= 3e-2 * want.norm()
+    if mask is None:
+        got = torch.func.vmap(lambda a: call(a, k, v))(torch.stack([q, q.flip(0)]))
+        assert (got[0].double() - _ref(q6, k.double(), v.double(), scale, None, causal)).norm() <= 1e-2 * got[0].double().norm()
