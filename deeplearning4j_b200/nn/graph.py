@@ -19,8 +19,8 @@ from .conf.graphconf import ElementWiseVertex
 from ..utils.crash import guard_fit
 
 
-def _dense_nhwc(t):
-    return t.dim() == 4 and t.dtype == torch.bfloat16 and t.is_cuda and t.numel() > 0 and t.is_contiguous(memory_format=torch.channels_last) \
+def _dense_nhwc(t, device):
+    return t.dim() == 4 and t.dtype == torch.bfloat16 and t.device == device and t.numel() > 0 and t.is_contiguous(memory_format=torch.channels_last) \
         and t.data_ptr() % 16 == 0
 
 
@@ -259,7 +259,8 @@ class ComputationGraph(BaseNetwork):
         from ..ops import native, nnops
         specs = self._fold_specs()
         if not specs or nnops._FORCE_TORCH or not x.is_cuda or x.dtype != torch.bfloat16 or not self.flat_params.is_cuda \
-                or self.flat_params.dtype != torch.float32 or not native.available():
+                or self.flat_params.dtype != torch.float32 or not native.available() \
+                or not native.on_current_device(x, self.flat_params):
             return ()
         sig = (self.flat_params.device,) + tuple((b.eps, b.useLogStd, b.lockGammaBeta, b.gamma, b.beta) for _, _, _, b in specs.values())
         t = getattr(self, "_fold_table", None)
@@ -306,7 +307,7 @@ class ComputationGraph(BaseNetwork):
             r = env.get(name)
             if r is None and name in acts:
                 t = acts[name]
-                if not _dense_nhwc(t):
+                if not _dense_nhwc(t, self.flat_params.device):
                     return None
                 if name not in ext:
                     ext.append(name)
@@ -419,7 +420,7 @@ class ComputationGraph(BaseNetwork):
         of the activations it starts from; the eight most recent are kept."""
         from ..ops import native
         plans = self.__dict__.setdefault("_run_plans", {})
-        key = (idx, len(folded_bn), self._fold_table["sig"]) + tuple((n, tuple(t.shape)) for n, t in acts.items() if t.dim() == 4 and _dense_nhwc(t))
+        key = (idx, len(folded_bn), self._fold_table["sig"]) + tuple((n, tuple(t.shape)) for n, t in acts.items() if _dense_nhwc(t, self.flat_params.device))
         plan = plans.get(key)
         if plan is None:
             while len(plans) >= 8:

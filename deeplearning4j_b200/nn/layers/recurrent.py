@@ -107,7 +107,7 @@ class LSTM(BaseRecurrentLayer):
         plain = isinstance(gate, ActivationSigmoid) and isinstance(act, ActivationTanH) and not self.PEEPHOLE
         if T == 1 and plain and mask is None and not training and x.is_cuda and not nnops._FORCE_TORCH:
             from ...ops import native as nat
-            if nat.lstm_step_supported(xt, W, RW, n, mb) and h.dtype == x.dtype and c.dtype == torch.float32 \
+            if nat.lstm_step_supported(xt, W, RW, n, mb, b, h, c) and h.dtype == x.dtype and c.dtype == torch.float32 \
                     and (b is None or b.dtype == torch.float32) and h.shape == c.shape == (mb, n):
                 h, c = nat.lstm_step(xt[0], W, RW, None if b is None else b.detach().reshape(-1), h, c)
                 self._store(ctx, key, (h, c))

@@ -193,7 +193,7 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
     heads and the last key block); other head sizes and fp16 on batched GEMMs with a materialised score matrix."""
     if not native.available() or q.dim() != 4 or q.dtype not in (torch.bfloat16, torch.float16):
         return None
-    if _bad_mask(q, k, mask) or not native._plain_autograd():
+    if _bad_mask(q, k, mask) or not native.on_current_device(q, k, v, mask) or not native._plain_autograd():
         return None
     D, Tk, Tq = q.shape[3], k.shape[2], q.shape[2]
     scale = float(scale) if scale is not None else D ** -0.5
@@ -215,7 +215,7 @@ def attention_grad(q, k, v, mask, scale, dout, causal=False):
     """(dq, dk, dv) without materialising the output: the forward kernel hands the row sums of dO * O straight to the backward kernel.
     None when the fused kernels do not cover the case."""
     if not USE_FLASH or not native.available() or not flash_supported(q, k, v) or _bad_mask(q, k, mask) or dout.dim() != 4 \
-            or not native._plain_autograd() or dout.device != q.device or dout.shape != (*q.shape[:3], v.shape[3]):
+            or not native.on_current_device(q, k, v, mask, dout) or not native._plain_autograd() or dout.shape != (*q.shape[:3], v.shape[3]):
         return None
     q, k, v, dout = _prep(q.detach()), _prep(k.detach()), _prep(v.detach()), _prep(dout.detach().to(q.dtype))
     Bn, H, Tq, D = q.shape

@@ -289,7 +289,7 @@ def _out_of_place_codec(x):
     if not (x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and 0 < x.numel() < 2 ** 31 - 1):
         return None
     from . import native
-    return native if native.available() else None
+    return native if native.available() and native.on_current_device(x) else None
 
 
 @op("encode_threshold", n_out=2, differentiable=False)

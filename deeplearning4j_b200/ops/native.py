@@ -134,6 +134,15 @@ def _stream():
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(dev))       # the raw handle: a Stream object costs 10 us a launch
 
 
+def on_current_device(*ts):
+    """Whether every given tensor (or None) lives on the current device, where ``_stream`` launches."""
+    dev = torch.cuda.current_device()
+    for t in ts:
+        if t is not None and t.get_device() != dev:          # -1: host memory
+            return False
+    return True
+
+
 def _check(rc, what):
     global LAUNCHES
     LAUNCHES += 1
@@ -701,7 +710,7 @@ class _OddLinearFn(torch.autograd.Function):
 
 def _linear_padded(x, W, b, act):
     """Layer widths that are not multiples of 8, see ``_OddLinearFn``; None when the case is not covered."""
-    if W.dim() != 2 or min(x.shape[0], W.shape[0], W.shape[1]) == 0 or W.dtype not in (x.dtype, torch.float32) or not W.is_cuda:
+    if W.dim() != 2 or min(x.shape[0], W.shape[0], W.shape[1]) == 0 or W.dtype not in (x.dtype, torch.float32) or not on_current_device(x, W, b):
         return None
     return _OddLinearFn.apply(x, W, b, act)
 
@@ -805,11 +814,11 @@ def linear32(x, W, b, relu):
     """fp32 dense layer on the small-problem kernel, or None when the case is not covered or the library does it better."""
     if not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.float32 or W.dtype != torch.float32 or W.dim() != 2 \
             or W.shape[0] != x.shape[1] or min(x.shape[0], *W.shape) == 0 or not _sgemm_wins(x.shape[0], W.shape[1]) \
-            or torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled() or not _unit(x) or not W.is_cuda:
+            or torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled() or not _unit(x) or not on_current_device(x, W, b):
         return None
     if not ((W.stride(0) == 1 and W.stride(1) >= W.shape[0]) or (W.stride(1) == 1 and W.stride(0) >= W.shape[1])):
         return None
-    if b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1] or not b.is_contiguous() or not b.is_cuda):
+    if b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1] or not b.is_contiguous()):
         return None
     if not _plain_autograd():
         return None
@@ -911,9 +920,9 @@ def layer_norm_grad(x, gain, bias, dy, eps):
         return None
     C = x.shape[-1]
     for p in (gain, bias):
-        if p is not None and (p.numel() != C or not p.is_floating_point() or p.dtype == torch.float64 or p.device != x.device):
+        if p is not None and (p.numel() != C or not p.is_floating_point() or p.dtype == torch.float64):
             return None
-    if dy.numel() != x.numel() or dy.device != x.device or not _plain_autograd():
+    if dy.numel() != x.numel() or not on_current_device(x, gain, bias, dy) or not _plain_autograd():
         return None
     l = _LIB
     x2 = x if x.is_contiguous() else x.contiguous()
@@ -1200,10 +1209,11 @@ def _f_ordered(w):
     return w.dim() == 2 and w.is_cuda and w.dtype in (torch.float32, torch.bfloat16) and w.stride(0) == 1 and w.stride(1) == w.shape[0]
 
 
-def lstm_step_supported(x, W, RW, n, mb):
-    """One inference step as one launch (``csrc/lstm_step.cu``) for mb * n up to LSTM_STEP_MAX."""
+def lstm_step_supported(x, W, RW, n, mb, *rest):
+    """One inference step as one launch (``csrc/lstm_step.cu``) for mb * n up to LSTM_STEP_MAX; ``rest``: its other operands."""
     return (available() and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled() and mb * n <= LSTM_STEP_MAX
-            and _f_ordered(W) and _f_ordered(RW) and W.dtype == RW.dtype and _plain_autograd())
+            and _f_ordered(W) and _f_ordered(RW) and W.dtype == RW.dtype and on_current_device(x, W, RW, *rest)
+            and _plain_autograd())
 
 
 # Measured per call for two layers (whole rnnTimeStep, device / wall us; step kernel against sequence kernel): 256 x 1: 17.7 / 195 against
@@ -1240,7 +1250,7 @@ def linear_small(x, W, b):
     """``x @ W + b`` without a gradient for up to 32 rows of bf16 activations on the parameters themselves, or None when not covered."""
     if torch.is_grad_enabled() or not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.bfloat16 or not 1 <= x.shape[0] <= 32 \
             or not _f_ordered(W) or W.shape[0] != x.shape[1] or W.numel() == 0 or (b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1])) \
-            or not _plain_autograd():
+            or not on_current_device(x, W, b) or not _plain_autograd():
         return None
     l = _small_sigs(require())
     x = x if x.stride(1) == 1 else x.contiguous()
@@ -1604,8 +1614,8 @@ def _avgpool_lib():
 
 def global_avgpool(x):
     """[N, C, H, W] 16-bit channels-last -> [N, C], or None when the case is not covered."""
-    if not available() or not x.is_cuda or x.dim() != 4 or x.dtype not in (torch.bfloat16, torch.float16) or x.numel() == 0 or x.shape[1] % 8 \
-            or x.shape[0] > 65535 or not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 or not _plain_autograd():
+    if not available() or x.dim() != 4 or x.dtype not in (torch.bfloat16, torch.float16) or x.numel() == 0 or x.shape[1] % 8 \
+            or not on_current_device(x) or x.shape[0] > 65535 or not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 or not _plain_autograd():
         return None
     return _GlobalAvgPoolFn.apply(x)
 
