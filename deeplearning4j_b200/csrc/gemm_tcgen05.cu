@@ -33,7 +33,8 @@ struct GemmParams {
   int bias_fp32;
   int out_fp32;           // C is float
   int act;                // 0 none, 1 relu, 2 gelu(erf), 3 gelu(tanh), 4 sigmoid, 5 tanh
-  int atomic_out;         // accumulate into fp32 C with vector reductions (split-K / grad accumulation)
+  int atomic_out;         // 1: accumulate into fp32 C with vector reductions (split-K / grad accumulation); 2: split s stores its
+                          // partial result in slab s of an fp32 [splits, M, ldc] buffer (staged epilogue only)
   int splits;             // split-K factor (>1 requires atomic_out)
   int fmt;                // 0 fp16, 1 bf16
   float alpha;
@@ -349,7 +350,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const uint32_t taddr_row = tmem_base + buf * BLOCK_N + ((uint32_t)(q * 32) << 16);
       if (p.tma_store) {
         // -------- staged epilogue: registers -> swizzled smem slab (32 rows x 128 B per warp) -> TMA store / reduce
-        const int b1 = batch % p.batch1, b2 = batch / p.batch1;
+        const int b1 = batch % p.batch1, b2 = p.atomic_out == 2 ? split : batch / p.batch1;
         uint8_t* ring = epi_smem + q * (2 * S::EPI_SLAB);
         const int sw = lane & 7;
         uint8_t* my_row0 = ring + lane * 128;
@@ -441,7 +442,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (r0 < p.M) {
               if (want_aux) tma_store_4d(&tmap_aux, ring, n0 + c, r0, b1, b2);
               uint8_t* src = ring + (want_aux ? S::EPI_SLAB : ring_idx * S::EPI_SLAB);
-              if (p.atomic_out) tma_reduce_add_4d(&tmap_c, src, n0 + c, r0, b1, b2);
+              if (p.atomic_out == 1) tma_reduce_add_4d(&tmap_c, src, n0 + c, r0, b1, b2);
               else tma_store_4d(&tmap_c, src, n0 + c, r0, b1, b2);
             }
             bulk_commit();
@@ -653,14 +654,16 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   p.tma_store = 0; p.tma_aux = 0;
   if (!(reinterpret_cast<uintptr_t>(C) & 15) && ((ldc * esz) % 16 == 0) && ((c_bs[0] * esz) % 16 == 0) && ((c_bs[1] * esz) % 16 == 0) &&
       (!aux || (!(reinterpret_cast<uintptr_t>(aux) & 15) && (ld_aux * 2) % 16 == 0))) {
-    r = encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * esz, out_fp32 ? 32 : 64, 32, nb1, nb2, c_bs[0] * esz,
-                  c_bs[1] * esz, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+    const bool slabs = atomic_out == 2;
+    r = encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * esz, out_fp32 ? 32 : 64, 32, nb1, slabs ? (uint64_t)splits : nb2,
+                  c_bs[0] * esz, slabs ? (uint64_t)M * ldc * esz : c_bs[1] * esz, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
     if (r == 0) p.tma_store = 1;
     if (r == 0 && aux) {
       r = encode_2d(&tx, aux, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux * 2, 64, 32, 1, 1, 0, 0);
       if (r == 0) p.tma_aux = 1; else p.tma_store = 0;
     }
   }
+  if (atomic_out == 2 && (!p.tma_store || batch1 != 1 || batch2 != 1)) return -DL4J_ERR_BAD_ARG;
   // bias on the tensor core: needs the bias in the operand format, 16-byte aligned, and alpha = 1 (the accumulator then
   // already holds A.B + bias); the epilogue's per-element broadcast of the bias competes with the MMA operand fetch for
   // the shared-memory path and costs a quarter of a short-K tile
@@ -703,6 +706,44 @@ DL4J_API int dl4j_gemm(const void* A, const void* B, void* C, void* aux, const v
   const long z[2] = {0, 0};
   return gemm_impl(A, B, C, aux, bias, residual, M, N, K, lda, ldb, ldc, ld_aux, ld_res, a_mn, b_mn, fmt, bias_fp32, out_fp32,
                    act, atomic_out, splits, alpha, block_n, num_sms, stream_, 1, 1, z, z, z);
+}
+
+// out[m, n] = sum over s of part[s][m][n] in order, rounded once.  Memory-bound, and what it reads has just been written: 7 slabs of
+// 2456 x 768 are 53 MB in L2.
+template <typename T>
+static __global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ part, T* __restrict__ out, int M, int N, long ldo, int splits) {
+  const long n4 = N / 4, total = (long)M * n4, slab = (long)M * N;
+  for (long g = blockIdx.x * 256L + threadIdx.x; g < total; g += (long)gridDim.x * 256) {
+    const long m = g / n4, n = (g - m * n4) * 4;
+    const float* s = part + m * N + n;
+    float4 a = __ldcs(reinterpret_cast<const float4*>(s));
+#pragma unroll 8
+    for (int i = 1; i < splits; ++i) {
+      const float4 b = __ldcs(reinterpret_cast<const float4*>(s + i * slab));
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    }
+    T* o = out + m * ldo + n;
+    o[0] = T(a.x); o[1] = T(a.y); o[2] = T(a.z); o[3] = T(a.w);
+  }
+}
+
+// C[M, N] (16-bit, row pitch ldc) = A B with the reduction split: each split stores its fp32 partial result, one kernel adds them in
+// order, so that the result does not depend on timing.  partial: [splits, M, N] fp32, 16-byte aligned, N a multiple of 4.
+DL4J_API int dl4j_gemm_split(const void* A, const void* B, float* partial, void* C, int M, int N, int K, long lda, long ldb, long ldc,
+                             int a_mn, int b_mn, int fmt, int splits, int num_sms, void* stream_) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (splits < 2 || N % 4 || (fmt != 0 && fmt != 1)) return -DL4J_ERR_BAD_ARG;
+  const long z[2] = {0, 0};
+  const int rc = gemm_impl(A, B, partial, nullptr, nullptr, nullptr, M, N, K, lda, ldb, N, 0, 0, a_mn, b_mn, fmt, 0, 1, 0, 2, splits, 1.0f, 256,
+                           num_sms, stream_, 1, 1, z, z, z);
+  if (rc) return rc;
+  const long blocks = ((long)M * (N / 4) + 255) / 256;
+  const int grid = (int)(blocks < 148 * 16 ? blocks : 148 * 16);
+  cudaStream_t st = (cudaStream_t)stream_;
+  if (fmt == 1) split_sum_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(partial, (__nv_bfloat16*)C, M, N, ldc, splits);
+  else split_sum_kernel<__half><<<grid, 256, 0, st>>>(partial, (__half*)C, M, N, ldc, splits);
+  return (int)cudaGetLastError();
 }
 
 // Batched form: batch index (b1, b2) with per-operand element strides {stride_b1, stride_b2} (multiples of 8 for A and B).

@@ -302,33 +302,57 @@ def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtyp
 
 
 def _long_k_splits(M, N, K):
-    """Split-K factor for a 16-bit-output GEMM with few output tiles and a long reduction (the data gradient of a vocabulary
-    projection: 2456 x 768 from K = 30522 is 60 tiles of 128 x 256 on 148 SMs).  The estimate: waves x k-blocks x 0.31 us (four MMAs
-    at one issue per ~147 clocks), against the passes a split adds over the fp32 partial result (zeroing, reductions, the cast).
-    2456 x 768 x 30522: 140 - 156 us unsplit (120 tiles of 128 x 128), 110 us split by 7, zeroing and cast included."""
+    """Split-K factor for a 16-bit-output GEMM with few output tiles and a long reduction (the data gradient of a wide output layer).
+    The estimate, fitted to the measurements below (us): a k-block of 64 takes 0.36 in a tile of 128 x 256 and 0.24 in one of
+    128 x 128, a product 11 and 7 besides; the partial results of a split cost 6 for a second launch and 2 per million of their
+    elements.  Measured unsplit / best split (factor): 128 x 768 x 30522 113 / 36 (16), 1000 x 768 x 30522 108 / 63 (6),
+    256 x 512 x 10001 68 / 26 (10), 1500 x 768 x 20000 82 / 56 (4), 2456 x 512 x 8192 39 / 38 (3), 2456 x 768 x 30522 113 / 110 (2),
+    1024 x 1024 x 4096 25 / 28 (3), 300 x 768 x 2048 16 / 20 (4).  A gain of less than a tenth is not worth the partial results."""
     sms, kb = num_sms(), (K + 63) // 64
-    tiles = ((M + 127) // 128) * ((N + 255) // 256)
+    rows, tiles = (M + 127) // 128, ((M + 127) // 128) * ((N + 255) // 256)
     if tiles >= sms or kb < 32:
         return 1
-    best, cost1 = 1, min((tiles + sms - 1) // sms, (((M + 127) // 128) * ((N + 127) // 128) + sms - 1) // sms) * kb * 0.31
-    best_cost = cost1
+    waves = lambda t: (t + sms - 1) // sms
+    best, best_cost = 1, 0.9 * min(7 + waves(rows * ((N + 127) // 128)) * kb * 0.24, 11 + kb * 0.36)
     for s in range(2, 17):
         if kb // s < 8:
             break
-        c = ((tiles * s + sms - 1) // sms) * ((kb + s - 1) // s) * 0.31 + M * N * (10 + 4 * s) / 5e6 + 6.0
+        c = 17 + waves(tiles * s) * ((kb + s - 1) // s) * 0.36 + s * M * N * 2e-6
         if c < best_cost:
             best, best_cost = s, c
     return best
 
 
 def _dgrad_gemm(a, b, out=None):
-    """``a @ b`` in a's type; a long reduction over few output tiles is split and summed in fp32 before the one rounding."""
+    """``a @ b`` in a's type; a long reduction over few output tiles is split and summed in fp32, in order, before the one rounding."""
     M, N = a.shape[0], b.shape[1]
     s = _long_k_splits(M, N, a.shape[1])
     if s == 1 or N % 4:
         return gemm_raw(a, b, out=out)
-    acc = gemm_raw(a, b, out_dtype=torch.float32, atomic=True, splits=s, block_n=256)
-    return acc.to(a.dtype) if out is None else out.copy_(acc)
+    return _split_gemm(a, b, s, out)
+
+
+def _split_gemm(a, b, s, out=None):
+    """``a @ b`` with the reduction in ``s`` parts, added in order: repeats bit for bit."""
+    l = require()
+    M, N = a.shape[0], b.shape[1]
+    if out is None:
+        out = torch.empty((M, N), dtype=a.dtype, device=a.device)
+    if not hasattr(l.dl4j_gemm_split, "_typed"):
+        vp, i32, lng = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
+        l.dl4j_gemm_split.argtypes = [vp, vp, vp, vp, i32, i32, i32, lng, lng, lng, i32, i32, i32, i32, i32, vp]
+        l.dl4j_gemm_split.restype = i32
+        l.dl4j_gemm_split._typed = True
+    oa, ob = _operand_a(a), _operand_b(b)
+    if oa is None or ob is None:
+        raise ValueError("operand layout not addressable by TMA (need unit stride in one dim, 16-byte alignment)")
+    part = torch.empty((s, M, N), dtype=torch.float32, device=a.device)
+    rc = l.dl4j_gemm_split(_ptr(oa[0]), _ptr(ob[0]), _ptr(part), _ptr(out), M, N, a.shape[1], oa[2], ob[2], out.stride(0), oa[1], ob[1],
+                           _DT[a.dtype], s, num_sms(), _stream())
+    global LAUNCHES
+    LAUNCHES += 1
+    _check(rc, "dl4j_gemm_split")
+    return out
 
 
 class _MatmulFn(torch.autograd.Function):

@@ -87,3 +87,26 @@ def test_cross_entropy_rows_with_infinities(C, sparse):
     grad = torch.autograd.grad(loss.sum(), z)[0]
     p = torch.softmax(z.detach().double(), -1) - torch.nn.functional.one_hot(lab if sparse else lab[4:], C)
     assert (grad.double() - p).abs().max() <= 2 ** -8
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(2456, 768, 30522), (1, 4, 2048), (130, 260, 4100), (300, 264, 2500), (7, 1000, 9001)])
+def test_split_reductions_repeat_bit_for_bit(M, N, K, dtype):
+    """Partial results are added in order: every call gives the same bits, and splits that get no part of K add zero."""
+    from deeplearning4j_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(K)
+    P = (K + 7) // 8 * 8
+    a, b = torch.randn(M, P, generator=g, device="cuda").to(dtype)[:, :K], torch.randn(N, P, generator=g, device="cuda").to(dtype)[:, :K].t()
+    want = a.double() @ b.double()
+    for s in (2, 7, 16, 30):
+        out = native._pitched(M, N, dtype, a.device)
+        first = native._split_gemm(a, b, s, out).clone()
+        assert (first.double() - want).norm() <= (4e-3 if dtype == torch.bfloat16 else 5e-4) * want.norm()
+        for _ in range(4):
+            assert torch.equal(native._split_gemm(a, b, s), first)
+    x = torch.randn(300, 768, generator=g, device="cuda").to(dtype).requires_grad_(True)
+    W = (torch.randn(768, 9001, generator=g, device="cuda") * 0.03).requires_grad_(True)
+    dy = torch.randn(300, 9001, generator=g, device="cuda").to(dtype)
+    grads = [torch.autograd.grad(native.linear(x, W, None, None), x, dy)[0] for _ in range(5)]
+    assert all(torch.equal(grads[0], t) for t in grads)
+    native.check_status()
