@@ -7,6 +7,7 @@
 // algebra (helpers/cuda/lstm.cu:45-110) and DL4J's LSTMHelpers.java:180-330 gate order [a, f, o, g].
 // Each op reads its operands once from HBM and writes once.
 #include "vec8.cuh"
+#include <cooperative_groups.h>
 
 namespace dl4j {
 
@@ -799,6 +800,58 @@ bias_act_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __
   }
 }
 
+// The fp32 form with a bias gradient of up to 4096 rows: every sum has one order, so that a layer's gradients repeat bit for bit (the
+// atomics of the other forms add in arrival order).  A block of 32 x 32 threads owns 32 columns and takes 128 rows at a time, four per
+// thread in flight; its column sums fold by shuffles.  More than 512 rows are split over the blocks of a cluster, whose first block adds
+// the slabs in order.
+// Latency-bound at these sizes (128 x 512: 262 KB in, 262 KB out).
+__global__ void __launch_bounds__(1024)
+bias_act_bwd_f32_kernel(const float* __restrict__ dy, const float* __restrict__ z, float* __restrict__ dz, float* __restrict__ dbias,
+                        int rows, int C, int act, int rows_per_block) {
+  __shared__ float red[32][33];
+  __shared__ float sums[32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + tx;
+  const int r0 = blockIdx.y * rows_per_block;
+  const int r1 = col < C ? min(r0 + rows_per_block, rows) : 0;
+  float s = 0.f;
+  for (int r = r0 + ty; r < r1; r += 128) {
+    float d[4], v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long o = (long long)(r + 32 * u) * C + col;
+      const bool in = r + 32 * u < r1;
+      d[u] = in ? __ldg(dy + o) : 0.f;
+      v[u] = in && act != 0 ? __ldg(z + o) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (r + 32 * u < r1) {
+        if (act != 0) d[u] *= act_grad(v[u], act);
+        if (dz) dz[(long long)(r + 32 * u) * C + col] = d[u];
+        s += d[u];
+      }
+    }
+  }
+  red[ty][tx] = s;
+  __syncthreads();
+  const float t = warp_sum(red[tx][ty]);                        // column ty of the block
+  const int c = blockIdx.x * 32 + ty;
+  if (gridDim.y == 1) {
+    if (tx == 0 && c < C) dbias[c] += t;
+    return;
+  }
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  if (tx == 0) sums[ty] = t;
+  cl.sync();
+  if (blockIdx.y == 0 && tx == 0 && c < C) {
+    float a = t;
+    for (int i = 1; i < (int)gridDim.y; ++i) a += cl.map_shared_rank(sums, i)[ty];
+    dbias[c] += a;
+  }
+  cl.sync();                                                    // nobody leaves while its sums are being read
+}
+
 // ----------------------------------------------------------------------------- attention softmax
 // In-place row softmax over scores S [rows, Tk] (already scaled by the GEMM epilogue) with an optional
 // key mask [B, Tk] (non-zero = keep); row r belongs to example r / rows_per_example.  One warp per row.
@@ -1074,6 +1127,21 @@ DL4J_API int dl4j_bias_act_bwd(const void* dy, const void* z, void* dz, float* d
   if (dy == nullptr || (act != 0 && z == nullptr)) return -DL4J_ERR_BAD_ARG;
   // a contiguous gradient may start anywhere: a one-row slice of a concatenation's gradient lies at the columns before it
   const bool aligned = (((uintptr_t)dy | (uintptr_t)(act != 0 ? z : nullptr) | (uintptr_t)dz) & 15) == 0;
+  if (dtype == 2 && dbias && rows <= 4096) {
+    int slabs = 1;
+    while (slabs * 512 < rows) slabs *= 2;                      // up to 8
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((C + 31) / 32, slabs);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = slabs; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = slabs > 1 ? 1 : 0;
+    return (int)cudaLaunchKernelEx(&cfg, bias_act_bwd_f32_kernel, (const float*)dy, (const float*)z, (float*)dz, dbias, rows, C, act,
+                                   (rows + slabs - 1) / slabs);
+  }
   if (C % 8 == 0 && aligned) {
     const int ct = (C + 255) / 256;
     int slabs = (148 * dl4j_launch_grid("BIAS_ACT_BWD", 6) + ct - 1) / ct;      // default: about two rounds of resident blocks (3 per SM)

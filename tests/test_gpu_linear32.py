@@ -79,3 +79,25 @@ def test_nan_and_inf_pass():
     y = nnops.linear(x, W, b, ActivationReLU())
     assert torch.isnan(y[0]).all() and not torch.isfinite(y[1]).any() == bool((W[0] > 0).all() and False) or torch.isinf(y[1]).any()
     assert torch.equal(torch.isnan(y), torch.isnan(torch.relu(x @ W + b)))
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 8, 8), (31, 5, 24), (128, 784, 512), (128, 512, 10), (257, 64, 63), (4096, 16, 64), (1000, 33, 200)])
+@pytest.mark.parametrize("relu", [True, False])
+def test_gradients_repeat_bit_for_bit(M, K, N, relu):
+    """Every sum of an fp32 layer has one order; the bias gradient is exact to a few units of the column's absolute sum."""
+    from deeplearning4j_b200.nn.activations import ActivationReLU
+    from deeplearning4j_b200.ops import native, nnops
+    x, W, b, dy = _case(M, K, N, True, M + N)
+    leaves = [t.detach().requires_grad_(True) for t in (x, W, b)]
+
+    def run():
+        before = native.LAUNCHES
+        y = nnops.linear(*leaves, ActivationReLU() if relu else None)
+        g = torch.autograd.grad(y, leaves, dy)
+        assert native.LAUNCHES >= before + 2
+        return (y.detach(), *g)
+    first = run()
+    for _ in range(10):
+        assert all(torch.equal(a, c) for a, c in zip(first, run()))
+    dz = dy.double() * (first[0] > 0) if relu else dy.double()
+    assert ((first[3].double() - dz.sum(0)).abs() <= 1e-6 * dz.abs().sum(0) + 1e-30).all()
