@@ -16,6 +16,7 @@ from .network import BaseNetwork, _as_tensor
 
 
 from .conf.graphconf import ElementWiseVertex
+from ..ops.native import TrainingStep
 from ..utils.crash import guard_fit
 
 
@@ -612,8 +613,9 @@ class ComputationGraph(BaseNetwork):
 
     def computeGradientAndScore(self, inputs, labels, fmasks=None, lmasks=None):
         self.flat_grads.zero_()
-        loss = self._loss(self._inputs(inputs), self._labels(labels))
-        loss.backward()
+        with TrainingStep() as step:
+            loss = self._loss(self._inputs(inputs), self._labels(labels))
+            step.backward(loss)
         reg = self._regularization_score()
         self._score = loss.detach() + (reg if reg is not None else 0.0)
         return self.gradient(), float(self._score)

@@ -16,6 +16,7 @@ from ..nd.ndarray import INDArray, wrap
 from .conf.base import BackpropType
 from .conf.neuralnet import MultiLayerConfiguration
 from .network import BaseNetwork, _as_tensor
+from ..ops.native import TrainingStep
 from ..utils.crash import guard_fit
 from ..utils import nvtx as _nvtx
 
@@ -174,8 +175,9 @@ class MultiLayerNetwork(BaseNetwork):
         x = self._prep_input(features if features is not None else self._input)
         y = _as_tensor(labels if labels is not None else self._labels, self.device)
         self.flat_grads.zero_()
-        loss = self._loss(x, y, _as_tensor(fmask, self.device), _as_tensor(lmask, self.device), True)
-        loss.backward()
+        with TrainingStep() as step:
+            loss = self._loss(x, y, _as_tensor(fmask, self.device), _as_tensor(lmask, self.device), True)
+            step.backward(loss)
         reg = self._regularization_score()
         self._score = loss.detach() + (reg if reg is not None else 0.0)
         self._last_batch = x.shape[0]
@@ -317,8 +319,9 @@ class MultiLayerNetwork(BaseNetwork):
                         x = self._forward(x, False, upto=idx - 1)
                     if idx in self.conf.inputPreProcessors:
                         x = self.conf.inputPreProcessors[idx].preProcess(x, x.shape[0], {})
-                loss = layer.pretrain_score(self.param_views[str(idx)], x)
-                loss.backward()
+                with TrainingStep() as step:
+                    loss = layer.pretrain_score(self.param_views[str(idx)], x)
+                    step.backward(loss)
                 self._score = loss.detach()
                 with torch.no_grad():
                     self._apply_update()

@@ -300,27 +300,29 @@ class BaseNetwork:
         ``tensors`` is a flat list of input / label (/ carried state) tensors; returns the detached loss.  ``aux`` is a
         dict that ``loss_fn`` fills with side outputs (carried recurrent state); on replay it receives the captured
         graph's output tensors."""
+        from ..ops import native
         cg = getattr(self, "_cg", None)
         if not (cg and cg["on"] and eager_ok and self.flat_params.is_cuda):
-            loss = loss_fn(tensors)
-            loss.backward()
+            with native.TrainingStep() as step:
+                loss = loss_fn(tensors)
+                step.backward(loss)
             return loss.detach()
-        from ..ops import native
         key = tuple((tuple(t.shape), t.dtype, tuple(t.stride())) for t in tensors)
         e = cg["entries"].setdefault(key, {"seen": 0, "graph": None})
         if e["graph"] is None:
             e["seen"] += 1
             if e["seen"] <= cg["warmup"]:
-                loss = loss_fn(tensors)
-                loss.backward()
+                with native.TrainingStep() as step:
+                    loss = loss_fn(tensors)
+                    step.backward(loss)
                 return loss.detach()
             e["static"] = [t.clone() for t in tensors]
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             n0 = native.LAUNCHES
-            with torch.cuda.graph(g):
+            with torch.cuda.graph(g), native.TrainingStep() as step:
                 loss = loss_fn(e["static"])
-                loss.backward()
+                step.backward(loss)
             e["launches"] = native.LAUNCHES - n0
             native.LAUNCHES = n0                    # capture launched nothing
             e["loss"] = loss.detach()

@@ -777,9 +777,41 @@ def _plain_autograd():
         and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
 
 
-def _own_grad(p):
-    """The parameter's preallocated fp32 gradient when the kernels may add to it in autograd's place (nobody hooked the leaf)."""
-    g = p.grad if p.is_leaf else None
+_STEP = threading.local()
+
+
+class TrainingStep:
+    """A trainer's forward and backward pass:
+
+        with TrainingStep() as step:
+            step.backward(loss_of(inputs))
+
+    While ``step.backward`` runs, the fp32 layers of that forward pass add their weight and bias gradients straight into the parameters'
+    preallocated ``.grad``.  Anywhere else (``torch.autograd.grad``, a user's own ``backward``) they return them to autograd, which
+    knows what was asked for."""
+    __slots__ = ("live", "outer")
+
+    def __enter__(self):
+        self.live, self.outer = False, getattr(_STEP, "current", None)
+        _STEP.current = self
+        return self
+
+    def __exit__(self, *exc):
+        _STEP.current = self.outer
+        return False
+
+    def backward(self, loss):
+        self.live = True
+        try:
+            loss.backward()
+        finally:
+            self.live = False
+
+
+def _own_grad(p, step):
+    """The parameter's preallocated fp32 gradient when the kernels may add to it in autograd's place (the trainer's own backward pass is
+    running and nobody hooked the leaf)."""
+    g = p.grad if step is not None and step.live and p.is_leaf else None
     if g is None or g.dtype != torch.float32 or p._backward_hooks or getattr(p, "_post_accumulate_grad_hooks", None) \
             or getattr(p, "_grad_ready", None) is not None:
         return None
@@ -794,7 +826,7 @@ class _Linear32Fn(torch.autograd.Function):
     def forward(ctx, x, W, b, relu):
         y = torch.empty((x.shape[0], W.shape[1]), dtype=torch.float32, device=x.device)
         _sgemm(x, W, y, bias=None if b is None else b.detach().reshape(-1), act=1 if relu else 0)
-        ctx.relu, ctx.refs = relu, (W, b)
+        ctx.relu, ctx.refs, ctx.step = relu, (W, b), getattr(_STEP, "current", None)
         ctx.save_for_backward(x, W, b, y if relu else None)
         return y
 
@@ -812,7 +844,7 @@ class _Linear32Fn(torch.autograd.Function):
         Wl, bl = ctx.refs
         db = acc = None
         if b is not None and need[2]:
-            acc = _own_grad(bl)
+            acc = _own_grad(bl, ctx.step)
             if acc is None or not acc.is_contiguous():
                 acc = db = torch.zeros(N, dtype=torch.float32, device=dy.device)
         dz = dy
@@ -824,7 +856,7 @@ class _Linear32Fn(torch.autograd.Function):
         if need[0]:
             dx = _sgemm(dz, W.t(), torch.empty_like(x, memory_format=torch.contiguous_format)) if _sgemm_wins(M, x.shape[1], 16) else dz @ W.t()
         if need[1]:
-            g = _own_grad(Wl)
+            g = _own_grad(Wl, ctx.step)
             if g is not None and _unit(g):
                 g.addmm_(x.t(), dz)
             elif W.stride(0) == 1 and W.shape[0] > 1:           # 'f' order

@@ -18,6 +18,7 @@ from ..nd.dtype import DataType
 from ..nn.conf.base import ParamSpec
 from ..nn.updater import MultiLayerUpdater, ParamEntry
 from ..nn.updaters import IUpdater, L1Regularization, L2Regularization, Regularization, Sgd, WeightDecay, updater_from_json, regularization_from_json
+from ..ops.native import TrainingStep
 from ..serde import jackson
 from .core import SDVariable, VariableType, _tensor
 
@@ -250,11 +251,12 @@ class TrainingState:
         if hook is not None and hasattr(hook, "pre_step"):
             hook.pre_step(tc.iterationCount, tc.epochCount)       # per-step device variables of an overlapped exchange
         def fwd_bwd(ph):
-            vals = InferenceSession(sd).run(ph, losses, self.values(), training=True)
-            loss = vals[losses[0]].sum() if len(losses) == 1 else sum(vals[l].sum() for l in losses)
-            if not tc.minimize:
-                loss = -loss
-            loss.backward()
+            with TrainingStep() as step:
+                vals = InferenceSession(sd).run(ph, losses, self.values(), training=True)
+                loss = vals[losses[0]].sum() if len(losses) == 1 else sum(vals[l].sum() for l in losses)
+                if not tc.minimize:
+                    loss = -loss
+                step.backward(loss)
             if hook is not None and hasattr(hook, "after_backward"):
                 hook.after_backward()                             # flush + join of the side stream (inside a graph capture too)
             return loss.detach()

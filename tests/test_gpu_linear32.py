@@ -101,3 +101,44 @@ def test_gradients_repeat_bit_for_bit(M, K, N, relu):
         assert all(torch.equal(a, c) for a, c in zip(first, run()))
     dz = dy.double() * (first[0] > 0) if relu else dy.double()
     assert ((first[3].double() - dz.sum(0)).abs() <= 1e-6 * dz.abs().sum(0) + 1e-30).all()
+
+
+@pytest.mark.parametrize("M,K,N", [(16, 24, 32), (5, 7, 3)])
+def test_autograd_grad_with_preallocated_gradients(M, K, N):
+    """``.grad`` belongs to the caller: only a trainer's own backward pass is added to behind autograd's back."""
+    from deeplearning4j_b200.nn.activations import ActivationReLU
+    from deeplearning4j_b200.ops import native, nnops
+    x, W, b, dy = _case(M, K, N, True, 9)
+    x, W, b = (t.detach().requires_grad_(True) for t in (x, W, b))
+    W.grad, b.grad = torch.full_like(W, 7.0), torch.full_like(b, 7.0)
+    ref = torch.autograd.grad(torch.relu(x.double() @ W.double() + b.double()), (x, W, b), dy.double())
+    call = lambda: nnops.linear(x, W, b, ActivationReLU())
+    for got, want in zip(torch.autograd.grad(call(), (x, W, b), dy), ref):
+        assert torch.allclose(got.double(), want.double(), rtol=1e-4, atol=1e-4)
+    assert torch.allclose(torch.autograd.grad(call(), x, dy)[0].double(), ref[0].double(), rtol=1e-4, atol=1e-4)
+    with native.TrainingStep() as step:
+        y = call()
+        inner = torch.autograd.grad(y, (W, b), dy, retain_graph=True)         # a layer's own gradient inside the forward pass
+        assert torch.allclose(inner[0].double(), ref[1].double(), rtol=1e-4, atol=1e-4)
+        assert (W.grad == 7).all() and (b.grad == 7).all()
+        step.backward((y * dy).sum())
+    for p, want in ((W, ref[1]), (b, ref[2])):
+        assert torch.allclose(p.grad.double(), want.double() + 7, rtol=1e-4, atol=1e-4)
+    got = torch.autograd.grad(call(), (W, b), dy)
+    assert torch.allclose(got[0].double(), ref[1].double(), rtol=1e-4, atol=1e-4)
+
+
+def test_a_network_trains_into_its_flat_gradient(monkeypatch):
+    """fit and computeGradientAndScore keep adding in place: autograd is handed no gradient for the dense parameters."""
+    from deeplearning4j_b200 import nn
+    from deeplearning4j_b200.nn.layers.core import DenseLayer, OutputLayer
+    from deeplearning4j_b200.ops import native
+    net = nn.MultiLayerNetwork(nn.NeuralNetConfiguration.Builder().seed(1).updater(nn.Sgd(0.1)).list().layer(DenseLayer(nIn=8, nOut=16, activation="RELU"))
+                               .layer(OutputLayer("MCXENT", nIn=16, nOut=4, activation="SOFTMAX")).build())
+    net.device = torch.device("cuda")
+    net.init()
+    seen, backward = [], native._Linear32Fn.backward
+    monkeypatch.setattr(native._Linear32Fn, "backward", staticmethod(lambda ctx, dy: seen.append(backward(ctx, dy)) or seen[-1]))
+    x, y = torch.randn(32, 8, device="cuda"), torch.eye(4, device="cuda")[torch.arange(32, device="cuda") % 4]
+    net.computeGradientAndScore(x, y)
+    assert len(seen) == 2 and all(g[1] is None and g[2] is None for g in seen)
