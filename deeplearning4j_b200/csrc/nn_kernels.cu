@@ -827,7 +827,8 @@ bias_act_bwd_f32_kernel(const float* __restrict__ dy, const float* __restrict__ 
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (r + 32 * u < r1) {
-        if (act != 0) d[u] *= act_grad(v[u], act);
+        if (act == 1) d[u] = v[u] <= 0.f ? 0.f : d[u];           // the library's rule: an infinite gradient stops at a unit that is off
+        else if (act != 0) d[u] *= act_grad(v[u], act);
         if (dz) dz[(long long)(r + 32 * u) * C + col] = d[u];
         s += d[u];
       }

@@ -835,7 +835,7 @@ class _Linear32Fn(torch.autograd.Function):
         x, W, b, y = ctx.saved_tensors
         need = ctx.needs_input_grad
         if torch.is_grad_enabled():                    # create_graph: the gradient has to be differentiable itself
-            dz = dy * (y > 0).to(dy.dtype) if ctx.relu else dy
+            dz = dy.masked_fill(y <= 0, 0.0) if ctx.relu else dy
             return (dz @ W.t() if need[0] else None, x.t() @ dz if need[1] else None,
                     dz.sum(0).reshape(b.shape) if b is not None and need[2] else None, None)
         l = require()

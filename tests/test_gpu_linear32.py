@@ -70,15 +70,32 @@ def test_hooks_create_graph_and_transforms():
     assert torch.allclose(t, torch.ones_like(x) @ W, atol=1e-5)
 
 
-def test_nan_and_inf_pass():
+@pytest.mark.parametrize("M,K,N", [(64, 8, 8), (70, 40, 24), (64, 8, 5)])
+def test_nan_and_inf_pass(M, K, N):
+    """Values and gradients have NaN and infinities of either sign where the library's operators have them."""
     from deeplearning4j_b200.nn.activations import ActivationReLU
-    from deeplearning4j_b200.ops import nnops
-    x, W, b, _ = _case(4, 8, 8, True, 1)
+    from deeplearning4j_b200.ops import native, nnops
+    x, W, b, dy = _case(M, K, N, True, 1)
     x[0, 0] = float("nan")
-    x[1, 0] = float("inf")
-    y = nnops.linear(x, W, b, ActivationReLU())
-    assert torch.isnan(y[0]).all() and not torch.isfinite(y[1]).any() == bool((W[0] > 0).all() and False) or torch.isinf(y[1]).any()
-    assert torch.equal(torch.isnan(y), torch.isnan(torch.relu(x @ W + b)))
+    x[1, 0], x[2, 0] = float("inf"), float("-inf")
+    dy[3, 1], dy[4, 2], dy[5, 3] = float("inf"), float("-inf"), float("nan")
+    dy[0, 4] = float("inf")
+
+    def same(u, v):
+        assert torch.equal(torch.isnan(u), torch.isnan(v)) and torch.equal(torch.isposinf(u), torch.isposinf(v)) \
+            and torch.equal(torch.isneginf(u), torch.isneginf(v))
+        fin = torch.isfinite(v)
+        assert torch.allclose(u[fin], v[fin], rtol=1e-4, atol=1e-4)
+    for create in (False, True):
+        leaves = [t.detach().requires_grad_(True) for t in (x, W, b)]
+        before = native.LAUNCHES
+        y = nnops.linear(*leaves, ActivationReLU())
+        assert native.LAUNCHES > before
+        ref = [t.detach().requires_grad_(True) for t in (x, W, b)]
+        z = torch.relu(ref[0] @ ref[1] + ref[2])
+        same(y.detach(), z.detach())
+        for u, v in zip(torch.autograd.grad(y, leaves, dy, create_graph=create), torch.autograd.grad(z, ref, dy)):
+            same(u.detach(), v)
 
 
 @pytest.mark.parametrize("M,K,N", [(1, 8, 8), (31, 5, 24), (128, 784, 512), (128, 512, 10), (257, 64, 63), (4096, 16, 64), (1000, 33, 200)])
