@@ -688,9 +688,8 @@ class _OddLinearFn(torch.autograd.Function):
         Wp = _on_pitch(Wd, dt) if rows else _on_pitch(Wd.t(), dt).t()
         y = _pitched(M, N, dt, x.device)
         z = _pitched(M, N, dt, x.device) if act in (2, 3, 4, 5, 6) and any(ctx.needs_input_grad) else None
-        b_fwd = _fwd_bias(b, dt)[0]
-        if b_fwd is not None:
-            b_fwd = _dense16(b_fwd.detach())
+        # the parameter itself, like the weights: in its own precision and as it is now (its 16-bit shadow is neither)
+        b_fwd = None if b is None else _dense16(b.detach().reshape(-1))
         gemm_raw(xp, Wp, out=y, bias=b_fwd, act=act, aux=z)
         ctx.act, ctx.rows, ctx.w_dtype, ctx.b_like = act, rows, W.dtype, None if b is None else (b.shape, b.dtype)
         ctx.save_for_backward(xp, Wp, z if z is not None else (y if act == 1 else None))
@@ -734,7 +733,8 @@ class _OddLinearFn(torch.autograd.Function):
 
 def _linear_padded(x, W, b, act):
     """Layer widths that are not multiples of 8, see ``_OddLinearFn``; None when the case is not covered."""
-    if W.dim() != 2 or min(x.shape[0], W.shape[0], W.shape[1]) == 0 or W.dtype not in (x.dtype, torch.float32) or not on_current_device(x, W, b):
+    if W.dim() != 2 or min(x.shape[0], W.shape[0], W.shape[1]) == 0 or W.dtype not in (x.dtype, torch.float32) or not on_current_device(x, W, b) \
+            or (b is not None and b.numel() != W.shape[1]):
         return None
     return _OddLinearFn.apply(x, W, b, act)
 

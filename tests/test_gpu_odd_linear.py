@@ -110,3 +110,25 @@ def test_split_reductions_repeat_bit_for_bit(M, N, K, dtype):
     grads = [torch.autograd.grad(native.linear(x, W, None, None), x, dy)[0] for _ in range(5)]
     assert all(torch.equal(grads[0], t) for t in grads)
     native.check_status()
+
+
+def test_bias_is_the_parameter_not_its_shadow():
+    """256.5 is not a bf16 number: what is left after the product's -256 shows the bits of the bias; a change in place is seen at once."""
+    from deeplearning4j_b200 import DataType, nn
+    from deeplearning4j_b200.nn.layers.core import DenseLayer, OutputLayer
+    net = nn.MultiLayerNetwork(nn.NeuralNetConfiguration.Builder().computeDataType(DataType.BFLOAT16).list()
+                               .layer(DenseLayer(nIn=8, nOut=10, activation="IDENTITY"))
+                               .layer(OutputLayer("MSE", nIn=10, nOut=8, activation="IDENTITY")).build())
+    net.device = torch.device("cuda")
+    net.init()
+    p = net.paramTable()
+    p["0_W"].t.fill_(-32.0)
+    p["0_b"].t.fill_(256.5)
+    p["1_W"].t.zero_()
+    p["1_W"].t[0, 0] = 1.0
+    p["1_b"].t.zero_()
+    x = torch.ones(300, 8, device="cuda")
+    net.setParams(net.params().t.clone())                     # the shadows are up to date
+    assert (net.output(x).t[:, 0] == 0.5).all()
+    net.paramTable()["0_b"].t.fill_(257.25)
+    assert (net.output(x).t[:, 0] == 1.25).all()
