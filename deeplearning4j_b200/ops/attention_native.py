@@ -67,7 +67,7 @@ class _AttentionFn(torch.autograd.Function):
         Bn, H, Tq, D = q.shape
         Tk = k.shape[2]
         dt = q.dtype
-        ctx.flash = (USE_FLASH or dropout_p > 0.0 or flags) and flash_supported(q, k, v)
+        ctx.flash = (USE_FLASH or dropout_p > 0.0 or flags) and scale >= 0.0 and flash_supported(q, k, v)
         if ctx.flash:
             # fused kernel: the score matrix stays in tensor memory; only O and the row log-sum-exp are written
             seed = _next_dropout_seed(q.device) if dropout_p > 0.0 else None
@@ -197,7 +197,8 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
         return None
     D, Tk, Tq = q.shape[3], k.shape[2], q.shape[2]
     scale = float(scale) if scale is not None else D ** -0.5
-    fused = flash_supported(q, k, v)
+    # the fused kernels take a row's maximum over raw scores: with a negative scale that is the smallest exponent, and exp overflows
+    fused = scale >= 0.0 and flash_supported(q, k, v)
     if dropout_p > 0.0 and (not fused or Tk % 128 or causal):
         return None
     if fused and (USE_FLASH or dropout_p > 0.0):
@@ -206,7 +207,8 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
             return flash_forward(q, k, v, mask, scale, flags=flags)[0].permute(0, 2, 1, 3)       # nothing to differentiate
         # laid out here and not in forward(): second derivatives go through the saved operands
         return _AttentionFn.apply(_prep(q), _prep(k), _prep(v), mask, scale, float(dropout_p), flags)
-    if causal or D % 8 or Tk % 8 or Tq % 8 or Tk > 1024:
+    if causal or D % 8 or Tk % 8 or Tq % 8 or Tk > 1024 or k.shape != v.shape or q.shape[:2] != k.shape[:2] or D != k.shape[3] \
+            or not q.dtype == k.dtype == v.dtype:
         return None
     return _AttentionFn.apply(q, k, v, mask, scale, float(dropout_p))
 
@@ -217,9 +219,11 @@ def attention_grad(q, k, v, mask, scale, dout, causal=False):
     if not USE_FLASH or not native.available() or not flash_supported(q, k, v) or _bad_mask(q, k, mask) or dout.dim() != 4 \
             or not native.on_current_device(q, k, v, mask, dout) or not native._plain_autograd() or dout.shape != (*q.shape[:3], v.shape[3]):
         return None
+    scale = float(scale) if scale is not None else q.shape[3] ** -0.5
+    if not scale >= 0.0:
+        return None
     q, k, v, dout = _prep(q.detach()), _prep(k.detach()), _prep(v.detach()), _prep(dout.detach().to(q.dtype))
     Bn, H, Tq, D = q.shape
-    scale = float(scale) if scale is not None else D ** -0.5
     flags = (1 if causal else 0) | (0 if _empty_rows_are_zero(D, Tq, k.shape[2]) and not causal else 2)
     mk = mask.detach().to(torch.float32).contiguous() if mask is not None else None
     stats = torch.empty((2, Bn, H, Tq), dtype=torch.float32, device=q.device)

@@ -121,3 +121,32 @@ def test_second_derivatives_forward_mode_and_vmap(T, masked, causal):
     if mask is None:
         got = torch.func.vmap(lambda a: call(a, k, v))(torch.stack([q, q.flip(0)]))
         assert (got[0].double() - _ref(q6, k.double(), v.double(), scale, None, causal)).norm() <= 1e-2 * got[0].double().norm()
+
+
+@pytest.mark.parametrize("T,causal", [(201, False), (64, False), (256, False), (130, True), (1032, False)])
+@pytest.mark.parametrize("scale", [-0.125, -8.0])
+def test_negative_scale(T, causal, scale):
+    """Scores are scaled before the row maximum is taken: large ones of the other sign do not overflow."""
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    q, k, v, do, _ = _inputs(2, 2, T, T, 64, T)
+    q = q * 4
+    q6, k6, v6 = (t.double().requires_grad_(True) for t in (q, k, v))
+    want = _ref(q6, k6, v6, scale, None, causal)
+    grads = torch.autograd.grad(want, (q6, k6, v6), do.double())
+    out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=scale, useCausalMask=causal).t
+    dq, dv, dk = (a.t for a in Nd4j.exec("dot_product_attention_v2_bp", q, v, k, do, scale=scale, useCausalMask=causal))
+    # scores reach the hundreds: bf16 scores (the operator path) carry an error of 2^-9 of them into the exponent
+    tol = 1e-2 if abs(scale) < 1 else 0.5
+    assert torch.isfinite(out).all() and (out.double() - want).norm() <= tol * want.norm()
+    for a, b in zip((dq, dk, dv), grads):
+        assert torch.isfinite(a).all() and (a.double() - b).norm() <= 3 * tol * (b.norm() + abs(scale) * do.double().norm())
+
+
+@pytest.mark.parametrize("kshape,vshape", [((1, 2, 64, 64), (1, 2, 64, 64)), ((2, 1, 64, 64), (2, 1, 64, 64)), ((2, 2, 64, 64), (2, 2, 64, 32))])
+def test_operands_that_broadcast(kshape, vshape):
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((2, 2, 64, 64), kshape, vshape))
+    out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=0.1).t
+    want = _ref(q.double(), k.double(), v.double(), 0.1, None, False)
+    assert out.shape == want.shape and (out.double() - want).norm() <= 1e-2 * want.norm()
