@@ -265,7 +265,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       xl[ch * FF_BM + r] = run_l;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       const float l = run_l + xl[(ch ^ 1) * FF_BM + r];
-      const float inv = l > 0.f ? 1.f / l : p.empty;
+      const float inv = l == 0.f ? p.empty : 1.f / l;               // l is 0, positive or NaN
       const int tq = q0 + r;
       if (p.dout) {            // uniform: D = sum over the head dimension of dO * O, this thread's 32 columns, then both halves
         float d = 0.f;
@@ -304,7 +304,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
         if (p.lse && ch == 0) {
           const float mref = (run_m == -INFINITY) ? 0.f : run_m;
-          p.lse[((long)b * p.H + h) * p.Tq + tq] = l > 0.f ? mref * p.scale + __logf(l) : -INFINITY;
+          p.lse[((long)b * p.H + h) * p.Tq + tq] = l == 0.f ? -INFINITY : mref * p.scale + __logf(l);      // NaN stays NaN for the backward pass
         }
       }
     }

@@ -150,3 +150,21 @@ def test_operands_that_broadcast(kshape, vshape):
     out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=0.1).t
     want = _ref(q.double(), k.double(), v.double(), 0.1, None, False)
     assert out.shape == want.shape and (out.double() - want).norm() <= 1e-2 * want.norm()
+
+
+@pytest.mark.parametrize("T,causal", [(201, False), (100, True), (130, True), (1032, False)])
+@pytest.mark.parametrize("where", ["q", "k"])
+def test_nan_reaches_the_gradients(T, causal, where):
+    """A NaN query makes its own row and dk, dv NaN; a NaN key makes every row that sees it NaN: as the operators have it."""
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    q, k, v, do, _ = _inputs(2, 2, T, T, 64, T)
+    bad = q if where == "q" else k
+    bad[1, 0, 3, 5] = float("nan")
+    q6, k6, v6 = (t.double().requires_grad_(True) for t in (q, k, v))
+    want = _ref(q6, k6, v6, 0.125, None, causal)
+    grads = torch.autograd.grad(want, (q6, k6, v6), do.double())
+    out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=0.125, useCausalMask=causal).t
+    dq, dv, dk = (a.t for a in Nd4j.exec("dot_product_attention_v2_bp", q, v, k, do, scale=0.125, useCausalMask=causal))
+    for a, b in zip((out, dq, dk, dv), (want, *grads)):
+        assert torch.equal(torch.isnan(a).any(-1).any(-1), torch.isnan(b).any(-1).any(-1))       # the same heads
+        assert (torch.isnan(a) >= torch.isnan(b)).all()                                          # nothing hidden
