@@ -7,7 +7,8 @@ using namespace dl4j;
 // One CTA per (batch, head, block of 128 keys); it walks the query blocks.  Per query block i:
 //     S = Q_i K_j^T and dP = dO_i V_j^T (TMEM)  ->  threads: P = exp(S * scale - lse), dS = scale * P * (dP - D)
 //     ->  P, dS staged in shared memory (bf16)  ->  dV += P^T dO_i, dK += dS^T Q_i (accumulated in TMEM over i),
-//     dQ_i = dS K_j (TMEM, added to the fp32 dQ buffer with vector atomics: four key blocks contribute to it).
+//     dQ_i = dS K_j (TMEM; every key block contributes, so it leaves for an fp32 buffer through the copy engine: added to one buffer in
+//     arrival order, or stored in a slab of its own and summed in order by the finishing kernel).
 // P^T and dS^T are the same shared-memory tiles read through MN-major descriptors, so nothing is transposed.
 // D = rowsum(dO * O) and the forward's log-sum-exp come from the caller.  Keys past Tk and causally hidden ones are taken out by the same
 // bits as masked keys; a causal key block starts at its own query block.  With a single key block nothing else contributes to dQ and
@@ -34,6 +35,7 @@ struct FlashBwdParams {
   const float* dvec;         // [B, H, Tq]  rowsum(dO * O)
   const float* key_mask;     // [B, Tk] or null
   float* dq;                 // [B, H, Tq, D] fp32, zero on entry; null: dq16 is written directly (one key block)
+  int dq_slabs;              // dq is [key blocks, B, H, Tq, D] instead: every key block stores its part, nothing is added
   __nv_bfloat16* dq16;       // [B, Tq, H, D]
   __nv_bfloat16* dk;         // [B, Tk, H, D]
   __nv_bfloat16* dv;         // [B, Tk, H, D]
@@ -238,7 +240,10 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         __syncwarp();
         const int row0 = (i0 + blk) * FB_BLK + q * 32;
         if (lane == 0) {
-          if (row0 < p.Tq && cq * 16 < p.D) tma_reduce_add_4d(&tmap_dq, slab, cq * 16, row0, h, b);
+          if (row0 < p.Tq && cq * 16 < p.D) {
+            if (p.dq_slabs) tma_store_4d(&tmap_dq, slab, cq * 16, row0, h, kb * p.B + b);
+            else tma_reduce_add_4d(&tmap_dq, slab, cq * 16, row0, h, b);
+          }
           bulk_commit();
         }
       }
@@ -348,7 +353,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 // q / k / v / dout: [B, H, T, D] bf16 views (element strides {sb, sh, st}), D a multiple of 8 up to 64; lse, dvec [B, H, Tq] fp32;
 // dq_acc [B, H, Tq, D] fp32 zeroed by the caller, or null with at most 128 keys: dq is then written here, addressed as
 // base + b * q_bs + query * q_ts + head * D; dk, dv bf16 addressed as base + b * o_bs + key * o_ts + head * D.
-// flags as in dl4j_flash_attn_fwd.
+// flags as in dl4j_flash_attn_fwd; 4: dq_acc is [key blocks, B, H, Tq, D], need not be zeroed, and every key block stores its part there.
 DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* dvec,
                                  const float* key_mask, float* dq_acc, void* dq, void* dk, void* dv, int B, int H, int Tq, int Tk, int D,
                                  const long* q_strides, const long* k_strides, const long* v_strides, const long* do_strides, long q_bs,
@@ -370,7 +375,7 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   if (dq_acc) {
     dl4j_PFN_encodeTiled enc = dl4j_get_encode_tiled();
     if (!enc || (reinterpret_cast<uintptr_t>(dq_acc) & 15)) return -DL4J_ERR_BAD_ARG;
-    cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)Tq, (cuuint64_t)H, (cuuint64_t)B};
+    cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)Tq, (cuuint64_t)H, (cuuint64_t)B * (flags & 4 ? (Tk + FB_BLK - 1) / FB_BLK : 1)};
     cuuint64_t strides[3] = {(cuuint64_t)D * 4, (cuuint64_t)Tq * D * 4, (cuuint64_t)H * Tq * D * 4};
     cuuint32_t box[4] = {16, 32, 1, 1}, es[4] = {1, 1, 1, 1};
     const CUresult cr = enc(&tdq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dq_acc, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -382,6 +387,7 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   FlashBwdParams p;
   p.lse = lse; p.dvec = dvec; p.key_mask = key_mask;
   p.dq = dq_acc;
+  p.dq_slabs = (flags >> 2) & 1;
   p.dq16 = reinterpret_cast<__nv_bfloat16*>(dq);
   p.q_bs = q_bs; p.q_ts = q_ts;
   p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
@@ -435,9 +441,11 @@ attn_dvec_kernel(const __nv_bfloat16* __restrict__ dO, long sb, long sh, long st
   if (row < rows && part == 0) dvec[row] = acc;
 }
 
-// dq (bf16, addressed base + b * o_bs + t * o_ts + h * D) = acc [B, H, T, D] fp32
+// dq (bf16, addressed base + b * o_bs + t * o_ts + h * D) = acc [slabs, B, H, T, D] fp32, slabs added in order; with a causal mask
+// query t has parts in the slabs 0 .. t / 128 only.
 __global__ void __launch_bounds__(256)
-attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long o_bs, long o_ts, int B, int H, int T, int D) {
+attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long o_bs, long o_ts, int B, int H, int T, int D,
+                      int slabs, int causal) {
   const int parts = D / 8;
   const long n8 = (long)B * H * T * parts;
   for (long g = blockIdx.x * 256L + threadIdx.x; g < n8; g += (long)gridDim.x * 256) {
@@ -447,7 +455,14 @@ attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__
     const int h = (int)((row / T) % H);
     const int b = (int)(row / ((long)T * H));
     const float4* src = reinterpret_cast<const float4*>(acc) + 2 * g;
-    const float4 x = __ldcs(src), y = __ldcs(src + 1);
+    float4 x = __ldcs(src), y = __ldcs(src + 1);
+    const int n = causal ? min(slabs, t / FB_BLK + 1) : slabs;
+#pragma unroll 4
+    for (int s = 1; s < n; ++s) {
+      const float4 a = __ldcs(src + s * 2 * n8), c = __ldcs(src + s * 2 * n8 + 1);
+      x.x += a.x; x.y += a.y; x.z += a.z; x.w += a.w;
+      y.x += c.x; y.y += c.y; y.z += c.z; y.w += c.w;
+    }
     uint4 u;
     __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&u);
     hh[0] = __floats2bfloat162_rn(x.x, x.y); hh[1] = __floats2bfloat162_rn(x.z, x.w);
@@ -466,10 +481,11 @@ DL4J_API int dl4j_attn_dvec(const void* dout, const long* do_strides, const void
   return (int)cudaGetLastError();
 }
 
-DL4J_API int dl4j_attn_dq_finish(const float* acc, void* out, long o_bs, long o_ts, int B, int H, int T, int D, void* stream) {
+DL4J_API int dl4j_attn_dq_finish(const float* acc, void* out, long o_bs, long o_ts, int B, int H, int T, int D, int slabs, int causal, void* stream) {
   const long n8 = (long)B * H * T * (D / 8);
   long blocks = (n8 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  attn_dq_finish_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(acc, reinterpret_cast<__nv_bfloat16*>(out), o_bs, o_ts, B, H, T, D);
+  attn_dq_finish_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(acc, reinterpret_cast<__nv_bfloat16*>(out), o_bs, o_ts, B, H, T, D,
+                                                                               slabs, causal);
   return (int)cudaGetLastError();
 }

@@ -274,7 +274,7 @@ def _flash_lib():
         l.dl4j_flash_attn_bwd.restype = ctypes.c_int
         l.dl4j_attn_dvec.argtypes = [vp, lp, vp, vp, i32, i32, i32, i32, vp]
         l.dl4j_attn_dvec.restype = ctypes.c_int
-        l.dl4j_attn_dq_finish.argtypes = [vp, vp, lng, lng, i32, i32, i32, i32, vp]
+        l.dl4j_attn_dq_finish.argtypes = [vp, vp, lng, lng, i32, i32, i32, i32, i32, i32, vp]
         l.dl4j_attn_dq_finish.restype = ctypes.c_int
         l.dl4j_flash_attn_bwd._typed = True
     return l
@@ -292,9 +292,17 @@ def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
         dq_t = torch.empty((Bn, Tq, H, D), dtype=q.dtype, device=q.device)
         dk_t = torch.empty((Bn, Tk, H, D), dtype=q.dtype, device=q.device)
         dv_t = torch.empty((Bn, Tk, H, D), dtype=q.dtype, device=q.device)
-    # more than one key block adds into a query's gradient: an fp32 accumulator, its own for every call (streams and threads may
-    # run the same shape at the same time)
-    acc = torch.zeros((Bn, H, Tq, D), dtype=torch.float32, device=q.device) if Tk > 128 else None
+    # more than one key block contributes to a query's gradient: an fp32 buffer, its own for every call (streams and threads may run the
+    # same shape at the same time).  The lengths that the batched products and the operators served before repeat bit for bit: their key
+    # blocks store slabs that are added in order.  The others always added in arrival order and keep the smaller buffer.
+    blocks = (Tk + 127) // 128
+    acc, slabs = None, 1
+    if blocks > 1 and (Tk % 128 or flags & 1):
+        slabs = blocks
+        acc = torch.empty((blocks, Bn, H, Tq, D), dtype=torch.float32, device=q.device)
+        flags |= 4
+    elif blocks > 1:
+        acc = torch.zeros((Bn, H, Tq, D), dtype=torch.float32, device=q.device)
     stream = native._stream()
     rc = l.dl4j_flash_attn_bwd(native._ptr(q), native._ptr(k), native._ptr(v), native._ptr(dO), native._ptr(lse), native._ptr(dvec),
                                native._ptr(mk), native._ptr(acc), native._ptr(dq_t), native._ptr(dk_t), native._ptr(dv_t), Bn, H, Tq, Tk, D,
@@ -303,7 +311,8 @@ def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
                                stream)
     native._check(rc, "dl4j_flash_attn_bwd")
     if acc is not None:
-        rc = l.dl4j_attn_dq_finish(native._ptr(acc), native._ptr(dq_t), dq_t.stride(0), dq_t.stride(1), Bn, H, Tq, D, stream)
+        rc = l.dl4j_attn_dq_finish(native._ptr(acc), native._ptr(dq_t), dq_t.stride(0), dq_t.stride(1), Bn, H, Tq, D, slabs,
+                                   flags & 1, stream)
         native._check(rc, "dl4j_attn_dq_finish")
     return dq_t.permute(0, 2, 1, 3), dk_t.permute(0, 2, 1, 3), dv_t.permute(0, 2, 1, 3)
 
