@@ -762,12 +762,38 @@ def _unit(t):
     return t.dim() == 2 and 1 in t.stride()
 
 
-def _sgemm_wins(M, N, most=64):
-    """Whether a product leaves a library kernel short of tiles.  A layer's forward (bias and ReLU in the epilogue) wins up to 64 tiles of
-    64 x 64: 512 x 512 x 512 15.6 us against 17.3, at 128 tiles (512 x 1024 x 1024) 47 against 36.  The bare data gradient up to 16:
-    128 x 512 x 512 8.7 us against 10.7, at 64 tiles 15 against 12.  The weight gradient stays a library product that adds into its
-    target: 7 us against 8 - 12 here."""
-    return ((M + 63) // 64) * ((N + 63) // 64) <= most
+def _sgemm_wins(M, N, K, relu):
+    """Whether the forward product of an fp32 layer (M rows, N units, a sum of K terms) leaves a library kernel short of tiles.  A tile of
+    64 x 64 has at most eight CTAs, so the time grows with K.  us of device time, here / library product [+ ReLU launch]:
+        M, N          K = 256    1024      2048      4096      8192      25088
+        64, 64        13 / 22    16 / 28   25 / 30   39 / 42   72 / 61   199 / 104
+        128, 512      12 / 22    19 / 38   29 / 41   49 / 56   90 / 88   254 / 150
+        512, 512      14 / 22    31 / 40   51 / 65   90 / 114  169 / 149 496 / 332
+        64, 4096      15 / 22    33 / 42   55 / 67   100 / 118 188 / 148 548 / 331
+        16, 512       12 / 22    16 / 17   25 / 23   41 / 30   72 / 34   203 / 75
+        32, 4096      15 / 22    33 / 40   55 / 47   98 / 74   186 / 111 543 / 319
+        1, 4096       14 / 13    31 / 17   53 / 22
+    Below 16 rows the library has matrix-vector kernels: 12 / 11 at K = 128, 12 / 13 at 256, 14 / 13 - 21 / 13 at 512.  Without a ReLU launch
+    to save: 128 x 512 x 10 6 / 9, 16 rows 12 / 8 at K = 128, 12 / 10 at 256, 12 / 12 at 512."""
+    if ((M + 63) // 64) * ((N + 63) // 64) > 64:
+        return False
+    if M < 16:
+        return relu and K <= 256
+    return K <= (4096 if M >= 64 else 1024) and (relu or K >= 256)
+
+
+def _sgemm_wins_dgrad(M, N, nIn):
+    """The same for the bare data gradient dz [M, N] @ W^T, up to 16 tiles; its sum has N terms.  here / library:
+        M, nIn        N = 256    512       1024      4096      8192
+        64, 64        12 / 12    12 / 18   16 / 21   39 / 40   71 / 57
+        128, 512      12 / 12    14 / 18   19 / 31   49 / 52   88 / 82
+        32, 1024                 14 / 15   20 / 19   51 / 44 - 53
+        16, 512       12 / 13    12 / 13   16 / 13   39 / 23
+        1, any        10 / 7     12 / 8
+    The weight gradient stays a library product that adds into its target: 7 us against 8 - 12 here."""
+    if ((M + 63) // 64) * ((nIn + 63) // 64) > 16 or M < 2:
+        return False
+    return N <= (4096 if M >= 64 else 512)
 
 
 def _plain_autograd():
@@ -854,7 +880,7 @@ class _Linear32Fn(torch.autograd.Function):
             _check(rc, "dl4j_bias_act_bwd")
         dx = dW = None
         if need[0]:
-            dx = _sgemm(dz, W.t(), torch.empty_like(x, memory_format=torch.contiguous_format)) if _sgemm_wins(M, x.shape[1], 16) else dz @ W.t()
+            dx = _sgemm(dz, W.t(), torch.empty_like(x, memory_format=torch.contiguous_format)) if _sgemm_wins_dgrad(M, N, x.shape[1]) else dz @ W.t()
         if need[1]:
             g = _own_grad(Wl, ctx.step)
             if g is not None and _unit(g):
@@ -869,7 +895,7 @@ class _Linear32Fn(torch.autograd.Function):
 def linear32(x, W, b, relu):
     """fp32 dense layer on the small-problem kernel, or None when the case is not covered or the library does it better."""
     if not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.float32 or W.dtype != torch.float32 or W.dim() != 2 \
-            or W.shape[0] != x.shape[1] or min(x.shape[0], *W.shape) == 0 or not _sgemm_wins(x.shape[0], W.shape[1]) \
+            or W.shape[0] != x.shape[1] or min(x.shape[0], *W.shape) == 0 or not _sgemm_wins(x.shape[0], W.shape[1], x.shape[1], relu) \
             or torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled() or not _unit(x) or not on_current_device(x, W, b):
         return None
     if not ((W.stride(0) == 1 and W.stride(1) >= W.shape[0]) or (W.stride(1) == 1 and W.stride(0) >= W.shape[1])):
