@@ -15,6 +15,7 @@ import threading
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 _LIB = None
 _LIB_ERR = None
@@ -120,6 +121,10 @@ def load_error():
     return _LIB_ERR
 
 
+# without the "is CUDA initialised" question of torch.cuda.current_device: asked where there are CUDA tensors
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+
+
 def _ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
@@ -127,7 +132,7 @@ def _ptr(t):
 def _stream():
     """Current torch stream handle; also binds the current device's context to this thread for the
     library's own CUDA runtime instance (autograd worker threads may not have one bound yet)."""
-    dev = torch.cuda.current_device()
+    dev = _current_device()
     rc = _LIB.dl4j_bind_device(dev)
     if rc != 0:
         raise RuntimeError(f"dl4j_bind_device failed with CUDA error {rc}")
@@ -136,7 +141,7 @@ def _stream():
 
 def on_current_device(*ts):
     """Whether every given tensor (or None) lives on the current device, where ``_stream`` launches."""
-    dev = torch.cuda.current_device()
+    dev = _current_device()
     for t in ts:
         if t is not None and t.get_device() != dev:          # -1: host memory
             return False
@@ -762,8 +767,8 @@ def _unit(t):
     return t.dim() == 2 and 1 in t.stride()
 
 
-def _sgemm_wins(M, N, K, relu):
-    """Whether the forward product of an fp32 layer (M rows, N units, a sum of K terms) leaves a library kernel short of tiles.  A tile of
+def _sgemm_wins(M, N, K, relu, grad):
+    """Whether an fp32 layer (M rows, N units, a sum of K terms) leaves a library kernel short of tiles.  A tile of
     64 x 64 has at most eight CTAs, so the time grows with K.  us of device time, here / library product [+ ReLU launch]:
         M, N          K = 256    1024      2048      4096      8192      25088
         64, 64        13 / 22    16 / 28   25 / 30   39 / 42   72 / 61   199 / 104
@@ -774,12 +779,14 @@ def _sgemm_wins(M, N, K, relu):
         32, 4096      15 / 22    33 / 40   55 / 47   98 / 74   186 / 111 543 / 319
         1, 4096       14 / 13    31 / 17   53 / 22
     Below 16 rows the library has matrix-vector kernels: 12 / 11 at K = 128, 12 / 13 at 256, 14 / 13 - 21 / 13 at 512.  Without a ReLU launch
-    to save: 128 x 512 x 10 6 / 9, 16 rows 12 / 8 at K = 128, 12 / 10 at 256, 12 / 12 at 512."""
+    to save: 128 x 512 x 10 6 / 9, 16 rows 12 / 8 at K = 128, 12 / 10 at 256, 12 / 12 at 512.
+    With a gradient to come the layer's backward saves what its product loses: replayed steps of 784-512-512-10 took 76 us here and 94 with
+    library products at 8 rows, 68 and 72 at one."""
     if ((M + 63) // 64) * ((N + 63) // 64) > 64:
         return False
-    if M < 16:
-        return relu and K <= 256
-    return K <= (4096 if M >= 64 else 1024) and (relu or K >= 256)
+    if not grad and (M < 16 and not (relu and K <= 256) or not relu and K < 256):
+        return False
+    return K <= (4096 if M >= 64 else 1024)
 
 
 def _sgemm_wins_dgrad(M, N, nIn):
@@ -796,11 +803,13 @@ def _sgemm_wins_dgrad(M, N, nIn):
     return N <= (4096 if M >= 64 else 512)
 
 
+_transforms, _tracing, _compiling = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state, torch.compiler.is_compiling
+
+
 def _plain_autograd():
     """No forward-mode level, functorch transform or tracer is active: the cases that differentiate or record through torch operators
     and that a custom autograd function does not serve."""
-    return torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None \
-        and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+    return forward_ad._current_level < 0 and _transforms() is None and _tracing() is None and not _compiling()
 
 
 _STEP = threading.local()
@@ -894,8 +903,11 @@ class _Linear32Fn(torch.autograd.Function):
 
 def linear32(x, W, b, relu):
     """fp32 dense layer on the small-problem kernel, or None when the case is not covered or the library does it better."""
-    if not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.float32 or W.dtype != torch.float32 or W.dim() != 2 \
-            or W.shape[0] != x.shape[1] or min(x.shape[0], *W.shape) == 0 or not _sgemm_wins(x.shape[0], W.shape[1], x.shape[1], relu) \
+    if not available() or x.dim() != 2 or x.dtype != torch.float32 or W.dtype != torch.float32 or W.dim() != 2 \
+            or W.shape[0] != x.shape[1] or min(x.shape[0], *W.shape) == 0:
+        return None
+    grad = torch.is_grad_enabled() and (x.requires_grad or W.requires_grad or (b is not None and b.requires_grad))
+    if not _sgemm_wins(x.shape[0], W.shape[1], x.shape[1], relu, grad) \
             or torch.backends.cuda.matmul.allow_tf32 or torch.is_autocast_enabled() or not _unit(x) or not on_current_device(x, W, b):
         return None
     if not ((W.stride(0) == 1 and W.stride(1) >= W.shape[0]) or (W.stride(1) == 1 and W.stride(0) >= W.shape[1])):
@@ -906,6 +918,8 @@ def linear32(x, W, b, relu):
         return None
     if x.stride(1) != 1:
         x = x.contiguous()
+    if not grad:
+        return _sgemm(x, W, torch.empty((x.shape[0], W.shape[1]), dtype=torch.float32, device=x.device), bias=b, act=1 if relu else 0)
     return _Linear32Fn.apply(x, W, b, bool(relu))
 
 

@@ -10,7 +10,7 @@ class _On:
 
 def test_rule(monkeypatch):
     from deeplearning4j_b200.ops import native
-    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    monkeypatch.setattr(native, "_current_device", lambda: 1)
     assert native.on_current_device(_On(1), None, _On(1))
     assert not native.on_current_device(_On(1), _On(0)) and not native.on_current_device(torch.zeros(2))
 
@@ -36,7 +36,7 @@ def test_routes_decline_tensors_of_another_device(monkeypatch):
         }
         for n, c in calls.items():
             assert c() is not None, n
-        monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+        monkeypatch.setattr(native, "_current_device", lambda: 1)
         for n, c in calls.items():
             assert c() is None, n
 

@@ -135,8 +135,8 @@ def test_negative_scale(T, causal, scale):
     grads = torch.autograd.grad(want, (q6, k6, v6), do.double())
     out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=scale, useCausalMask=causal).t
     dq, dv, dk = (a.t for a in Nd4j.exec("dot_product_attention_v2_bp", q, v, k, do, scale=scale, useCausalMask=causal))
-    # scores reach the hundreds: bf16 scores (the operator path) carry an error of 2^-9 of them into the exponent
-    tol = 1e-2 if abs(scale) < 1 else 0.5
+    # the operator path rounds the scores to bf16, 2^-9 of them, and that error goes into the exponent: scores to 16 and to 1000
+    tol = 4e-2 if abs(scale) < 1 else 0.5
     assert torch.isfinite(out).all() and (out.double() - want).norm() <= tol * want.norm()
     for a, b in zip((dq, dk, dv), grads):
         assert torch.isfinite(a).all() and (a.double() - b).norm() <= 3 * tol * (b.norm() + abs(scale) * do.double().norm())

@@ -25,7 +25,7 @@ def test_forward_and_gradients(M, K, N, f_order, act):
     leaves = [t.detach().requires_grad_(True) for t in (x, W, b)]
     before = native.LAUNCHES
     y = nnops.linear(*leaves, {None: None, "relu": ActivationReLU(), "tanh": ActivationTanH()}[act])
-    assert (native.LAUNCHES > before) == native._sgemm_wins(M, N, K, act == "relu")
+    assert (native.LAUNCHES > before) == native._sgemm_wins(M, N, K, act == "relu", True)
     got = torch.autograd.grad(y, leaves, dy)
     ref_leaves = [t.detach().double().requires_grad_(True) for t in (x, W, b)]
     z = ref_leaves[0] @ ref_leaves[1] + ref_leaves[2]
@@ -51,9 +51,10 @@ def test_both_sides_of_the_rule(M, N, K):
     from deeplearning4j_b200.nn.activations import ActivationReLU
     from deeplearning4j_b200.ops import native, nnops
     x, W, b, dy = _case(M, K, N, True, M + K + N)
-    before = native.LAUNCHES
-    y = nnops.linear(x, W, b, ActivationReLU())
-    assert (native.LAUNCHES > before) == (M * N <= 64 * 4096 and K <= (256 if M < 16 else 1024 if M < 64 else 4096))
+    for grad in (True, False):
+        before = native.LAUNCHES
+        y = nnops.linear(x, W.detach().requires_grad_(grad), b, ActivationReLU()).detach()
+        assert (native.LAUNCHES > before) == (M * N <= 64 * 4096 and K <= (256 if M < 16 and not grad else 1024 if M < 64 else 4096))
     want = torch.relu(x.double() @ W.double() + b.double())
     direct = native._sgemm(x, W, torch.empty(M, N, device="cuda"), bias=b, act=1)
     for u in (y, direct):
@@ -130,7 +131,7 @@ def test_gradients_repeat_bit_for_bit(M, K, N, relu):
         before = native.LAUNCHES
         y = nnops.linear(*leaves, ActivationReLU() if relu else None)
         g = torch.autograd.grad(y, leaves, dy)
-        assert native.LAUNCHES > before or not native._sgemm_wins(M, N, K, relu)
+        assert native.LAUNCHES > before or not native._sgemm_wins(M, N, K, relu, True)
         return (y.detach(), *g)
     first = run()
     for _ in range(10):
