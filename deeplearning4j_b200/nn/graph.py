@@ -416,17 +416,31 @@ class ComputationGraph(BaseNetwork):
         return {"steps": blob, "n": len(steps), "bytes": max(total, 256), "ext": ext, "region": inside,
                 "keep": [(n,) + env[n] + (where(env[n][0]),) for n in keep]}
 
+    def _run_plan(self, shape, start, compile_):
+        """The plan kept for a run that begins at ``start`` in a call of ``shape``, or what ``compile_`` gives.  One call may try several
+        starts, most of them without a run: the limit counts shapes, not starts."""
+        shapes = self.__dict__.setdefault("_run_plans", {})
+        plans = shapes.pop(shape, None)
+        if plans is None:
+            plans = {}
+        shapes[shape] = plans                                # the latest is last
+        while len(shapes) > 8:
+            try:
+                shapes.pop(next(iter(shapes)), None)
+            except (StopIteration, RuntimeError):            # another thread was at it
+                break
+        plan = plans.get(start)
+        if plan is None:
+            plan = plans[start] = compile_()
+        return plan
+
     def _folded_run(self, idx, acts, folded, folded_bn, fuse):
         """Runs the planned vertices from ``order[idx]`` on; returns them as a set (empty: nothing was run).  A plan depends on the shapes
-        of the activations it starts from; the eight most recent are kept."""
+        of the activations it starts from; those of the eight most recently used shapes are kept.  Threads may share the network."""
         from ..ops import native
-        plans = self.__dict__.setdefault("_run_plans", {})
-        key = (idx, len(folded_bn), self._fold_table["sig"]) + tuple((n, tuple(t.shape)) for n, t in acts.items() if _dense_nhwc(t, self.flat_params.device))
-        plan = plans.get(key)
-        if plan is None:
-            while len(plans) >= 8:
-                plans.pop(next(iter(plans)), None)
-            plan = plans[key] = self._compile_run(idx, acts, folded, folded_bn, fuse) or {"n": 0}
+        plan = self._run_plan((tuple(next(iter(acts.values())).shape), self._fold_table["sig"]),
+                              (idx, len(folded_bn)) + tuple((n, tuple(t.shape)) for n, t in acts.items() if _dense_nhwc(t, self.flat_params.device)),
+                              lambda: self._compile_run(idx, acts, folded, folded_bn, fuse) or {"n": 0})
         if not plan["n"]:
             return ()
         ins = [acts[n] for n in plan["ext"]]
