@@ -1271,8 +1271,10 @@ def transpose16(m):
 
 
 def lstm_seq_supported(zx, n, mb):
-    """Hidden sizes off the 64 grid run zero-padded (``lstm_seq``)."""
-    return (available() and zx.is_cuda and zx.dtype == torch.bfloat16 and 1 <= n <= 1280 and 1 <= mb <= 128)
+    """Hidden sizes off the 64 grid run zero-padded (``lstm_seq``) from two steps on; for a single one the padding costs more than the
+    general step (two layers of 500 units, 100 rows: inference 595 against 457 us, training 1934 against 1535; at two steps 594 against
+    620 and 1958 against 1982)."""
+    return (available() and zx.is_cuda and zx.dtype == torch.bfloat16 and 1 <= n <= 1280 and 1 <= mb <= 128 and (n % 64 == 0 or zx.shape[0] > 1))
 
 
 def lstm_seq(zx, rw, h0, c0, reverse=False):

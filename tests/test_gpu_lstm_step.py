@@ -108,3 +108,19 @@ def test_sequence_kernels_repeat_bit_for_bit(n, mb):
         got = run()
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     native.check_status()
+
+
+@pytest.mark.parametrize("n,mb,T,seq", [(300, 120, 1, False), (300, 120, 2, True), (320, 120, 1, True), (1000, 40, 1, False)])
+def test_route_of_a_single_step(monkeypatch, n, mb, T, seq):
+    """One step of a size off the 64 grid takes the general path, two take the padded sequence kernel; same values either way."""
+    from deeplearning4j_b200.ops import native
+    calls, apply = [], native._LstmSeqFn.apply
+    monkeypatch.setattr(native._LstmSeqFn, "apply", lambda *a: calls.append(1) or apply(*a))
+    net = _net(16, n, 1)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(T, mb, 16, generator=g, device="cuda").bfloat16().float()
+    out = net.output(x.permute(1, 2, 0)).t
+    with torch.no_grad():
+        logits, _, _ = _ref(net, x.double(), 1, n)
+    want = torch.softmax(logits, -1).permute(1, 2, 0)
+    assert (len(calls) > 0) == seq and (out.double() - want).norm() <= 1.5e-2 * want.norm()
