@@ -4,7 +4,7 @@
 //
 // One block per hidden unit, one warp per gate (order a | f | o | g): the gate's column of W and of RW is contiguous in the 'f'-ordered
 // parameters, the lanes split it and keep eight batch rows' partial sums, the columns are re-read from L1 for the next eight rows.
-// The weights are the parameters themselves (fp32, or bf16 where the network holds them so): no shadow to be stale, no rounding.
+// The weights are the fp32 parameters themselves: no shadow to be stale, no rounding.
 // Sums, bias and cell are fp32 throughout; only h is rounded.  h_out may not alias h.
 // The same dot product serves a dense layer of a few rows whose width the tensor-core kernels cannot address (a 77-symbol alphabet),
 // which took two casts of the parameters and a library product.
@@ -40,9 +40,8 @@ __device__ __forceinline__ void lt_dot(const TW* __restrict__ w, const __nv_bflo
   }
 }
 
-template <typename TW>
 __global__ void __launch_bounds__(128)
-lstm_step_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const TW* __restrict__ W, const TW* __restrict__ RW,
+lstm_step_kernel(const __nv_bfloat16* __restrict__ x, long ldx, const float* __restrict__ W, const float* __restrict__ RW,
                  const float* __restrict__ bias, const __nv_bfloat16* __restrict__ h, const float* __restrict__ c,
                  __nv_bfloat16* __restrict__ h_out, float* __restrict__ c_out, int mb, int nIn, int n, int vec_x, int vec_h) {
   __shared__ float z[4][LT_ROWS];
@@ -101,19 +100,14 @@ using namespace dl4j;
 
 static bool lt_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// x [mb, nIn] bf16 (row stride ldx), W [nIn, 4n] and RW [n, 4n] column-major ('f'), fp32 or bf16; bias fp32 [4n] or null, h [mb, n]
-// bf16, c [mb, n] fp32.
-DL4J_API int dl4j_lstm_step(const void* x, long ldx, const void* W, const void* RW, int w_fp32, const float* bias, const void* h,
-                            const float* c, void* h_out, float* c_out, int mb, int nIn, int n, void* stream) {
+// x [mb, nIn] bf16 (row stride ldx), W [nIn, 4n] and RW [n, 4n] fp32 column-major ('f'), bias fp32 [4n] or null, h [mb, n] bf16, c [mb, n] fp32.
+DL4J_API int dl4j_lstm_step(const void* x, long ldx, const float* W, const float* RW, const float* bias, const void* h, const float* c,
+                            void* h_out, float* c_out, int mb, int nIn, int n, void* stream) {
   if (mb < 1 || nIn < 1 || n < 1 || h == h_out) return -DL4J_ERR_BAD_ARG;
   const int vec_x = nIn % 8 == 0 && ldx % 8 == 0 && lt_aligned(x) && lt_aligned(W), vec_h = n % 8 == 0 && lt_aligned(h) && lt_aligned(RW);
   using B = __nv_bfloat16;
-  if (w_fp32)
-    lstm_step_kernel<float><<<n, 128, 0, (cudaStream_t)stream>>>((const B*)x, ldx, (const float*)W, (const float*)RW, bias, (const B*)h, c,
-                                                                (B*)h_out, c_out, mb, nIn, n, vec_x, vec_h);
-  else
-    lstm_step_kernel<B><<<n, 128, 0, (cudaStream_t)stream>>>((const B*)x, ldx, (const B*)W, (const B*)RW, bias, (const B*)h, c, (B*)h_out,
-                                                            c_out, mb, nIn, n, vec_x, vec_h);
+  lstm_step_kernel<<<n, 128, 0, (cudaStream_t)stream>>>((const B*)x, ldx, W, RW, bias, (const B*)h, c, (B*)h_out, c_out, mb, nIn, n, vec_x,
+                                                        vec_h);
   return (int)cudaGetLastError();
 }
 

@@ -56,11 +56,8 @@ def _load():
             "dl4j_threshold_encode": [vp, i64, f32, vp, i32, vp],
             "dl4j_threshold_decode": [vp, i32, vp, i64, f32, i32, vp],
             "dl4j_bitmap_encode_to": [vp, vp, i64, f32, vp, vp],
-            "dl4j_bitmap_encode": [vp, i64, f32, vp, vp],
             "dl4j_bitmap_decode_to": [vp, vp, vp, i64, f32, vp],
-            "dl4j_bitmap_decode": [vp, vp, i64, f32, vp],
             "dl4j_layer_norm_fwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, f32, i32, vp],
-            "dl4j_layer_norm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp],
             "dl4j_layer_norm_grad": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, f32, i32, i32, i32, vp],
             "dl4j_softmax_xent": [vp, vp, vp, vp, vp, i32, i32, i64, i32, i32, vp],
             "dl4j_scatter_add_rows": [vp, vp, vp, i64, i32, i64, i64, i32, vp],
@@ -670,11 +667,6 @@ def _on_pitch(t, dtype):
     if t.stride(1) != 1 or (t.dtype != dtype and t.dtype != torch.float32):
         t = t.to(dtype).contiguous()
     return pitch_copy(t, _pitched(t.shape[0], t.shape[1], dtype, t.device))
-
-
-def _full_rows(t):
-    """A pitched matrix with its padding columns (whatever they hold)."""
-    return t.as_strided((t.shape[0], t.stride(0)), (t.stride(0), 1))
 
 
 class _OddLinearFn(torch.autograd.Function):
@@ -1302,15 +1294,15 @@ def lstm_seq(zx, rw, h0, c0, reverse=False):
     return hs[..., :n], h[:, :n].contiguous(), c[:, :n].contiguous()
 
 
-def _f_ordered(w):
-    """A weight whose columns are contiguous (the 'f'-ordered parameter views), in a type the small kernels read."""
-    return w.dim() == 2 and w.is_cuda and w.dtype in (torch.float32, torch.bfloat16) and w.stride(0) == 1 and w.stride(1) == w.shape[0]
+def _f_ordered(w, *types):
+    """A weight of one of the given types whose columns are contiguous (the 'f'-ordered parameter views)."""
+    return w.dim() == 2 and w.is_cuda and w.dtype in types and w.stride(0) == 1 and w.stride(1) == w.shape[0]
 
 
 def lstm_step_supported(x, W, RW, n, mb, *rest):
     """One inference step as one launch (``csrc/lstm_step.cu``) for mb * n up to LSTM_STEP_MAX; ``rest``: its other operands."""
     return (available() and x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled() and mb * n <= LSTM_STEP_MAX
-            and _f_ordered(W) and _f_ordered(RW) and W.dtype == RW.dtype and on_current_device(x, W, RW, *rest)
+            and _f_ordered(W, torch.float32) and _f_ordered(RW, torch.float32) and on_current_device(x, W, RW, *rest)
             and _plain_autograd())
 
 
@@ -1323,7 +1315,7 @@ LSTM_STEP_MAX = 32768
 def _small_sigs(l):
     if not hasattr(l.dl4j_lstm_step, "_typed"):
         vp, i32, lng = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
-        l.dl4j_lstm_step.argtypes = [vp, lng, vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, vp]
+        l.dl4j_lstm_step.argtypes = [vp, lng, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, vp]
         l.dl4j_lstm_step.restype = i32
         l.dl4j_linear_small.argtypes = [vp, lng, vp, i32, vp, vp, i32, i32, i32, vp]
         l.dl4j_linear_small.restype = i32
@@ -1332,13 +1324,13 @@ def _small_sigs(l):
 
 
 def lstm_step(x, W, RW, b, h, c):
-    """(h', c') of one LSTM step: x [mb, nIn] bf16, W [nIn, 4n] / RW [n, 4n] column-major, b fp32, h [mb, n] bf16, c [mb, n] fp32."""
+    """(h', c') of one LSTM step: x [mb, nIn] bf16, W [nIn, 4n] / RW [n, 4n] fp32 column-major, b fp32, h [mb, n] bf16, c [mb, n] fp32."""
     l = _small_sigs(require())
     mb, nIn = x.shape
     x = x if x.stride(1) == 1 else x.contiguous()
     h, c = h.contiguous(), c.contiguous()
     h_out, c_out = torch.empty_like(h), torch.empty_like(c)
-    rc = l.dl4j_lstm_step(_ptr(x), x.stride(0), _ptr(W), _ptr(RW), int(W.dtype == torch.float32), _ptr(b), _ptr(h), _ptr(c), _ptr(h_out),
+    rc = l.dl4j_lstm_step(_ptr(x), x.stride(0), _ptr(W), _ptr(RW), _ptr(b), _ptr(h), _ptr(c), _ptr(h_out),
                           _ptr(c_out), mb, nIn, h.shape[1], _stream())
     _check(rc, "dl4j_lstm_step")
     return h_out, c_out
@@ -1347,7 +1339,7 @@ def lstm_step(x, W, RW, b, h, c):
 def linear_small(x, W, b):
     """``x @ W + b`` without a gradient for up to 32 rows of bf16 activations on the parameters themselves, or None when not covered."""
     if torch.is_grad_enabled() or not available() or not x.is_cuda or x.dim() != 2 or x.dtype != torch.bfloat16 or not 1 <= x.shape[0] <= 32 \
-            or not _f_ordered(W) or W.shape[0] != x.shape[1] or W.numel() == 0 or (b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1])) \
+            or not _f_ordered(W, torch.float32, torch.bfloat16) or W.shape[0] != x.shape[1] or W.numel() == 0 or (b is not None and (b.dtype != torch.float32 or b.numel() != W.shape[1])) \
             or not on_current_device(x, W, b) or not _plain_autograd():
         return None
     l = _small_sigs(require())

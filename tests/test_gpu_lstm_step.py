@@ -63,8 +63,7 @@ def test_padded_hidden_sizes_train(n, mb, T):
 
 
 @pytest.mark.parametrize("n,mb,n_in", [(1, 1, 1), (8, 2, 5), (33, 9, 77), (256, 1, 77), (200, 64, 98), (512, 33, 16), (1024, 32, 40)])
-@pytest.mark.parametrize("bf16_params", [False])
-def test_one_step_matches_fp64(n, mb, n_in, bf16_params):
+def test_one_step_matches_fp64(n, mb, n_in):
     """Three consecutive steps: h is rounded to bf16 once per layer and step, nothing else is."""
     from deeplearning4j_b200.ops import native
     net = _net(n_in, n, 2)
@@ -124,3 +123,20 @@ def test_route_of_a_single_step(monkeypatch, n, mb, T, seq):
         logits, _, _ = _ref(net, x.double(), 1, n)
     want = torch.softmax(logits, -1).permute(1, 2, 0)
     assert (len(calls) > 0) == seq and (out.double() - want).norm() <= 1.5e-2 * want.norm()
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (3, 24, 77), (8, 77, 10), (9, 256, 5), (32, 131, 33)])
+@pytest.mark.parametrize("wdtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("bias", [True, False])
+def test_small_dense_layers_without_a_gradient(M, K, N, wdtype, bias):
+    """A few rows on the parameters themselves, in either type they are held in: one rounding of the result."""
+    from deeplearning4j_b200.ops import native
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    base = torch.randn(M * K + 1, generator=g, device="cuda").bfloat16()
+    W = torch.randn(N, K, generator=g, device="cuda").to(wdtype).t()
+    b = torch.randn(1, N, generator=g, device="cuda") if bias else None
+    with torch.no_grad():
+        for x in (base[:M * K].view(M, K), base[1:].view(M, K)):
+            y = native.linear_small(x, W, b)
+            want = x.double() @ W.double() + (b.double() if bias else 0.0)
+            assert y.dtype == torch.bfloat16 and (y.double() - want).norm() <= 2 ** -8 * want.norm()
