@@ -57,9 +57,9 @@ __device__ __forceinline__ float relu_f(float v) {
   return y;
 }
 
-// One thread of a converged warp.  Code that issues tcgen05.mma sits under this and not under `lane == 0`: the compiler knows that a
-// single thread is active after elect.sync and keeps the instruction's descriptors in uniform registers; after a plain comparison it
-// does not, and one thread gets an instruction out per ~147 clocks instead of ~64 (mma_issue_probe.cu).  512 x 512 x 2048 GEMM:
+// One thread of a converged warp.  Code that issues tcgen05.mma sits under this and not under `lane == 0`: measured, a thread chosen by
+// elect.sync gets an instruction out per ~64 clocks (127 at N = 256, the tensor core's own rate), one under `lane == 0` per ~147.
+// 512 x 512 x 2048 GEMM:
 // 14.5 -> 10.3 us, 16384 x 768 x 3072 in 128-column tiles: 99 -> 70 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;

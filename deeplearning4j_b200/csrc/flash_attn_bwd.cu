@@ -310,12 +310,12 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
-      // dQ of the previous block: read out of tensor memory and reduced into global memory now, while the MMA thread issues
-      // the dV / dK products of this block (the reductions stall their warp on the L2 atomics queue for about a microsecond)
+      // dQ of the previous block: read out of tensor memory and handed to the copy engine now, while the MMA threads issue the dV / dK
+      // products of this block
       if (i > 0 && !dq_flush(i - 1)) { ok = false; break; }
     }
     if (ok && nq > 0) ok = dq_flush(nq - 1);
-    if (lane == 0) bulk_wait<0>();                    // the reductions are done before the shared memory goes
+    if (lane == 0) bulk_wait<0>();                    // the copies are done before the shared memory goes
     if (ok && mbar_wait_bounded(fin_full, 0, p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) {
       tc_fence_after();
       // accumulator rows are keys here: thread r owns key k0 + r; column groups 0, 1 -> dV, 2, 3 -> dK

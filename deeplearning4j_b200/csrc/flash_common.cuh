@@ -1,4 +1,4 @@
-// Shared pieces of the fused attention kernels (head size 64, bf16).
+// Shared pieces of the fused attention kernels (head sizes up to 64, bf16).
 #pragma once
 #include "common.cuh"
 

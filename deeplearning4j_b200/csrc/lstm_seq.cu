@@ -58,7 +58,7 @@ __device__ __forceinline__ void epilogue_bar_sync() { asm volatile("bar.sync 1, 
 
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-// Acquire loads: once the target is seen, the other CTAs' stores that preceded their (fenced) arrivals are visible to this thread;
+// Acquire loads: once the target is seen, the other CTAs' stores that preceded their arrivals (released) are visible to this thread;
 // no separate fence is needed after the wait.
 __device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
   unsigned int v;
