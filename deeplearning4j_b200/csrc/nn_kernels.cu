@@ -801,10 +801,10 @@ bias_act_bwd_vec_kernel(const T* __restrict__ dy, const T* __restrict__ z, T* __
 }
 
 // The fp32 form with a bias gradient of up to 4096 rows: every sum has one order, so that a layer's gradients repeat bit for bit (the
-// atomics of the other forms add in arrival order).  A block of 32 x 32 threads owns 32 columns and takes 256 rows at a time, eight per
+// atomics of the other forms add in arrival order).  A block of 32 x 32 threads owns 32 columns and takes 128 rows at a time, four per
 // thread in flight; its column sums fold by shuffles.  More than 512 rows are split over the blocks of a cluster, whose first block adds
-// the slabs in order (two cluster barriers: 1.5 us).
-// Latency-bound at these sizes: a round of four rows per thread took 0.8 us; 128 x 512 in 2.6 us, with atomics 3.1.
+// the slabs in order.
+// Latency-bound at these sizes (128 x 512: 262 KB in, 262 KB out).
 __global__ void __launch_bounds__(1024)
 bias_act_bwd_f32_kernel(const float* __restrict__ dy, const float* __restrict__ z, float* __restrict__ dz, float* __restrict__ dbias,
                         int rows, int C, int act, int rows_per_block) {
@@ -815,18 +815,17 @@ bias_act_bwd_f32_kernel(const float* __restrict__ dy, const float* __restrict__ 
   const int r0 = blockIdx.y * rows_per_block;
   const int r1 = col < C ? min(r0 + rows_per_block, rows) : 0;
   float s = 0.f;
-  constexpr int U = 8;
-  for (int r = r0 + ty; r < r1; r += 32 * U) {
-    float d[U], v[U];
+  for (int r = r0 + ty; r < r1; r += 128) {
+    float d[4], v[4];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < 4; ++u) {
       const long long o = (long long)(r + 32 * u) * C + col;
       const bool in = r + 32 * u < r1;
       d[u] = in ? __ldg(dy + o) : 0.f;
       v[u] = in && act != 0 ? __ldg(z + o) : 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < 4; ++u) {
       if (r + 32 * u < r1) {
         if (act == 1) d[u] = v[u] <= 0.f ? 0.f : d[u];           // the library's rule: an infinite gradient stops at a unit that is off
         else if (act != 0) d[u] *= act_grad(v[u], act);
@@ -1131,7 +1130,7 @@ DL4J_API int dl4j_bias_act_bwd(const void* dy, const void* z, void* dz, float* d
   const bool aligned = (((uintptr_t)dy | (uintptr_t)(act != 0 ? z : nullptr) | (uintptr_t)dz) & 15) == 0;
   if (dtype == 2 && dbias && rows <= 4096) {
     int slabs = 1;
-    while (rows > 512 && slabs < 8 && slabs * 256 < rows) slabs *= 2;
+    while (slabs * 512 < rows) slabs *= 2;                      // up to 8
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((C + 31) / 32, slabs);
     cfg.blockDim = dim3(1024);
