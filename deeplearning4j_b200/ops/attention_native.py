@@ -21,16 +21,14 @@ _LONG2 = ctypes.c_long * 2
 
 
 def _ok_view(t):
-    """[B, H, T, D] view usable by a rank-4 tensor map: unit inner stride, 16-byte aligned strides."""
+    """[B, H, T, D] view usable by a rank-4 tensor map: unit inner stride, 16-byte aligned strides, none of them 0 (an expanded axis)."""
     s = t.stride()
-    return len(s) == 4 and s[3] == 1 and not (s[0] | s[1] | s[2]) & 7 and t.data_ptr() % 16 == 0 and t.shape[3] % 8 == 0
+    return len(s) == 4 and s[3] == 1 and not (s[0] | s[1] | s[2]) & 7 and s[0] and s[1] and s[2] and t.data_ptr() % 16 == 0 and t.shape[3] % 8 == 0
 
 
 def _prep(t):
-    if _ok_view(t):
-        return t
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
+    # a copy also where the tensor counts as contiguous: an extent of one leaves its stride open, and the map wants all of them aligned
+    return t if _ok_view(t) else t.clone(memory_format=torch.contiguous_format)
 
 
 def _bgemm(l, A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, alpha, H, Bn, a_bs, b_bs, c_bs, dtype, out_fp32=0):

@@ -36,3 +36,20 @@ def test_is_differentiable():
     q, k, v, do = (torch.randn(1, 1, 3, 8, dtype=torch.float64, requires_grad=True) for _ in range(4))
     out = _grad_in_ops(q, k, v, do, None, 0.3, 1)
     assert all(t is not None for t in torch.autograd.grad([(o ** 2).sum() for o in out], (q, k, v, do)))
+
+
+@pytest.mark.parametrize("make", [
+    lambda: torch.randn(1, 1, 1, 33)[..., :32],                                     # one row: any pitch counts as contiguous
+    lambda: torch.randn(2, 1, 5, 32).expand(2, 3, 5, 32),                           # one head for all
+    lambda: torch.randn(1, 1, 1, 32).expand(2, 3, 5, 32),
+    lambda: torch.randn(2, 3, 5, 36)[..., :32],
+    lambda: torch.randn(2 * 3 * 5 * 32 + 1)[1:].view(2, 3, 5, 32),
+    lambda: torch.randn(2, 3, 32, 5).transpose(-1, -2),
+])
+def test_operands_are_laid_out_for_the_tensor_map(make):
+    from deeplearning4j_b200.ops.attention_native import _ok_view, _prep
+    t = make()
+    p = _prep(t)
+    assert torch.equal(p, t) and _ok_view(p) and p.is_contiguous()
+    ok = torch.randn(2, 5, 3, 32).permute(0, 2, 1, 3)
+    assert _prep(ok) is ok

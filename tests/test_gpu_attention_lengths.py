@@ -195,3 +195,22 @@ def test_gradients_repeat_bit_for_bit(Tq, Tk, causal, D, masked):
     ok = slice(1, 2) if masked and causal else slice(None)                          # example 0 has rows without keys there
     for a, b in zip((first[0], first[2]), want[:2]):
         assert (a.double() - b)[ok].norm() <= 1e-2 * (b[ok].norm() + size)
+
+
+@pytest.mark.parametrize("Tq,Tk", [(1, 1), (1, 37), (33, 33), (128, 128)])
+def test_expanded_and_oddly_pitched_operands(Tq, Tk):
+    """One key head for all query heads, and single rows cut from a buffer of an odd pitch."""
+    from deeplearning4j_b200.nd.nd4j import Nd4j
+    g = torch.Generator(device="cuda").manual_seed(Tk)
+    t = lambda H, T: torch.randn(1, H, T, 35, generator=g, device="cuda").bfloat16()[..., :32]
+    H = 1 if Tq == Tk == 1 else 4
+    q, k, v, do = t(H, Tq), t(1, Tk).expand(1, H, Tk, 32), t(1, Tk).expand(1, H, Tk, 32), t(H, Tq)
+    q6, k6, v6 = (a.double().requires_grad_(True) for a in (q, k, v))
+    want = _ref(q6, k6, v6, 0.2, None, False)
+    grads = torch.autograd.grad(want, (q6, k6, v6), do.double())
+    out = Nd4j.exec("dot_product_attention_v2", q, v, k, scale=0.2).t
+    assert (out.double() - want).norm() <= 1e-2 * want.norm()
+    dq, dv, dk = (a.t for a in Nd4j.exec("dot_product_attention_v2_bp", q, v, k, do, scale=0.2))
+    size = do.double().norm() * 0.2
+    for a, b in zip((dq, dk, dv), grads):
+        assert a.shape == b.shape and (a.double() - b).norm() <= 1e-2 * (b.norm() + size)
