@@ -23,7 +23,7 @@ _LONG2 = ctypes.c_long * 2
 def _ok_view(t):
     """[B, H, T, D] view usable by a rank-4 tensor map: unit inner stride, 16-byte aligned strides, none of them 0 (an expanded axis)."""
     s = t.stride()
-    return len(s) == 4 and s[3] == 1 and not (s[0] | s[1] | s[2]) & 7 and s[0] and s[1] and s[2] and t.data_ptr() % 16 == 0 and t.shape[3] % 8 == 0
+    return len(s) == 4 and s[3] == 1 and not (s[0] | s[1] | s[2]) & 7 and s[0] and s[1] and s[2] and t.data_ptr() % 16 == 0 and t.size(3) % 8 == 0
 
 
 def _prep(t):
@@ -193,7 +193,8 @@ def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
         return None
     if _bad_mask(q, k, mask) or not native.on_current_device(q, k, v, mask) or not native._plain_autograd():
         return None
-    D, Tk, Tq = q.shape[3], k.shape[2], q.shape[2]
+    _, _, Tq, D = q.shape
+    Tk = k.size(2)
     scale = float(scale) if scale is not None else D ** -0.5
     # the fused kernels take a row's maximum over raw scores: with a negative scale that is the smallest exponent, and exp overflows
     fused = scale >= 0.0 and flash_supported(q, k, v)
@@ -226,9 +227,9 @@ def attention_grad(q, k, v, mask, scale, dout, causal=False):
     mk = mask.detach().to(torch.float32).contiguous() if mask is not None else None
     stats = torch.empty((2, Bn, H, Tq), dtype=torch.float32, device=q.device)
     lse, dvec = stats[0], stats[1]
-    rc = _flash_lib().dl4j_flash_attn_fwd(native._ptr(q), native._ptr(k), native._ptr(v), None, native._ptr(lse), native._ptr(mk), Bn, H, Tq,
-                                          k.shape[2], D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), scale,
-                                          flags, native._ptr(dout), _LONG3(*dout.stride()[:3]), native._ptr(dvec), 0.0, None,
+    rc = _flash_lib().dl4j_flash_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), None, lse.data_ptr(), native._ptr(mk), Bn, H, Tq,
+                                          k.size(2), D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), scale,
+                                          flags, dout.data_ptr(), _LONG3(*dout.stride()[:3]), dvec.data_ptr(), 0.0, None,
                                           native._stream())
     native._check(rc, "dl4j_flash_attn_fwd")
     return _flash_backward(q, k, v, dout, lse, dvec, mk, scale, flags, 0.0, None)
@@ -302,8 +303,8 @@ def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
     elif blocks > 1:
         acc = torch.zeros((Bn, H, Tq, D), dtype=torch.float32, device=q.device)
     stream = native._stream()
-    rc = l.dl4j_flash_attn_bwd(native._ptr(q), native._ptr(k), native._ptr(v), native._ptr(dO), native._ptr(lse), native._ptr(dvec),
-                               native._ptr(mk), native._ptr(acc), native._ptr(dq_t), native._ptr(dk_t), native._ptr(dv_t), Bn, H, Tq, Tk, D,
+    rc = l.dl4j_flash_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), dO.data_ptr(), lse.data_ptr(), dvec.data_ptr(),
+                               native._ptr(mk), native._ptr(acc), dq_t.data_ptr(), dk_t.data_ptr(), dv_t.data_ptr(), Bn, H, Tq, Tk, D,
                                _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), _LONG3(*dO.stride()[:3]),
                                dq_t.stride(0), dq_t.stride(1), dk_t.stride(0), dk_t.stride(1), scale, flags, dropout_p, native._ptr(seed),
                                stream)
@@ -331,8 +332,8 @@ def flash_forward(q, k, v, key_mask, scale, dropout_p=0.0, seed=None, flags=0):
     out = torch.empty((Bn, Tq, H, D), dtype=q.dtype, device=q.device)
     lse = torch.empty((Bn, H, Tq), dtype=torch.float32, device=q.device)
     mk = key_mask.to(torch.float32).contiguous() if key_mask is not None else None
-    rc = l.dl4j_flash_attn_fwd(native._ptr(q), native._ptr(k), native._ptr(v), native._ptr(out), native._ptr(lse), native._ptr(mk), Bn, H, Tq,
-                               k.shape[2], D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), float(scale), flags,
+    rc = l.dl4j_flash_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), native._ptr(mk), Bn, H, Tq,
+                               k.size(2), D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), float(scale), flags,
                                None, None, None, float(dropout_p), native._ptr(seed), native._stream())
     native._check(rc, "dl4j_flash_attn_fwd")
     return out, lse

@@ -795,13 +795,13 @@ def _sgemm_wins_dgrad(M, N, nIn):
     return N <= (4096 if M >= 64 else 512)
 
 
-_transforms, _tracing, _compiling = torch._C._functorch.peek_interpreter_stack, torch._C._get_tracing_state, torch.compiler.is_compiling
+_transforms, _tracing, _compiling = torch._C._functorch.peek_interpreter_stack, torch._C._is_tracing, torch.compiler.is_compiling
 
 
 def _plain_autograd():
     """No forward-mode level, functorch transform or tracer is active: the cases that differentiate or record through torch operators
     and that a custom autograd function does not serve."""
-    return forward_ad._current_level < 0 and _transforms() is None and _tracing() is None and not _compiling()
+    return forward_ad._current_level < 0 and _transforms() is None and not _tracing() and not _compiling()
 
 
 _STEP = threading.local()
