@@ -14,6 +14,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
+from ...ops import native as nat
 from ...ops import nnops
 from ..activations import Activation, ActivationSigmoid, ActivationTanH
 from ..conf.base import BaseLayer, FeedForwardLayer, InputType, Layer, ParamSpec, RNNFormat, _L
@@ -106,7 +107,6 @@ class LSTM(BaseRecurrentLayer):
         gate, act = self.gateActivationFn, self.activation
         plain = isinstance(gate, ActivationSigmoid) and isinstance(act, ActivationTanH) and not self.PEEPHOLE
         if T == 1 and plain and mask is None and not training and x.is_cuda and not nnops._FORCE_TORCH:
-            from ...ops import native as nat
             if nat.lstm_step_supported(xt, W, RW, n, mb, b, h, c) and h.dtype == x.dtype and c.dtype == torch.float32 \
                     and (b is None or b.dtype == torch.float32) and h.shape == c.shape == (mb, n):
                 h, c = nat.lstm_step(xt[0], W, RW, None if b is None else b.detach().reshape(-1), h, c)
@@ -115,7 +115,6 @@ class LSTM(BaseRecurrentLayer):
         # one GEMM for all time steps' input contributions
         zx = nnops.linear(xt.reshape(T * mb, -1), W, b).reshape(T, mb, 4 * n)
         if plain and mask is None and c.dtype == torch.float32 and not nnops._FORCE_TORCH:
-            from ...ops import native as nat
             if nat.lstm_seq_supported(zx, n, mb) and h.dtype == zx.dtype:
                 # whole sequence in one persistent kernel (recurrent weights resident on chip)
                 hs, h, c = nat.lstm_seq(zx, RW if RW.shape[1] == 4 * n else RW4, h, c, reverse)

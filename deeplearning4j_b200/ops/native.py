@@ -1855,12 +1855,10 @@ def add_relu(a, b):
 
 
 def attention(q, k, v, mask, scale, dropout_p=0.0, causal=False):
-    from . import attention_native
     return attention_native.attention(q, k, v, mask, scale, dropout_p, causal)
 
 
 def attention_grad(q, k, v, mask, scale, dout, causal=False):
-    from . import attention_native
     return attention_native.attention_grad(q, k, v, mask, scale, dout, causal)
 
 
@@ -2088,3 +2086,6 @@ def barnes_edge_forces(row_p, col_p, val_p, y):
     rc = l.dl4j_barnes_edge_forces(_ptr(row_p), _ptr(col_p), _ptr(val_p), _ptr(y), _ptr(out), N, D, _stream())
     _check(rc, "dl4j_barnes_edge_forces")
     return out
+
+
+from . import attention_native  # noqa: E402  (it imports this module; a relative import inside the two calls above costs 1 us each time)
