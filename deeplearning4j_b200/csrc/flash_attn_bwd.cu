@@ -35,6 +35,7 @@ struct FlashBwdParams {
   const float* dvec;         // [B, H, Tq]  rowsum(dO * O)
   const float* key_mask;     // [B, Tk] or null
   float* dq;                 // [B, H, Tq, D] fp32, zero on entry; null: dq16 is written directly (one key block)
+  int dq_slabs;              // dq is [key blocks, B, H, Tq, D] instead: every key block stores its part, nothing is added
   __nv_bfloat16* dq16;       // [B, Tq, H, D]
   __nv_bfloat16* dk;         // [B, Tk, H, D]
   __nv_bfloat16* dv;         // [B, Tk, H, D]
@@ -50,9 +51,7 @@ struct FlashBwdParams {
   float inv_keep;
 };
 
-// SLABS: dq is [key blocks, B, H, Tq, D], every key block stores its part and nothing is added (decided at compile time: as a branch in the
-// flush it cost the adding form 2.5 of 264 us)
-template <bool DROP, bool SLABS>
+template <bool DROP>
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -242,7 +241,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         const int row0 = (i0 + blk) * FB_BLK + q * 32;
         if (lane == 0) {
           if (row0 < p.Tq && cq * 16 < p.D) {
-            if constexpr (SLABS) tma_store_4d(&tmap_dq, slab, cq * 16, row0, h, kb * p.B + b);
+            if (p.dq_slabs) tma_store_4d(&tmap_dq, slab, cq * 16, row0, h, kb * p.B + b);
             else tma_reduce_add_4d(&tmap_dq, slab, cq * 16, row0, h, b);
           }
           bulk_commit();
@@ -354,8 +353,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 // q / k / v / dout: [B, H, T, D] bf16 views (element strides {sb, sh, st}), D a multiple of 8 up to 64; lse, dvec [B, H, Tq] fp32;
 // dq_acc [B, H, Tq, D] fp32 zeroed by the caller, or null with at most 128 keys: dq is then written here, addressed as
 // base + b * q_bs + query * q_ts + head * D; dk, dv bf16 addressed as base + b * o_bs + key * o_ts + head * D.
-// flags as in dl4j_flash_attn_fwd; 4: dq_acc is [key blocks, B, H, Tq, D], need not be zeroed, and every key block stores its part there
-// (not with dropout).
+// flags as in dl4j_flash_attn_fwd; 4: dq_acc is [key blocks, B, H, Tq, D], need not be zeroed, and every key block stores its part there.
 DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* dvec,
                                  const float* key_mask, float* dq_acc, void* dq, void* dk, void* dv, int B, int H, int Tq, int Tk, int D,
                                  const long* q_strides, const long* k_strides, const long* v_strides, const long* do_strides, long q_bs,
@@ -389,6 +387,7 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   FlashBwdParams p;
   p.lse = lse; p.dvec = dvec; p.key_mask = key_mask;
   p.dq = dq_acc;
+  p.dq_slabs = (flags >> 2) & 1;
   p.dq16 = reinterpret_cast<__nv_bfloat16*>(dq);
   p.q_bs = q_bs; p.q_ts = q_ts;
   p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
@@ -403,9 +402,7 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   p.drop_thr = dropout_p > 0.f ? (uint32_t)(dropout_p * 65536.f + 0.5f) : 0u;
   p.inv_keep = p.drop_thr ? 65536.f / (65536.f - (float)p.drop_thr) : 1.f;
   const size_t smem = 6 * FB_TILE + 2 * FB_PS + FB_DQ + FB_BLK * sizeof(float) + 256 + 1024;
-  const bool slabs = (flags & 4) != 0;
-  if (slabs && p.drop_thr) return -DL4J_ERR_BAD_ARG;
-  auto kern = p.drop_thr ? flash_attn_bwd_kernel<true, false> : (slabs ? flash_attn_bwd_kernel<false, true> : flash_attn_bwd_kernel<false, false>);
+  auto kern = p.drop_thr ? flash_attn_bwd_kernel<true> : flash_attn_bwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   kern<<<B * H * ((Tk + FB_BLK - 1) / FB_BLK), FB_THREADS, smem, (cudaStream_t)stream_>>>(tq, tk, tv, tdo, tdq, p);
