@@ -442,7 +442,9 @@ attn_dvec_kernel(const __nv_bfloat16* __restrict__ dO, long sb, long sh, long st
 }
 
 // dq (bf16, addressed base + b * o_bs + t * o_ts + h * D) = acc [slabs, B, H, T, D] fp32, slabs added in order; with a causal mask
-// query t has parts in the slabs 0 .. t / 128 only.
+// query t has parts in the slabs 0 .. t / 128 only.  One buffer is a kernel of its own: the loop's loads in flight take registers that
+// a plain conversion needs as resident warps.
+template <bool SLABS>
 __global__ void __launch_bounds__(256)
 attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ out, long o_bs, long o_ts, int B, int H, int T, int D,
                       int slabs, int causal) {
@@ -456,7 +458,7 @@ attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__
     const int b = (int)(row / ((long)T * H));
     const float4* src = reinterpret_cast<const float4*>(acc) + 2 * g;
     float4 x = __ldcs(src), y = __ldcs(src + 1);
-    const int n = causal ? min(slabs, t / FB_BLK + 1) : slabs;
+    const int n = !SLABS ? 1 : (causal ? min(slabs, t / FB_BLK + 1) : slabs);
 #pragma unroll 4
     for (int s = 1; s < n; ++s) {
       const float4 a = __ldcs(src + s * 2 * n8), c = __ldcs(src + s * 2 * n8 + 1);
@@ -485,7 +487,7 @@ DL4J_API int dl4j_attn_dq_finish(const float* acc, void* out, long o_bs, long o_
   const long n8 = (long)B * H * T * (D / 8);
   long blocks = (n8 + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
-  attn_dq_finish_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(acc, reinterpret_cast<__nv_bfloat16*>(out), o_bs, o_ts, B, H, T, D,
-                                                                               slabs, causal);
+  auto kern = slabs > 1 ? attn_dq_finish_kernel<true> : attn_dq_finish_kernel<false>;
+  kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(acc, reinterpret_cast<__nv_bfloat16*>(out), o_bs, o_ts, B, H, T, D, slabs, causal);
   return (int)cudaGetLastError();
 }
