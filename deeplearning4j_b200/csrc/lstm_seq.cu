@@ -1,4 +1,5 @@
-// Persistent LSTM sequence kernel: all time steps of one layer in a single cooperative launch.
+// Persistent LSTM sequence kernel: all time steps of one layer in a single cooperative launch.  Batches that fit its limits run on the
+// kernels of lstm_split.cu; these take the rest (more than 48 rows a group, or no room for a group's h beside the weights).
 //
 // Math per step (DL4J gate order a|f|o|g along the 4n axis, libnd4j lstmLayer / LSTMHelpers.java):
 //   z_t = zx_t + h_{t-1} RW          zx_t = x_t W + b is computed beforehand by one large GEMM
@@ -14,14 +15,12 @@
 // epilogue warps (one thread per batch row) apply the cell non-linearities with c_t held in registers across
 // steps, then publish their slice of h_t.  Steps are separated by a grid-wide arrive/wait on a global counter;
 // every wait is bounded and reports through the status word.
-#include "common.cuh"
+#include "lstm_common.cuh"
 
 namespace dl4j {
 
-constexpr int LS_UNITS = 16;                 // hidden units per CTA
 constexpr int LS_N = 4 * LS_UNITS;           // MMA N: gate rows per CTA
 constexpr int LS_M = 128;                    // MMA M: batch rows (zero padded)
-constexpr int LS_BK = 64;                    // K elements per stage (128 bytes, SWIZZLE_128B)
 constexpr int LS_ISSUERS = 3;                // MMA-issuing warps.  One elected thread gets a tcgen05.mma into the pipe per ~64 clocks, while
                                              // an M 128 x N 64 x K 16 instruction occupies the tensor core for ~48 clocks and N = 16 for ~39;
                                              // with the producer warp and four epilogue warps the CTA stays at 256 threads (a ninth warp
@@ -53,63 +52,6 @@ struct LstmSeqParams {
 // acquire, orders the generic-proxy stores before the async-proxy reads; a second one on the writer's side (every epilogue thread waited
 // there for its own stores before the release did so again) cost 0.6 us of each step: batch 64, n 1024: 6.16 -> 5.59 us forward,
 // 7.53 -> 6.92 us backward.
-// Named barrier over the four epilogue warps (barrier 0 is __syncthreads).
-__device__ __forceinline__ void epilogue_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-
-// Acquire loads: once the target is seen, the other CTAs' stores that preceded their arrivals (released) are visible to this thread;
-// no separate fence is needed after the wait.
-__device__ __forceinline__ unsigned int ld_acquire_gpu(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void red_release_add(unsigned int* p) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
-}
-__device__ __forceinline__ bool wait_counter(const unsigned int* counter, unsigned int target, int* status) {
-  if (ld_acquire_gpu(counter) >= target) return true;
-  const long long t0 = clock64();
-  uint32_t spins = 0;
-  while (ld_acquire_gpu(counter) < target) {
-    if ((++spins & 0xff) == 0 && (clock64() - t0 > 4000000000LL || *((volatile int*)status) != 0)) {
-      atomicCAS(status, 0, DL4J_ERR_TIMEOUT_PEER);
-      return false;
-    }
-  }
-  return true;
-}
-
-// Timeline of one CTA: slot `i` of step `s` receives this SM's clock.  Slots: 0 producer saw the step's grid barrier open,
-// 1 producer issued the step's last load, 2..17 MMA thread saw k-block (slot - 2) land (first 16 k-blocks), 18 MMA thread
-// committed the accumulator, 19 epilogue saw the accumulator, 20 after the TMEM loads, 21 after the global stores, 22 after the
-// fences, 23 after the barrier arrive.
-__device__ __forceinline__ void ls_stamp(long long* trace, int s, int slot) {
-  if (trace != nullptr && blockIdx.x == gridDim.x / 2) trace[s * 32 + slot] = clock64();
-}
-
-__device__ __forceinline__ float tanh_fast(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// sigmoid(x) = 0.5 tanh(x / 2) + 0.5: one special-function instruction
-__device__ __forceinline__ float sigm_fast(float x) { return fmaf(0.5f, tanh_fast(0.5f * x), 0.5f); }
-
-__device__ __forceinline__ void unpack8(const uint4& u, float* o) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); o[2 * i] = f.x; o[2 * i + 1] = f.y; }
-}
-__device__ __forceinline__ uint4 pack8(const float* v) {
-  uint4 u;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-  return u;
-}
-
 __global__ void __launch_bounds__(LS_THREADS, 1)
 lstm_seq_fwd_kernel(const __grid_constant__ CUtensorMap tmap_h, const __grid_constant__ CUtensorMap tmap_w, const LstmSeqParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -556,57 +498,6 @@ lstm_seq_bwd_kernel(const __grid_constant__ CUtensorMap tmap_dz, const __grid_co
   }
 }
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t mapa_cluster(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-// release at cluster scope: the stores above are visible to the peer thread that observes this arrival with an acquire
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_bounded_cluster(uint64_t* bar, uint32_t parity, int* status, int code) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = clock64();
-  uint32_t spins = 0;
-  while (!mbar_try_wait_cluster(bar, parity)) {
-    if ((++spins & 0x3ff) == 0 && (clock64() - t0 > 4000000000LL || *((volatile int*)status) != 0)) {
-      atomicCAS(status, 0, code);
-      return false;
-    }
-  }
-  return true;
-}
-// shared memory of this CTA -> shared memory of a CTA of the cluster; the bytes are counted on that CTA's mbarrier
-__device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst_cluster, uint32_t src_cta, uint32_t bytes, uint32_t bar_cluster) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_cluster), "r"(src_cta),
-               "r"(bytes), "r"(bar_cluster)
-               : "memory");
-}
-// every thread of every CTA of the cluster
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // Cluster form of the backward kernel: the CS (2 or 4) CTAs of a cluster own 16 CS hidden units together and split the reduction
 // over the 4n gate columns.  CTA `rank` keeps RW[16 CS units, its 1/CS of the columns] resident (the same 128 KB as 16 units x all
 // columns), streams only its share of dz per step (the L2 -> SM stream is what bounds the single-CTA form) and issues N = 16 CS
@@ -947,19 +838,28 @@ static int ls_encode(CUtensorMap* map, const void* base, uint64_t inner, uint64_
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
+// lstm_split.cu; 1: not covered there
+int dl4j_lstm_split_fwd(const void* zx, const void* rw, void* h_all, const float* c0, float* cs, void* gates, int T, int mb, int n, int reverse,
+                        int sms, int* status, long long* trace, cudaStream_t stream);
+int dl4j_lstm_split_bwd(const void* dout, const void* gates, const float* cs, const float* c0, const void* rwt, void* dzx, const float* dc_last,
+                        void* dh0, float* dc0, int T, int mb, int n, int reverse, int sms, int* status, long long* trace, cudaStream_t stream);
+
 // zx [T, mb, 4n] bf16; rw [4n, n] bf16 (row g*n + j = recurrent weights into gate g of unit j); h_all [T+1, mb, n] bf16 with slot 0 = h_0;
 // c0 [mb, n] fp32; cs [T, mb, n] fp32; gates [T, mb, 4n] bf16; counter: one unsigned int of device scratch.
 // Limits: n % 64 == 0, n <= 1216 (weights resident in shared memory), n / 16 <= SM count, 1 <= mb <= 128.
 DL4J_API int dl4j_lstm_seq_fwd(const void* zx, const void* rw, void* h_all, const float* c0, float* cs, void* gates, int T, int mb, int n,
                                int reverse, unsigned int* counter, void* stream_) {
   if (T < 1 || mb < 1 || mb > LS_M || n < 64 || n % 64 != 0) return -DL4J_ERR_BAD_ARG;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int rc = dl4j_lstm_split_fwd(zx, rw, h_all, c0, cs, gates, T, mb, n, reverse, sms, dl4j_status_word(dev), g_lstm_trace, (cudaStream_t)stream_);
+  if (rc == 0) return 0;
+  if (rc != 1) (void)cudaGetLastError();       // a refused launch leaves a (non-sticky) error behind
   const int kblocks = n / LS_BK;
   int a_rows, stages;
   const size_t smem = ls_ring((size_t)kblocks * LS_B_KB, mb, &a_rows, &stages);
   if (!smem) return -DL4J_ERR_BAD_ARG;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = n / LS_UNITS;
   if (grid > sms) return -DL4J_ERR_BAD_ARG;
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -1051,7 +951,10 @@ DL4J_API int dl4j_lstm_seq_bwd(const void* dout, const void* gates, const float*
   // Cluster form first (CS CTAs share 16 CS units and split the gate columns: the same resident bytes, 1 / CS of the L2 -> SM stream
   // per CTA); a form that does not fit the problem, or whose launch the driver refuses (a cooperative launch needs every cluster
   // resident at once, which a partly occupied device or a profiler may not grant), gives way to the next smaller one.
-  int rc = 1;
+  int rc = dl4j_lstm_split_bwd(dout, gates, cs, c0, rwt, dzx, dc_last, dh0, dc0, T, mb, n, reverse, sms, dl4j_status_word(dev), g_lstm_trace,
+                               (cudaStream_t)stream_);
+  if (rc == 0) return 0;
+  if (rc != 1) (void)cudaGetLastError();
   for (int csz = lstm_cluster_size(); csz >= 1; csz /= 2) {
     rc = lstm_bwd_launch(csz, dout, gates, cs, c0, rwt, dzx, dc_last, dh0, dc0, T, mb, n, reverse, counter, (cudaStream_t)stream_);
     if (rc == 0) return 0;
