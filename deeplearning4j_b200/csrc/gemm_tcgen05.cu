@@ -4,12 +4,12 @@
 // (libnd4j/include/helpers/cuda/MmulHelper.cu:41-129 usualCudaGemm, :501-517 cublas*gemm) and the
 // matmul+addBias+activation sequences of xw_plus_b / relu_layer / DenseLayer.
 //
-// Structure (one persistent CTA per SM, 192 threads):
+// Structure (one persistent CTA per SM, 320 threads):
 //   warp 0      : TMA producer  - cp.async.bulk.tensor tiles of A and B into a multi-stage smem ring
 //   warp 1      : MMA issuer    - one elected lane issues tcgen05.mma (128 x BLOCK_N x 16), accumulators
 //                                 live in TMEM, double-buffered (2 x BLOCK_N columns) so the epilogue of
 //                                 tile i overlaps the main loop of tile i+1
-//   warps 2..5  : epilogue      - tcgen05.ld 32 lanes x 32 columns, bias / activation / residual,
+//   warps 2..9  : epilogue      - tcgen05.ld 32 lanes x 32 columns, bias / activation / residual,
 //                                 16-byte global stores (or fp32 vector reductions for split-K)
 // Operands may be K-major (reduction dimension contiguous) or MN-major (output dimension contiguous),
 // which covers forward (X·Wᵀ), data-gradient (dY·W) and weight-gradient (dYᵀ·X) without transposes.
@@ -20,7 +20,8 @@ namespace dl4j {
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_K = 64;         // 64 x 2 bytes = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-constexpr int GEMM_THREADS = 192;
+constexpr int GEMM_EPI_WARPS = 8;   // two per TMEM lane quadrant: they take every second group of 32 columns
+constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI_WARPS;
 
 struct GemmParams {
   int M, N, K;
@@ -69,9 +70,10 @@ struct GemmSmem {
   static constexpr int B_BYTES = BLOCK_N * BLOCK_K * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (BLOCK_N == 256) ? 4 : 6;
-  static constexpr int EPI_SLAB = 32 * 128;                 // one warp's 32 rows x 128 bytes
-  static constexpr int EPI_BYTES = 4 * 2 * EPI_SLAB;        // 4 epilogue warps x 2 ring buffers
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+  static constexpr int EPI_SLAB = 32 * 64;                  // one warp's 32 rows x 32 16-bit columns (fp32: both slabs)
+  static constexpr int EPI_BYTES = GEMM_EPI_WARPS * 2 * EPI_SLAB;
+  static constexpr int BIAS_BYTES = GEMM_EPI_WARPS * 32 * 4;   // one group of 32 columns per warp
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + BIAS_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 };
 
 __device__ __forceinline__ float apply_act(float v, int act) {
@@ -155,19 +157,47 @@ __device__ __forceinline__ float unpack_lo(uint32_t u, int fmt) {
   return __half2float(*reinterpret_cast<__half*>(&u));
 }
 
-// bias[col] as float (0 beyond N); the bias vector is fp32 or the operand type
-__device__ __forceinline__ float load_bias(const GemmParams& p, int col) {
-  if (col >= p.N) return 0.f;
-  return p.bias_fp32 ? __ldg(reinterpret_cast<const float*>(p.bias) + col)
-                     : unpack_lo((uint32_t)__ldg(reinterpret_cast<const uint16_t*>(p.bias) + col), p.fmt);
-}
 __device__ __forceinline__ float unpack_hi(uint32_t u, int fmt) {
   uint32_t h = u >> 16;
   if (fmt == 1) return __bfloat162float(*reinterpret_cast<__nv_bfloat16*>(&h));
   return __half2float(*reinterpret_cast<__half*>(&h));
 }
 
-template <int BLOCK_N, bool A_MN, bool B_MN>
+// 32 values of a row as four 16-byte units of the 64-byte swizzle, the format decided once
+template <bool BF16>
+__device__ __forceinline__ void store_row32(uint8_t* row, int sw64, const float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    constexpr int F = BF16 ? 1 : 0;
+    const uint4 u = make_uint4(pack2(v[8 * j], v[8 * j + 1], F), pack2(v[8 * j + 2], v[8 * j + 3], F), pack2(v[8 * j + 4], v[8 * j + 5], F),
+                               pack2(v[8 * j + 6], v[8 * j + 7], F));
+    *reinterpret_cast<uint4*>(row + ((j ^ sw64) << 4)) = u;
+  }
+}
+template <bool BF16>
+__device__ __forceinline__ void unpack_row32(const uint4 (&z)[4], float (&f)[32]) {
+  constexpr int F = BF16 ? 1 : 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t w[4] = {z[j].x, z[j].y, z[j].z, z[j].w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { f[8 * j + 2 * e] = unpack_lo(w[e], F); f[8 * j + 2 * e + 1] = unpack_hi(w[e], F); }
+  }
+}
+
+// bias[col] as float (0 beyond N); the bias vector is fp32 or the operand type
+__device__ __forceinline__ float load_bias(const GemmParams& p, int col) {
+  if (col >= p.N) return 0.f;
+  return p.bias_fp32 ? __ldg(reinterpret_cast<const float*>(p.bias) + col)
+                     : unpack_lo((uint32_t)__ldg(reinterpret_cast<const uint16_t*>(p.bias) + col), p.fmt);
+}
+
+// FULL: pre-activation output, activations other than ReLU, activation gradients.  The other form knows bias, residual and ReLU only: what an
+// epilogue warp executes per 32 columns is then one short run of code.  With both kinds in one kernel, four epilogue warps, the operand
+// format looked at for every pair of values and the bias broadcast by shuffles, 32 columns took 310 instructions and 1900 clocks, most of
+// them waits for the instruction fetch and for dependent results.  Before / now, us (N = 256 tiles): 200704 x 256 x 64 53 / 33, with fp32
+// bias 70 / 41, with residual 156 / 74; 16384 x 3072 x 768 with bias, GELU and pre-activations 99 / 85, with residual 179 / 89.
+template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_aux,
@@ -178,7 +208,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* epi_smem = smem + STAGES * S::STAGE_BYTES;       // 1024-byte aligned (stage sizes are multiples of 1024)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + S::EPI_BYTES);
+  float* bias_smem = reinterpret_cast<float*>(epi_smem + S::EPI_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + S::EPI_BYTES + S::BIAS_BYTES);
   uint64_t* full_bar = bars;                    // [STAGES]
   uint64_t* empty_bar = bars + STAGES;          // [STAGES]
   uint64_t* tmem_full = bars + 2 * STAGES;      // [2]
@@ -204,7 +235,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 4);   // one arrive per epilogue warp
+      mbar_init(&tmem_empty[i], GEMM_EPI_WARPS);   // one arrive per epilogue warp
     }
     mbar_fence_init();
   }
@@ -323,8 +354,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..9)
     const int q = warp & 3;                 // TMEM lane quadrant this warp may access
+    const int c_first = ((warp - 2) >> 2) * 32;
     int it = 0;
     bool ok = true;
     for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++it) {
@@ -339,111 +371,118 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       const bool lead_split = split == 0;
-      // lane L of the warp fetches bias[col0 + L] one 32-column group ahead of its use (first group here, before the
-      // wait for the accumulator), and the group is broadcast with shuffles: no load latency inside the tile loop
+      // lane L of the warp fetches bias[col0 + L] one group ahead of its use (first group here, before the wait for the
+      // accumulator), and the group is broadcast through the warp's own 32 floats: no load latency inside the tile loop
       const bool use_bias = p.bias != nullptr && lead_split && !p.bias_mma;
-      float bias_cur = use_bias ? load_bias(p, n0 + lane) : 0.f;
+      float bias_cur = use_bias ? load_bias(p, n0 + c_first + lane) : 0.f;
+      // the residual's 64 bytes of this thread's row likewise travel one group ahead (rows 16-byte aligned, whole groups)
+      const bool use_res = p.residual != nullptr && lead_split && m0 + q * 32 + lane < p.M;
+      const uint16_t* res_row = reinterpret_cast<const uint16_t*>(p.residual) + (long)(m0 + q * 32 + lane) * p.ld_res + n0;
+      const bool res_vec = use_res && p.tma_store && (reinterpret_cast<uintptr_t>(res_row) & 15) == 0;
+      uint4 rz[4];
+      auto load_res = [&](int c) {
+        if (res_vec && c < BLOCK_N && n0 + c + 32 <= p.N) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) rz[j] = *reinterpret_cast<const uint4*>(res_row + c + 8 * j);
+        }
+      };
+      load_res(c_first);
       if (!mbar_wait_bounded(&tmem_full[buf], acc_phase, p.status, DL4J_ERR_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
       const bool row_ok = row < p.M;
       const uint32_t taddr_row = tmem_base + buf * BLOCK_N + ((uint32_t)(q * 32) << 16);
       if (p.tma_store) {
-        // -------- staged epilogue: registers -> swizzled smem slab (32 rows x 128 B per warp) -> TMA store / reduce
+        // -------- staged epilogue: registers -> swizzled smem slab (32 rows x 64 B, fp32 128 B, per warp) -> TMA store / reduce
         const int b1 = batch % p.batch1, b2 = p.atomic_out == 2 ? split : batch / p.batch1;
-        uint8_t* ring = epi_smem + q * (2 * S::EPI_SLAB);
-        const int sw = lane & 7;
-        uint8_t* my_row0 = ring + lane * 128;
-        const int cols_per_store = p.out_fp32 ? 32 : 64;
+        uint8_t* ring = epi_smem + (warp - 2) * (2 * S::EPI_SLAB);
+        float* my_bias = bias_smem + (warp - 2) * 32;
+        const bool rescale = !has_k || p.alpha != 1.0f;
+        const bool want_aux = FULL && p.aux != nullptr && p.tma_aux;
+        const bool two_slabs = want_aux || p.out_fp32;        // an iteration fills both slabs: every earlier store must have been read
         int ring_idx = 0;
 #pragma unroll 1
-        for (int c = 0; c < BLOCK_N; c += cols_per_store) {
-          if (n0 + c >= p.N) break;                                   // warp-uniform
-          const bool want_aux = p.aux != nullptr && p.tma_aux;
-          // buffers: without aux alternate the ring (one store may still be reading the other slab);
-          // with aux both slabs are filled in this iteration, so every earlier store must have been read.
-          if (lane == 0) { if (want_aux) bulk_wait_read<0>(); else bulk_wait_read<1>(); }
-          __syncwarp();
-          uint8_t* slab_out = my_row0 + (want_aux ? S::EPI_SLAB : ring_idx * S::EPI_SLAB);
-          uint8_t* slab_aux = my_row0;
-          const int halves = p.out_fp32 ? 1 : 2;
-#pragma unroll 1
-          for (int hf = 0; hf < halves; ++hf) {
-            const int col0 = n0 + c + hf * 32;
-            if (col0 >= p.N) break;                                   // warp-uniform; TMA clips the unwritten half
-            uint32_t r[32];
-            tmem_ld_32x32(taddr_row + c + hf * 32, r);
-            tmem_ld_wait();
-            float v[32];
+        for (int c = c_first; c < BLOCK_N; c += 64) {
+          const int col0 = n0 + c;
+          if (col0 >= p.N) break;                                     // warp-uniform
+          uint32_t r[32];
+          tmem_ld_32x32(taddr_row + c, r);
+          tmem_ld_wait();
+          float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = has_k ? __uint_as_float(r[j]) * p.alpha : 0.0f;
-            if (use_bias) {
-              const int next_col0 = hf + 1 < halves ? col0 + 32 : n0 + c + cols_per_store;
-              const float bias_next = load_bias(p, next_col0 + lane);
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+          if (rescale) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += __shfl_sync(0xffffffffu, bias_cur, j);
-              bias_cur = bias_next;
+            for (int j = 0; j < 32; ++j) v[j] = has_k ? v[j] * p.alpha : 0.0f;
+          }
+          if (use_bias) {
+            my_bias[lane] = bias_cur;
+            __syncwarp();
+            bias_cur = load_bias(p, col0 + 64 + lane);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float4 b4 = reinterpret_cast<const float4*>(my_bias)[j];
+              v[4 * j] += b4.x; v[4 * j + 1] += b4.y; v[4 * j + 2] += b4.z; v[4 * j + 3] += b4.w;
             }
+          }
+          if (lane == 0) { if (two_slabs) bulk_wait_read<0>(); else bulk_wait_read<1>(); }
+          __syncwarp();
+          uint8_t* slab_out = ring + (p.out_fp32 ? 0 : want_aux ? S::EPI_SLAB : ring_idx * S::EPI_SLAB);
+          const int sw64 = (lane >> 1) & 3;                           // 64-byte swizzle: 16-byte unit ^ (row / 2 % 4)
+          if constexpr (FULL) {
             if (want_aux) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 u = make_uint4(pack2(v[8 * j], v[8 * j + 1], p.fmt), pack2(v[8 * j + 2], v[8 * j + 3], p.fmt),
-                                           pack2(v[8 * j + 4], v[8 * j + 5], p.fmt), pack2(v[8 * j + 6], v[8 * j + 7], p.fmt));
-                *reinterpret_cast<uint4*>(slab_aux + (((hf * 4 + j) ^ sw) << 4)) = u;
-              }
+              if (p.fmt == 1) store_row32<true>(ring + lane * 64, sw64, v);
+              else store_row32<false>(ring + lane * 64, sw64, v);
             }
             if (p.act != 0) apply_act32(v, p.act);
-            if (p.residual != nullptr && lead_split && row_ok) {
-              const uint16_t* rs = reinterpret_cast<const uint16_t*>(p.residual) + (long)row * p.ld_res + col0;
-              if (col0 + 32 <= p.N && ((reinterpret_cast<uintptr_t>(rs) & 15) == 0)) {
+          } else if (p.act == 1) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 8) {
-                  const uint4 u = *reinterpret_cast<const uint4*>(rs + j);
-                  const float z8[8] = {unpack_lo(u.x, p.fmt), unpack_hi(u.x, p.fmt), unpack_lo(u.y, p.fmt), unpack_hi(u.y, p.fmt),
-                                       unpack_lo(u.z, p.fmt), unpack_hi(u.z, p.fmt), unpack_lo(u.w, p.fmt), unpack_hi(u.w, p.fmt)};
-                  if (p.res_act) {
+            for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
+          }
+          if (use_res) {
+            if (res_vec && col0 + 32 <= p.N) {
+              float z[32];
+              if (p.fmt == 1) unpack_row32<true>(rz, z);
+              else unpack_row32<false>(rz, z);
+              if (FULL && p.res_act) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[j + e] = mul_act_grad(v[j + e], z8[e], p.res_act);
-                  } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[j + e] += z8[e];
-                  }
-                }
+                for (int j = 0; j < 32; ++j) v[j] = mul_act_grad(v[j], z[j], p.res_act);
               } else {
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (col0 + j < p.N) {
-                    const float z = unpack_lo((uint32_t)rs[j], p.fmt);
-                    v[j] = p.res_act ? mul_act_grad(v[j], z, p.res_act) : v[j] + z;
-                  }
+                for (int j = 0; j < 32; ++j) v[j] += z[j];
               }
-            }
-            if (p.relu_last) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
-            }
-            if (p.out_fp32) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<float4*>(slab_out + ((j ^ sw) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+              load_res(c + 64);
             } else {
+              const uint16_t* rs = res_row + c;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 u = make_uint4(pack2(v[8 * j], v[8 * j + 1], p.fmt), pack2(v[8 * j + 2], v[8 * j + 3], p.fmt),
-                                           pack2(v[8 * j + 4], v[8 * j + 5], p.fmt), pack2(v[8 * j + 6], v[8 * j + 7], p.fmt));
-                *reinterpret_cast<uint4*>(slab_out + (((hf * 4 + j) ^ sw) << 4)) = u;
-              }
+              for (int j = 0; j < 32; ++j)
+                if (col0 + j < p.N) {
+                  const float z = unpack_lo((uint32_t)rs[j], p.fmt);
+                  v[j] = FULL && p.res_act ? mul_act_grad(v[j], z, p.res_act) : v[j] + z;
+                }
             }
+          }
+          if (p.relu_last) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = relu_f(v[j]);
+          }
+          if (p.out_fp32) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<float4*>(slab_out + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          } else if (p.fmt == 1) {
+            store_row32<true>(slab_out + lane * 64, sw64, v);
+          } else {
+            store_row32<false>(slab_out + lane * 64, sw64, v);
           }
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
             const int r0 = m0 + q * 32;
             if (r0 < p.M) {
-              if (want_aux) tma_store_4d(&tmap_aux, ring, n0 + c, r0, b1, b2);
-              uint8_t* src = ring + (want_aux ? S::EPI_SLAB : ring_idx * S::EPI_SLAB);
-              if (p.atomic_out == 1) tma_reduce_add_4d(&tmap_c, src, n0 + c, r0, b1, b2);
-              else tma_store_4d(&tmap_c, src, n0 + c, r0, b1, b2);
+              if (want_aux) tma_store_4d(&tmap_aux, ring, col0, r0, b1, b2);
+              if (p.atomic_out == 1) tma_reduce_add_4d(&tmap_c, slab_out, col0, r0, b1, b2);
+              else tma_store_4d(&tmap_c, slab_out, col0, r0, b1, b2);
             }
             bulk_commit();
           }
@@ -455,7 +494,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         continue;
       }
 #pragma unroll 1
-      for (int c = 0; c < BLOCK_N; c += 32) {
+      for (int c = c_first; c < BLOCK_N; c += 64) {
         const int col0 = n0 + c;
         if (col0 >= p.N) break;             // warp-uniform
         uint32_t r[32];
@@ -576,7 +615,8 @@ using namespace dl4j;
 
 static int encode_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
                      uint32_t box_inner, uint32_t box_outer, uint64_t nb1 = 1, uint64_t nb2 = 1, uint64_t sb1_bytes = 0,
-                     uint64_t sb2_bytes = 0, CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16) {
+                     uint64_t sb2_bytes = 0, CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                     CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   dl4j_PFN_encodeTiled enc = dl4j_get_encode_tiled();
   if (!enc) return -1;
   // rank-4 map {inner, outer, batch1, batch2}; unit batch dims get a harmless 16-byte-multiple stride
@@ -587,7 +627,7 @@ static int encode_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_
   cuuint32_t box[4] = {box_inner, box_outer, 1, 1};
   cuuint32_t es[4] = {1, 1, 1, 1};
   CUresult r = enc(map, dt, 4, const_cast<void*>(base), dims, strides, box, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
@@ -598,11 +638,11 @@ static int encode_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_
 static __device__ __align__(128) uint16_t g_ones_bf16[128] = {DL4J_REP128(0x3F80)};
 static __device__ __align__(128) uint16_t g_ones_f16[128] = {DL4J_REP128(0x3C00)};
 
-template <int BLOCK_N, bool A_MN, bool B_MN>
+template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx,
                        const CUtensorMap& tones, const CUtensorMap& tbias, const GemmParams& p, int grid, cudaStream_t stream) {
   using S = GemmSmem<BLOCK_N, A_MN, B_MN>;
-  auto kern = gemm_tcgen05_kernel<BLOCK_N, A_MN, B_MN>;
+  auto kern = gemm_tcgen05_kernel<BLOCK_N, A_MN, B_MN, FULL>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
   if (e != cudaSuccess) return (int)e;
   kern<<<grid, GEMM_THREADS, S::TOTAL, stream>>>(ta, tb, tc, tx, tones, tbias, p);
@@ -646,7 +686,7 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   if (!b_mn) r = encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, BLOCK_K, (uint32_t)block_n, nb1, nb2, b_bs[0] * 2, b_bs[1] * 2);
   else       r = encode_2d(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, 64, BLOCK_K, nb1, nb2, b_bs[0] * 2, b_bs[1] * 2);
   if (r) return r > 0 ? -1000 - r : r;
-  // output maps: a 32-row x 128-byte box per epilogue warp (64 16-bit or 32 fp32 columns)
+  // output maps: a box of 32 rows x 32 columns per epilogue warp (64 bytes a row, fp32 128)
   CUtensorMap tc, tx;
   memset(&tc, 0, sizeof(tc));
   memset(&tx, 0, sizeof(tx));
@@ -655,11 +695,13 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   if (!(reinterpret_cast<uintptr_t>(C) & 15) && ((ldc * esz) % 16 == 0) && ((c_bs[0] * esz) % 16 == 0) && ((c_bs[1] * esz) % 16 == 0) &&
       (!aux || (!(reinterpret_cast<uintptr_t>(aux) & 15) && (ld_aux * 2) % 16 == 0))) {
     const bool slabs = atomic_out == 2;
-    r = encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * esz, out_fp32 ? 32 : 64, 32, nb1, slabs ? (uint64_t)splits : nb2,
-                  c_bs[0] * esz, slabs ? (uint64_t)M * ldc * esz : c_bs[1] * esz, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+    r = encode_2d(&tc, C, (uint64_t)N, (uint64_t)M, (uint64_t)ldc * esz, 32, 32, nb1, slabs ? (uint64_t)splits : nb2,
+                  c_bs[0] * esz, slabs ? (uint64_t)M * ldc * esz : c_bs[1] * esz, out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                  out_fp32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
     if (r == 0) p.tma_store = 1;
     if (r == 0 && aux) {
-      r = encode_2d(&tx, aux, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux * 2, 64, 32, 1, 1, 0, 0);
+      r = encode_2d(&tx, aux, (uint64_t)N, (uint64_t)M, (uint64_t)ld_aux * 2, 32, 32, 1, 1, 0, 0, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                    CU_TENSOR_MAP_SWIZZLE_64B);
       if (r == 0) p.tma_aux = 1; else p.tma_store = 0;
     }
   }
@@ -687,8 +729,11 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   const int tiles = (int)tiles_l;
   if (num_sms <= 0) num_sms = 148;
   const int grid = tiles < num_sms ? tiles : num_sms;
-#define DL4J_GEMM_CASE(BN, AM, BM) \
-  if (block_n == BN && a_mn == AM && b_mn == BM) return launch_gemm<BN, AM != 0, BM != 0>(ta, tb, tc, tx, tones, tbias, p, grid, stream);
+  const bool full = p.aux || p.act > 1 || p.res_act;
+#define DL4J_GEMM_CASE(BN, AM, BM)                                                                                              \
+  if (block_n == BN && a_mn == AM && b_mn == BM)                                                                               \
+    return full ? launch_gemm<BN, AM != 0, BM != 0, true>(ta, tb, tc, tx, tones, tbias, p, grid, stream)                       \
+                : launch_gemm<BN, AM != 0, BM != 0, false>(ta, tb, tc, tx, tones, tbias, p, grid, stream);
   DL4J_GEMM_CASE(256, 0, 0) DL4J_GEMM_CASE(256, 0, 1) DL4J_GEMM_CASE(256, 1, 0) DL4J_GEMM_CASE(256, 1, 1)
   DL4J_GEMM_CASE(128, 0, 0) DL4J_GEMM_CASE(128, 0, 1) DL4J_GEMM_CASE(128, 1, 0) DL4J_GEMM_CASE(128, 1, 1)
 #undef DL4J_GEMM_CASE
