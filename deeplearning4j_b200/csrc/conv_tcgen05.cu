@@ -180,6 +180,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait_and_release();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -388,6 +389,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap tmap_a,     // activation {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait_and_release();
   const uint32_t tmem_base = *tmem_slot;
   // with resident weights every CTA keeps one column tile for its whole life: work items are strided so that nt is fixed
   // (the host launches a grid that is a multiple of tiles_n in that case)
@@ -634,6 +636,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_dy,    // {Cout, OW, 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait_and_release();
   const uint32_t tmem_base = *tmem_slot;
 
   // work item -> (split, tap, m tile, n tile); splits of one output tile are neighbours so they run at the same time
@@ -838,20 +841,24 @@ template <int BN>
 static int launch_conv(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const ConvParams& p, int grid,
                        cudaStream_t stream) {
   auto kern = conv_igemm_kernel<BN>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ConvSmem<BN>::TOTAL);
+  static SmemLimit limit;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const cudaError_t e = raise_smem_limit((const void*)kern, dev, ConvSmem<BN>::TOTAL, limit);
   if (e != cudaSuccess) return (int)e;
-  kern<<<grid, CV_THREADS, ConvSmem<BN>::TOTAL, stream>>>(ta, tb, tc, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(kern, dim3(grid), dim3(CV_THREADS), ConvSmem<BN>::TOTAL, stream, ta, tb, tc, p);
 }
 
 template <int BN>
 static int launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const WgradParams& p, int grid,
                         cudaStream_t stream) {
   auto kern = conv_wgrad_kernel<BN>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ConvSmem<BN>::TOTAL);
+  static SmemLimit limit;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const cudaError_t e = raise_smem_limit((const void*)kern, dev, ConvSmem<BN>::TOTAL, limit);
   if (e != cudaSuccess) return (int)e;
-  kern<<<grid, CV_THREADS, ConvSmem<BN>::TOTAL, stream>>>(ta, tb, tc, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(kern, dim3(grid), dim3(CV_THREADS), ConvSmem<BN>::TOTAL, stream, ta, tb, tc, p);
 }
 
 
@@ -859,10 +866,12 @@ template <int BN>
 static int launch_halo(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const HaloParams& p, int grid,
                        int smem_bytes, cudaStream_t stream) {
   auto kern = conv_halo_kernel<BN>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  static SmemLimit limit;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const cudaError_t e = raise_smem_limit((const void*)kern, dev, smem_bytes, limit);
   if (e != cudaSuccess) return (int)e;
-  kern<<<grid, CV_HALO_THREADS, smem_bytes, stream>>>(ta, tb, tc, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(kern, dim3(grid), dim3(CV_HALO_THREADS), smem_bytes, stream, ta, tb, tc, p);
 }
 
 static bool conv_halo_auto() {

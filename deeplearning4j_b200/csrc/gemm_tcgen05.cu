@@ -246,6 +246,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait_and_release();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -640,13 +641,13 @@ static __device__ __align__(128) uint16_t g_ones_f16[128] = {DL4J_REP128(0x3C00)
 
 template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx,
-                       const CUtensorMap& tones, const CUtensorMap& tbias, const GemmParams& p, int grid, cudaStream_t stream) {
+                       const CUtensorMap& tones, const CUtensorMap& tbias, const GemmParams& p, int grid, int dev, cudaStream_t stream) {
   using S = GemmSmem<BLOCK_N, A_MN, B_MN>;
   auto kern = gemm_tcgen05_kernel<BLOCK_N, A_MN, B_MN, FULL>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+  static SmemLimit limit;
+  const cudaError_t e = raise_smem_limit((const void*)kern, dev, S::TOTAL, limit);
   if (e != cudaSuccess) return (int)e;
-  kern<<<grid, GEMM_THREADS, S::TOTAL, stream>>>(ta, tb, tc, tx, tones, tbias, p);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(kern, dim3(grid), dim3(GEMM_THREADS), S::TOTAL, stream, ta, tb, tc, tx, tones, tbias, p);
 }
 
 // C[M,N] = act(alpha * A·B + bias) (+ residual)
@@ -732,8 +733,8 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   const bool full = p.aux || p.act > 1 || p.res_act;
 #define DL4J_GEMM_CASE(BN, AM, BM)                                                                                              \
   if (block_n == BN && a_mn == AM && b_mn == BM)                                                                               \
-    return full ? launch_gemm<BN, AM != 0, BM != 0, true>(ta, tb, tc, tx, tones, tbias, p, grid, stream)                       \
-                : launch_gemm<BN, AM != 0, BM != 0, false>(ta, tb, tc, tx, tones, tbias, p, grid, stream);
+    return full ? launch_gemm<BN, AM != 0, BM != 0, true>(ta, tb, tc, tx, tones, tbias, p, grid, dev, stream)                       \
+                : launch_gemm<BN, AM != 0, BM != 0, false>(ta, tb, tc, tx, tones, tbias, p, grid, dev, stream);
   DL4J_GEMM_CASE(256, 0, 0) DL4J_GEMM_CASE(256, 0, 1) DL4J_GEMM_CASE(256, 1, 0) DL4J_GEMM_CASE(256, 1, 1)
   DL4J_GEMM_CASE(128, 0, 0) DL4J_GEMM_CASE(128, 0, 1) DL4J_GEMM_CASE(128, 1, 0) DL4J_GEMM_CASE(128, 1, 1)
 #undef DL4J_GEMM_CASE

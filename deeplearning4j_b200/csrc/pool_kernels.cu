@@ -28,6 +28,7 @@ __device__ __forceinline__ uint4 pl_pack8(const float* v) {
 
 __global__ void __launch_bounds__(PL_THREADS)
 maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, unsigned char* __restrict__ idx, const PoolShape s) {
+  pdl_wait_and_release();
   const int cv_n = s.C >> 3;
   const long long total = (long long)s.N * s.OH * s.OW * cv_n;
   for (long long g = blockIdx.x * (long long)PL_THREADS + threadIdx.x; g < total; g += (long long)gridDim.x * PL_THREADS) {
@@ -111,6 +112,7 @@ maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const unsigned char* __
 // writes the zeros and the scattered gradient in one pass.
 __global__ void __launch_bounds__(PL_THREADS)
 subsample_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, const PoolShape s) {
+  pdl_wait_and_release();
   const int cv_n = s.C >> 3;
   const long long total = (long long)s.N * s.OH * s.OW * cv_n;
   for (long long g = blockIdx.x * (long long)PL_THREADS + threadIdx.x; g < total; g += (long long)gridDim.x * PL_THREADS) {
@@ -166,9 +168,8 @@ DL4J_API int dl4j_maxpool_fwd(const void* x, void* y, void* idx, const int* shap
   memcpy(&s, shape, sizeof(s));
   if (!pl_ok(s)) return -DL4J_ERR_BAD_ARG;
   const long long total = (long long)s.N * s.OH * s.OW * (s.C >> 3);
-  maxpool_fwd_kernel<<<pl_grid(total), PL_THREADS, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<__nv_bfloat16*>(y), reinterpret_cast<unsigned char*>(idx), s);
-  return (int)cudaGetLastError();
+  return (int)launch_dependent(maxpool_fwd_kernel, dim3(pl_grid(total)), dim3(PL_THREADS), 0, (cudaStream_t)stream,
+                               reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<__nv_bfloat16*>(y), reinterpret_cast<unsigned char*>(idx), s);
 }
 
 DL4J_API int dl4j_maxpool_bwd(const void* dy, const void* idx, void* dx, const int* shape, void* stream) {
@@ -194,8 +195,8 @@ DL4J_API int dl4j_subsample(const void* in, void* out, const int* shape, int bac
                                                                                  reinterpret_cast<__nv_bfloat16*>(out), s);
   } else {
     const long long total = (long long)s.N * s.OH * s.OW * (s.C >> 3);
-    subsample_fwd_kernel<<<pl_grid(total), PL_THREADS, 0, (cudaStream_t)stream>>>(reinterpret_cast<const __nv_bfloat16*>(in),
-                                                                                 reinterpret_cast<__nv_bfloat16*>(out), s);
+    return (int)launch_dependent(subsample_fwd_kernel, dim3(pl_grid(total)), dim3(PL_THREADS), 0, (cudaStream_t)stream,
+                                 reinterpret_cast<const __nv_bfloat16*>(in), reinterpret_cast<__nv_bfloat16*>(out), s);
   }
   return (int)cudaGetLastError();
 }
