@@ -302,3 +302,55 @@ DL4J_API int dl4j_stem_space_to_depth(const void* x, void* out, int N, int C, in
   else return -DL4J_ERR_BAD_ARG;
   return (int)cudaGetLastError();
 }
+
+namespace dl4j {
+// Patches of a few-channel image as the rows of a matrix: out[(n, oh, ow), (c, kh, kw)] = x[n, c, oh sH + kh dH - pH, ow sW + kw dW - pW], zero
+// outside the image and in the columns C kH kW .. KP - 1.  A convolution over three channels is then one GEMM with a reduction of 32
+// forward and one with 32 columns for the weights, each of which reads or writes the large operand once.  Eight columns per thread,
+// consecutive threads along a row: 16-byte stores, and the reads of neighbouring threads share cache lines.
+constexpr int SI_MAX = 64;
+struct PatchShape { int N, C, H, W, OH, OW, kH, kW, sH, sW, pH, pW, dH, dW, KP; long long sn, sc, sh, sw; };
+__global__ void __launch_bounds__(256)
+stem_patches_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ out, const PatchShape s) {
+  __shared__ int2 tap[SI_MAX];          // row and column shift of a matrix column
+  __shared__ long long off[SI_MAX];     // element offset of its channel and shift; -1: padding column
+  for (int j = threadIdx.x; j < s.KP; j += 256) {
+    const int kw = j % s.kW, kh = (j / s.kW) % s.kH, c = j / (s.kW * s.kH);
+    tap[j] = make_int2(kh * s.dH - s.pH, kw * s.dW - s.pW);
+    off[j] = c < s.C ? c * s.sc : -1;
+  }
+  __syncthreads();
+  const unsigned chunks = s.KP / 8, total = (unsigned)s.N * s.OH * s.OW * chunks;      // below 2^31
+  for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+    const unsigned px = i / chunks, line = px / s.OW, n = line / s.OH;
+    const int ch = i - px * chunks, ow = px - line * s.OW, oh = line - n * s.OH;
+    const uint16_t* base = x + n * s.sn;
+    __align__(16) uint16_t v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int2 sh = tap[ch * 8 + j];
+      const int ih = oh * s.sH + sh.x, iw = ow * s.sW + sh.y;
+      const long long o = off[ch * 8 + j];
+      v[j] = o >= 0 && ih >= 0 && ih < s.H && iw >= 0 && iw < s.W ? __ldg(base + o + ih * s.sh + iw * s.sw) : (uint16_t)0;
+    }
+    reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(v);
+  }
+}
+}  // namespace dl4j
+
+// x: 16-bit elements [N, C, H, W] with element strides {sn, sc, sh, sw}; geom: 15 ints {N, C, H, W, OH, OW, kH, kW, sH, sW, pH, pW, dH, dW, KP};
+// out [N * OH * OW, KP] on a 16-byte boundary, KP a multiple of 8, C kH kW <= KP <= 64, N * OH * OW * KP / 8 < 2^31.
+DL4J_API int dl4j_stem_patches(const void* x, void* out, const int* geom, const long long* strides, void* stream) {
+  PatchShape s;
+  memcpy(&s, geom, 15 * sizeof(int));
+  s.sn = strides[0]; s.sc = strides[1]; s.sh = strides[2]; s.sw = strides[3];
+  if (s.N < 1 || s.C < 1 || s.H < 1 || s.W < 1 || s.OH < 1 || s.OW < 1 || s.kH < 1 || s.kW < 1 || s.sH < 1 || s.sW < 1 || s.dH < 1 || s.dW < 1 ||
+      s.KP % 8 || s.KP > SI_MAX || s.C * s.kH * s.kW > s.KP || ((uintptr_t)out & 15))
+    return -DL4J_ERR_BAD_ARG;
+  const long long total = (long long)s.N * s.OH * s.OW * (s.KP / 8);
+  if (total >= 1LL << 31) return -DL4J_ERR_BAD_ARG;
+  const long long blocks = (total + 255) / 256;
+  stem_patches_kernel<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const uint16_t*>(x), reinterpret_cast<uint16_t*>(out), s);
+  return (int)cudaGetLastError();
+}

@@ -157,7 +157,15 @@ class ConvolutionLayer(FeedForwardLayer):
                 z = _stem_space_to_depth(x, W, b, tuple(self.kernelSize), tuple(pad))
                 z = self.activation(z, training)
                 return z.permute(0, 2, 3, 1) if nhwc else z
-            # an RGB stem has too few input channels for the tensor-core convolution kernels: zero-pad them to 8
+            from ...ops import native as nat
+            from ...ops import nnops as _nn
+            if not _nn._FORCE_TORCH:
+                z = nat.conv_few_channels(x, p["W"], p["b"].reshape(-1) if self.hasBias and not skip_bias else None, tuple(self.stride), tuple(pad),
+                                          tuple(self.dilation))
+                if z is not None:
+                    z = self.activation(z, training)
+                    return z.permute(0, 2, 3, 1) if nhwc else z
+            # otherwise an RGB stem has too few input channels for the tensor-core convolution kernels: zero-pad them to 8
             extra = 8 - x.shape[1]
             x = F.pad(x, (0, 0, 0, 0, 0, extra)).contiguous(memory_format=torch.channels_last)
             W = F.pad(W, (0, 0, 0, 0, 0, extra))
