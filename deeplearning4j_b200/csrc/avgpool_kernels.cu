@@ -50,9 +50,10 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 avgpool_bwd_kernel(const T* __restrict__ dy, T* __restrict__ dx, int S, int cv, long long n_vec, float inv) {
   for (long long g = blockIdx.x * 256LL + threadIdx.x; g < n_vec; g += (long long)gridDim.x * 256) {
-    const long long row = g / cv;
+    int c, px;
+    const long long image = div_mod(div_mod(g, cv, c), S, px);
     float v[8];
-    Vec8<T>::load(dy + (row / S) * (cv * 8LL) + (g - row * cv) * 8, v);
+    Vec8<T>::load(dy + image * (cv * 8LL) + c * 8, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] *= inv;
     Vec8<T>::store(dx + g * 8, v);

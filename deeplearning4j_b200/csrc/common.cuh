@@ -52,6 +52,18 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// a = q * b + r for 0 <= a, 0 < b; the index arithmetic of the element-wise kernels, 32 bits wide wherever the value allows it
+__device__ __forceinline__ long long div_mod(long long a, int b, int& r) {
+  if (a <= 0xffffffffLL) {
+    const unsigned q = (unsigned)a / (unsigned)b;
+    r = (int)((unsigned)a - q * (unsigned)b);
+    return q;
+  }
+  const long long q = a / b;
+  r = (int)(a - q * b);
+  return q;
+}
+
 // ReLU as the library has it: NaN passes (fmaxf returns its other operand), infinities and signs as fmaxf.
 __device__ __forceinline__ float relu_f(float v) {
   float y;

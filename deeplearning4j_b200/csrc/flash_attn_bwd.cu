@@ -422,9 +422,8 @@ attn_dvec_kernel(const __nv_bfloat16* __restrict__ dO, long sb, long sh, long st
   const int part = (int)(g & 7);
   float acc = 0.f;
   if (row < rows && part * 8 < D) {
-    const int t = (int)(row % T);
-    const int h = (int)((row / T) % H);
-    const int b = (int)(row / ((long)T * H));
+    int t, h;
+    const int b = (int)div_mod(div_mod(row, T, t), H, h);
     const uint4 a = __ldg(reinterpret_cast<const uint4*>(dO + b * sb + h * sh + t * st) + part);
     const uint4 c = __ldg(reinterpret_cast<const uint4*>(O + (((long)b * T + t) * H + h) * D) + part);
     const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&a);
@@ -451,11 +450,8 @@ attn_dq_finish_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__
   const int parts = D / 8;
   const long n8 = (long)B * H * T * parts;
   for (long g = blockIdx.x * 256L + threadIdx.x; g < n8; g += (long)gridDim.x * 256) {
-    const int part = (int)(g % parts);
-    const long row = g / parts;
-    const int t = (int)(row % T);
-    const int h = (int)((row / T) % H);
-    const int b = (int)(row / ((long)T * H));
+    int part, t, h;
+    const int b = (int)div_mod(div_mod(div_mod(g, parts, part), T, t), H, h);
     const float4* src = reinterpret_cast<const float4*>(acc) + 2 * g;
     float4 x = __ldcs(src), y = __ldcs(src + 1);
     const int n = !SLABS ? 1 : (causal ? min(slabs, t / FB_BLK + 1) : slabs);

@@ -32,11 +32,8 @@ maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restric
   const int cv_n = s.C >> 3;
   const long long total = (long long)s.N * s.OH * s.OW * cv_n;
   for (long long g = blockIdx.x * (long long)PL_THREADS + threadIdx.x; g < total; g += (long long)gridDim.x * PL_THREADS) {
-    const int cv = (int)(g % cv_n);
-    long long t = g / cv_n;
-    const int ow = (int)(t % s.OW); t /= s.OW;
-    const int oh = (int)(t % s.OH);
-    const int n = (int)(t / s.OH);
+    int cv, ow, oh;
+    const int n = (int)div_mod(div_mod(div_mod(g, cv_n, cv), s.OW, ow), s.OH, oh);
     float best[8];
     unsigned char bi[8];
 #pragma unroll
@@ -73,11 +70,8 @@ maxpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const unsigned char* __
   const int cv_n = s.C >> 3;
   const long long total = (long long)s.N * s.H * s.W * cv_n;
   for (long long g = blockIdx.x * (long long)PL_THREADS + threadIdx.x; g < total; g += (long long)gridDim.x * PL_THREADS) {
-    const int cv = (int)(g % cv_n);
-    long long t = g / cv_n;
-    const int iw = (int)(t % s.W); t /= s.W;
-    const int ih = (int)(t % s.H);
-    const int n = (int)(t / s.H);
+    int cv, iw, ih;
+    const int n = (int)div_mod(div_mod(div_mod(g, cv_n, cv), s.W, iw), s.H, ih);
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
@@ -116,11 +110,8 @@ subsample_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restr
   const int cv_n = s.C >> 3;
   const long long total = (long long)s.N * s.OH * s.OW * cv_n;
   for (long long g = blockIdx.x * (long long)PL_THREADS + threadIdx.x; g < total; g += (long long)gridDim.x * PL_THREADS) {
-    const int cv = (int)(g % cv_n);
-    long long t = g / cv_n;
-    const int ow = (int)(t % s.OW); t /= s.OW;
-    const int oh = (int)(t % s.OH);
-    const int n = (int)(t / s.OH);
+    int cv, ow, oh;
+    const int n = (int)div_mod(div_mod(div_mod(g, cv_n, cv), s.OW, ow), s.OH, oh);
     const long long xo = (((long long)n * s.H + (long long)oh * s.sH) * s.W + (long long)ow * s.sW) * cv_n + cv;
     if (!DL4J_IN_BOUNDS(xo, (long long)s.N * s.H * s.W * cv_n)) continue;
     reinterpret_cast<uint4*>(y)[g] = __ldg(reinterpret_cast<const uint4*>(x) + xo);
@@ -132,11 +123,8 @@ subsample_bwd_kernel(const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __rest
   const int cv_n = s.C >> 3;
   const long long total = (long long)s.N * s.H * s.W * cv_n;
   for (long long g = blockIdx.x * (long long)PL_THREADS + threadIdx.x; g < total; g += (long long)gridDim.x * PL_THREADS) {
-    const int cv = (int)(g % cv_n);
-    long long t = g / cv_n;
-    const int iw = (int)(t % s.W); t /= s.W;
-    const int ih = (int)(t % s.H);
-    const int n = (int)(t / s.H);
+    int cv, iw, ih;
+    const int n = (int)div_mod(div_mod(div_mod(g, cv_n, cv), s.W, iw), s.H, ih);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (ih % s.sH == 0 && iw % s.sW == 0) {
       const int oh = ih / s.sH, ow = iw / s.sW;
