@@ -323,14 +323,21 @@ static inline cudaError_t raise_smem_limit(const void* kern, int dev, int bytes,
 }
 // Launch of a kernel that calls `pdl_wait_and_release`.  ResNet-50 inference, 32 images (70 dependent launches of 5 - 20 us): 896 -> 766 us.
 template <typename... K, typename... A>
-static inline cudaError_t launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+static inline cudaError_t launch_dependent_clusters(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                                                    const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at; cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, K(args)...);
+}
+template <typename... K, typename... A>
+static inline cudaError_t launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const A&... args) {
+  return launch_dependent_clusters(kern, grid, block, smem, stream, 1, args...);
 }
 typedef CUresult (*dl4j_PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                          const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,

@@ -20,6 +20,7 @@ namespace dl4j {
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_K = 64;         // 64 x 2 bytes = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
+constexpr int GEMM_PAIR_TILE = 512;  // `block_n` of the 256 x 256 tiles on CTA pairs
 constexpr int GEMM_EPI_WARPS = 8;   // two per TMEM lane quadrant: they take every second group of 32 columns
 constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI_WARPS;
 
@@ -64,12 +65,63 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   nt = n_base + (r - mt * gw);
 }
 
-template <int BLOCK_N, bool A_MN, bool B_MN>
+// ------------------------------------------------------------------ CTA pairs
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of `local` (a shared::cta address of this CTA) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc2(uint32_t* smem_dst, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish2() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// D[tmem of both CTAs] (+)= A * B over the CTA pair: 256 rows (128 per CTA), N columns (each CTA stages N / 2 of B)
+__device__ __forceinline__ void umma2_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :
+      : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the mbarrier at shared::cluster address `bar` once all MMAs issued so far by this thread have completed
+__device__ __forceinline__ void umma2_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// a load into this CTA's shared memory that completes on a barrier of either CTA of the pair (shared::cluster address)
+__device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+
+template <int BLOCK_N, bool A_MN, bool B_MN, bool PAIR>
 struct GemmSmem {
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
-  static constexpr int B_BYTES = BLOCK_N * BLOCK_K * 2;
+  static constexpr int B_COLS = PAIR ? BLOCK_N / 2 : BLOCK_N;      // columns of the tile that this CTA stages
+  static constexpr int B_BYTES = B_COLS * BLOCK_K * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BLOCK_N == 256) ? 4 : 6;
+  static constexpr int STAGES = B_COLS == 256 ? 4 : 6;
   static constexpr int EPI_SLAB = 32 * 64;                  // one warp's 32 rows x 32 16-bit columns (fp32: both slabs)
   static constexpr int EPI_BYTES = GEMM_EPI_WARPS * 2 * EPI_SLAB;
   static constexpr int BIAS_BYTES = GEMM_EPI_WARPS * 32 * 4;   // one group of 32 columns per warp
@@ -197,13 +249,21 @@ __device__ __forceinline__ float load_bias(const GemmParams& p, int col) {
 // format looked at for every pair of values and the bias broadcast by shuffles, 32 columns took 310 instructions and 1900 clocks, most of
 // them waits for the instruction fetch and for dependent results.  Before / now, us (N = 256 tiles): 200704 x 256 x 64 53 / 33, with fp32
 // bias 70 / 41, with residual 156 / 74; 16384 x 3072 x 768 with bias, GELU and pre-activations 99 / 85, with residual 179 / 89.
-template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL>
+// PAIR: the two CTAs of a cluster work on one tile of 256 rows.  Each stages its own 128 rows of A and half of B's columns, 32 KB per 64 of K
+// instead of 48: what a k-step takes is the time its operands need from L2.  The leader's MMA thread issues tcgen05.mma.cta_group::2 for
+// both (each tensor core produces its own 128 rows in its own tensor memory); both CTAs' loads complete on the leader's barrier, commits
+// free the stage and announce the accumulator in both CTAs, and both epilogues release the accumulator on the leader's barrier.
+// 256 wide / pair, us: 16384 x 3072 x 768 67 / 58, 16384 x 768 x 3072 62 / 57, 16384 x 2304 x 768 51 / 44, 2456 x 30520 x 768 150 / 122,
+// 8192 x 8192 x 8192 796 / 768.  With the peer's loads on its own barrier and a thread that forwarded their arrival the form was no faster.
+template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_aux,
                     const __grid_constant__ CUtensorMap tmap_ones, const __grid_constant__ CUtensorMap tmap_bias,
                     const GemmParams p) {
-  using S = GemmSmem<BLOCK_N, A_MN, B_MN>;
+  using S = GemmSmem<BLOCK_N, A_MN, B_MN, PAIR>;
+  constexpr int TILE_M = PAIR ? 2 * BLOCK_M : BLOCK_M;
+  constexpr int B_COLS = S::B_COLS;
   constexpr int STAGES = S::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -219,7 +279,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  const int tiles_m = (p.M + BLOCK_M - 1) / BLOCK_M;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;      // 0: the leader, issues the MMAs
+  const int first_work = PAIR ? blockIdx.x >> 1 : blockIdx.x, work_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
   const int tiles_n = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int kb_total = (p.K + BLOCK_K - 1) / BLOCK_K;
   const int kb_per_split = (kb_total + p.splits - 1) / p.splits;
@@ -235,16 +297,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], GEMM_EPI_WARPS);   // one arrive per epilogue warp
+      mbar_init(&tmem_empty[i], (PAIR ? 2 : 1) * GEMM_EPI_WARPS);   // one arrive per epilogue warp
     }
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 2 * BLOCK_N);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc2(tmem_slot, 2 * BLOCK_N);
+      tmem_relinquish2();
+    } else {
+      tmem_alloc(tmem_slot, 2 * BLOCK_N);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();       // both CTAs' barriers exist before anybody arrives on a remote one
   tc_fence_after();
   pdl_wait_and_release();
   const uint32_t tmem_base = *tmem_slot;
@@ -255,13 +323,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
+      auto expect = [&](uint32_t bytes) {              // of both CTAs of a pair, on the leader's barrier
+        if (!PAIR || rank == 0) mbar_expect_tx(&full_bar[stage], PAIR ? 2 * bytes : bytes);
+      };
+      auto load = [&](void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+        if constexpr (PAIR) tma_load_4d_pair(dst, map, mapa(smem_u32(&full_bar[stage]), 0), c0, c1, c2, c3);
+        else tma_load_4d(dst, map, &full_bar[stage], c0, c1, c2, c3);
+      };
+      for (int w = first_work; w < num_work && ok; w += work_step) {
         const int batch = w / per_batch, wr = w % per_batch;
         const int b1 = batch % p.batch1, b2 = batch / p.batch1;
         const int tile = wr / p.splits, split = wr % p.splits;
         int mt, nt;
         tile_coords(tile, tiles_m, tiles_n, p.raster_gn, mt, nt);
-        const int m0 = mt * BLOCK_M, n0 = nt * BLOCK_N;
+        const int m0 = mt * TILE_M + (int)rank * BLOCK_M, n0 = nt * BLOCK_N + (int)rank * B_COLS;
         const int kb0 = split * kb_per_split;
         const int kb1 = min(kb0 + kb_per_split, kb_total);
         if (p.bias_mma) {
@@ -271,43 +346,60 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1, p.status, DL4J_ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
           uint8_t* sa = smem + stage * S::STAGE_BYTES;
           uint8_t* sb = sa + S::A_BYTES;
-          mbar_expect_tx(&full_bar[stage], (BLOCK_M / 64 + BLOCK_N / 64) * (64 * UMMA_K * 2));
+          expect((BLOCK_M / 64 + B_COLS / 64) * (64 * UMMA_K * 2));
 #pragma unroll
           for (int i = 0; i < BLOCK_M / 64; ++i)
-            tma_load_4d(sa + i * (64 * BLOCK_K * 2), &tmap_ones, &full_bar[stage], i * 64, 0, 0, 0);
+            load(sa + i * (64 * BLOCK_K * 2), &tmap_ones, i * 64, 0, 0, 0);
 #pragma unroll
-          for (int i = 0; i < BLOCK_N / 64; ++i)
-            tma_load_4d(sb + i * (64 * BLOCK_K * 2), &tmap_bias, &full_bar[stage], n0 + i * 64, 0, 0, 0);
+          for (int i = 0; i < B_COLS / 64; ++i)
+            load(sb + i * (64 * BLOCK_K * 2), &tmap_bias, n0 + i * 64, 0, 0, 0);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1, p.status, DL4J_ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
           uint8_t* sa = smem + stage * S::STAGE_BYTES;
           uint8_t* sb = sa + S::A_BYTES;
-          mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
+          expect(S::STAGE_BYTES);
           const int k0 = kb * BLOCK_K;
           if (!A_MN) {
-            tma_load_4d(sa, &tmap_a, &full_bar[stage], k0, m0, b1, b2);
+            load(sa, &tmap_a, k0, m0, b1, b2);
           } else {
 #pragma unroll
             for (int i = 0; i < BLOCK_M / 64; ++i)
-              tma_load_4d(sa + i * (64 * BLOCK_K * 2), &tmap_a, &full_bar[stage], m0 + i * 64, k0, b1, b2);
+              load(sa + i * (64 * BLOCK_K * 2), &tmap_a, m0 + i * 64, k0, b1, b2);
           }
           if (!B_MN) {
-            tma_load_4d(sb, &tmap_b, &full_bar[stage], k0, n0, b1, b2);
+            load(sb, &tmap_b, k0, n0, b1, b2);
           } else {
 #pragma unroll
-            for (int i = 0; i < BLOCK_N / 64; ++i)
-              tma_load_4d(sb + i * (64 * BLOCK_K * 2), &tmap_b, &full_bar[stage], n0 + i * 64, k0, b1, b2);
+            for (int i = 0; i < B_COLS / 64; ++i)
+              load(sb + i * (64 * BLOCK_K * 2), &tmap_b, n0 + i * 64, k0, b1, b2);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      if constexpr (PAIR)              // every commit of the leader has arrived here before this CTA may go
+        for (int i = 0; i < STAGES; ++i) {
+          mbar_wait_bounded(&empty_bar[stage], phase ^ 1, p.status, DL4J_ERR_TIMEOUT_PRODUCER);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
-      const uint32_t idesc = make_idesc(p.fmt, A_MN ? 1 : 0, B_MN ? 1 : 0, BLOCK_M, BLOCK_N);
+    if (rank == 0 && elect_one()) {
+      const uint32_t idesc = make_idesc(p.fmt, A_MN ? 1 : 0, B_MN ? 1 : 0, TILE_M, BLOCK_N);
+      auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate) {
+        if constexpr (PAIR) umma2_f16(d, a, b, id, accumulate);
+        else umma_f16(d, a, b, id, accumulate);
+      };
+      auto commit = [&](uint64_t* bar) {
+        if constexpr (PAIR) {
+          umma2_commit(mapa(smem_u32(bar), 0));
+          umma2_commit(mapa(smem_u32(bar), 1));
+        } else {
+          umma_commit(bar);
+        }
+      };
       // K-major: 8-row groups are 1024 B apart (SBO); MN-major: 64-element column blocks are one
       // TMA box apart (LBO = 64 rows x 128 B) and 8-row K groups 1024 B apart (SBO).
       constexpr uint32_t LBO_A = A_MN ? 64 * BLOCK_K * 2 : 16, LBO_B = B_MN ? 64 * BLOCK_K * 2 : 16;
@@ -316,7 +408,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++it) {
+      for (int w = first_work; w < num_work && ok; w += work_step, ++it) {
         const int split = (w % per_batch) % p.splits;
         const int kb0 = split * kb_per_split;
         const int kb1 = min(kb0 + kb_per_split, kb_total);
@@ -331,9 +423,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * S::STAGE_BYTES);
           const uint32_t sb = sa + S::A_BYTES;
-          umma_f16(tmem_d, make_smem_desc_sw128(sa, 64 * BLOCK_K * 2, 1024), make_smem_desc_sw128(sb, 64 * BLOCK_K * 2, 1024),
-                   make_idesc(p.fmt, 1, 1, BLOCK_M, BLOCK_N), 0u);
-          umma_commit(&empty_bar[stage]);
+          mma(tmem_d, make_smem_desc_sw128(sa, 64 * BLOCK_K * 2, 1024), make_smem_desc_sw128(sb, 64 * BLOCK_K * 2, 1024),
+                   make_idesc(p.fmt, 1, 1, TILE_M, BLOCK_N), 0u);
+          commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -345,13 +437,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           const uint64_t db = make_smem_desc_sw128(sb, LBO_B, 1024);
 #pragma unroll
           for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-            umma_f16(tmem_d, da + ((uint64_t)(k * KSTEP_A) >> 4), db + ((uint64_t)(k * KSTEP_B) >> 4), idesc,
+            mma(tmem_d, da + ((uint64_t)(k * KSTEP_A) >> 4), db + ((uint64_t)(k * KSTEP_B) >> 4), idesc,
                      (kb > kb0 || k > 0 || p.bias_mma) ? 1u : 0u);
           }
-          umma_commit(&empty_bar[stage]);   // frees the smem stage once these MMAs have read it
+          commit(&empty_bar[stage]);   // frees the smem stage once these MMAs have read it
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        umma_commit(&tmem_full[buf]);       // accumulator ready for the epilogue
+        commit(&tmem_full[buf]);       // accumulator ready for the epilogue
       }
     }
   } else {
@@ -360,13 +452,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int c_first = ((warp - 2) >> 2) * 32;
     int it = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++it) {
+    auto release = [&](int buf) {           // the accumulator has been read
+      if constexpr (PAIR) mbar_arrive_cluster(mapa(smem_u32(&tmem_empty[buf]), 0));
+      else mbar_arrive(&tmem_empty[buf]);
+    };
+    for (int w = first_work; w < num_work && ok; w += work_step, ++it) {
       const int batch = w / per_batch, wr = w % per_batch;
       const long c_off = (long)(batch % p.batch1) * p.c_stride_b1 + (long)(batch / p.batch1) * p.c_stride_b2;
       const int tile = wr / p.splits, split = wr % p.splits;
       int mt, nt;
       tile_coords(tile, tiles_m, tiles_n, p.raster_gn, mt, nt);
-      const int m0 = mt * BLOCK_M, n0 = nt * BLOCK_N;
+      const int m0 = mt * TILE_M + (int)rank * BLOCK_M, n0 = nt * BLOCK_N;
       const int kb0 = split * kb_per_split;
       const bool has_k = kb0 < min(kb0 + kb_per_split, kb_total);
       const int buf = it & 1;
@@ -491,7 +587,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+        if (lane == 0) release(buf);
         continue;
       }
 #pragma unroll 1
@@ -595,7 +691,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+      if (lane == 0) release(buf);
     }
     if (lane == 0) bulk_wait<0>();          // staged tiles must have left shared memory before the CTA exits
   }
@@ -603,9 +699,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();   // the partner's shared and tensor memory stay until the pair is done
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * BLOCK_N);
+    if constexpr (PAIR) tmem_dealloc2(tmem_base, 2 * BLOCK_N);
+    else tmem_dealloc(tmem_base, 2 * BLOCK_N);
   }
 }
 
@@ -639,15 +737,15 @@ static int encode_2d(CUtensorMap* map, const void* base, uint64_t inner, uint64_
 static __device__ __align__(128) uint16_t g_ones_bf16[128] = {DL4J_REP128(0x3F80)};
 static __device__ __align__(128) uint16_t g_ones_f16[128] = {DL4J_REP128(0x3C00)};
 
-template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL>
+template <int BLOCK_N, bool A_MN, bool B_MN, bool FULL, bool PAIR = false>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx,
                        const CUtensorMap& tones, const CUtensorMap& tbias, const GemmParams& p, int grid, int dev, cudaStream_t stream) {
-  using S = GemmSmem<BLOCK_N, A_MN, B_MN>;
-  auto kern = gemm_tcgen05_kernel<BLOCK_N, A_MN, B_MN, FULL>;
+  using S = GemmSmem<BLOCK_N, A_MN, B_MN, PAIR>;
+  auto kern = gemm_tcgen05_kernel<BLOCK_N, A_MN, B_MN, FULL, PAIR>;
   static SmemLimit limit;
   const cudaError_t e = raise_smem_limit((const void*)kern, dev, S::TOTAL, limit);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_dependent(kern, dim3(grid), dim3(GEMM_THREADS), S::TOTAL, stream, ta, tb, tc, tx, tones, tbias, p);
+  return (int)launch_dependent_clusters(kern, dim3(grid), dim3(GEMM_THREADS), S::TOTAL, stream, PAIR ? 2 : 1, ta, tb, tc, tx, tones, tbias, p);
 }
 
 // C[M,N] = act(alpha * A·B + bias) (+ residual)
@@ -678,13 +776,14 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
   p.batch1 = batch1; p.batch2 = batch2; p.c_stride_b1 = c_bs[0]; p.c_stride_b2 = c_bs[1];
   if ((a_bs[0] & 7) || (a_bs[1] & 7) || (b_bs[0] & 7) || (b_bs[1] & 7)) return -DL4J_ERR_BAD_ARG;
   const uint64_t nb1 = batch1, nb2 = batch2;
+  const bool pair = block_n == GEMM_PAIR_TILE;
   if (block_n != 128 && block_n != 256) block_n = 256;
   CUtensorMap ta, tb;
   int r;
   if (!a_mn) r = encode_2d(&ta, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda * 2, BLOCK_K, BLOCK_M, nb1, nb2, a_bs[0] * 2, a_bs[1] * 2);
   else       r = encode_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, 64, BLOCK_K, nb1, nb2, a_bs[0] * 2, a_bs[1] * 2);
   if (r) return r > 0 ? -1000 - r : r;
-  if (!b_mn) r = encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, BLOCK_K, (uint32_t)block_n, nb1, nb2, b_bs[0] * 2, b_bs[1] * 2);
+  if (!b_mn) r = encode_2d(&tb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb * 2, BLOCK_K, (uint32_t)(pair ? 128 : block_n), nb1, nb2, b_bs[0] * 2, b_bs[1] * 2);
   else       r = encode_2d(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, 64, BLOCK_K, nb1, nb2, b_bs[0] * 2, b_bs[1] * 2);
   if (r) return r > 0 ? -1000 - r : r;
   // output maps: a box of 32 rows x 32 columns per epilogue warp (64 bytes a row, fp32 128)
@@ -725,12 +824,23 @@ static int gemm_impl(const void* A, const void* B, void* C, void* aux, const voi
     const int tn = (N + block_n - 1) / block_n;
     p.raster_gn = tn < 16 ? tn : 16;
   }
-  const long tiles_l = (long)((M + BLOCK_M - 1) / BLOCK_M) * ((N + block_n - 1) / block_n) * splits * batch1 * batch2;
+  const int tile_m = pair ? 2 * BLOCK_M : BLOCK_M;
+  const long tiles_l = (long)((M + tile_m - 1) / tile_m) * ((N + block_n - 1) / block_n) * splits * batch1 * batch2;
   if (tiles_l > 0x7fffffffL) return -DL4J_ERR_BAD_ARG;
   const int tiles = (int)tiles_l;
   if (num_sms <= 0) num_sms = 148;
-  const int grid = tiles < num_sms ? tiles : num_sms;
   const bool full = p.aux || p.act > 1 || p.res_act;
+  if (pair) {
+    const int pairs = num_sms / 2 > 0 ? num_sms / 2 : 1, grid2 = 2 * (tiles < pairs ? tiles : pairs);
+#define DL4J_GEMM_PAIR(AM, BM)                                                                                                   \
+    if (a_mn == AM && b_mn == BM)                                                                                                \
+      return full ? launch_gemm<256, AM != 0, BM != 0, true, true>(ta, tb, tc, tx, tones, tbias, p, grid2, dev, stream)    \
+                  : launch_gemm<256, AM != 0, BM != 0, false, true>(ta, tb, tc, tx, tones, tbias, p, grid2, dev, stream);
+    DL4J_GEMM_PAIR(0, 0) DL4J_GEMM_PAIR(0, 1) DL4J_GEMM_PAIR(1, 0) DL4J_GEMM_PAIR(1, 1)
+#undef DL4J_GEMM_PAIR
+    return -DL4J_ERR_BAD_ARG;
+  }
+  const int grid = tiles < num_sms ? tiles : num_sms;
 #define DL4J_GEMM_CASE(BN, AM, BM)                                                                                              \
   if (block_n == BN && a_mn == AM && b_mn == BM)                                                                               \
     return full ? launch_gemm<BN, AM != 0, BM != 0, true>(ta, tb, tc, tx, tones, tbias, p, grid, dev, stream)                       \
@@ -781,8 +891,11 @@ DL4J_API int dl4j_gemm_split(const void* A, const void* B, float* partial, void*
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (splits < 2 || N % 4 || (fmt != 0 && fmt != 1)) return -DL4J_ERR_BAD_ARG;
   const long z[2] = {0, 0};
-  const int rc = gemm_impl(A, B, partial, nullptr, nullptr, nullptr, M, N, K, lda, ldb, N, 0, 0, a_mn, b_mn, fmt, 0, 1, 0, 2, splits, 1.0f, 256,
-                           num_sms, stream_, 1, 1, z, z, z);
+  // pairs from 36 steps of K per CTA on, unless their rows are mostly padding, as everywhere
+  const long pairs = num_sms > 1 ? num_sms / 2 : 74, tiles = (long)((M + 255) / 256) * ((N + 255) / 256) * splits;
+  const long steps = (tiles + pairs - 1) / pairs * (((K + 63) / 64 + splits - 1) / splits);
+  const int rc = gemm_impl(A, B, partial, nullptr, nullptr, nullptr, M, N, K, lda, ldb, N, 0, 0, a_mn, b_mn, fmt, 0, 1, 0, 2, splits, 1.0f,
+                           steps >= 36 && (M + 255) / 256 * 8 <= (M + 127) / 128 * 5 ? GEMM_PAIR_TILE : 256, num_sms, stream_, 1, 1, z, z, z);
   if (rc) return rc;
   const long blocks = ((long)M * (N / 4) + 255) / 256;
   const int grid = (int)(blocks < 148 * 16 ? blocks : 148 * 16);

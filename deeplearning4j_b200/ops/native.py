@@ -222,29 +222,32 @@ def gemm_supported(a, b) -> bool:
     return _operand_a(a) is not None and _operand_b(b) is not None
 
 
-def _pick_block_n(M, N, splits=1):
+_PAIR_TILE = 512          # `block_n` code of the 256 x 256 tiles on pairs of CTAs
+
+
+def _pair_rows(M):
+    """Whether 256-row tiles cover M rows with at most a quarter more padding than 128-row tiles."""
+    return (M + 255) // 256 * 8 <= (M + 127) // 128 * 5
+
+
+def _pick_block_n(M, N, splits=1, K=0):
+    """Tile of a GEMM by waves x columns: 128 x 256, 128 x 128 (pays 4 - 14 % more per column: 16384 rows, N and K 768 - 3072) or, with K
+    given, 256 x 256 on a pair of CTAs.  A pair needs a third fewer bytes from L2 per step of K and about 1 us more to start and end, so it
+    takes problems with at least 36 steps of 64 per CTA.  256 wide / pair, us: 16384 x 3072 x 768 67 / 58, 16384 x 768 x 3072 62 / 57,
+    16384 x 768 x 768 (36 steps) 21.3 / 19.8, 3200 x 4096 x 1024 (48) 24.6 / 22.9, 2456 x 30520 x 768 150 / 122; with fewer steps 32768 x 512 x
+    512 (32) 20.2 / 19.1, but its GELU form 30.9 / 31.3, 4096 x 1024 x 1024 (16) 11.6 / 12.4, 25088 x 512 x 128 (6) 11.6 / 12.6."""
     sms = num_sms()
     best, best_cost = 256, None
-    for bn in (256, 128):
-        tiles = ((M + 127) // 128) * ((N + bn - 1) // bn) * splits
-        waves = (tiles + sms - 1) // sms
-        cost = waves * bn * (1.0 if bn == 256 else 1.08)     # 128-wide tiles pay 4 - 14 % more per column (16384 rows, N and K 768 - 3072)
+    for bn, rows, units, f in ((256, 128, sms, 1.0), (128, 128, sms, 1.08), (_PAIR_TILE, 256, sms // 2, 0.9)):
+        cols = min(bn, 256)
+        tiles = ((M + rows - 1) // rows) * ((N + cols - 1) // cols) * splits
+        waves = (tiles + units - 1) // units
+        if bn == _PAIR_TILE and (waves * (((K + 63) // 64 + splits - 1) // splits) < 36 or not _pair_rows(M)):
+            continue
+        cost = waves * cols * f
         if best_cost is None or cost < best_cost:
             best, best_cost = bn, cost
     return best
-
-
-_PAIR_MODE = os.environ.get("DL4J_GEMM_PAIR", "0")     # 0 | 1: 256x256 tiles on CTA pairs (cta_group::2) for large problems
-
-
-def _use_pair(M, N, K, splits):
-    """Whether a GEMM runs on CTA pairs (``csrc/gemm_pair_tcgen05.cu``).  Off unless requested: measured on the BERT-base shapes
-    the pair kernel ties the single-CTA kernel (30 / 75 / 71 / 58 us against 30 / 71 / 71 / 54 us for out / ffn1 / ffn2 / qkv) and
-    loses on 8192^3 (1058 against 790 us): the kernels are bound by the depth of the shared-memory ring over the load latency,
-    not by the shared-memory bandwidth a pair saves, and the pair's "stage landed" hand-off between the CTAs adds to that latency."""
-    if _PAIR_MODE != "1":
-        return False
-    return M >= 2048 and N >= 512 and ((M + 255) // 256) * ((N + 255) // 256) * max(splits, 1) >= 74
 
 
 def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtype=None, atomic=False, splits=1,
@@ -256,7 +259,6 @@ def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtyp
         if residual is None or act:
             raise ValueError("res_act needs the pre-activations as `residual` and no forward activation")
         act = int(res_act) << 8
-        pair = False
     oa, ob = _operand_a(a), _operand_b(b)
     if oa is None or ob is None:
         raise ValueError("operand layout not addressable by TMA (need unit stride in one dim, 16-byte alignment)")
@@ -274,27 +276,12 @@ def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtyp
     splits = max(1, min(int(splits), kb))
     if splits > 1 and not (atomic and out_fp32):
         splits = 1
-    bn = block_n or _pick_block_n(M, N, splits)
+    bn = block_n or (_PAIR_TILE if pair else _pick_block_n(M, N, splits, K if pair is None else 0))
     bias_fp32 = 1 if (bias is not None and bias.dtype == torch.float32) else 0
     if bias is not None and not bias_fp32 and bias.dtype != a.dtype:
         bias = bias.to(a.dtype)
     if bias is not None and not bias.is_contiguous():
         bias = bias.contiguous()
-    if pair is None:
-        pair = block_n is None and _use_pair(M, N, K, splits)
-    if pair:
-        if not getattr(l, "_pair_typed", False):
-            vp, i32, lng, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_long, ctypes.c_float
-            l.dl4j_gemm_pair.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, lng, lng, lng, lng, lng, i32, i32, i32, i32, i32, i32,
-                                         i32, i32, f32, i32, vp]
-            l.dl4j_gemm_pair.restype = i32
-            l._pair_typed = True
-        rc = l.dl4j_gemm_pair(_ptr(oa[0]), _ptr(ob[0]), _ptr(out), _ptr(aux), _ptr(bias), _ptr(residual), M, N, K, oa[2], ob[2],
-                              out.stride(0), 0 if aux is None else aux.stride(0), 0 if residual is None else residual.stride(0),
-                              oa[1], ob[1], _DT[a.dtype], bias_fp32, out_fp32, int(act), 1 if atomic else 0, splits, float(alpha),
-                              num_sms(), _stream())
-        _check(rc, "dl4j_gemm_pair")
-        return out
     rc = l.dl4j_gemm(_ptr(oa[0]), _ptr(ob[0]), _ptr(out), _ptr(aux), _ptr(bias), _ptr(residual), M, N, K, oa[2], ob[2],
                      out.stride(0), 0 if aux is None else aux.stride(0), 0 if residual is None else residual.stride(0),
                      oa[1], ob[1], _DT[a.dtype], bias_fp32, out_fp32, int(act), 1 if atomic else 0, splits, float(alpha),
@@ -305,21 +292,28 @@ def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtyp
 
 def _long_k_splits(M, N, K):
     """Split-K factor for a 16-bit-output GEMM with few output tiles and a long reduction (the data gradient of a wide output layer).
-    The estimate, fitted to the measurements below (us): a k-block of 64 takes 0.36 in a tile of 128 x 256 and 0.24 in one of
-    128 x 128, a product 11 and 7 besides; the partial results of a split cost 6 for a second launch and 2 per million of their
-    elements.  Measured unsplit / best split (factor): 128 x 768 x 30522 113 / 36 (16), 1000 x 768 x 30522 108 / 63 (6),
-    256 x 512 x 10001 68 / 26 (10), 1500 x 768 x 20000 82 / 56 (4), 2456 x 512 x 8192 39 / 38 (3), 2456 x 768 x 30522 113 / 110 (2),
-    1024 x 1024 x 4096 25 / 28 (3), 300 x 768 x 2048 16 / 20 (4).  A gain of less than a tenth is not worth the partial results."""
+    The estimate, fitted to the measurements below (us): a k-block of 64 takes 0.36 in a tile of 128 x 256, 0.24 in one of 128 x 128 and 0.30
+    in one of 256 x 256 on a pair of CTAs, a product 11, 7 and 12 besides; the partial results of a split cost 6 for a second launch and 2
+    per million of their elements.  Measured unsplit / best split (factor): 128 x 768 x 30522 73 / 23 (16), 1000 x 768 x 30522 95 / 44 (6),
+    256 x 512 x 10001 63 / 19 (16), 1500 x 768 x 20000 75 / 43 (4), 2456 x 512 x 8192 28 / 29 (3), 2456 x 768 x 30522 106 / 97 (2),
+    3000 x 512 x 30000 131 / 76 (3), 4000 x 768 x 16000 87 / 83 (3), 1024 x 1024 x 4096 15 / 19 (4), 300 x 768 x 2048 9 / 15.  A gain of
+    less than a tenth by the estimate is not worth the partial results."""
     sms, kb = num_sms(), (K + 63) // 64
-    rows, tiles = (M + 127) // 128, ((M + 127) // 128) * ((N + 255) // 256)
+    rows, cols = (M + 127) // 128, (N + 255) // 256
+    tiles, pair_tiles = rows * cols, ((M + 255) // 256) * cols
     if tiles >= sms or kb < 32:
         return 1
-    waves = lambda t: (t + sms - 1) // sms
-    best, best_cost = 1, 0.9 * min(7 + waves(rows * ((N + 127) // 128)) * kb * 0.24, 11 + kb * 0.36)
+
+    def wide(s):                # k-block time of the 256-wide tiles that `s` parts run on
+        steps, pair_waves = (kb + s - 1) // s, -(-pair_tiles * s // (sms // 2))
+        if pair_waves * steps >= 36 and _pair_rows(M):
+            return pair_waves * steps * 0.30
+        return -(-tiles * s // sms) * steps * 0.36
+    best, best_cost = 1, 0.9 * min(7 + -(-rows * ((N + 127) // 128) // sms) * kb * 0.24, 12 + wide(1))
     for s in range(2, 17):
         if kb // s < 8:
             break
-        c = 17 + waves(tiles * s) * ((kb + s - 1) // s) * 0.36 + s * M * N * 2e-6
+        c = 17 + wide(s) + s * M * N * 2e-6
         if c < best_cost:
             best, best_cost = s, c
     return best
