@@ -403,7 +403,8 @@ DL4J_API int dl4j_flash_attn_bwd(const void* q, const void* k, const void* v, co
   p.inv_keep = p.drop_thr ? 65536.f / (65536.f - (float)p.drop_thr) : 1.f;
   const size_t smem = 6 * FB_TILE + 2 * FB_PS + FB_DQ + FB_BLK * sizeof(float) + 256 + 1024;
   auto kern = p.drop_thr ? flash_attn_bwd_kernel<true> : flash_attn_bwd_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limits[2];
+  const cudaError_t e = raise_smem_limit((const void*)kern, dev, (int)smem, limits[p.drop_thr ? 1 : 0]);
   if (e != cudaSuccess) return (int)e;
   kern<<<B * H * ((Tk + FB_BLK - 1) / FB_BLK), FB_THREADS, smem, (cudaStream_t)stream_>>>(tq, tk, tv, tdo, tdq, p);
   return (int)cudaGetLastError();

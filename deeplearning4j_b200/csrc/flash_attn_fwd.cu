@@ -392,7 +392,8 @@ DL4J_API int dl4j_flash_attn_fwd(const void* q, const void* k, const void* v, vo
   p.inv_keep = p.drop_thr ? 65536.f / (65536.f - (float)p.drop_thr) : 1.f;
   const size_t smem = FF_TILE * (1 + FF_SLOTS) + FF_P_BYTES + (2 * FF_BN + 4 * FF_BM + 4) * sizeof(float) + 256 + 1024;
   auto kern = p.drop_thr ? flash_attn_fwd_kernel<true> : flash_attn_fwd_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemLimit limits[2];
+  const cudaError_t e = raise_smem_limit((const void*)kern, dev, (int)smem, limits[p.drop_thr ? 1 : 0]);
   if (e != cudaSuccess) return (int)e;
   const int q_blocks = (Tq + FF_BM - 1) / FF_BM;
   int sms = 0;

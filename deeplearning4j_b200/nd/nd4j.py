@@ -61,6 +61,7 @@ class Nd4j:
     _default_dtype = DataType.FLOAT
     _device = torch.device("cpu")
     _random = _Random()
+    _executioner = None         # the OpExecutioner class, imported at the first call (its package imports this one)
 
     # ------------------------------------------------------------------ environment
     @classmethod
@@ -91,8 +92,10 @@ class Nd4j:
 
     @classmethod
     def getExecutioner(cls):
-        from ..ops.executioner import OpExecutioner
-        return OpExecutioner.instance()
+        if cls._executioner is None:
+            from ..ops.executioner import OpExecutioner
+            cls._executioner = OpExecutioner
+        return cls._executioner.instance()
 
     @classmethod
     def getMemoryManager(cls):

@@ -225,7 +225,7 @@ def attention_grad(q, k, v, mask, scale, dout, causal=False):
     Bn, H, Tq, D = q.shape
     flags = (1 if causal else 0) | (0 if _empty_rows_are_zero(D, Tq, k.shape[2]) and not causal else 2)
     mk = mask.detach().to(torch.float32).contiguous() if mask is not None else None
-    stats = torch.empty((2, Bn, H, Tq), dtype=torch.float32, device=q.device)
+    stats = q.new_empty((2, Bn, H, Tq), dtype=torch.float32)
     lse, dvec = stats[0], stats[1]
     rc = _flash_lib().dl4j_flash_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), None, lse.data_ptr(), native._ptr(mk), Bn, H, Tq,
                                           k.size(2), D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), scale,
@@ -285,12 +285,10 @@ def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
     Tk = k.shape[2]
     if Tq == Tk:
         # one packed [B, T, 3, H, D] gradient buffer, so the gradient of the fused q/k/v projection is a plain view
-        dqkv = torch.empty((Bn, Tq, 3, H, D), dtype=q.dtype, device=q.device)
+        dqkv = q.new_empty((Bn, Tq, 3, H, D))
         dq_t, dk_t, dv_t = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
     else:
-        dq_t = torch.empty((Bn, Tq, H, D), dtype=q.dtype, device=q.device)
-        dk_t = torch.empty((Bn, Tk, H, D), dtype=q.dtype, device=q.device)
-        dv_t = torch.empty((Bn, Tk, H, D), dtype=q.dtype, device=q.device)
+        dq_t, dk_t, dv_t = q.new_empty((Bn, Tq, H, D)), q.new_empty((Bn, Tk, H, D)), q.new_empty((Bn, Tk, H, D))
     # more than one key block contributes to a query's gradient: an fp32 buffer, its own for every call (streams and threads may run the
     # same shape at the same time).  The lengths that the batched products and the operators served before repeat bit for bit: their key
     # blocks store slabs that are added in order.  The others always added in arrival order and keep the smaller buffer.
@@ -298,7 +296,7 @@ def _flash_backward(q, k, v, dO, lse, dvec, mk, scale, flags, dropout_p, seed):
     acc, slabs = None, 1
     if blocks > 1 and (Tk % 128 or flags & 1):
         slabs = blocks
-        acc = torch.empty((blocks, Bn, H, Tq, D), dtype=torch.float32, device=q.device)
+        acc = q.new_empty((blocks, Bn, H, Tq, D), dtype=torch.float32)
         flags |= 4
     elif blocks > 1:
         acc = torch.zeros((Bn, H, Tq, D), dtype=torch.float32, device=q.device)
@@ -329,8 +327,8 @@ def flash_forward(q, k, v, key_mask, scale, dropout_p=0.0, seed=None, flags=0):
     l = _flash_lib()
     q, k, v = _prep(q), _prep(k), _prep(v)
     Bn, H, Tq, D = q.shape
-    out = torch.empty((Bn, Tq, H, D), dtype=q.dtype, device=q.device)
-    lse = torch.empty((Bn, H, Tq), dtype=torch.float32, device=q.device)
+    out = q.new_empty((Bn, Tq, H, D))
+    lse = q.new_empty((Bn, H, Tq), dtype=torch.float32)
     mk = key_mask.to(torch.float32).contiguous() if key_mask is not None else None
     rc = l.dl4j_flash_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), native._ptr(mk), Bn, H, Tq,
                                k.size(2), D, _LONG3(*q.stride()[:3]), _LONG3(*k.stride()[:3]), _LONG3(*v.stride()[:3]), float(scale), flags,

@@ -13,17 +13,16 @@ import time
 import torch
 
 from . import argschema, registry
+from ..nd.ndarray import INDArray
 
 
 def _t(x):
-    from ..nd.ndarray import INDArray
-    if x is None:
-        return None
-    return x.t if isinstance(x, INDArray) else (x if isinstance(x, torch.Tensor) else torch.as_tensor(x))
+    if x is None or isinstance(x, torch.Tensor):
+        return x
+    return x.t if isinstance(x, INDArray) else torch.as_tensor(x)
 
 
 def _wrap(x):
-    from ..nd.ndarray import INDArray
     return INDArray(x) if isinstance(x, torch.Tensor) else x
 
 
@@ -244,6 +243,13 @@ class OpExecutioner:
     def exec(self, op, *inputs, context=None, **kw):
         """``exec(op)`` / ``exec(op, context)`` for op objects (returns the output arrays; preallocated outputs are filled), or
         ``exec("name", *inputs, **kwargs)`` for a registry op by name."""
+        if isinstance(op, str) and self.profilingMode == ProfilingMode.DISABLED and not self.verbose:
+            out = registry.get(op).fn(*[_t(x) for x in inputs], **kw)       # what a loop over small ops pays for: nothing but the call
+            self.lastOp = op
+            if isinstance(out, (tuple, list)):
+                res = [_wrap(o) for o in out]
+                return res if len(res) > 1 else res[0]
+            return _wrap(out)
         t0 = time.perf_counter() if self.profilingMode in (ProfilingMode.OPERATIONS, ProfilingMode.ALL) else None
         if isinstance(op, str):
             name = op
