@@ -9,6 +9,7 @@ cannot masquerade as the native path.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import struct
 import threading
@@ -230,6 +231,7 @@ def _pair_rows(M):
     return (M + 255) // 256 * 8 <= (M + 127) // 128 * 5
 
 
+@functools.lru_cache(maxsize=4096)      # of sizes alone; small networks ask for it as often as they launch
 def _pick_block_n(M, N, splits=1, K=0):
     """Tile of a GEMM by waves x columns: 128 x 256, 128 x 128 (pays 4 - 14 % more per column: 16384 rows, N and K 768 - 3072) or, with K
     given, 256 x 256 on a pair of CTAs.  A pair needs a third fewer bytes from L2 per step of K and about 1 us more to start and end, so it
@@ -290,6 +292,7 @@ def gemm_raw(a, b, out=None, bias=None, act=0, aux=None, residual=None, out_dtyp
     return out
 
 
+@functools.lru_cache(maxsize=4096)
 def _long_k_splits(M, N, K):
     """Split-K factor for a 16-bit-output GEMM with few output tiles and a long reduction (the data gradient of a wide output layer).
     The estimate, fitted to the measurements below (us): a k-block of 64 takes 0.36 in a tile of 128 x 256, 0.24 in one of 128 x 128 and 0.30
